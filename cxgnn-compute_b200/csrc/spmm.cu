@@ -20,6 +20,7 @@
 // segment order. No atomics touch feature data, so results are reproducible.
 #include "common.cuh"
 #include "spmm_stream.cuh"
+#include "spmm_walk.cuh"
 
 namespace cxg {
 namespace {
@@ -488,7 +489,11 @@ extern "C" int cxg_spmm_csr_workspace_size(int64_t n_dst, int64_t nnz, int32_t f
   int tile = split_edges > 0 ? split_edges : 64;
   rc = stream_layout(nnz, static_cast<int64_t>(feat) * heads, tile, &S);
   CXG_REQUIRE(rc == CXG_OK, rc, "cxg_spmm_csr_workspace_size: graph too large for 32-bit tile ids");
+  WalkLayout W;
+  rc = walk_layout(nnz, static_cast<int64_t>(feat) * heads, tile, &W);
+  CXG_REQUIRE(rc == CXG_OK, rc, "cxg_spmm_csr_workspace_size: graph too large for 32-bit tile ids");
   *bytes = L.total > S.total ? L.total : S.total;
+  if (W.total > *bytes) *bytes = W.total;
   return CXG_OK;
 }
 
@@ -517,6 +522,12 @@ extern "C" int cxg_spmm_csr(const cxg_spmm_desc *d, void *workspace, size_t work
   CXG_REQUIRE(d->edge_rel == nullptr || d->rel_stride > 0, CXG_EINVAL,
               "cxg_spmm_csr: edge_rel needs rel_stride > 0");
 
+  const uint32_t variant = CXG_SPMM_BULK_ROWS | CXG_SPMM_TMA_INDEX | CXG_SPMM_GENERIC_WALK;
+  if (!(d->flags & variant) && walk_eligible(d)) {
+    CXG_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 16 == 0, CXG_EINVAL,
+                "cxg_spmm_csr: workspace must be 16-byte aligned");
+    return walk_launch(d, !stream_eligible(d), workspace, workspace_bytes, as_stream(stream));
+  }
   if (stream_eligible(d)) {
     CXG_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 16 == 0, CXG_EINVAL,
                 "cxg_spmm_csr: workspace must be 16-byte aligned");

@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "spmm_stream.cuh"
+#include "spmm_walk.cuh"
 
 namespace cxg {
 namespace {
@@ -71,7 +72,12 @@ extern "C" int cxg_spmm_csr_static(const cxg_spmm_desc *d, void *stream) {
               (long long)d->nnz, d->feat, d->heads);
   // Scratch this request needs: exact for the tiled kernel, the published upper bound otherwise.
   size_t need = 0;
-  if (stream_eligible(d)) {
+  if (!(d->flags & (CXG_SPMM_BULK_ROWS | CXG_SPMM_TMA_INDEX | CXG_SPMM_GENERIC_WALK)) && walk_eligible(d)) {
+    WalkLayout L;
+    int rc = walk_layout(d->nnz, static_cast<int64_t>(d->feat) * d->heads, walk_tile_edges(d), &L);
+    CXG_REQUIRE(rc == CXG_OK, rc, "cxg_spmm_csr_static: graph too large for 32-bit tile ids");
+    need = L.total;
+  } else if (stream_eligible(d)) {
     StreamLayout L;
     int rc = stream_layout(d->nnz, static_cast<int64_t>(d->feat) * d->heads, stream_tile_edges(d), &L);
     CXG_REQUIRE(rc == CXG_OK, rc, "cxg_spmm_csr_static: graph too large for 32-bit tile ids");

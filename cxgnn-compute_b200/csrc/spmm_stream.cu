@@ -1,4 +1,6 @@
-// Edge-tiled streaming CSR SpMM for sm_100a (the fast path of cxg_spmm_csr).
+// Edge-tiled streaming CSR SpMM for sm_100a with the rows staged in shared memory: the measured variants of
+// cxg_spmm_csr that its flags select (bulk row copies, an id ring, the general walk). Without flags the
+// register-staged walk of spmm_walk_impl.cuh runs, same tiles and same bits.
 //
 // Work is cut by EDGES, not by rows: tile t owns edges [t*T, (t+1)*T) of the CSR
 // edge array, whatever rows they belong to, so every warp gets the same number of
@@ -564,7 +566,7 @@ __global__ void __launch_bounds__(kSThreads, kCtasPerSM) spmm_stream(StreamArgs 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Lean variant of the walk for the shapes that carry the large graphs: rows of exactly 32 * CB bytes
+// Variant of the walk with an id ring (CXG_SPMM_TMA_INDEX), for rows of exactly 32 * CB bytes
 // (128 / 256 / 512 bytes: every lane owns CB bytes of every row), no edge values, relations or targets,
 // 16-byte cp.async staging, one stage per warp. Same tiles, same order of additions, same
 // partials as spmm_stream (results are bit-identical); what differs is the instruction count per edge:
@@ -637,17 +639,13 @@ struct FastAcc<__nv_bfloat16, CB> {
   }
 };
 
-// NS = stages in flight per warp: 2 (two stages of 4 KiB, the default) or 1 (the whole 8 KiB as one stage).
-#ifndef CXG_FAST_CTAS
-#define CXG_FAST_CTAS kCtasPerSM  // resident CTAs per SM of the lean walk (7 measured 25 % slower: more warps, more L2 misses)
-#endif
-// IDXS: the tile's source ids are not loaded by the lanes but staged by the bulk-copy unit (TMA): one
+// Two stages of 4 KiB are in flight per warp. The tile's source ids are staged by the bulk-copy unit (TMA): one
 // `cp.async.bulk` of 512 bytes (128 int32 / 64 int64 ids) per chunk into a two-slot ring per warp, completion on an
 // mbarrier, the next chunk (of this tile or of the warp's next tile) requested when a chunk is first read. The
-// copy lanes then take the id of their row from shared memory instead of a shuffle. The waits are bounded like
-// those of the bulk-row variant.
-template <typename T, int CB, typename IdxT, bool ACC, int NS, bool IDXS>
-__global__ void __launch_bounds__(kSThreads, CXG_FAST_CTAS) spmm_stream_fast(StreamArgs a) {
+// copy lanes take the id of their row from shared memory. The waits are bounded like those of the bulk-row variant.
+template <typename T, int CB, typename IdxT, bool ACC>
+__global__ void __launch_bounds__(kSThreads, kCtasPerSM) spmm_stream_fast(StreamArgs a) {
+  constexpr int NS = 2;
   using C = Chunk<T, CB>;
   using Acc = FastAcc<T, CB>;
   constexpr int EL = C::kElems;
@@ -674,20 +672,18 @@ __global__ void __launch_bounds__(kSThreads, CXG_FAST_CTAS) spmm_stream_fast(Str
   const int jrow = lane / CPR;
   const uint8_t *xlane = x + (lane % CPR) * 16;
   const uint32_t cdst = sl + lane * 16;
-  // id ring (IDXS): two slots of kIdxChunkBytes per warp behind the row slots of all warps, then two barriers per warp
+  // id ring: two slots of kIdxChunkBytes per warp behind the row slots of all warps, then two barriers per warp
   constexpr int CH = kIdxChunkBytes / static_cast<int>(sizeof(IdxT));  // ids per chunk; a multiple of B
   const uint32_t ibuf = smem_u32(smem + static_cast<size_t>(kSWarps) * (NS * B * RB) + warp * (2 * kIdxChunkBytes));
   const uint32_t ibar = smem_u32(smem + static_cast<size_t>(kSWarps) * (NS * B * RB + 2 * kIdxChunkBytes) + warp * 16);
   uint32_t g_issue = 0, g_wait = 0;  // chunks requested / consumed by this warp so far (slot = number & 1)
   bool dead = false;
-  if (IDXS) {
-    if (lane == 0) {
-      mbar_init(ibar, 1);
-      mbar_init(ibar + 8, 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
+  if (lane == 0) {
+    mbar_init(ibar, 1);
+    mbar_init(ibar + 8, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncwarp();
 
   auto zero_row = [&](int64_t r) {
     if (ACC) return;  // y[r] += 0
@@ -723,7 +719,7 @@ __global__ void __launch_bounds__(kSThreads, CXG_FAST_CTAS) spmm_stream_fast(Str
     }
     ++g_issue;
   };
-  if (IDXS && gwarp < n_tiles) request_chunk(gwarp, 0);
+  if (gwarp < n_tiles) request_chunk(gwarp, 0);
 
   for (int64_t t = gwarp; t < n_tiles; t += nwarps) {
     const int64_t tb = t * a.tile;
@@ -747,18 +743,13 @@ __global__ void __launch_bounds__(kSThreads, CXG_FAST_CTAS) spmm_stream_fast(Str
     int rstart = rs64 < -kFar ? -kFar : static_cast<int>(rs64);
     const IdxT *idx_t = idx + tb;
 
-    auto load_nid = [&](int k) -> uint32_t {
-      if (IDXS) return 0u;
-      const int pos = k * B + lane;
-      return (lane < B && pos < tile_len) ? static_cast<uint32_t>(load_idx_stream(idx_t + pos)) : 0u;
-    };
     // stage k goes to slot k % NS; exactly one group is committed per call (an empty one past the last stage), so
     // "all but the newest NS - 1 groups complete" means stage k has landed
-    auto fill = [&](int k, uint32_t nid) {
+    auto fill = [&](int k) {
       const int cnt = tile_len - k * B;
-      const uint32_t dst = cdst + (NS == 1 ? 0 : (k & (NS - 1)) * (B * RB));
-      uint32_t ids = 0;  // IDXS: shared address of the id of this lane's row of the stage's first copy group
-      if (IDXS && cnt > 0 && !dead) {
+      const uint32_t dst = cdst + (k & (NS - 1)) * (B * RB);
+      uint32_t ids = 0;  // shared address of the id of this lane's row of the stage's first copy group
+      if (cnt > 0 && !dead) {
         const int in_chunk = (k * B) % CH;
         if (in_chunk == 0) {  // first stage of a chunk: wait for it, then request the one after it
           const uint32_t bar = ibar + (g_wait & 1u) * 8;
@@ -784,49 +775,42 @@ __global__ void __launch_bounds__(kSThreads, CXG_FAST_CTAS) spmm_stream_fast(Str
         }
         ids = ibuf + ((g_wait - 1) & 1u) * kIdxChunkBytes + (in_chunk + jrow) * static_cast<uint32_t>(sizeof(IdxT));
       }
-      if (IDXS && dead) {
+      if (dead) {
         // the stage's copies are not issued; the group below stays empty
       } else if (cnt >= B) {  // full stage: no bounds test per copy
 #pragma unroll
         for (int c = 0; c < NCOPY; ++c) {
           uint32_t nj;
-          if (IDXS)
-            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(nj) : "r"(ids + c * RPI * static_cast<uint32_t>(sizeof(IdxT))));
-          else
-            nj = __shfl_sync(0xffffffffu, nid, c * RPI + jrow);
+          asm volatile("ld.shared.b32 %0, [%1];" : "=r"(nj) : "r"(ids + c * RPI * static_cast<uint32_t>(sizeof(IdxT))));
           cp_async16(dst + c * 512, xlane + static_cast<uint64_t>(nj) * RB);
         }
       } else if (cnt > 0) {
 #pragma unroll
         for (int c = 0; c < NCOPY; ++c) {
           uint32_t nj = 0;
-          if (IDXS) {
-            if (c * RPI + jrow < cnt)
-              asm volatile("ld.shared.b32 %0, [%1];" : "=r"(nj) : "r"(ids + c * RPI * static_cast<uint32_t>(sizeof(IdxT))));
-          } else {
-            nj = __shfl_sync(0xffffffffu, nid, (c * RPI + jrow) & 31);
+          if (c * RPI + jrow < cnt) {
+            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(nj) : "r"(ids + c * RPI * static_cast<uint32_t>(sizeof(IdxT))));
+            cp_async16(dst + c * 512, xlane + static_cast<uint64_t>(nj) * RB);
           }
-          if (c * RPI + jrow < cnt) cp_async16(dst + c * 512, xlane + static_cast<uint64_t>(nj) * RB);
         }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    fill(0, load_nid(0));
-    if (NS == 2) fill(1, load_nid(1));
+    fill(0);
+    fill(1);
     Acc acc;
     acc.zero();
     float f[EL];
 
     for (int k = 0; k < n_stage; ++k) {
-      if (IDXS && dead) break;
-      const uint32_t nid_next = load_nid(k + NS);
+      if (dead) break;
       asm volatile("cp.async.wait_group %0;" ::"n"(NS - 1) : "memory");
       __syncwarp();
       const int sbase = k * B;
       const int send = min(sbase + B, tile_len);
       int pos = sbase;
-      uint32_t p = my + (NS == 1 ? 0 : (k & (NS - 1)) * (B * RB));  // shared address of this lane's bytes of edge `pos`
+      uint32_t p = my + (k & (NS - 1)) * (B * RB);  // shared address of this lane's bytes of edge `pos`
       while (pos < send) {
         const int stop = min(send, rend);
         int n = stop - pos;
@@ -886,13 +870,10 @@ __global__ void __launch_bounds__(kSThreads, CXG_FAST_CTAS) spmm_stream_fast(Str
         }
       }
       __syncwarp();
-      if (NS == 2)
-        fill(k + 2, nid_next);  // also past the last stage: an empty group keeps the group count in step
-      else if (k + 1 < n_stage)
-        fill(k + 1, nid_next);
+      fill(k + 2);  // also past the last stage: an empty group keeps the group count in step
     }
-    if (NS == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");  // only empty groups are left
-    if (IDXS && dead) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");  // only empty groups are left
+    if (dead) {
       // An id chunk did not arrive within the limit. The row copies of this warp have been waited for above and no
       // other chunk is requested; the tile's tail_row keeps the -1 of the plan kernel and the fix-up kernels do
       // nothing once the error word is set.
@@ -1108,16 +1089,9 @@ cudaError_t launch_stream1(const StreamArgs &a, int cb, int nv, int valmode, int
 template <typename T, int CB, typename IdxT>
 cudaError_t launch_fast3(const StreamArgs &a, int grid, cudaStream_t st) {
   constexpr int RB = 32 * CB;
-  // two half-size stages in flight per warp (measured 2-3 % faster than one 8 KiB stage on every graph size)
-  const bool two = kStageBytes / 2 / RB >= 4;
-  const int rows = two ? 2 * ((kStageBytes / 2) / RB > 32 ? 32 : (kStageBytes / 2) / RB)
-                       : (kStageBytes / RB > 32 ? 32 : kStageBytes / RB);
-  const bool idxs = two && a.tma_index;
-  const size_t smem = static_cast<size_t>(rows) * RB * kSWarps + (idxs ? kSWarps * (2 * kIdxChunkBytes + 16) : 0);
-  auto k = idxs ? (a.accumulate ? spmm_stream_fast<T, CB, IdxT, true, 2, true> : spmm_stream_fast<T, CB, IdxT, false, 2, true>)
-           : a.accumulate
-               ? (two ? spmm_stream_fast<T, CB, IdxT, true, 2, false> : spmm_stream_fast<T, CB, IdxT, true, 1, false>)
-               : (two ? spmm_stream_fast<T, CB, IdxT, false, 2, false> : spmm_stream_fast<T, CB, IdxT, false, 1, false>);
+  constexpr int rows = 2 * ((kStageBytes / 2) / RB > 32 ? 32 : (kStageBytes / 2) / RB);
+  const size_t smem = static_cast<size_t>(rows) * RB * kSWarps + kSWarps * (2 * kIdxChunkBytes + 16);
+  auto k = a.accumulate ? spmm_stream_fast<T, CB, IdxT, true> : spmm_stream_fast<T, CB, IdxT, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   k<<<grid, kSThreads, smem, st>>>(a);
@@ -1202,7 +1176,6 @@ int stream_launch(const cxg_spmm_desc *d, void *workspace, size_t workspace_byte
   a.n_dst = d->n_dst, a.nnz = d->nnz, a.rel_stride = d->rel_stride;
   a.wait_cycles = wait_limit_cycles();
   a.test_stall = (d->flags & CXG_SPMM_TEST_STALL) ? 1 : 0;
-  a.tma_index = 0;
   a.feat = d->feat, a.heads = d->heads, a.width = d->feat * d->heads;
   a.ptr_bytes = d->ptr_bytes, a.reduce = d->reduce;
   a.accumulate = (d->flags & CXG_SPMM_ACCUMULATE) ? 1 : 0;
@@ -1250,16 +1223,13 @@ int stream_launch(const cxg_spmm_desc *d, void *workspace, size_t workspace_byte
   // collective's copy kernel) finds registers and shared memory on every SM while this one runs
   int grid = kNumSM * ((d->flags & CXG_SPMM_SHARE_SMS) ? 4 : kCtasPerSM);
   cudaError_t e;
-  // the lean kernel covers full-warp rows without per-edge extras; ids are kept as 32-bit there (a feature matrix
-  // of 2^32 rows of 128 bytes would not fit the device)
-  const bool fast = row_bytes == 32 * cb && valmode == 0 && a.mode == kModeCpAsync && d->edge_rel == nullptr &&
+  // The id ring covers full-warp rows without per-edge extras; ids are kept as 32-bit there (a feature matrix of 2^32
+  // rows of 128 bytes would not fit the device). Its bulk copies need 16-byte aligned sources: tiles are multiples of 32
+  // ids, so the base decides.
+  const bool ring = (d->flags & CXG_SPMM_TMA_INDEX) && reinterpret_cast<uintptr_t>(d->idx) % 16 == 0 && a.tile % 32 == 0 &&
+                    row_bytes == 32 * cb && valmode == 0 && a.mode == kModeCpAsync && d->edge_rel == nullptr &&
                     d->targets == nullptr && !(d->flags & CXG_SPMM_GENERIC_WALK);
-  if (fast) {
-    if (!(d->flags & CXG_SPMM_SHARE_SMS)) {
-      grid = kNumSM * CXG_FAST_CTAS;
-    }
-    // the bulk copies of the id ring need 16-byte aligned sources: tiles are multiples of 32 ids, so the base decides
-    a.tma_index = (d->flags & CXG_SPMM_TMA_INDEX) && reinterpret_cast<uintptr_t>(d->idx) % 16 == 0 && a.tile % 32 == 0;
+  if (ring) {
     e = launch_fast(a, d->dtype, cb, d->idx_bytes, grid, st);
   } else if (d->dtype == CXG_F32)
     e = d->idx_bytes == 8 ? launch_stream1<float, int64_t>(a, cb, nv, valmode, grid, smem, st)

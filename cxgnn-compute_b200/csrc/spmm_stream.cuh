@@ -38,7 +38,6 @@ struct StreamArgs {
   int max_blocks;
   int cpr_shift;  // log2(16-byte chunks per row), -1 when not a power of two
   int mode;       // how feature rows are fetched: kModeCpAsync / kModeBulk
-  int tma_index;  // lean walk: source ids staged by bulk copies into a ring in shared memory
   int32_t *hdr;
   int64_t *tile_row;    // row that owns the first edge of each tile
   int64_t *tail_row;    // row left unfinished at the end of each tile, or -1

@@ -1,0 +1,87 @@
+// Interface between cxg_spmm_csr and its register-staged tiled walk (spmm_walk*.cu).
+#pragma once
+#include "common.cuh"
+
+namespace cxg {
+
+// Longer chains of partial rows are added in ordered blocks of this many partials.
+constexpr int kWalkSeqPartials = 64;
+
+// What the plan leaves per tile: its first row and its first edge. The entry behind the last tile ends the last one.
+struct WalkTile {
+  int64_t row, begin;
+};
+
+struct WalkArgs {
+  const void *ptr;
+  const void *idx;
+  const void *x;
+  void *y;
+  const float *edge_val;
+  const int32_t *edge_rel;
+  int64_t n_dst;
+  int64_t nnz;  // edges the caller declared: no kernel goes beyond
+  int64_t rel_stride;
+  int64_t max_tiles;
+  int row_bytes, width, feat, heads, ptr_bytes, idx_bytes, reduce;
+  int tile;       // edges per tile
+  int whole_rows; // 1: rows of up to `tile` edges are never cut (see spmm_walk_impl.cuh)
+  uint64_t tile_magic;  // ceil(2^64 / tile), 0: divide
+  int32_t *hdr;
+  WalkTile *tiles;  // [tile + 1]
+  int32_t *count;   // [tile] finished blocks of the long chain that starts in the tile
+  float *partials;  // [tile][2][width]: head partial, tail partial
+};
+
+struct WalkLayout {
+  size_t hdr, tiles, count, partials, total;
+  int64_t max_tiles;
+};
+
+int walk_layout(int64_t nnz, int64_t width, int tile, WalkLayout *L);
+// True when the walk covers the descriptor: no edge mask, output rows in order and overwritten, rows that fit its lane
+// layouts.
+bool walk_eligible(const cxg_spmm_desc *d);
+// Edges per tile for this call (desc->split_edges when set).
+int walk_tile_edges(const cxg_spmm_desc *d);
+int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t workspace_bytes, cudaStream_t st);
+
+// One launcher per element type and vector width, each in a translation unit of its own. False: no kernel for it. With
+// resident_tiles set nothing is launched: it receives the number of tiles that are walked at the same time.
+bool walk_launch_f32_16(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
+bool walk_launch_f32_8(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
+bool walk_launch_f32_4(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
+bool walk_launch_bf16_16(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
+bool walk_launch_bf16_8(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
+bool walk_launch_bf16_4(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
+bool walk_launch_bf16_2(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
+
+#ifdef __CUDACC__
+// Edges the kernels walk: ptr[n_dst], but never more than the caller declared.
+__device__ __forceinline__ int64_t edge_total(const WalkArgs &a) {
+  const int64_t e = load_ptr(a.ptr, a.n_dst, a.ptr_bytes);
+  return e > a.nnz ? a.nnz : e;
+}
+
+// Waits for the kernel in front (launch_dependent lets a kernel start before that one has ended).
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launch whose blocks may become resident while the kernel in front of it in the stream drains; that kernel's writes
+// are visible behind dependency_wait(). Takes about 2 us out of a chain of three short kernels.
+template <typename Kernel, typename... Args>
+cudaError_t launch_dependent(Kernel kernel, unsigned grid, int threads, size_t smem, cudaStream_t st, const Args &...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+#endif
+
+}  // namespace cxg

@@ -1,0 +1,455 @@
+// The tiled walk of cxg_spmm_csr: y[t(r),:] (+)= red_{e in row r} v[e] * x[s(e),:].
+//
+// Work is cut by EDGES: tile t owns the edges [t*T, (t+1)*T) of the CSR edge array. A tile is walked by a GROUP of G
+// lanes, 32 / G tiles side by side in a warp. A lane holds NV vectors of VB bytes of every row, so that narrow rows do
+// not cost a whole warp instruction per load and rows of any width (F = 47, 100 ...) keep most of their lanes busy.
+// Feature rows go global -> registers through L1 (where the hub rows of a power-law graph are found again: 32 % of the
+// sectors), U edges in flight per lane, and are added strictly in edge order, one fp32 accumulator per column. When the walk passes the end of a row the accumulators are written and reset; rows
+// without edges get zeros on the way.
+//
+// A row inside one tile is therefore summed like a sequential loop. A row that crosses tile borders leaves one fp32
+// partial per tile; walk_fix adds the partials in tile order (sequentially up to 64; longer chains in blocks of 64
+// consecutive partials, whose sums are then added in block order). No atomics touch feature data. (Letting the tile that
+// arrives last add them inside this kernel measured 30 % slower: the fence and the counter cost every tile two round
+// trips to L2 while the gather saturates it. The same holds for a search of the tile's first row in here: walk_plan
+// leaves it, and the record of a group's next tile is fetched a tile ahead.)
+// whole_rows: tile borders are moved so that only rows longer than T are cut, at multiples of T from their own start:
+// tile t then owns the pieces that START in [t*T, (t+1)*T).
+//
+// Every edge of a step has its own copy of the code at a row's end, which therefore holds nothing that is not needed there:
+// scattered (targets) and accumulating outputs take spmm_stream / spmm_rows.
+//
+// What bounds it: L2 and DRAM where rows are wide, the instructions per edge below 256 bytes a row (so no bounds test, no
+// address arithmetic and no wait for a row pointer per edge). Staging the rows in shared memory with 16-byte
+// asynchronous copies was the form before: it needs a load, an address and a barrier more per edge, and rows that do not
+// start at a multiple of 128 bytes land there at half the rate (F = 100: 12.9 ms for 126 M edges; here 4.9 ms).
+// Measured, whole call, before -> now: 126 M edges, F = 100 fp32 12.9 -> 4.9 ms, F = 64 3.8 -> 2.9, F = 128 5.5 -> 5.1,
+// F = 128 bf16 3.8 -> 3.2 ms; 12.6 M edges, F = 47 1.20 -> 0.43 ms; 2.3 M edges, F = 128 172 -> 131 us, F = 256 562 -> 205 us.
+#pragma once
+#include "spmm_stream.cuh"
+#include "spmm_walk.cuh"
+
+namespace cxg {
+namespace walk {
+
+constexpr int kThreads = 128;
+constexpr int kFar = 1 << 30;  // "no row end in sight" in tile-relative positions
+
+template <int W>
+struct Words {
+  uint32_t w[W];
+};
+template <int VB>
+__device__ __forceinline__ void load_row_bytes(Words<(VB + 3) / 4> &r, const uint8_t *p) {
+  if constexpr (VB == 16) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
+    r.w[0] = v.x, r.w[1] = v.y, r.w[2] = v.z, r.w[3] = v.w;
+  } else if constexpr (VB == 8) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
+    r.w[0] = v.x, r.w[1] = v.y;
+  } else if constexpr (VB == 4) {
+    r.w[0] = __ldg(reinterpret_cast<const uint32_t *>(p));
+  } else {
+    r.w[0] = __ldg(reinterpret_cast<const uint16_t *>(p));
+  }
+}
+
+__device__ __forceinline__ int64_t load_id_stream(const int64_t *p) {
+  int64_t v;
+  asm volatile("ld.global.nc.L1::no_allocate.s64 %0, [%1];" : "=l"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int32_t load_id_stream(const int32_t *p) {
+  int32_t v;
+  asm volatile("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+// EL = fp32 values in VB bytes of T
+template <typename T, int VB>
+struct Acc {
+  static constexpr int EL = VB / static_cast<int>(sizeof(T));
+  static constexpr int W = (VB + 3) / 4;
+  static constexpr int P = EL / 2;
+  unsigned long long p[P > 0 ? P : 1];  // packed pairs (add.rn.f32x2 rounds each half like the scalar add)
+  float s;                              // EL == 1
+  __device__ __forceinline__ static unsigned long long pair(uint32_t lo, uint32_t hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1,%2};" : "=l"(v) : "r"(lo), "r"(hi));
+    return v;
+  }
+  __device__ __forceinline__ static unsigned long long operand(const Words<W> &r, int i) {
+    if (sizeof(T) == 4) return pair(r.w[(2 * i) % W], r.w[(2 * i + 1) % W]);
+    return pair(r.w[i % W] << 16, r.w[i % W] & 0xffff0000u);
+  }
+  __device__ __forceinline__ static float scalar(const Words<W> &r) {
+    return __uint_as_float(sizeof(T) == 4 ? r.w[0] : r.w[0] << 16);
+  }
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < P; ++i) p[i] = 0ull;
+    s = 0.f;
+  }
+  __device__ __forceinline__ void add(const Words<W> &r) {
+    if (EL == 1) {
+      s += scalar(r);
+    } else if (sizeof(T) == 2) {
+      // fp32 += bf16 in one instruction per value (the same rounding as widening first, which takes twice as many)
+#pragma unroll
+      for (int i = 0; i < P; ++i)
+        asm("{\n\t.reg .b16 a0, a1;\n\t.reg .f32 f0, f1;\n\tmov.b32 {a0, a1}, %1;\n\tmov.b64 {f0, f1}, %0;\n\t"
+            "add.rn.f32.bf16 f0, a0, f0;\n\tadd.rn.f32.bf16 f1, a1, f1;\n\tmov.b64 %0, {f0, f1};\n\t}"
+            : "+l"(p[i])
+            : "r"(r.w[i % W]));
+    } else {
+#pragma unroll
+      for (int i = 0; i < P; ++i) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(p[i]) : "l"(operand(r, i)));
+    }
+  }
+  __device__ __forceinline__ void fma(const Words<W> &r, float v) {
+    if (EL == 1) {
+      s = fmaf(scalar(r), v, s);
+    } else {
+      const unsigned long long vv = pair(__float_as_uint(v), __float_as_uint(v));
+#pragma unroll
+      for (int i = 0; i < P; ++i) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(p[i]) : "l"(operand(r, i)), "l"(vv));
+    }
+  }
+  __device__ __forceinline__ void get(float *f) const {
+    if (EL == 1) {
+      f[0] = s;
+    } else {
+#pragma unroll
+      for (int i = 0; i < P; ++i) asm("mov.b64 {%0,%1}, %2;" : "=f"(f[2 * i]), "=f"(f[(2 * i + 1) % EL]) : "l"(p[i]));
+    }
+  }
+};
+
+// f[i] / d, rounded to nearest, for a whole number d >= 1. With r the correctly rounded reciprocal, q = f r and the
+// residual f - q d taken exactly by an fma, q + r (f - q d) is the correctly rounded quotient as long as nothing
+// underflows (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990); below
+// 1e-28 the last bit can differ. One step of Newton's method makes r exact from the hardware's estimate for every
+// mantissa (checked over all 2^23 of them). A full division per value is a dozen instructions and, in every copy of the
+// row end, half of the kernel where eight lanes share a row.
+template <int N>
+__device__ __forceinline__ void divide_by_count(float (&f)[N], float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(fmaf(-d, r, 1.f), r, r);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float q = f[i] * r;
+    const float rest = fmaf(-q, d, f[i]);
+    f[i] = rest == rest ? fmaf(rest, r, q) : q;  // infinities and NaN stay what they are
+  }
+}
+
+template <typename T, int VB>
+__device__ __forceinline__ void store_row_bytes(uint8_t *dst, const float *f) {
+  constexpr int EL = VB / static_cast<int>(sizeof(T));
+  if (sizeof(T) == 4) {
+    if (VB == 16)
+      __stcs(reinterpret_cast<float4 *>(dst), make_float4(f[0], f[1 % EL], f[2 % EL], f[3 % EL]));
+    else if (VB == 8)
+      __stcs(reinterpret_cast<float2 *>(dst), make_float2(f[0], f[1 % EL]));
+    else
+      __stcs(reinterpret_cast<float *>(dst), f[0]);
+  } else if (EL == 1) {
+    *reinterpret_cast<__nv_bfloat16 *>(dst) = __float2bfloat16_rn(f[0]);
+  } else {
+    constexpr int W = EL / 2 > 0 ? EL / 2 : 1;
+    uint32_t w[W];
+#pragma unroll
+    for (int i = 0; i < EL / 2; ++i) {
+      const __nv_bfloat162 t = __floats2bfloat162_rn(f[2 * i], f[(2 * i + 1) % EL]);
+      w[i] = *reinterpret_cast<const uint32_t *>(&t);
+    }
+    if (W == 4)
+      __stcs(reinterpret_cast<uint4 *>(dst), make_uint4(w[0], w[1 % W], w[2 % W], w[3 % W]));
+    else if (W == 2)
+      __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(w[0], w[1 % W]));
+    else
+      __stcs(reinterpret_cast<unsigned int *>(dst), w[0]);
+  }
+}
+
+// VB: bytes per load of a lane; NV loads per row, G lanes per tile, U edges in flight per lane. VALMODE: 0 no
+// edge values, 1 one per edge, 2 one per (edge, head), 3 none and the mean of the row.
+template <typename T, int VB, int G, int NV, int U, int VALMODE, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constant__ WalkArgs a) {
+  using A = Acc<T, VB>;
+  constexpr int W = (VB + 3) / 4;
+  constexpr int EL = A::EL;
+  constexpr int NG = 32 / G;
+  const int lane = threadIdx.x & 31;
+  const int lg = lane & (G - 1);
+  dependency_wait();
+  const int64_t e_total = edge_total(a);
+  const int64_t n_tiles = (e_total + a.tile - 1) / a.tile;
+  const int64_t wid = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
+  const int64_t n_warps = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
+  const int rb = a.row_bytes;
+  // vector q of this lane covers bytes [(lg + q * G) * VB, +VB) of a row; one that lies behind the row reads the lane's
+  // first vector again (or the row's; no other sectors) and is not stored
+  auto on = [&](int q) { return (lg + q * G) * VB < rb; };
+  const uint8_t *xq[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q)
+    xq[q] = static_cast<const uint8_t *>(a.x) + (on(q) ? (lg + q * G) * VB : (on(0) ? lg * VB : 0));
+  uint8_t *y0 = static_cast<uint8_t *>(a.y) + lg * VB;
+  int head[NV];
+  if (VALMODE == 2) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) head[q] = on(q) ? ((lg + q * G) * VB / static_cast<int>(sizeof(T))) / a.feat : 0;
+  }
+
+  auto store = [&](uint8_t *dst, float (&f)[NV][EL]) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+      if (on(q)) store_row_bytes<T, VB>(dst + q * G * VB, f[q]);
+  };
+  auto zero_row = [&](uint8_t *dst) {
+    float z[NV][EL];
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+#pragma unroll
+      for (int i = 0; i < EL; ++i) z[q][i] = 0.f;
+    store(dst, z);
+  };
+  if (e_total == 0) {  // no edge at all: every row is empty
+    for (int64_t r = wid * NG + lane / G; r < a.n_dst; r += n_warps * NG) zero_row(y0 + r * rb);
+    return;
+  }
+
+  // what the plan left for this group's next tile: its first row and first edge, and the first edge behind it
+  int64_t next_row = 0, next_begin = 0, next_stop = 0;
+  auto fetch = [&](int64_t t) {
+    next_begin = next_stop = 0;
+    if (t < n_tiles) {
+      next_row = a.tiles[t].row;
+      next_begin = a.tiles[t].begin;
+      next_stop = a.tiles[t + 1].begin;
+    }
+  };
+  fetch(wid * NG + lane / G);
+  for (int64_t t0 = wid * NG; t0 < n_tiles; t0 += n_warps * NG) {
+    const int64_t t = t0 + lane / G;
+    const int64_t begin = next_begin;
+    int64_t row = next_row;
+    const int len = next_stop > begin ? static_cast<int>(next_stop - begin) : 0;
+    fetch(t + n_warps * NG);
+
+    // Source ids (and edge values) are requested a whole batch of 32 edges ahead: lane lg holds edges j * G + lg.
+    constexpr int IB = 32 / G;
+    uint32_t id_cur[IB], id_nxt[IB];
+    float val_cur[IB], val_nxt[IB];
+    auto load_batch = [&](int first) {
+#pragma unroll
+      for (int j = 0; j < IB; ++j) {
+        const int pos = first + j * G + lg;
+        id_nxt[j] = 0u;
+        val_nxt[j] = 0.f;
+        if (pos < len) {
+          if (a.idx_bytes == 8)
+            id_nxt[j] = static_cast<uint32_t>(load_id_stream(static_cast<const int64_t *>(a.idx) + begin + pos));
+          else
+            id_nxt[j] = static_cast<uint32_t>(load_id_stream(static_cast<const int32_t *>(a.idx) + begin + pos));
+          if (a.edge_rel != nullptr)
+            id_nxt[j] += static_cast<uint32_t>(static_cast<int64_t>(__ldg(a.edge_rel + begin + pos)) * a.rel_stride);
+          if (VALMODE == 1) val_nxt[j] = __ldg(a.edge_val + begin + pos);
+        }
+      }
+    };
+
+    // Row ends are positions relative to `begin`. The end of the row after the current one is requested a row ahead and
+    // kept as it was loaded, so that nothing waits for it before it is used.
+    auto end_raw = [&](int64_t r) -> int64_t { return load_ptr(a.ptr, min(r + 1, a.n_dst), a.ptr_bytes); };
+    auto end_rel = [&](int64_t r, int64_t raw) -> int {
+      const int64_t v = raw - begin;
+      return r >= a.n_dst || v > kFar ? kFar : static_cast<int>(v);
+    };
+    int rend = kFar, rstart = 0, stop = kFar;
+    int64_t next_raw = 0;
+    if (len > 0) {
+      if (t == 0)
+        for (int64_t r = 0; r < row; ++r) zero_row(y0 + r * rb);  // leading rows without edges
+      rend = end_rel(row, end_raw(row));
+      while (rend == 0) ++row, rend = end_rel(row, end_raw(row));  // empty rows that the previous tile's walk wrote
+      next_raw = end_raw(row + 1);
+      const int64_t s = load_ptr(a.ptr, row, a.ptr_bytes) - begin;
+      rstart = s < -kFar ? -kFar : static_cast<int>(s);
+      stop = min(rend, len);
+    }
+    uint8_t *yr = y0 + row * rb;
+    A acc[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) acc[q].zero();
+
+    // the walk stands at a row end, at the end of the tile, or at both
+    auto event = [&](int pos) {
+      const bool row_done = pos == rend;
+      if (row_done && rstart >= 0) {
+        const float d = static_cast<float>(rend - rstart);
+        float f[NV][EL];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          acc[q].get(f[q]);
+          if (VALMODE == 3) divide_by_count<EL>(f[q], d);
+        }
+        store(yr, f);
+      } else if (row < a.n_dst) {
+        // the row began in an earlier tile, or goes on in the next one
+        float *p = a.partials + (t * 2 + (rstart < 0 ? 0 : 1)) * a.width + lg * EL;
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+          if (on(q)) {
+            float f[EL];
+            acc[q].get(f);
+#pragma unroll
+            for (int i = 0; i < EL; ++i) p[q * G * EL + i] = f[i];
+          }
+      }
+#pragma unroll
+      for (int q = 0; q < NV; ++q) acc[q].zero();
+      if (row_done) {
+        rstart = pos;
+        for (;;) {
+          ++row;
+          yr += rb;
+          rend = end_rel(row, next_raw);
+          next_raw = end_raw(row + 1);
+          if (rend != pos) break;
+          zero_row(yr);  // a row without edges
+        }
+      }
+      stop = pos == len ? kFar : min(rend, len);
+    };
+
+    const int longest = G == 32 ? len : __reduce_max_sync(0xffffffffu, len);
+    struct Step {
+      Words<W> v[U][NV];
+      float ev[U][VALMODE == 2 ? NV : 1];
+    };
+    // requests the rows of edges [p, p + U)
+    auto issue = [&](Step &st, int p) {
+      const int in_batch = p & 31;
+      if (in_batch == 0) {
+#pragma unroll
+        for (int j = 0; j < IB; ++j) id_cur[j] = id_nxt[j], val_cur[j] = val_nxt[j];
+        load_batch(p + 32);
+      }
+      uint32_t id = id_cur[0];
+      float val = val_cur[0];
+#pragma unroll
+      for (int j = 1; j < IB; ++j) {
+        id = in_batch >= j * G ? id_cur[j] : id;
+        if (VALMODE == 1) val = in_batch >= j * G ? val_cur[j] : val;
+      }
+      const int lane0 = in_batch & (G - 1);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t nid = __shfl_sync(0xffffffffu, id, lane0 + u, G);
+        const uint64_t off = static_cast<uint64_t>(nid) * static_cast<uint32_t>(rb);
+#pragma unroll
+        for (int q = 0; q < NV; ++q) load_row_bytes<VB>(st.v[u][q], xq[q] + off);
+        if (VALMODE == 1) st.ev[u][0] = __shfl_sync(0xffffffffu, val, lane0 + u, G);
+        if (VALMODE == 2) {
+          const int pos = min(p + u, len - 1);
+#pragma unroll
+          for (int q = 0; q < NV; ++q) st.ev[u][q] = len > 0 ? __ldg(a.edge_val + (begin + pos) * a.heads + head[q]) : 0.f;
+        }
+      }
+    };
+    // adds them; groups that have passed the end of their tile add into accumulators that nobody reads
+    auto consume = [&](const Step &st, int p) {
+      auto add = [&](int u) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          if (VALMODE == 0 || VALMODE == 3)
+            acc[q].add(st.v[u][q]);
+          else
+            acc[q].fma(st.v[u][q], st.ev[u][VALMODE == 2 ? q : 0]);
+        }
+      };
+      // no row ends among the U edges of any group (not worth asking with four groups: one of them nearly always has one)
+      if (NG <= 2 && !__any_sync(0xffffffffu, stop - p <= U)) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) add(u);
+        return;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        add(u);
+        if (p + u + 1 == stop) event(p + u + 1);
+      }
+    };
+    load_batch(0);
+    Step s;
+    for (int p = 0; p < longest; p += U) {
+      issue(s, p);
+      consume(s, p);
+    }
+  }
+}
+
+// Lane layouts: vectors per row -> (lanes per tile, loads per lane, edges in flight per lane, resident CTAs per SM).
+// 512 bytes in flight per row and lane group and 32 warps per SM where 64 registers hold them: 7, 6 and 5 CTAs measured
+// 3 to 25 % slower on 128- to 512-byte rows, twice the edges per step (128 registers) 40 %, and two steps in flight with
+// half the edges each 30 %. Narrow fp32 rows read one word at a time (F = 47) want four edges per step, not eight.
+// With resident_tiles set nothing is launched: it receives the tiles that are walked at the same time.
+template <typename T, int VB, int VALMODE>
+bool launch_width(const WalkArgs &a, bool share, cudaStream_t st, int *resident_tiles) {
+  const int n = (a.row_bytes + VB - 1) / VB;
+  auto go = [&](auto kernel, int g, int ctas) {
+    const int per_cta = kThreads / g;
+    if (resident_tiles != nullptr) {
+      *resident_tiles = kNumSM * ctas * per_cta;
+      return true;
+    }
+    int64_t grid = (a.max_tiles + per_cta - 1) / per_cta;
+    const int64_t resident = kNumSM * (share ? ctas / 2 : ctas);
+    if (grid > resident) grid = resident;
+    return launch_dependent(kernel, static_cast<unsigned>(grid < 1 ? 1 : grid), kThreads, 0, st, a) == cudaSuccess;
+  };
+  constexpr int kMost = VALMODE == 2 ? 6 : 8;  // a value per edge and vector: more registers
+#define CXG_WALK(G, NV, U, CTAS) \
+  if (n <= G * NV)               \
+  return go(spmm_walk<T, VB, G, NV, U, VALMODE, (CTAS < kMost ? CTAS : kMost)>, G, CTAS < kMost ? CTAS : kMost)
+  if constexpr (VB == 16) {
+    CXG_WALK(8, 1, 8, 8);
+    CXG_WALK(16, 1, 8, 8);
+    CXG_WALK(32, 1, 8, 8);
+    CXG_WALK(32, 2, 4, 8);
+    CXG_WALK(32, 4, 2, 6);
+  } else if constexpr (VB == 8) {
+    CXG_WALK(8, 1, 8, 8);
+    CXG_WALK(16, 1, 8, 8);
+    CXG_WALK(16, 2, 4, 8);
+    CXG_WALK(32, 2, 4, 8);
+    CXG_WALK(32, 4, 4, 6);
+    CXG_WALK(32, 8, 2, 5);
+  } else {
+    CXG_WALK(8, 1, 8, 8);
+    CXG_WALK(8, 2, 8, 8);
+    CXG_WALK(16, 2, 8, 8);
+    CXG_WALK(16, 3, 4, 8);
+    CXG_WALK(16, 4, 4, 8);
+    CXG_WALK(32, 3, 4, 8);
+    CXG_WALK(32, 4, 4, 7);
+    CXG_WALK(32, 6, 4, 6);
+    CXG_WALK(32, 8, 4, 5);
+  }
+#undef CXG_WALK
+  return false;
+}
+
+template <typename T, int VB>
+bool launch(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles) {
+  if (valmode == 0) return launch_width<T, VB, 0>(a, share, st, resident_tiles);
+  if (valmode == 1) return launch_width<T, VB, 1>(a, share, st, resident_tiles);
+  if (valmode == 3) return launch_width<T, VB, 3>(a, share, st, resident_tiles);
+  return launch_width<T, VB, 2>(a, share, st, resident_tiles);
+}
+
+}  // namespace walk
+}  // namespace cxg
