@@ -1,17 +1,22 @@
-"""Builds libcxgnn_b200.so from the .cu files in this directory with nvcc for sm_100a.
+"""Builds libcxgnn_b200.so from the .cu files in this directory with nvcc for sm_100a, and the Python backend's host
+module (native.cpp, g++ against torch's headers) that calls it.
 
 Usage: python build.py [--force] [--verbose]
-The library is written next to this file; nothing is installed.
+The library is written next to this file, the module next to the backend; nothing is installed.
 """
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB = os.path.join(HERE, "libcxgnn_b200.so")
+NATIVE_SRC = os.path.join(HERE, "native.cpp")
+NATIVE = os.path.join(HERE, "..", "cxgnncomp_backend", "_native.so")
 OBJ_DIR = os.path.join(HERE, "build")
-NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+NVCC = os.environ.get("NVCC", os.path.join(CUDA_HOME, "bin", "nvcc"))
 FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
@@ -36,6 +41,16 @@ def stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def native_command():
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+            + ["-I" + p for p in include_paths() + [sysconfig.get_paths()["include"], os.path.join(CUDA_HOME, "include")]]
+            + [NATIVE_SRC, "-o", NATIVE, "-L" + libs, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-ldl"])
+
+
 def build(force=False, verbose=False):
     os.makedirs(OBJ_DIR, exist_ok=True)
     hdrs = headers() + [os.path.abspath(__file__)]
@@ -52,12 +67,15 @@ def build(force=False, verbose=False):
         r = subprocess.run(cmd, capture_output=True, text=True)
         return cmd, r
 
+    if force or stale(NATIVE, [NATIVE_SRC] + hdrs):
+        jobs.append(native_command())
+
     with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
         for cmd, r in ex.map(run, jobs):
             if verbose or r.returncode != 0:
                 sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
             if r.returncode != 0:
-                raise RuntimeError("nvcc failed for " + cmd[-3])
+                raise RuntimeError("the compiler failed: " + " ".join(cmd))
     if jobs or force or stale(LIB, objs):
         cmd = [NVCC, "-shared", "-o", LIB] + objs
         r = subprocess.run(cmd, capture_output=True, text=True)

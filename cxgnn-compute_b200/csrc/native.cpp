@@ -1,0 +1,408 @@
+// Host path of the Python backend in C++: argument checks, scratch, descriptor, launch and autograd of the operators that
+// are called often and on small inputs, where the interpreter cost more than the kernels (an aggregation of 11,000 edges:
+// 32 us per call through ctypes and a Python autograd function, 20 us of it kernels).
+//
+// The kernels stay behind the C ABI of libcxgnn_b200.so: this module opens the library it is told to (init) and calls its
+// entry points. No CUDA code, no other state than the scratch buffers per stream and the transposed graphs.
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/extension.h>
+
+#include <list>
+#include <map>
+#include <mutex>
+
+#include "../../include/cxgnn_b200.h"
+
+namespace {
+
+using at::Tensor;
+using c10::optional;
+using torch::autograd::AutogradContext;
+using torch::autograd::Variable;
+using torch::autograd::variable_list;
+
+// ---- the library -----------------------------------------------------------------------------------------------------
+struct Lib {
+  void *handle = nullptr;
+#define CXG_FN(name) decltype(&::name) name = nullptr
+  CXG_FN(cxg_last_error_string);
+  CXG_FN(cxg_spmm_csr_workspace_size);
+  CXG_FN(cxg_spmm_csr);
+  CXG_FN(cxg_spmm_csr_backward);
+  CXG_FN(cxg_csr_transpose_workspace_size);
+  CXG_FN(cxg_csr_transpose);
+  CXG_FN(cxg_gather_edges);
+  CXG_FN(cxg_gather_rows);
+  CXG_FN(cxg_sample_batch_bounds);
+  CXG_FN(cxg_sample_batch);
+#undef CXG_FN
+} lib;
+
+void init(const std::string &path) {
+  lib.handle = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  if (lib.handle == nullptr) throw std::runtime_error(std::string("cannot open ") + path + ": " + dlerror());
+#define CXG_FN(name)                                                                \
+  lib.name = reinterpret_cast<decltype(&::name)>(dlsym(lib.handle, #name));         \
+  if (lib.name == nullptr) throw std::runtime_error(std::string("no ") + #name + " in " + path)
+  CXG_FN(cxg_last_error_string);
+  CXG_FN(cxg_spmm_csr_workspace_size);
+  CXG_FN(cxg_spmm_csr);
+  CXG_FN(cxg_spmm_csr_backward);
+  CXG_FN(cxg_csr_transpose_workspace_size);
+  CXG_FN(cxg_csr_transpose);
+  CXG_FN(cxg_gather_edges);
+  CXG_FN(cxg_gather_rows);
+  CXG_FN(cxg_sample_batch_bounds);
+  CXG_FN(cxg_sample_batch);
+#undef CXG_FN
+}
+
+[[noreturn]] void fail(const std::string &text) { throw std::runtime_error(text); }
+
+void check(int rc, const char *what) {
+  if (rc != 0) fail(std::string(what) + " failed with status " + std::to_string(rc) + ": " + lib.cxg_last_error_string());
+}
+
+const Tensor &cuda(const Tensor &t, const char *name) {
+  if (!t.is_cuda()) fail(std::string(name) + " must be a CUDA tensor (this backend has no CPU path)");
+  if (!t.is_contiguous()) fail(std::string(name) + " must be contiguous");
+  return t;
+}
+const Tensor &of_type(const Tensor &t, const char *name, std::initializer_list<at::ScalarType> types) {
+  cuda(t, name);
+  for (auto s : types)
+    if (t.scalar_type() == s) return t;
+  fail(std::string(name) + " has dtype " + c10::toString(t.scalar_type()) + ", which this operator does not take");
+}
+const Tensor &feature(const Tensor &t, const char *name) { return of_type(t, name, {at::kFloat, at::kBFloat16}); }
+const Tensor &index_of(const Tensor &t, const char *name) { return of_type(t, name, {at::kLong, at::kInt}); }
+const Tensor &f32(const Tensor &t, const char *name) { return of_type(t, name, {at::kFloat}); }
+
+void *stream_of(const Tensor &t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+// ---- scratch ---------------------------------------------------------------------------------------------------------
+// One buffer per (device, stream), grown on demand; contents never carry over. `kind` names the entry point family that
+// used it last (whose status word check_device_status can ask for). Calls of one stream are ordered, and this module runs
+// with the interpreter's lock held, so two threads on one stream do not interleave their launches.
+struct Scratch {
+  Tensor buf;
+  std::string kind;
+};
+std::mutex scratch_lock;
+std::map<std::pair<int, void *>, Scratch> scratch;
+
+Tensor workspace_on(int device, void *stream, int64_t bytes, const char *kind) {
+  std::lock_guard<std::mutex> hold(scratch_lock);
+  Scratch &s = scratch[{device, stream}];
+  if (!s.buf.defined() || s.buf.numel() < bytes)
+    s.buf = at::empty({std::max<int64_t>(bytes, 1 << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
+  if (s.kind != kind) s.kind = kind;
+  return s.buf;
+}
+
+Tensor workspace(int device, int64_t bytes, const std::string &kind) {
+  return workspace_on(device, c10::cuda::getCurrentCUDAStream(device).stream(), bytes, kind.c_str());
+}
+
+// (buffer or None, kind) of the current stream
+std::pair<optional<Tensor>, std::string> last_workspace(int device) {
+  std::lock_guard<std::mutex> hold(scratch_lock);
+  auto it = scratch.find({device, c10::cuda::getCurrentCUDAStream(device).stream()});
+  if (it == scratch.end()) return {c10::nullopt, ""};
+  return {it->second.buf, it->second.kind};
+}
+
+// ---- aggregation -----------------------------------------------------------------------------------------------------
+int64_t rows_of(const Tensor &ptr, int64_t num_node) {
+  const int64_t all = ptr.size(0) - 1;
+  const int64_t n = num_node > 0 ? num_node : all;  // 0 means all rows
+  if (n > all) fail("num_node " + std::to_string(n) + " exceeds the " + std::to_string(all) + " rows of ptr");
+  return n;
+}
+
+cxg_spmm_desc describe(const Tensor &ptr, const Tensor &idx, int64_t n, int64_t heads, int64_t feat, at::ScalarType type,
+                       int64_t reduce, int64_t flags, int64_t split) {
+  cxg_spmm_desc d = {};
+  d.ptr = ptr.data_ptr();
+  d.idx = idx.data_ptr();
+  d.n_dst = n;
+  d.nnz = idx.size(0);
+  d.feat = static_cast<int32_t>(feat);
+  d.heads = static_cast<int32_t>(heads);
+  d.dtype = type == at::kFloat ? CXG_F32 : CXG_BF16;
+  d.ptr_bytes = static_cast<int32_t>(ptr.element_size());
+  d.idx_bytes = static_cast<int32_t>(idx.element_size());
+  d.reduce = static_cast<int32_t>(reduce);
+  d.flags = static_cast<uint32_t>(flags);
+  d.split_edges = static_cast<int32_t>(split);
+  return d;
+}
+
+void run_spmm(cxg_spmm_desc &d, const Tensor &on) {
+  size_t need = 0;
+  check(lib.cxg_spmm_csr_workspace_size(d.n_dst, d.nnz, d.feat, d.heads, d.split_edges, &need), "cxg_spmm_csr_workspace_size");
+  void *st = stream_of(on);
+  const Tensor ws = workspace_on(on.device().index(), st, static_cast<int64_t>(need), "spmm");
+  check(lib.cxg_spmm_csr(&d, ws.data_ptr(), static_cast<size_t>(ws.numel()), st), "cxg_spmm_csr");
+}
+
+// y = A x for the first rows of the graph; x [N, F] or [N, H, F]
+Tensor spmm(const Tensor &x, const Tensor &ptr, const Tensor &idx, int64_t num_node, const optional<Tensor> &edge_val,
+            int64_t reduce, const optional<Tensor> &out, const optional<Tensor> &edge_mask, const optional<Tensor> &edge_rel,
+            int64_t rel_stride, const optional<Tensor> &targets, int64_t flags, int64_t split) {
+  feature(x, "x");
+  index_of(ptr, "ptr");
+  index_of(idx, "idx");
+  const int64_t n = rows_of(ptr, num_node);
+  if (x.dim() != 2 && x.dim() != 3) fail("x must be [N, F] or [N, H, F]");
+  const int64_t heads = x.dim() == 3 ? x.size(1) : 1, feat = x.size(-1);
+  if (edge_val) {
+    f32(*edge_val, "edge_value");
+    const int64_t vh = edge_val->dim() == 2 ? edge_val->size(1) : 1;
+    if (vh != heads) fail("edge_value has " + std::to_string(vh) + " heads, x has " + std::to_string(heads));
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor y = out ? *out : (x.dim() == 3 ? at::empty({n, heads, feat}, x.options()) : at::empty({n, feat}, x.options()));
+  cxg_spmm_desc d = describe(ptr, idx, n, heads, feat, x.scalar_type(), reduce, flags, split);
+  d.x = x.data_ptr();
+  d.y = y.data_ptr();
+  if (edge_val) d.edge_val = static_cast<const float *>(edge_val->data_ptr());
+  if (edge_mask) d.edge_mask = static_cast<const uint8_t *>(edge_mask->data_ptr());
+  if (edge_rel) d.edge_rel = static_cast<const int32_t *>(edge_rel->data_ptr());
+  if (targets) d.targets = static_cast<const int64_t *>(targets->data_ptr());
+  d.rel_stride = rel_stride;
+  run_spmm(d, x);
+  return y;
+}
+
+// ---- transposed graphs -----------------------------------------------------------------------------------------------
+struct Transposed {
+  Tensor t_ptr, t_idx, t_eid, inv_deg;
+};
+
+Transposed transpose(const Tensor &ptr, const Tensor &idx, int64_t num_node, int64_t n_src, bool want_eid) {
+  index_of(ptr, "ptr");
+  index_of(idx, "idx");
+  const int64_t n = rows_of(ptr, num_node), nnz = idx.size(0);
+  c10::cuda::CUDAGuard guard(ptr.device());
+  Transposed t;
+  t.t_ptr = at::empty({n_src + 1}, ptr.options().dtype(at::kLong));
+  t.t_idx = at::empty({nnz}, idx.options());
+  if (want_eid) t.t_eid = at::empty({nnz}, idx.options());
+  t.inv_deg = at::empty({n}, ptr.options().dtype(at::kFloat));
+  size_t need = 0;
+  check(lib.cxg_csr_transpose_workspace_size(nnz, &need), "cxg_csr_transpose_workspace_size");
+  void *st = stream_of(ptr);
+  const Tensor ws = workspace_on(ptr.device().index(), st, static_cast<int64_t>(need), "");
+  check(lib.cxg_csr_transpose(ptr.data_ptr(), idx.data_ptr(), static_cast<int>(ptr.element_size()),
+                              static_cast<int>(idx.element_size()), n, n_src, nnz, t.t_ptr.data_ptr<int64_t>(),
+                              t.t_idx.data_ptr(), want_eid ? t.t_eid.data_ptr() : nullptr, t.inv_deg.data_ptr<float>(),
+                              ws.data_ptr(), static_cast<size_t>(ws.numel()), st),
+        "cxg_csr_transpose");
+  return t;
+}
+
+// The last eight transposed graphs, by the tensors they came from. An entry keeps ptr and idx alive, so their addresses
+// cannot be handed to another graph.
+struct CachedGraph {
+  const void *ptr_data, *idx_data;
+  int64_t n, n_src;
+  uint32_t ptr_version, idx_version;
+  int device;
+  Tensor ptr, idx;
+  Transposed t;
+};
+std::mutex graphs_lock;
+std::list<CachedGraph> graphs;
+constexpr size_t kMostGraphs = 8;
+
+Transposed transposed_graph(const Tensor &ptr, const Tensor &idx, int64_t n, int64_t n_src) {
+  const uint32_t pv = ptr._version(), iv = idx._version();
+  {
+    std::lock_guard<std::mutex> hold(graphs_lock);
+    for (const auto &g : graphs)
+      if (g.ptr_data == ptr.data_ptr() && g.idx_data == idx.data_ptr() && g.n == n && g.n_src == n_src && g.ptr_version == pv &&
+          g.idx_version == iv && g.device == ptr.device().index())
+        return g.t;
+  }
+  CachedGraph g{ptr.data_ptr(), idx.data_ptr(), n, n_src, pv, iv, ptr.device().index(), ptr, idx, transpose(ptr, idx, n, n_src, true)};
+  Transposed t = g.t;
+  std::lock_guard<std::mutex> hold(graphs_lock);
+  while (graphs.size() >= kMostGraphs) graphs.pop_front();
+  graphs.push_back(std::move(g));
+  return t;
+}
+void forget_graphs() {
+  std::lock_guard<std::mutex> hold(graphs_lock);
+  graphs.clear();
+}
+size_t count_graphs() {
+  std::lock_guard<std::mutex> hold(graphs_lock);
+  return graphs.size();
+}
+
+// dX = A^T dY on the cached transposed graph, in dY's type
+Tensor spmm_transposed(const Tensor &grad, const Tensor &ptr, const Tensor &idx, int64_t n, int64_t n_src,
+                       const optional<Tensor> &edge_val, int64_t reduce, int64_t flags, int64_t split) {
+  const Transposed t = transposed_graph(ptr, idx, n, n_src);
+  Tensor dy = grad.size(0) == n ? grad : grad.narrow(0, 0, n);
+  if (reduce == CXG_MEAN) {
+    std::vector<int64_t> shape(dy.dim(), 1);
+    shape[0] = n;
+    const Tensor w = t.inv_deg.view(shape);
+    dy = dy.scalar_type() == at::kFloat ? at::mul(dy, w) : at::mul(dy.to(at::kFloat), w).to(dy.scalar_type());
+  }
+  optional<Tensor> tv;
+  if (edge_val) {  // the edge values in transposed order
+    const Tensor ev = edge_val->contiguous();
+    tv = at::empty_like(ev);
+    check(lib.cxg_gather_edges(ev.data_ptr<float>(), t.t_eid.data_ptr(), static_cast<int>(t.t_eid.element_size()),
+                               tv->data_ptr<float>(), std::min(t.t_eid.size(0), ev.size(0)),
+                               static_cast<int>(ev.dim() == 2 ? ev.size(1) : 1), 1, stream_of(ev)),
+          "cxg_gather_edges");
+  }
+  return spmm(dy.contiguous(), t.t_ptr, t.t_idx, n_src, tv, CXG_SUM, c10::nullopt, c10::nullopt, c10::nullopt, 0, c10::nullopt,
+              flags, split);
+}
+
+// Sum or mean aggregation with its gradients: x over the transposed graph (or, `scatter`, with atomics over the forward
+// edges), the edge values by a second pass over the forward edges.
+class SageFunction : public torch::autograd::Function<SageFunction> {
+ public:
+  static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &ptr, const Tensor &idx,
+                        const optional<Tensor> &edge_val, int64_t num_node, int64_t reduce, int64_t flags, int64_t split,
+                        bool scatter) {
+    ctx->save_for_backward({x, ptr, idx, edge_val ? *edge_val : Tensor()});
+    ctx->saved_data["n"] = num_node;
+    ctx->saved_data["reduce"] = reduce;
+    ctx->saved_data["flags"] = flags;
+    ctx->saved_data["split"] = split;
+    ctx->saved_data["scatter"] = scatter;
+    return spmm(x, ptr, idx, num_node, edge_val, reduce, c10::nullopt, c10::nullopt, c10::nullopt, 0, c10::nullopt, flags, split);
+  }
+  static variable_list backward(AutogradContext *ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &ptr = saved[1], &idx = saved[2];
+    optional<Tensor> edge_val;
+    if (saved[3].defined()) edge_val = saved[3];
+    const Tensor g = grads[0].contiguous();
+    const int64_t n = rows_of(ptr, ctx->saved_data["n"].toInt()), reduce = ctx->saved_data["reduce"].toInt();
+    const int64_t flags = ctx->saved_data["flags"].toInt(), split = ctx->saved_data["split"].toInt();
+    c10::cuda::CUDAGuard guard(g.device());
+    Tensor dx, dval;
+    bool need_dx = ctx->needs_input_grad(0);
+    const bool need_dval = edge_val && ctx->needs_input_grad(3);
+    if (need_dx && !ctx->saved_data["scatter"].toBool() && n > 0 && idx.size(0) > 0) {
+      dx = spmm_transposed(g, ptr, idx, n, x.size(0), edge_val, reduce, flags, split);
+      need_dx = false;
+    }
+    if (need_dx || need_dval) {
+      cxg_spmm_desc d = describe(ptr, idx, n, g.dim() == 3 ? g.size(1) : 1, g.size(-1), g.scalar_type(), reduce, flags, split);
+      Tensor xs;
+      if (edge_val) d.edge_val = static_cast<const float *>(edge_val->data_ptr());
+      if (need_dx) dx = at::zeros(x.sizes(), x.options().dtype(at::kFloat));
+      if (need_dval) {
+        dval = at::zeros(edge_val->sizes(), edge_val->options());
+        xs = x.scalar_type() == g.scalar_type() ? x : x.to(g.scalar_type());
+        d.x = xs.data_ptr();
+      }
+      check(lib.cxg_spmm_csr_backward(&d, g.data_ptr(), need_dx ? dx.data_ptr<float>() : nullptr,
+                                      need_dval ? dval.data_ptr<float>() : nullptr, stream_of(g)),
+            "cxg_spmm_csr_backward");
+    }
+    if (dx.defined() && dx.scalar_type() != x.scalar_type()) dx = dx.to(x.scalar_type());
+    return {dx, Tensor(), Tensor(), dval, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor sage(const Tensor &x, const Tensor &ptr, const Tensor &idx, const optional<Tensor> &edge_val, int64_t num_node,
+            int64_t reduce, int64_t flags, int64_t split, bool scatter) {
+  if (at::GradMode::is_enabled() && (x.requires_grad() || (edge_val && edge_val->requires_grad())))
+    return SageFunction::apply(x, ptr, idx, edge_val, num_node, reduce, flags, split, scatter);
+  return spmm(x, ptr, idx, num_node, edge_val, reduce, c10::nullopt, c10::nullopt, c10::nullopt, 0, c10::nullopt, flags, split);
+}
+
+Tensor gather_rows(const Tensor &x, const Tensor &rows) {
+  cuda(x, "x");
+  of_type(rows, "rows", {at::kLong});
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = at::empty({rows.size(0), x.size(1)}, x.options());
+  check(lib.cxg_gather_rows(x.data_ptr(), rows.data_ptr<int64_t>(), out.data_ptr(), rows.size(0),
+                            x.size(1) * static_cast<int64_t>(x.element_size()), stream_of(x)),
+        "cxg_gather_rows");
+  return out;
+}
+
+// ---- neighbour sampling ----------------------------------------------------------------------------------------------
+// The most a call may reserve for the nodes and edges a batch can reach; above it the hops are run one by one.
+constexpr int64_t kMostSampled = 1 << 27;
+
+bool sample_batch_fits(int64_t n_seeds, std::vector<int> fanouts, int64_t n_nodes, int64_t nnz) {
+  int64_t nodes = 0, rows = 0, edges = 0;
+  size_t bytes = 0;
+  if (n_seeds < 1 || lib.cxg_sample_batch_bounds(n_seeds, fanouts.data(), static_cast<int>(fanouts.size()), n_nodes, nnz, &nodes,
+                                                 &rows, &edges, &bytes) != 0)
+    return false;
+  return nodes + edges <= kMostSampled;
+}
+
+// (nodes, ptr, idx, nodes after every hop, edges after every hop): one host synchronisation, at the end, for the sizes.
+std::tuple<Tensor, Tensor, Tensor, std::vector<int64_t>, std::vector<int64_t>> sample_batch(
+    const Tensor &gptr, const Tensor &gidx, const Tensor &seeds, std::vector<int> fanouts, std::vector<uint64_t> hop_seeds,
+    const Tensor &local_of, const Tensor &bitmap, const Tensor &host_sizes) {
+  index_of(gptr, "graph_ptr");
+  index_of(gidx, "graph_idx");
+  of_type(seeds, "seeds", {at::kLong});
+  const int hops = static_cast<int>(fanouts.size());
+  const int64_t n_nodes = gptr.size(0) - 1, nnz = gidx.size(0);
+  int64_t max_nodes = 0, max_rows = 0, max_edges = 0;
+  size_t bytes = 0;
+  check(lib.cxg_sample_batch_bounds(seeds.size(0), fanouts.data(), hops, n_nodes, nnz, &max_nodes, &max_rows, &max_edges, &bytes),
+        "cxg_sample_batch_bounds");
+  c10::cuda::CUDAGuard guard(seeds.device());
+  const auto opt = seeds.options();
+  Tensor nodes = at::empty({max_nodes}, opt), ptr = at::empty({max_rows + 1}, opt), idx = at::empty({max_edges}, opt);
+  Tensor sizes = at::empty({2 * (hops + 1)}, opt);
+  void *st = stream_of(seeds);
+  const Tensor ws = workspace_on(seeds.device().index(), st, static_cast<int64_t>(bytes), "");
+  check(lib.cxg_sample_batch(gptr.data_ptr(), gidx.data_ptr(), static_cast<int>(gptr.element_size()),
+                             static_cast<int>(gidx.element_size()), n_nodes, nnz, seeds.data_ptr<int64_t>(), seeds.size(0),
+                             fanouts.data(), hops, hop_seeds.data(), local_of.data_ptr<int64_t>(),
+                             reinterpret_cast<uint32_t *>(bitmap.data_ptr()), nodes.data_ptr<int64_t>(), ptr.data_ptr<int64_t>(),
+                             idx.data_ptr<int64_t>(), sizes.data_ptr<int64_t>(), ws.data_ptr(), static_cast<size_t>(ws.numel()), st),
+        "cxg_sample_batch");
+  host_sizes.narrow(0, 0, sizes.size(0)).copy_(sizes, /*non_blocking=*/true);
+  {
+    py::gil_scoped_release other_threads;
+    c10::cuda::getCurrentCUDAStream(seeds.device().index()).synchronize();
+  }
+  const int64_t *h = host_sizes.data_ptr<int64_t>();
+  std::vector<int64_t> known(h, h + hops + 1), edges(h + hops + 2, h + 2 * (hops + 1));
+  const int64_t rows = known[hops - 1];
+  return {nodes.narrow(0, 0, known[hops]), ptr.narrow(0, 0, rows + 1), idx.narrow(0, 0, edges[hops - 1]), known, edges};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("init", &init);
+  m.def("workspace", &workspace);
+  m.def("last_workspace", &last_workspace);
+  m.def("spmm", &spmm);
+  m.def("sage", &sage);
+  m.def("transpose", [](const Tensor &ptr, const Tensor &idx, int64_t n, int64_t n_src, bool want_eid) {
+    const Transposed t = transpose(ptr, idx, n, n_src, want_eid);
+    return std::make_tuple(t.t_ptr, t.t_idx, want_eid ? optional<Tensor>(t.t_eid) : c10::nullopt, t.inv_deg);
+  });
+  m.def("transposed_graph", [](const Tensor &ptr, const Tensor &idx, int64_t n, int64_t n_src) {
+    const Transposed t = transposed_graph(ptr, idx, n, n_src);
+    return std::make_tuple(t.t_ptr, t.t_idx, t.t_eid, t.inv_deg);
+  });
+  m.def("forget_graphs", &forget_graphs);
+  m.def("count_graphs", &count_graphs);
+  m.def("gather_rows", &gather_rows);
+  m.def("sample_batch_fits", &sample_batch_fits);
+  m.def("sample_batch", &sample_batch);
+}

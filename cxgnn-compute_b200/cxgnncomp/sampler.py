@@ -24,6 +24,9 @@ class NeighborSampler:
         self.num_nodes = graph_ptr.shape[0] - 1
         # global id -> position in the batch, -1 outside the batch; cleared after every batch
         self.local_of = torch.full((self.num_nodes,), -1, dtype=torch.int64, device=graph_ptr.device)
+        # one bit per node, zero between batches; the sizes of a batch as the host reads them
+        self._marks = torch.zeros((self.num_nodes + 31) // 32, dtype=torch.int32, device=graph_ptr.device)
+        self._sizes = torch.empty(64, dtype=torch.int64, pin_memory=graph_ptr.is_cuda)
         self.n_fresh = torch.zeros(1, dtype=torch.int64, device=graph_ptr.device)
         self._fresh_buf = torch.empty(0, dtype=torch.int64, device=graph_ptr.device)
 
@@ -36,6 +39,10 @@ class NeighborSampler:
     def sample(self, seeds, seed=0):
         """seeds: distinct int64 global ids on the graph's device. Returns (nodes, ptr, idx, num_node_in_layer,
         num_edge_in_layer) with ptr / idx int64 on the device."""
+        if cxgnncomp_backend.sample_batch_fits(seeds.shape[0], self.fanouts, self.num_nodes, self.idx.shape[0]):
+            # all hops in one call, sizes read back once
+            return cxgnncomp_backend.sample_batch(self.ptr, self.idx, seeds, self.fanouts, seed, self.local_of,
+                                                  self._marks, self._sizes)
         dev = seeds.device
         local_of = self.local_of
         nodes = [seeds]
@@ -67,4 +74,4 @@ class NeighborSampler:
     def batch(self, x, seeds, seed=0, y=None):
         """A `Batch` with the features (and labels of the seeds) gathered for the sampled nodes."""
         nodes, ptr, idx, num_node, num_edge = self.sample(seeds, seed)
-        return Batch(x[nodes], ptr, idx, num_node, num_edge, target=nodes, y=None if y is None else y[seeds])
+        return Batch(cxgnncomp_backend.take_rows(x, nodes), ptr, idx, num_node, num_edge, target=nodes, y=None if y is None else y[seeds])

@@ -31,10 +31,16 @@ def _load():
         raise ImportError(
             f"{path} is missing: build it with `python {os.path.join(os.path.dirname(path), 'build.py')}` "
             "(nvcc, sm_100a). There is no CPU or PyTorch fallback for these operators.")
-    return ctypes.CDLL(path)
+    return ctypes.CDLL(path), path
 
 
-_lib = _load()
+_lib, _lib_file = _load()
+try:
+    from . import _native  # argument checks, scratch, launches and autograd of the frequent operators, in C++
+except ImportError as e:
+    raise ImportError(f"the backend's host module is missing or does not load ({e}): build it with "
+                      f"`python {os.path.join(os.path.dirname(os.path.abspath(_LIB_PATH)), 'build.py')}`") from e
+_native.init(_lib_file)
 _vp, _i64, _i32, _u32, _sz = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32, ctypes.c_uint32, ctypes.c_size_t
 
 
@@ -130,7 +136,6 @@ _on = _OnDevice
 
 _FEAT_DTYPES = (torch.float32, torch.bfloat16)
 _INDEX_DTYPES = (torch.int64, torch.int32)
-_workspaces = {}
 
 # Rows with more edges than this are split into segments; 0 keeps the library default.
 # Tests lower it to exercise the split path on small graphs.
@@ -147,20 +152,10 @@ CXG_TMM_GATHER4 = 32  # gathered rows through the bulk tensor copy unit (tile::g
 EXTRA_SPMM_FLAGS = int(os.environ.get("CXG_SPMM_FLAGS", "0"))
 
 
-_last_kind = {}
-
-
-def _workspace(device, nbytes, kind=None):
+def _workspace(device, nbytes, kind=""):
     """Scratch buffer per (device, stream); grows on demand, contents never carry over. `kind` names the entry
     point family that uses it now (its status word is the one check_device_status can answer for)."""
-    idx = _dev_index(device)
-    key = (idx, _raw_stream(idx))
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    _last_kind[key] = kind
-    return buf
+    return _native.workspace(_dev_index(device), nbytes, kind)
 
 
 def _dtype_code(t):
@@ -213,10 +208,8 @@ def check_device_status(kind="spmm", device=None):
     of spinning forever) or, for "spmm", ptr[num_node] exceeded the length of idx. The calls of one stream share
     a scratch buffer, so only the last call can be asked about; for any other kind nothing is checked."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    idx = _dev_index(device)
-    key = (idx, _raw_stream(idx))
-    ws = _workspaces.get(key)
-    if ws is None or _last_kind.get(key) != kind:
+    ws, last = _native.last_workspace(_dev_index(device))
+    if ws is None or last != kind:
         return
     fn, name = (_spmm_status, "cxg_spmm_csr_status") if kind == "spmm" else (_tmm_status, "cxg_typed_matmul_status")
     with _on(device):
@@ -233,39 +226,11 @@ def set_wait_limit_cycles(cycles):
     _check(_set_wait(int(cycles)), "cxg_set_wait_limit_cycles")
 
 
-def _run_spmm(desc, device):
-    need = _sz(0)
-    _check(_spmm_ws(desc.n_dst, desc.nnz, desc.feat, desc.heads, desc.split_edges, ctypes.byref(need)),
-           "cxg_spmm_csr_workspace_size")
-    ws = _workspace(device, need.value, "spmm")
-    with _on(device):
-        _check(_spmm_fwd(ctypes.byref(desc), _p(ws), ws.numel(), _stream()), "cxg_spmm_csr")
-
-
 def _spmm_forward(x, ptr, idx, num_node, *, edge_val=None, reduce=CXG_SUM, out=None, accumulate=False,
                   edge_mask=None, edge_rel=None, rel_stride=0, targets=None, flags=0):
     """y = A x for the first `num_node` rows; x is [N_s, F] or [N_s, H, F]."""
-    _cuda(x, "x", _FEAT_DTYPES)
-    n = _num_rows(ptr, num_node)
-    heads = 1
-    if x.dim() == 3:
-        heads = x.shape[1]
-    elif x.dim() != 2:
-        raise RuntimeError("x must be [N, F] or [N, H, F]")
-    feat = x.shape[-1]
-    if edge_val is not None:
-        _cuda(edge_val, "edge_value", (torch.float32,))
-        ev_heads = edge_val.shape[1] if edge_val.dim() == 2 else 1
-        if ev_heads != heads and not (heads == 1 and ev_heads == 1):
-            raise RuntimeError(f"edge_value has {ev_heads} heads, x has {heads}")
-    if out is None:
-        shape = (n, heads, feat) if x.dim() == 3 else (n, feat)
-        out = torch.empty(shape, dtype=x.dtype, device=x.device)
-    desc = _make_desc(ptr, idx, x, out, n, heads=heads, feat=feat, edge_val=edge_val, edge_mask=edge_mask,
-                      edge_rel=edge_rel, rel_stride=rel_stride, targets=targets, reduce=reduce,
-                      accumulate=accumulate, flags=flags)
-    _run_spmm(desc, x.device)
-    return out
+    return _native.spmm(x, ptr, idx, int(num_node), edge_val, reduce, out, edge_mask, edge_rel, rel_stride, targets,
+                        (CXG_SPMM_ACCUMULATE if accumulate else 0) | EXTRA_SPMM_FLAGS | flags, SPLIT_EDGES)
 
 
 # dX = A^T dY is a forward aggregation over the transposed graph: deterministic and on the fast forward
@@ -274,11 +239,19 @@ def _spmm_forward(x, ptr, idx, num_node, *, edge_val=None, reduce=CXG_SUM, out=N
 # of the edges by source) the first time a backward is asked for a graph and kept in a small cache keyed by the
 # ptr / idx tensors. BACKWARD_MODE: "auto" (= "transpose" wherever it applies) | "scatter" | "transpose".
 BACKWARD_MODE = os.environ.get("CXG_BACKWARD_MODE", "auto")
-_TRANSPOSE_CACHE = {}
-_TRANSPOSE_CACHE_MAX = 8
-_transpose_ws = _sig("cxg_csr_transpose_workspace_size", [_i64, ctypes.POINTER(_sz)])
-_transpose = _sig("cxg_csr_transpose", [_vp, _vp, ctypes.c_int, ctypes.c_int, _i64, _i64, _i64, _vp, _vp, _vp, _vp,
-                                        _vp, _sz, _vp])
+
+
+class _TransposeCache:
+    """The transposed graphs the backward keeps (the last eight), as far as callers look at them."""
+
+    def __len__(self):
+        return _native.count_graphs()
+
+    def clear(self):
+        _native.forget_graphs()
+
+
+_TRANSPOSE_CACHE = _TransposeCache()
 
 
 def csr_transpose(ptr, idx, num_node, num_src, want_eid=True):
@@ -286,36 +259,12 @@ def csr_transpose(ptr, idx, num_node, num_src, want_eid=True):
     graph (ptr, idx): row s of the transposed graph lists the destinations of source s in ascending order, t_eid
     the forward edge of every transposed edge (what a stable sort of idx returns), inv_deg 1 / in-degree per
     destination. t_idx / t_eid have the dtype and length of idx; entries past ptr[num_node] are not written."""
-    _cuda(ptr, "ptr", _INDEX_DTYPES)
-    _cuda(idx, "idx", _INDEX_DTYPES)
-    n = _num_rows(ptr, num_node)
-    nnz = idx.shape[0]
-    dev = ptr.device
-    t_ptr = torch.empty(num_src + 1, dtype=torch.int64, device=dev)
-    t_idx = torch.empty(nnz, dtype=idx.dtype, device=dev)
-    t_eid = torch.empty(nnz, dtype=idx.dtype, device=dev) if want_eid else None
-    inv_deg = torch.empty(n, dtype=torch.float32, device=dev)
-    need = _sz(0)
-    _check(_transpose_ws(nnz, ctypes.byref(need)), "cxg_csr_transpose_workspace_size")
-    ws = _workspace(dev, need.value)
-    with _on(dev):
-        _check(_transpose(_p(ptr), _p(idx), ptr.element_size(), idx.element_size(), n, int(num_src), nnz, _p(t_ptr),
-                          _p(t_idx), _p(t_eid), _p(inv_deg), _p(ws), ws.numel(), _stream()), "cxg_csr_transpose")
-    return t_ptr, t_idx, t_eid, inv_deg
+    return _native.transpose(ptr, idx, int(num_node), int(num_src), bool(want_eid))
 
 
 def _transposed_graph(ptr, idx, n, n_src):
     """Cached csr_transpose of the first n rows."""
-    key = (ptr.data_ptr(), idx.data_ptr(), n, n_src, ptr._version, idx._version, str(ptr.device))
-    hit = _TRANSPOSE_CACHE.get(key)
-    if hit is not None:
-        return hit[:4]
-    entry = csr_transpose(ptr, idx, n, n_src)
-    while len(_TRANSPOSE_CACHE) >= _TRANSPOSE_CACHE_MAX:
-        _TRANSPOSE_CACHE.pop(next(iter(_TRANSPOSE_CACHE)))
-    # ptr and idx are kept alive with the entry, so their addresses cannot be handed to another graph
-    _TRANSPOSE_CACHE[key] = entry + (ptr, idx)
-    return entry
+    return _native.transposed_graph(ptr, idx, n, n_src)
 
 
 def _spmm_backward(grad_out, x, ptr, idx, num_node, *, edge_val=None, reduce=CXG_SUM, need_dx=True,
@@ -372,42 +321,21 @@ def _spmm_backward(grad_out, x, ptr, idx, num_node, *, edge_val=None, reduce=CXG
 # --------------------------------------------------------------------------------------
 # autograd-aware aggregation (reference: C++ torch::autograd::Function, src/cpp/include/aggr.h:13-33)
 # --------------------------------------------------------------------------------------
-class _SageFunction(torch.autograd.Function):
-    """SAGEFunction / SAGEEdgeValueFunction (src/cpp/src/aggr.cu:275-303).
-
-    The reference stashes raw device pointers of ptr/idx between forward and backward
-    (aggr.cu:116-117); the tensors themselves are saved here, so they cannot dangle.
-    """
-
-    @staticmethod
-    def forward(ctx, x, ptr, idx, edge_val, num_node, reduce):
-        ctx.num_node = num_node
-        ctx.reduce = reduce
-        ctx.save_for_backward(x, ptr, idx, edge_val if edge_val is not None else torch.empty(0))
-        ctx.has_val = edge_val is not None
-        return _spmm_forward(x, ptr, idx, num_node, edge_val=edge_val, reduce=reduce)
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        x, ptr, idx, edge_val = ctx.saved_tensors
-        edge_val = edge_val if ctx.has_val else None
-        need_dx = ctx.needs_input_grad[0]
-        need_dval = ctx.has_val and ctx.needs_input_grad[3]
-        dx, dval = _spmm_backward(grad_out, x, ptr, idx, ctx.num_node, edge_val=edge_val, reduce=ctx.reduce,
-                                  need_dx=need_dx, need_dval=need_dval)
-        if dx is not None and dx.dtype != x.dtype:
-            dx = dx.to(x.dtype)
-        return dx, None, None, dval, None, None
+def _sage(x, ptr, idx, edge_value, num_node, reduce):
+    """SAGEFunction / SAGEEdgeValueFunction (src/cpp/src/aggr.cu:275-303): forward and gradients in one C++ autograd
+    function. The reference stashes raw device pointers of ptr/idx between forward and backward (aggr.cu:116-117);
+    the tensors themselves are saved there, so they cannot dangle."""
+    return _native.sage(x, ptr, idx, edge_value, num_node, reduce, EXTRA_SPMM_FLAGS, SPLIT_EDGES, BACKWARD_MODE == "scatter")
 
 
 def sage_sum_forward(x, ptr, idx, num_node):
     """out[r] = sum of x[idx[e]] over row r (binding.cpp:20, aggr.cu:390-393)."""
-    return _SageFunction.apply(x, ptr, idx, None, num_node, CXG_SUM)
+    return _sage(x, ptr, idx, None, num_node, CXG_SUM)
 
 
 def sage_mean_forward(x, ptr, idx, num_node):
     """out[r] = mean of x[idx[e]] over row r, 0 for empty rows (binding.cpp:19, aggr.cu:385-388)."""
-    return _SageFunction.apply(x, ptr, idx, None, num_node, CXG_MEAN)
+    return _sage(x, ptr, idx, None, num_node, CXG_MEAN)
 
 
 def sage_sum_forward_edge_value(x, ptr, idx, edge_value, num_node):
@@ -415,7 +343,7 @@ def sage_sum_forward_edge_value(x, ptr, idx, edge_value, num_node):
     (binding.cpp:17, aggr.cu:377-383)."""
     if edge_value.dim() == 2 and x.dim() == 2 and edge_value.shape[1] == 1:
         edge_value = edge_value.reshape(-1)
-    return _SageFunction.apply(x, ptr, idx, edge_value, num_node, CXG_SUM)
+    return _sage(x, ptr, idx, edge_value, num_node, CXG_SUM)
 
 
 def sage_mean_forward_edge_value(x, ptr, idx, edge_value, num_node):
@@ -573,6 +501,26 @@ def sample_neighbors(graph_ptr, graph_idx, frontier, fanout, seed):
                        int(fanout), _p(out_ptr), _p(out), int(seed) & 0xFFFFFFFFFFFFFFFF, _stream()),
                "cxg_sample_neighbors")
     return out_ptr, out
+
+
+sample_batch_fits = _native.sample_batch_fits
+
+
+def sample_batch(graph_ptr, graph_idx, seeds, fanouts, seed, local_of, marks, host_sizes):
+    """(nodes, ptr, idx, nodes after every hop, edges after every hop) of a batch: all hops in one call
+    (cxg_sample_batch), hop h drawn with seed * 1000003 + h. local_of: -1 per node, marks: a zero bit per node, both as
+    before when the call returns; host_sizes: pinned int64, at least 2 * (hops + 1)."""
+    return _native.sample_batch(graph_ptr, graph_idx, seeds, fanouts,
+                                [(seed * 1000003 + h) & 0xFFFFFFFFFFFFFFFF for h in range(len(fanouts))], local_of, marks,
+                                host_sizes)
+
+
+def take_rows(x, rows):
+    """x[rows] for a 2-D x: one gathering kernel where no gradient is asked for."""
+    if (isinstance(x, torch.Tensor) and x.is_cuda and x.dim() == 2 and x.is_contiguous() and not x.requires_grad
+            and x.element_size() % 2 == 0):
+        return _native.gather_rows(x, rows)
+    return x[rows]
 
 
 _claim = _sig("cxg_renumber_claim", [_vp, _i64, _vp, _vp, _vp, _vp])

@@ -434,6 +434,24 @@ int cxg_put_rows(const void *in, const int64_t *rows, void *const *peer_base_hos
  * d <= fanout, else a uniform subset drawn by Floyd's algorithm from a counter-based generator keyed by
  * (seed, v). out_ptr is the caller's exclusive prefix sum of min(d, fanout). fanout <= 64.
  */
+/*
+ * A whole batch of layer-wise sampling in one call, nothing read back in between: hop h draws fanouts[h] neighbours
+ * (cxg_sample_neighbors with hop_seeds[h]) of the nodes first reached at hop h - 1 (the seeds at hop 0), new nodes get
+ * batch ids in ascending order of their node id behind the ones before. nodes[batch id], row_ptr / edges = CSR rows of
+ * the expanded nodes in batch ids, sizes[0 .. hops] = nodes known before hop 0, after hop 0, ..., sizes[hops + 1 ..
+ * 2 hops + 1] = edges before hop 0, after hop 0, ... (device memory). local_of[n_nodes] is -1 and bitmap[ceil(n_nodes /
+ * 32)] zero before and after the call. Up to 16 hops of fanout 1 to 64. cxg_sample_batch_bounds gives the lengths the
+ * output arrays need (nodes: max_nodes, row_ptr: max_rows + 1, edges: max_edges) and the scratch bytes; fanouts and
+ * hop_seeds are host memory.
+ */
+int cxg_sample_batch_bounds(int64_t n_seeds, const int *fanouts, int hops, int64_t n_nodes, int64_t nnz,
+                            int64_t *max_nodes, int64_t *max_rows, int64_t *max_edges, size_t *workspace_bytes);
+int cxg_sample_batch(const void *graph_ptr, const void *graph_idx, int ptr_bytes, int idx_bytes, int64_t n_nodes,
+                     int64_t nnz, const int64_t *seeds, int64_t n_seeds, const int *fanouts, int hops,
+                     const uint64_t *hop_seeds, int64_t *local_of, uint32_t *bitmap, int64_t *nodes,
+                     int64_t *row_ptr, int64_t *edges, int64_t *sizes, void *workspace, size_t workspace_bytes,
+                     void *stream);
+
 /* counts[i] = min(in-degree of frontier[i], fanout): the row lengths whose prefix sum is out_ptr below. */
 int cxg_sample_counts(const void *graph_ptr, int ptr_bytes, const int64_t *frontier, int64_t n_front,
                       int fanout, int64_t *counts, void *stream);
