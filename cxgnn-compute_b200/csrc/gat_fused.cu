@@ -8,9 +8,9 @@
 // Here per-edge values never reach memory:
 //
 //   forward   y[r,h,:] = sum_e p[e,h] x[s(e),h,:],  p = softmax over the edges of row r of
-//             t[e,h] = leaky(a_dst[r,h] + a_src[s(e),h]).  The walk is the edge-tiled one of the
-//             streaming SpMM (tiles of consecutive edges, one warp per tile, feature rows staged
-//             with 16-byte cp.async); per (row, head) it keeps a running maximum m and a running
+//             t[e,h] = leaky(a_dst[r,h] + a_src[s(e),h]).  The walk is the register-staged tiled one
+//             of the SpMM (spmm_walk_impl.cuh: tiles of consecutive edges, a group of lanes per tile,
+//             rows of any width); per (row, head) it keeps a running maximum m and a running
 //             sum s and rescales the fp32 accumulator when the maximum grows (online softmax):
 //                 m' = max(m, t);  acc = acc * exp(m - m') + exp(t - m') * x;  s likewise.
 //             Outputs y, row_max = m and row_sum = s per (row, head): [N, H] each instead of [E, H].
@@ -29,531 +29,910 @@
 //                 destination then adds its edges' values in a fixed order (same bits on every run); without
 //                 it, one atomic add per edge and head (order not fixed, as the reference's grad_src atomics).
 //
-// Shapes covered: fp32 features, heads a power of two <= 16, a feature row (heads * c floats) of exactly
-// 128, 256 or 512 bytes (every lane owns 4, 8 or 16 bytes of it, inside one head). Everything else stays on
+// Shapes covered: fp32 features, heads a power of two <= 16, a feature row (heads * c floats) of up to 2 KiB (c a
+// multiple of 4), 1 KiB (c even) or 1.5 KiB (any c); backward with c a power of two, at most 128. Everything else stays on
 // the separate kernels (cxg_gat_scores, cxg_edge_softmax_forward, cxg_spmm_csr).
-#include "common.cuh"
+//
+// What bounds it: instructions per edge and per row end, with an IPC of 0.55 to 0.65 per scheduler; the gather stays in L2
+// for graphs of this kind. 2.33 M edges, 4 heads x 32: forward 203 -> 178 us and its fix-up 52 -> 17, backward 407 -> 288
+// us and 42 -> 17 (before: rows and scores staged in shared memory, a whole warp per edge). 4 heads x 47 ran on the edge
+// softmax and the weighted aggregation before (0.79 ms; now 0.52).
+#include "spmm_walk_impl.cuh"
 
 namespace cxg {
 namespace {
 
-constexpr int kGWarps = 4;
-constexpr int kGThreads = kGWarps * 32;
-constexpr int kGCtasPerSM = 5;
-constexpr int kGStageBytes = 8192;
-constexpr int kGFar = 1 << 30;
+using walk::kFar;
+using walk::kThreads;
+using walk::load_id_stream;
+
 constexpr float kNegBig = -1e30f;  // "no edge yet": exp(kNegBig - t) is 0 for every finite t
-constexpr int kFixSeq = 32;        // chains of more partials are joined by a whole CTA
 constexpr int kLongRowEdges = 256;  // ordered d a_dst: destinations with more edges are summed piecewise by CTAs
                                     // (a single warp on a longer row is the tail of the kernel)
 
 struct GatArgs {
-  const void *ptr;       // graph that is walked: CSR (forward) or transposed CSR (backward)
-  const void *idx;
-  const float *gathered; // rows fetched per edge: x [n_src, H, C] (forward), dy [n_dst, H, C] (backward)
+  WalkArgs w;            // graph that is walked (CSR forward, transposed CSR backward) and its plan; w.x = rows fetched per
+                         // edge: x [n_src, H, C] (forward), dy [n_dst, H, C] (backward); w.y = y (forward), dx (backward)
   const float *g_small;  // small per-node record fetched per edge: a_src [n_src, H] (forward),
                          // stats [n_dst, H, 4] = {a_dst, row_max, 1 / row_sum, D} (backward)
   const float *r_small;  // per walked row: a_dst [n_dst, H] (forward), a_src [n_src, H] (backward)
   const float *r_feat;   // backward: x [n_src, H, C]
-  float *out;            // y [n_dst, H, C] (forward), dx [n_src, H, C] (backward)
   float *row_max;        // forward [n_dst, H]
   float *row_sum;        // forward [n_dst, H]
   float *d_r_small;      // backward: d a_src [n_src, H]
   float *d_g_small;      // backward: d a_dst [n_dst, H], added into atomically (when d_edge is NULL)
   const void *eid;       // backward, ordered mode: forward edge of every transposed edge (width of idx)
   float *d_edge;         // backward, ordered mode: [nnz, H] score gradient of every edge at its forward position
-  int64_t n_rows, nnz, max_tiles;
-  int heads, hshift, c, ptr_bytes, idx_bytes, tile;
+  int heads, c;
   float slope;
-  int32_t *hdr;
-  int64_t *tile_row, *tail_row;
-  int64_t *long_tiles;  // first tile of every chain of more than kFixSeq partials
-  int max_long;
-  float *part_acc;  // [tile][2][width]
-  float *part_ms;   // [tile][2][heads][2]: forward (m, s); backward (d a_src partial, unused)
+  float *part_ms;        // [tile][2][heads][2]: forward (m, s); backward (unused, d a_src partial)
+  float *block_ms;       // [tile][heads][2]: those of a block of a long chain
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+// exp(x): as __expf, with results below 2^-126 flushed to zero (three instructions instead of six)
+__device__ __forceinline__ float exp_flush(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.4426950408889634f));
+  return r;
 }
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ float lds_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-template <int EL>
-__device__ __forceinline__ void lds_row(float *f, uint32_t addr) {
-  if (EL == 1) {
-    f[0] = lds_f32(addr);
-  } else if (EL == 2) {
-    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(f[0]), "=f"(f[EL > 1 ? 1 : 0]) : "r"(addr));
-  } else {
-    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(f[0]), "=f"(f[EL > 1 ? 1 : 0]), "=f"(f[EL > 2 ? 2 : 0]), "=f"(f[EL > 3 ? 3 : 0])
-                 : "r"(addr));
-  }
-}
-template <int EL>
-__device__ __forceinline__ void stg_row(float *p, const float *f) {
-  if (EL == 1)
-    *p = f[0];
-  else if (EL == 2)
-    *reinterpret_cast<float2 *>(p) = make_float2(f[0], f[EL > 1 ? 1 : 0]);
-  else
-    *reinterpret_cast<float4 *>(p) = make_float4(f[0], f[EL > 1 ? 1 : 0], f[EL > 2 ? 2 : 0], f[EL > 3 ? 3 : 0]);
-}
-template <int EL>
-__device__ __forceinline__ void ldg_row(float *f, const float *p) {
-  if (EL == 1) {
-    f[0] = __ldg(p);
-  } else if (EL == 2) {
-    const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
-    f[0] = v.x, f[EL > 1 ? 1 : 0] = v.y;
-  } else {
-    const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
-    f[0] = v.x, f[EL > 1 ? 1 : 0] = v.y, f[EL > 2 ? 2 : 0] = v.z, f[EL > 3 ? 3 : 0] = v.w;
-  }
-}
-__device__ __forceinline__ float leaky(float t, float slope) { return fmaxf(t, t * slope); }
 
-// acc = acc * sc + w * f over EL floats; pairs go through the packed f32x2 pipe (each half rounded like the
-// scalar operation).
-template <int EL>
-__device__ __forceinline__ void scale_fma(float *acc, const float *f, float sc, float w) {
-  if (EL == 1) {
-    acc[0] = fmaf(w, f[0], acc[0] * sc);
-  } else {
-    unsigned long long s2, w2;
-    asm("mov.b64 %0, {%1,%1};" : "=l"(s2) : "f"(sc));
-    asm("mov.b64 %0, {%1,%1};" : "=l"(w2) : "f"(w));
-#pragma unroll
-    for (int i = 0; i < EL; i += 2) {
-      unsigned long long a2, f2;
-      asm("mov.b64 %0, {%1,%2};" : "=l"(a2) : "f"(acc[i]), "f"(acc[(i + 1) % EL]));
-      asm("mov.b64 %0, {%1,%2};" : "=l"(f2) : "f"(f[i]), "f"(f[(i + 1) % EL]));
-      asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(a2) : "l"(s2));
-      asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a2) : "l"(w2), "l"(f2));
-      asm("mov.b64 {%0,%1}, %2;" : "=f"(acc[i]), "=f"(acc[(i + 1) % EL]) : "l"(a2));
+// Per-tile state of a walk: where the walk stands in the rows. Positions are relative to the tile's first edge.
+struct TileWalk {
+  const GatArgs &a;
+  int64_t begin, row;
+  int len, rend, rstart, stop;
+  int64_t next_raw;  // end of the row behind the walked one, requested a row ahead
+  __device__ __forceinline__ int64_t end_raw(int64_t r) const {
+    return load_ptr(a.w.ptr, min(r + 1, a.w.n_dst), a.w.ptr_bytes);
+  }
+  __device__ __forceinline__ int end_rel(int64_t r, int64_t raw) const {
+    const int64_t v = raw - begin;
+    return r >= a.w.n_dst || v > kFar ? kFar : static_cast<int>(v);
+  }
+  __device__ __forceinline__ void start() {
+    rend = end_rel(row, end_raw(row));
+    next_raw = end_raw(row + 1);
+    const int64_t s = load_ptr(a.w.ptr, row, a.w.ptr_bytes) - begin;
+    rstart = s < -kFar ? -kFar : static_cast<int>(s);
+    stop = min(rend, len);
+  }
+  __device__ __forceinline__ void next() {
+    ++row;
+    rend = end_rel(row, next_raw);
+    next_raw = end_raw(row + 1);
+  }
+  __device__ __forceinline__ uint32_t load_id(int pos) const {
+    if (pos >= len) return 0u;
+    return a.w.idx_bytes == 8 ? static_cast<uint32_t>(load_id_stream(static_cast<const int64_t *>(a.w.idx) + begin + pos))
+                              : static_cast<uint32_t>(load_id_stream(static_cast<const int32_t *>(a.w.idx) + begin + pos));
+  }
+  // backward: the score gradient of the edge at `pos`, whose destination is `dst`
+  __device__ __forceinline__ void edge_gradient(int pos, uint32_t dst, int head, float dt) const {
+    if (a.d_edge != nullptr) {
+      const int64_t e = a.w.idx_bytes == 8 ? __ldg(static_cast<const int64_t *>(a.eid) + begin + pos)
+                                           : __ldg(static_cast<const int32_t *>(a.eid) + begin + pos);
+      a.d_edge[e * a.heads + head] = dt;
+    } else {
+      asm volatile("red.global.add.f32 [%0], %1;" ::"l"(a.d_g_small + static_cast<int64_t>(dst) * a.heads + head), "f"(dt)
+                   : "memory");
     }
   }
-}
-__device__ __forceinline__ void red_add_f32(float *addr, float v) {
-  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
-}
+};
 
-__device__ __forceinline__ int64_t edge_total(const GatArgs &a) {
-  const int64_t e = load_ptr(a.ptr, a.n_rows, a.ptr_bytes);
-  return e > a.nnz ? a.nnz : e;
-}
-
-__global__ void gat_plan(GatArgs a) {
-  const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (t == 0) {
-    a.hdr[0] = 0;  // number of long chains
-    a.hdr[1] = 0;  // number of long destinations (ordered d a_dst)
+template <int VB>
+__device__ __forceinline__ void load_floats(float (&f)[VB / 4], const float *p) {
+  if constexpr (VB == 16) {
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
+    f[0] = v.x, f[1] = v.y, f[2] = v.z, f[3] = v.w;
+  } else if constexpr (VB == 8) {
+    const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
+    f[0] = v.x, f[1] = v.y;
+  } else {
+    f[0] = __ldg(p);
   }
-  if (t >= a.max_tiles) return;
-  a.tail_row[t] = -1;
-  const int64_t e_total = edge_total(a);
-  const int64_t pos = t * a.tile;
-  if (pos >= e_total) return;
-  int64_t lo = 0, hi = a.n_rows;  // ptr[lo] <= pos < ptr[hi]
-  while (hi - lo > 1) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (load_ptr(a.ptr, mid, a.ptr_bytes) <= pos)
-      lo = mid;
-    else
-      hi = mid;
-  }
-  a.tile_row[t] = lo;
+}
+template <int W>
+__device__ __forceinline__ void store_floats(float *dst, const float (&f)[W]) {
+  if constexpr (W == 4)
+    __stcs(reinterpret_cast<float4 *>(dst), make_float4(f[0], f[1], f[2], f[3]));
+  else if constexpr (W == 2)
+    __stcs(reinterpret_cast<float2 *>(dst), make_float2(f[0], f[1]));
+  else
+    __stcs(dst, f[0]);
 }
 
-// The walk shared by both directions. CB = bytes of a feature row per lane (row = 32 * CB bytes).
-// BWD = false: forward (online softmax). BWD = true: backward on the transposed graph.
-template <int CB, typename IdxT, bool BWD>
-__global__ void __launch_bounds__(kGThreads, kGCtasPerSM) gat_walk(GatArgs a) {
-  constexpr int EL = CB / 4;
-  constexpr int RB = 32 * CB;
-  constexpr int B = kGStageBytes / RB > 32 ? 32 : kGStageBytes / RB;
-  constexpr int CPR = RB / 16, RPI = 32 / CPR, NCOPY = B * CPR / 32;
-  constexpr int WIDTH = RB / 4;
-  extern __shared__ __align__(128) uint8_t smem[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int H = a.heads;
-  const int small_bytes = BWD ? H * 16 : H * 4;  // per-edge record
-  const int warp_smem = B * RB + B * small_bytes;
-  const uint32_t sl = smem_u32(smem + static_cast<size_t>(warp) * warp_smem);
-  const uint32_t sv = sl + B * RB;
-  const uint32_t my = sl + lane * CB;
-  const int lph = (a.c * 4) / CB;  // lanes per head
-  const int h = lane / lph;        // this lane's head
-  const bool head_lead = (lane % lph) == 0;
-  const IdxT *idx = reinterpret_cast<const IdxT *>(a.idx);
-  const uint8_t *xg = reinterpret_cast<const uint8_t *>(a.gathered);
-  const int64_t e_total = edge_total(a);
-  const int64_t n_tiles = (e_total + a.tile - 1) / a.tile;
-  const int64_t gwarp = static_cast<int64_t>(blockIdx.x) * kGWarps + warp;
-  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kGWarps;
-  const int jrow = lane / CPR;
-  const uint8_t *xlane = xg + (lane % CPR) * 16;
-  const uint32_t cdst = sl + lane * 16;
-  const float slope = a.slope;
-
-  // a row of the walked graph without entries: zeros (and "no edge" statistics in the forward direction)
-  auto empty_row = [&](int64_t r) {
-    float z[EL];
+// acc = acc * keep + prob * f and acc += prob * f, two columns per instruction
+template <int W>
+__device__ __forceinline__ void scale_add(float (&acc)[W], float keep, const float (&f)[W], float prob) {
+  if constexpr (W == 1) {
+    acc[0] = fmaf(acc[0], keep, prob * f[0]);
+  } else {
 #pragma unroll
-    for (int i = 0; i < EL; ++i) z[i] = 0.f;
-    stg_row<EL>(a.out + r * WIDTH + lane * EL, z);
-    if (head_lead) {
+    for (int i = 0; i < W; i += 2)
+      asm("{\n\t.reg .b64 a, k, v, p;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 k, {%2, %2};\n\tmov.b64 v, {%3, %4};\n\t"
+          "mov.b64 p, {%5, %5};\n\tmul.rn.f32x2 v, v, p;\n\tfma.rn.f32x2 a, a, k, v;\n\tmov.b64 {%0, %1}, a;\n\t}"
+          : "+f"(acc[i]), "+f"(acc[(i + 1) % W])
+          : "f"(keep), "f"(f[i]), "f"(f[(i + 1) % W]), "f"(prob));
+  }
+}
+template <int W>
+__device__ __forceinline__ void scale_add(float (&acc)[W], const float (&f)[W], float prob) {
+  if constexpr (W == 1) {
+    acc[0] = fmaf(prob, f[0], acc[0]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < W; i += 2)
+      asm("{\n\t.reg .b64 a, v, p;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 p, {%4, %4};\n\t"
+          "fma.rn.f32x2 a, v, p, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+          : "+f"(acc[i]), "+f"(acc[(i + 1) % W])
+          : "f"(f[i]), "f"(f[(i + 1) % W]), "f"(prob));
+  }
+}
+
+// Rows of up to 32 vectors: a group of G lanes per tile, one vector of VB bytes per lane, U edges in flight; see
+// spmm_walk. What a row needs besides its edges (its score, in the backward its features) is requested a row ahead.
+template <int VB, int G, int U, bool BWD, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB) gat_walk(const __grid_constant__ GatArgs a) {
+  constexpr int W = VB / 4;
+  constexpr int NG = 32 / G;
+  const int lane = threadIdx.x & 31;
+  const int lg = lane & (G - 1);
+  const int H = a.heads;
+  dependency_wait();
+  const int64_t e_total = edge_total(a.w);
+  const int64_t n_tiles = (e_total + a.w.tile - 1) / a.w.tile;
+  const int64_t wid = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
+  const int64_t n_warps = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
+  const int width = a.w.width;
+  const int64_t n_rows = a.w.n_dst;
+  // a lane behind the row reads column 0 again and is not stored
+  const bool on = lg * W < width;
+  const int col = on ? lg * W : 0;
+  const int head = col / a.c;
+  const bool lead = on && col == head * a.c;  // first lane of its head
+  const int lanes_per_head = BWD ? a.c / W : 0;
+  const float *x = static_cast<const float *>(a.w.x) + col;
+  const float *small_of = a.g_small + head * (BWD ? 4 : 1);
+  float *y = static_cast<float *>(a.w.y) + col;
+  auto empty_row = [&](int64_t r) {
+    float z[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) z[i] = 0.f;
+    if (on) store_floats<W>(y + r * width, z);
+    if (lead) {
       if (BWD) {
-        a.d_r_small[r * H + h] = 0.f;
+        a.d_r_small[r * H + head] = 0.f;
       } else {
-        a.row_max[r * H + h] = kNegBig;
-        a.row_sum[r * H + h] = 0.f;
+        a.row_max[r * H + head] = kNegBig;
+        a.row_sum[r * H + head] = 0.f;
       }
     }
   };
-
   if (e_total == 0) {
-    for (int64_t r = gwarp; r < a.n_rows; r += nwarps) empty_row(r);
+    for (int64_t r = wid * NG + lane / G; r < n_rows; r += n_warps * NG) empty_row(r);
     return;
   }
 
-  for (int64_t t = gwarp; t < n_tiles; t += nwarps) {
-    const int64_t tb = t * a.tile;
-    const int tile_len = static_cast<int>(min(static_cast<int64_t>(a.tile), e_total - tb));
-    const int n_stage = (tile_len + B - 1) / B;
-    int64_t row = a.tile_row[t];
-    if (t == 0)
-      for (int64_t r = 0; r < row; ++r) empty_row(r);
-    int64_t pbase = row;
-    auto load_ends = [&]() -> int {
-      const int64_t r = pbase + lane;
-      if (r >= a.n_rows) return kGFar;
-      const int64_t v = load_ptr(a.ptr, r + 1, a.ptr_bytes) - tb;
-      return v > kGFar ? kGFar : static_cast<int>(v);
-    };
-    int pc = load_ends();
-    int rrel = 0;
-    int rend = __shfl_sync(0xffffffffu, pc, 0);
-    const int64_t rs64 = load_ptr(a.ptr, row, a.ptr_bytes) - tb;
-    int rstart = rs64 < -kGFar ? -kGFar : static_cast<int>(rs64);
-    const IdxT *idx_t = idx + tb;
-
-    auto load_nid = [&](int k) -> uint32_t {
-      const int pos = k * B + lane;
-      return (lane < B && pos < tile_len) ? static_cast<uint32_t>(__ldg(idx_t + pos)) : 0u;
-    };
-    auto fill = [&](int k, uint32_t nid) {
-      const int cnt = min(B, tile_len - k * B);
+  int64_t next_row = 0, next_begin = 0, next_stop = 0;
+  auto fetch = [&](int64_t t) {
+    next_begin = next_stop = 0;
+    if (t < n_tiles) {
+      next_row = a.w.tiles[t].row;
+      next_begin = a.w.tiles[t].begin;
+      next_stop = a.w.tiles[t + 1].begin;
+    }
+  };
+  fetch(wid * NG + lane / G);
+  for (int64_t t0 = wid * NG; t0 < n_tiles; t0 += n_warps * NG) {
+    const int64_t t = t0 + lane / G;
+    TileWalk w{a};
+    w.begin = next_begin;
+    w.row = next_row;
+    w.len = next_stop > next_begin ? static_cast<int>(next_stop - next_begin) : 0;
+    fetch(t + n_warps * NG);
+    constexpr int IB = 32 / G;
+    uint32_t id_cur[IB], id_nxt[IB];
+    auto load_batch = [&](int first) {
 #pragma unroll
-      for (int c = 0; c < NCOPY; ++c) {
-        const uint32_t nj = __shfl_sync(0xffffffffu, nid, (c * RPI + jrow) & 31);
-        if (c * RPI + jrow < cnt) cp_async16(cdst + c * 512, xlane + static_cast<uint64_t>(nj) * RB);
+      for (int j = 0; j < IB; ++j) id_nxt[j] = w.load_id(first + j * G + lg);
+    };
+    w.rend = w.stop = kFar;
+    w.rstart = 0;
+    w.next_raw = 0;
+    if (w.len > 0) {
+      if (t == 0)
+        for (int64_t r = 0; r < w.row; ++r) empty_row(r);  // leading rows without edges
+      w.start();
+    }
+    float score, score_next;  // of the walked row and of the one after it
+    float xr[W], xr_next[W];
+    auto load_row = [&](int64_t r) {
+      const int64_t k = min(r, n_rows - 1);
+      score_next = __ldg(a.r_small + k * H + head);
+      if constexpr (BWD) load_floats<VB>(xr_next, a.r_feat + k * width + col);
+    };
+    auto take_row = [&]() {
+      score = score_next;
+      if constexpr (BWD) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) xr[i] = xr_next[i];
       }
-      // the small record of every edge of the stage
-      for (int q0 = 0; q0 < B * H; q0 += 32) {
-        const int q = q0 + lane;
-        const int e = q >> a.hshift;
-        const uint32_t nj = __shfl_sync(0xffffffffu, nid, e & 31);
-        if (e < cnt) {
-          if (BWD)
-            cp_async16(sv + q * 16, a.g_small + (static_cast<uint64_t>(nj) * H + (q & (H - 1))) * 4);
-          else
-            cp_async4(sv + q * 4, a.g_small + static_cast<uint64_t>(nj) * H + (q & (H - 1)));
+    };
+    load_row(w.row);
+    take_row();
+    load_row(w.row + 1);
+
+    float *yr = y + w.row * width;
+    // forward: acc = sum of exp(t - m) x, m = largest t so far, s = sum of exp(t - m); backward: acc = dx, s = d a_src
+    float acc[W], m, s;
+    auto reset = [&]() {
+      m = kNegBig;
+      s = 0.f;
+#pragma unroll
+      for (int i = 0; i < W; ++i) acc[i] = 0.f;
+    };
+    reset();
+    auto event = [&](int pos) {
+      const bool row_done = pos == w.rend;
+      if (row_done && w.rstart >= 0) {
+        if (!BWD) {
+          const float inv = 1.f / s;
+#pragma unroll
+          for (int i = 0; i < W; ++i) acc[i] *= inv;
         }
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-
-    // per-row state
-    float acc[EL];
-    float m = kNegBig, s = 0.f;  // forward: running max and sum; backward: s = d a_src accumulator
-    float rsm = 0.f;             // a_dst[row, h] (forward) / a_src[row, h] (backward)
-    float xr[EL];                // backward: x[row, h, this lane's columns]
-    auto begin_row = [&](int64_t r) {
-#pragma unroll
-      for (int i = 0; i < EL; ++i) acc[i] = 0.f;
-      m = kNegBig, s = 0.f;
-      if (r < a.n_rows) {
-        rsm = __ldg(a.r_small + r * H + h);
-        if (BWD) ldg_row<EL>(xr, a.r_feat + r * WIDTH + lane * EL);
-      }
-    };
-    begin_row(row);
-    uint32_t nid_cur = load_nid(0);
-    fill(0, nid_cur);
-    // ordered d a_dst: the forward position of every transposed edge, fetched like the ids
-    const IdxT *eid_t = reinterpret_cast<const IdxT *>(a.eid) + tb;
-    const bool ordered = BWD && a.d_edge != nullptr;
-    auto load_eid = [&](int k) -> uint32_t {
-      const int pos = k * B + lane;
-      return (ordered && lane < B && pos < tile_len) ? static_cast<uint32_t>(__ldg(eid_t + pos)) : 0u;
-    };
-    uint32_t eid_cur = load_eid(0);
-
-    for (int k = 0; k < n_stage; ++k) {
-      const uint32_t nid_next = load_nid(k + 1);
-      const uint32_t eid_next = load_eid(k + 1);
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncwarp();
-      const int sbase = k * B;
-      const int send = min(sbase + B, tile_len);
-      int pos = sbase;
-      uint32_t p = my;
-      uint32_t pv = sv + h * (BWD ? 16 : 4);
-      while (pos < send) {
-        const int stop = min(send, rend);
-        for (; pos < stop; ++pos) {
-          float f[EL];
-          lds_row<EL>(f, p);
-          if (!BWD) {
-            const float tt = leaky(lds_f32(pv) + rsm, slope);
-            const float mn = fmaxf(m, tt);
-            const float sc = __expf(m - mn), w = __expf(tt - mn);
-            s = fmaf(s, sc, w);
-            m = mn;
-            scale_fma<EL>(acc, f, sc, w);
+        if (on) store_floats<W>(yr, acc);
+        if (lead) {
+          if (BWD) {
+            a.d_r_small[w.row * H + head] = s;
           } else {
-            float st[4];
-            lds_row<4>(st, pv);  // {a_dst, row_max, 1 / row_sum, D} of the destination, this lane's head
-            const float t0 = st[0] + rsm;
-            const float w = __expf(leaky(t0, slope) - st[1]) * st[2];
-            float dp = 0.f;
-#pragma unroll
-            for (int i = 0; i < EL; ++i) dp = fmaf(f[i], xr[i], dp);
-            for (int o = lph >> 1; o > 0; o >>= 1) dp += __shfl_xor_sync(0xffffffffu, dp, o);
-            const float dt = w * (dp - st[3]) * (t0 > 0.f ? 1.f : slope);
-            s += dt;
-#pragma unroll
-            for (int i = 0; i < EL; ++i) acc[i] = fmaf(w, f[i], acc[i]);
-            if (ordered) {  // left at the edge's forward position; the destinations add theirs up afterwards
-              const uint32_t fe = __shfl_sync(0xffffffffu, eid_cur, pos - sbase);
-              if (head_lead) a.d_edge[static_cast<uint64_t>(fe) * H + h] = dt;
-            } else {
-              const uint32_t dst_node = __shfl_sync(0xffffffffu, nid_cur, pos - sbase);
-              if (head_lead) red_add_f32(a.d_g_small + static_cast<uint64_t>(dst_node) * H + h, dt);
-            }
+            a.row_max[w.row * H + head] = m;
+            a.row_sum[w.row * H + head] = s;
           }
-          p += RB;
-          pv += small_bytes;
         }
-        if (pos == rend) {
-          if (rstart < 0) {
-            stg_row<EL>(a.part_acc + (t * 2) * WIDTH + lane * EL, acc);
-            if (head_lead) {
-              a.part_ms[((t * 2) * H + h) * 2] = m;
-              a.part_ms[((t * 2) * H + h) * 2 + 1] = s;
-            }
-          } else {
-            if (!BWD) {
-              const float inv = 1.f / s;
-              float o[EL];
+      } else if (w.row < n_rows) {
+        const int64_t slot = t * 2 + (w.rstart < 0 ? 0 : 1);
+        if (on) {
+          float *p = a.w.partials + slot * width + col;
 #pragma unroll
-              for (int i = 0; i < EL; ++i) o[i] = acc[i] * inv;
-              stg_row<EL>(a.out + row * WIDTH + lane * EL, o);
-              if (head_lead) {
-                a.row_max[row * H + h] = m;
-                a.row_sum[row * H + h] = s;
-              }
-            } else {
-              stg_row<EL>(a.out + row * WIDTH + lane * EL, acc);
-              if (head_lead) a.d_r_small[row * H + h] = s;
-            }
-          }
-          rstart = rend;
-          for (;;) {
-            ++row;
-            if (++rrel == 32) {
-              pbase = row;
-              rrel = 0;
-              pc = load_ends();
-            }
-            rend = __shfl_sync(0xffffffffu, pc, rrel);
-            if (rend != rstart) break;
-            empty_row(row);
-          }
-          begin_row(row);
+          for (int i = 0; i < W; ++i) p[i] = acc[i];
+        }
+        if (lead) *reinterpret_cast<float2 *>(a.part_ms + (slot * H + head) * 2) = make_float2(m, s);
+      }
+      reset();
+      if (row_done) {
+        w.rstart = pos;
+        for (;;) {
+          w.next();
+          yr += width;
+          take_row();
+          load_row(w.row + 1);
+          if (w.rend != pos) break;
+          empty_row(w.row);
         }
       }
-      __syncwarp();
-      if (k + 1 < n_stage) fill(k + 1, nid_next);
-      nid_cur = nid_next;
-      eid_cur = eid_next;
-    }
-    int64_t tail = -1;
-    if (row < a.n_rows && rstart < tile_len && rend > tile_len) {
-      const int which = rstart < 0 ? 0 : 1;
-      stg_row<EL>(a.part_acc + (t * 2 + which) * WIDTH + lane * EL, acc);
-      if (head_lead) {
-        a.part_ms[((t * 2 + which) * H + h) * 2] = m;
-        a.part_ms[((t * 2 + which) * H + h) * 2 + 1] = s;
+      w.stop = pos == w.len ? kFar : min(w.rend, w.len);
+    };
+
+    const int longest = G == 32 ? w.len : __reduce_max_sync(0xffffffffu, w.len);
+    load_batch(0);
+    for (int p = 0; p < longest; p += U) {
+      const int in_batch = p & 31;
+      if (in_batch == 0) {
+#pragma unroll
+        for (int j = 0; j < IB; ++j) id_cur[j] = id_nxt[j];
+        load_batch(p + 32);
       }
-      if (which) tail = row;
-    }
-    if (lane == 0) a.tail_row[t] = tail;
-  }
-}
-
-// One partial of a chain: element 0 is the tail partial of tile t, element k > 0 the head partial of tile t + k.
-template <int EL, int WIDTH>
-__device__ __forceinline__ void load_partial(const GatArgs &a, int64_t t, int64_t k, int lane, int h, float *f, float &m,
-                                             float &s) {
-  const int64_t slot = k == 0 ? t * 2 + 1 : (t + k) * 2;
-  ldg_row<EL>(f, a.part_acc + slot * WIDTH + lane * EL);
-  m = a.part_ms[(slot * a.heads + h) * 2];
-  s = a.part_ms[(slot * a.heads + h) * 2 + 1];
-}
-
-// (acc, m, s) <- (acc, m, s) joined with (f, mu, su). Forward: online-softmax merge; backward: plain sums.
-template <int EL, bool BWD>
-__device__ __forceinline__ void join(float *acc, float &m, float &s, const float *f, float mu, float su) {
-  if (BWD) {
+      uint32_t id = id_cur[0];
 #pragma unroll
-    for (int i = 0; i < EL; ++i) acc[i] += f[i];
-    s += su;
-  } else {
-    const float mn = fmaxf(m, mu);
-    const float ca = __expf(m - mn), cb = __expf(mu - mn);
-    scale_fma<EL>(acc, f, ca, cb);
-    s = fmaf(s, ca, su * cb);
-    m = mn;
-  }
-}
-
-template <int EL, int WIDTH, bool BWD>
-__device__ __forceinline__ void finish_chain(const GatArgs &a, int64_t r, int lane, int h, bool head_lead, float *acc,
-                                             float m, float s) {
-  if (BWD) {
-    stg_row<EL>(a.out + r * WIDTH + lane * EL, acc);
-    if (head_lead) a.d_r_small[r * a.heads + h] = s;
-  } else {
-    const float inv = 1.f / s;
+      for (int j = 1; j < IB; ++j) id = in_batch >= j * G ? id_cur[j] : id;
+      const int lane0 = in_batch & (G - 1);
+      float v[U][W], small[U][BWD ? 4 : 1];
+      uint32_t from[U];
 #pragma unroll
-    for (int i = 0; i < EL; ++i) acc[i] *= inv;
-    stg_row<EL>(a.out + r * WIDTH + lane * EL, acc);
-    if (head_lead) {
-      a.row_max[r * a.heads + h] = m;
-      a.row_sum[r * a.heads + h] = s;
+      for (int u = 0; u < U; ++u) {
+        from[u] = __shfl_sync(0xffffffffu, id, lane0 + u, G);
+        load_floats<VB>(v[u], x + static_cast<uint64_t>(from[u]) * static_cast<uint32_t>(width));
+        const float *gs = small_of + static_cast<uint64_t>(from[u]) * static_cast<uint32_t>(H * (BWD ? 4 : 1));
+        if constexpr (BWD)
+          load_floats<16>(small[u], gs);
+        else
+          small[u][0] = __ldg(gs);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int pos = p + u;
+        const float z = score + small[u][0];
+        const float tl = z > 0.f ? z : z * a.slope;
+        if constexpr (BWD) {
+          const float prob = exp_flush(tl - small[u][1]) * small[u][2];
+          float dot = 0.f;
+#pragma unroll
+          for (int i = 0; i < W; ++i) dot = fmaf(v[u][i], xr[i], dot);
+          if (!on) dot = 0.f;
+          for (int o = lanes_per_head >> 1; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+          float dt = prob * (dot - small[u][3]);
+          dt = z > 0.f ? dt : dt * a.slope;
+          s += dt;
+          scale_add<W>(acc, v[u], prob);
+          if (lead && pos < w.len) w.edge_gradient(pos, from[u], head, dt);
+        } else {
+          const float mn = fmaxf(m, tl);
+          const float keep = exp_flush(m - mn), prob = exp_flush(tl - mn);
+          m = mn;
+          s = fmaf(s, keep, prob);
+          scale_add<W>(acc, keep, v[u], prob);
+        }
+        if (pos + 1 == w.stop) event(pos + 1);
+      }
     }
   }
 }
 
-// Joins the partials of rows that cross tile borders, in tile order: one warp per chain of up to kFixSeq
-// partials; longer chains are listed for gat_fix_long.
-template <int CB, bool BWD>
-__global__ void __launch_bounds__(256) gat_fix(GatArgs a) {
-  constexpr int EL = CB / 4;
-  constexpr int WIDTH = 32 * CB / 4;
+// Rows of 17 to 384 vectors: a whole warp per tile. Scores, maxima and exponentials are computed once per (edge, head), one
+// of them per lane, instead of by every lane that holds columns of the head: with 4 heads of 32 the walk above would spend
+// 53 warp instructions per edge on the forward and 99 on the backward. The U edges of a step are taken segment by segment:
+// the edges of one row.
+//
+// Forward. Lane l scores the edges (l >> log2 H) + j * (32 >> log2 H) of a step for head l & (H - 1); P = scores per lane.
+template <int VB, int NV, int U, int P, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB) gat_wide_forward(const __grid_constant__ GatArgs a) {
+  constexpr int W = VB / 4;
+  __shared__ float probs[kThreads / 32][P * 32];
   const int lane = threadIdx.x & 31;
-  const int lph = (a.c * 4) / CB;
-  const int h = lane / lph;
-  const bool head_lead = (lane % lph) == 0;
-  const int64_t e_total = edge_total(a);
-  const int64_t n_tiles = (e_total + a.tile - 1) / a.tile;
-  const int64_t gwarp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t t = gwarp; t < n_tiles; t += nwarps) {
-    const int64_t r = a.tail_row[t];
-    if (r < 0 || r >= a.n_rows) continue;
-    const int64_t re = min(load_ptr(a.ptr, r + 1, a.ptr_bytes), e_total);
-    const int64_t n_part = (re - 1) / a.tile - t + 1;
-    if (n_part > kFixSeq) {
-      if (lane == 0) {
-        const int slot = atomicAdd(a.hdr, 1);
-        if (slot < a.max_long) a.long_tiles[slot] = t;
+  const int H = a.heads, hs = __ffs(H) - 1;
+  const int my_head = lane & (H - 1);
+  float *prob = probs[threadIdx.x >> 5];
+  dependency_wait();
+  const int64_t e_total = edge_total(a.w);
+  const int64_t n_tiles = (e_total + a.w.tile - 1) / a.w.tile;
+  const int64_t wid = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
+  const int64_t n_warps = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
+  const int width = a.w.width;
+  const int64_t n_rows = a.w.n_dst;
+  int col[NV], head[NV];  // vectors behind the row read column 0 again and are not stored
+  bool on[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    const int c = (lane + q * 32) * W;
+    on[q] = c < width;
+    col[q] = on[q] ? c : 0;
+    head[q] = col[q] / a.c;
+  }
+  const float *prob_of[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) prob_of[q] = prob + head[q];
+  const float *x = static_cast<const float *>(a.w.x);
+  float *y = static_cast<float *>(a.w.y);
+  auto empty_row = [&](int64_t r) {
+    float z[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) z[i] = 0.f;
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+      if (on[q]) store_floats<W>(y + r * width + col[q], z);
+    if (lane < H) {
+      a.row_max[r * H + lane] = kNegBig;
+      a.row_sum[r * H + lane] = 0.f;
+    }
+  };
+  if (e_total == 0) {
+    for (int64_t r = wid; r < n_rows; r += n_warps) empty_row(r);
+    return;
+  }
+  for (int64_t t = wid; t < n_tiles; t += n_warps) {
+    TileWalk w{a};
+    w.begin = a.w.tiles[t].begin;
+    w.row = a.w.tiles[t].row;
+    const int64_t end = a.w.tiles[t + 1].begin;
+    if (end <= w.begin) continue;
+    w.len = static_cast<int>(end - w.begin);
+    if (t == 0)
+      for (int64_t r = 0; r < w.row; ++r) empty_row(r);  // leading rows without edges
+    uint32_t id_next = w.load_id(lane);
+    w.start();
+    auto row_score = [&](int64_t r) { return __ldg(a.r_small + min(r, n_rows - 1) * H + my_head); };
+    float score = row_score(w.row), score_next = row_score(w.row + 1);
+    // acc = sum of exp(t - m) x; m = largest t so far of the lane's scoring head, s = this lane's part of sum of exp(t - m)
+    float acc[NV][W], m = kNegBig, s = 0.f;
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+#pragma unroll
+      for (int i = 0; i < W; ++i) acc[q][i] = 0.f;
+    uint32_t id = 0u;
+    for (int p = 0; p < w.len; p += U) {
+      const int lane0 = p & 31;
+      if (lane0 == 0) {
+        id = id_next;
+        id_next = w.load_id(p + 32 + lane);
       }
-      continue;
+      float v[U][NV][W], small[P];
+#pragma unroll
+      for (int j = 0; j < P; ++j) {
+        const int e = (lane >> hs) + j * (32 >> hs);
+        const uint32_t nid = __shfl_sync(0xffffffffu, id, lane0 + (e & (U - 1)));
+        small[j] = __ldg(a.g_small + static_cast<uint64_t>(nid) * static_cast<uint32_t>(H) + my_head);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t nid = __shfl_sync(0xffffffffu, id, lane0 + u);
+        const float *xs = x + static_cast<uint64_t>(nid) * static_cast<uint32_t>(width);
+#pragma unroll
+        for (int q = 0; q < NV; ++q) load_floats<VB>(v[u][q], xs + col[q]);
+      }
+      int q0 = 0;
+#pragma unroll 1
+      do {
+        const int q1 = min(w.stop - p, U);
+        const unsigned edges = ((2u << (q1 - 1)) - 1u) & (~0u << q0);  // the segment's edges, a bit each
+        float tl[P], mx = kNegBig;
+        bool in[P];
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+          const int e = (lane >> hs) + j * (32 >> hs);
+          in[j] = (edges >> e) & 1u;
+          const float z = score + small[j];
+          tl[j] = z > 0.f ? z : z * a.slope;
+          if (in[j]) mx = fmaxf(mx, tl[j]);
+        }
+        for (int o = H; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (__any_sync(0xffffffffu, mx > m)) {  // seldom after a row's first edges
+          const float mn = fmaxf(m, mx);
+          const float keep = exp_flush(m - mn);
+          m = mn;
+          s *= keep;
+#pragma unroll
+          for (int q = 0; q < NV; ++q) {
+            const float k = __shfl_sync(0xffffffffu, keep, head[q]);
+#pragma unroll
+            for (int i = 0; i < W; ++i) acc[q][i] *= k;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+          const float pr = in[j] ? exp_flush(tl[j] - m) : 0.f;
+          s += pr;
+          prob[j * 32 + lane] = pr;
+        }
+        __syncwarp();
+        auto add = [&](int u) {
+#pragma unroll
+          for (int q = 0; q < NV; ++q) scale_add<W>(acc[q], v[u][q], prob_of[q][u << hs]);
+        };
+        if (edges == (1u << U) - 1u) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) add(u);
+        } else {
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if ((edges >> u) & 1u) add(u);
+        }
+        __syncwarp();
+        q0 = q1;
+        if (p + q1 != w.stop) break;
+        // the end of a row, of the tile, or of both
+        for (int o = H; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const bool row_done = p + q1 == w.rend;
+        if (row_done && w.rstart >= 0) {
+          const float inv = 1.f / s;
+#pragma unroll
+          for (int q = 0; q < NV; ++q) {
+            const float k = __shfl_sync(0xffffffffu, inv, head[q]);
+#pragma unroll
+            for (int i = 0; i < W; ++i) acc[q][i] *= k;
+            if (on[q]) store_floats<W>(y + w.row * width + col[q], acc[q]);
+          }
+          if (lane < H) {
+            a.row_max[w.row * H + lane] = m;
+            a.row_sum[w.row * H + lane] = s;
+          }
+        } else if (w.row < n_rows) {
+          const int64_t slot = t * 2 + (w.rstart < 0 ? 0 : 1);
+#pragma unroll
+          for (int q = 0; q < NV; ++q)
+            if (on[q]) {
+              float *pp = a.w.partials + slot * width + col[q];
+#pragma unroll
+              for (int i = 0; i < W; ++i) pp[i] = acc[q][i];
+            }
+          if (lane < H) *reinterpret_cast<float2 *>(a.part_ms + (slot * H + lane) * 2) = make_float2(m, s);
+        }
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+#pragma unroll
+          for (int i = 0; i < W; ++i) acc[q][i] = 0.f;
+        m = kNegBig;
+        s = 0.f;
+        if (row_done) {
+          w.rstart = w.rend;
+          for (;;) {
+            w.next();
+            score = score_next;
+            score_next = row_score(w.row + 1);
+            if (w.rend != w.rstart) break;
+            empty_row(w.row);
+          }
+        }
+        w.stop = p + q1 == w.len ? kFar : min(w.rend, w.len);
+      } while (q0 < U);
     }
-    float acc[EL], m, s;
-    load_partial<EL, WIDTH>(a, t, 0, lane, h, acc, m, s);
-    for (int64_t k = 1; k < n_part; ++k) {
-      float f[EL], mu, su;
-      load_partial<EL, WIDTH>(a, t, k, lane, h, f, mu, su);
-      join<EL, BWD>(acc, m, s, f, mu, su);
-    }
-    finish_chain<EL, WIDTH, BWD>(a, r, lane, h, head_lead, acc, m, s);
   }
 }
 
-// Long chains: the n partials are dealt to the 8 warps of a CTA in contiguous blocks [n w / 8, n (w + 1) / 8); each
-// warp joins its block in order, then warp 0 joins the 8 block results in block order.
-template <int CB, bool BWD>
-__global__ void __launch_bounds__(256) gat_fix_long(GatArgs a) {
-  constexpr int EL = CB / 4;
-  constexpr int WIDTH = 32 * CB / 4;
-  __shared__ float sh_acc[8][WIDTH];
-  __shared__ float sh_ms[8][32][2];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int lph = (a.c * 4) / CB;
-  const int h = lane / lph;
-  const bool head_lead = (lane % lph) == 0;
-  const int64_t e_total = edge_total(a);
-  const int n_long = min(a.hdr[0], a.max_long);
-  for (int i = blockIdx.x; i < n_long; i += gridDim.x) {
-    const int64_t t = a.long_tiles[i];
-    const int64_t r = a.tail_row[t];
-    if (r < 0 || r >= a.n_rows) continue;  // uniform over the CTA
-    const int64_t re = min(load_ptr(a.ptr, r + 1, a.ptr_bytes), e_total);
-    const int64_t n_part = (re - 1) / a.tile - t + 1;
-    const int64_t kb = n_part * warp / 8, ke = n_part * (warp + 1) / 8;  // n_part > 32: no block is empty
-    float acc[EL], m, s;
-    load_partial<EL, WIDTH>(a, t, kb, lane, h, acc, m, s);
-#pragma unroll 4
-    for (int64_t k = kb + 1; k < ke; ++k) {
-      float f[EL], mu, su;
-      load_partial<EL, WIDTH>(a, t, k, lane, h, f, mu, su);
-      join<EL, BWD>(acc, m, s, f, mu, su);
-    }
+// Backward. The dot products of U edges are reduced over a head's lanes and spread over them at the same time (at every
+// step a lane keeps half of the edges and hands the other half to its partner): 7 exchanges for 8 edges where a reduction
+// per edge takes 24. R = min(lanes per head, U); afterwards a lane holds E = U / R edges of its head, from first_edge on.
+template <int U, int R>
+__device__ __forceinline__ int first_edge(int lane) {
+  int e = 0;
 #pragma unroll
-    for (int j = 0; j < EL; ++j) sh_acc[warp][lane * EL + j] = acc[j];
-    sh_ms[warp][lane][0] = m;
-    sh_ms[warp][lane][1] = s;
-    __syncthreads();
-    if (warp == 0) {
-      for (int w = 1; w < 8; ++w) {
-        float f[EL];
+  for (int o = 1, n = U / 2; o < R; o <<= 1, n >>= 1) e += (lane & o) ? n : 0;
+  return e;
+}
+template <int U, int R>
+__device__ __forceinline__ constexpr int lane_of_edge(int u) {
+  int l = 0;
+  for (int o = 1, n = U / 2; o < R; o <<= 1, n >>= 1) l += (u & n) ? o : 0;
+  return l;
+}
+
+template <int NV, int U, int R, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB) gat_wide_backward(const __grid_constant__ GatArgs a) {
+  constexpr int W = 4;
+  constexpr int E = U / R;
+  const int lane = threadIdx.x & 31;
+  const int H = a.heads;
+  const int lph = a.c / W;  // lanes per head, a power of two >= R
+  const int group = lane & ~(lph - 1) & 31;
+  const bool own = (lane & (lph - 1)) < R;  // the head's other lanes hold copies
+  const bool lead = (lane & (lph - 1)) == 0;
+  const int e0 = first_edge<U, R>(lane);
+  dependency_wait();
+  const int64_t e_total = edge_total(a.w);
+  const int64_t n_tiles = (e_total + a.w.tile - 1) / a.w.tile;
+  const int64_t wid = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
+  const int64_t n_warps = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
+  const int width = a.w.width;
+  const int64_t n_rows = a.w.n_dst;
+  int col[NV], head[NV];
+  bool on[NV];
 #pragma unroll
-        for (int j = 0; j < EL; ++j) f[j] = sh_acc[w][lane * EL + j];
-        join<EL, BWD>(acc, m, s, f, sh_ms[w][lane][0], sh_ms[w][lane][1]);
+  for (int q = 0; q < NV; ++q) {
+    const int c = (lane + q * 32) * W;
+    on[q] = c < width;
+    col[q] = on[q] ? c : 0;
+    head[q] = col[q] / a.c;
+  }
+  const float *dy = static_cast<const float *>(a.w.x);
+  float *dx = static_cast<float *>(a.w.y);
+  auto empty_row = [&](int64_t r) {
+    const float z[W] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+      if (on[q]) {
+        store_floats<W>(dx + r * width + col[q], z);
+        if (lead) a.d_r_small[r * H + head[q]] = 0.f;
       }
-      finish_chain<EL, WIDTH, BWD>(a, r, lane, h, head_lead, acc, m, s);
+  };
+  if (e_total == 0) {
+    for (int64_t r = wid; r < n_rows; r += n_warps) empty_row(r);
+    return;
+  }
+  for (int64_t t = wid; t < n_tiles; t += n_warps) {
+    TileWalk w{a};
+    w.begin = a.w.tiles[t].begin;
+    w.row = a.w.tiles[t].row;
+    const int64_t end = a.w.tiles[t + 1].begin;
+    if (end <= w.begin) continue;
+    w.len = static_cast<int>(end - w.begin);
+    if (t == 0)
+      for (int64_t r = 0; r < w.row; ++r) empty_row(r);
+    uint32_t id_next = w.load_id(lane);
+    w.start();
+    float score[NV], score_next[NV], xr[NV][W], xr_next[NV][W];
+    auto load_row = [&](int64_t r) {
+      const int64_t k = min(r, n_rows - 1);
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        score_next[q] = __ldg(a.r_small + k * H + head[q]);
+        load_floats<16>(xr_next[q], a.r_feat + k * width + col[q]);
+        if (!on[q])
+#pragma unroll
+          for (int i = 0; i < W; ++i) xr_next[q][i] = 0.f;
+      }
+    };
+    auto take_row = [&]() {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        score[q] = score_next[q];
+#pragma unroll
+        for (int i = 0; i < W; ++i) xr[q][i] = xr_next[q][i];
+      }
+    };
+    load_row(w.row);
+    take_row();
+    load_row(w.row + 1);
+    float acc[NV][W], s[NV];  // dx and this lane's part of d a_src of the walked row
+    auto reset = [&]() {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        s[q] = 0.f;
+#pragma unroll
+        for (int i = 0; i < W; ++i) acc[q][i] = 0.f;
+      }
+    };
+    reset();
+    uint32_t id = 0u;
+    for (int p = 0; p < w.len; p += U) {
+      const int lane0 = p & 31;
+      if (lane0 == 0) {
+        id = id_next;
+        id_next = w.load_id(p + 32 + lane);
+      }
+      float v[U][NV][W];
+      float4 stat[E][NV];
+      uint32_t mine[E];
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        mine[i] = __shfl_sync(0xffffffffu, id, lane0 + e0 + i);
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+          stat[i][q] = __ldg(reinterpret_cast<const float4 *>(a.g_small) + static_cast<uint64_t>(mine[i]) * static_cast<uint32_t>(H) + head[q]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t nid = __shfl_sync(0xffffffffu, id, lane0 + u);
+        const float *src = dy + static_cast<uint64_t>(nid) * static_cast<uint32_t>(width);
+#pragma unroll
+        for (int q = 0; q < NV; ++q) load_floats<16>(v[u][q], src + col[q]);
+      }
+      int q0 = 0;
+#pragma unroll 1
+      do {
+        const int q1 = min(w.stop - p, U);
+        const unsigned edges = ((2u << (q1 - 1)) - 1u) & (~0u << q0);  // the segment's edges, a bit each
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          float d[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            d[u] = v[u][q][0] * xr[q][0];
+#pragma unroll
+            for (int i = 1; i < W; ++i) d[u] = fmaf(v[u][q][i], xr[q][i], d[u]);
+          }
+#pragma unroll
+          for (int o = 1, n = U / 2; o < R; o <<= 1, n >>= 1) {
+            const bool upper = lane & o;
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+              const float other = __shfl_xor_sync(0xffffffffu, upper ? d[i] : d[i + n], o);
+              d[i] = (upper ? d[i + n] : d[i]) + other;
+            }
+          }
+          for (int o = R; o < lph; o <<= 1) {
+#pragma unroll
+            for (int i = 0; i < E; ++i) d[i] += __shfl_xor_sync(0xffffffffu, d[i], o);
+          }
+          float prob[E];
+#pragma unroll
+          for (int i = 0; i < E; ++i) {
+            const float4 r = stat[i][q];
+            const float z = score[q] + r.x;
+            const float tl = z > 0.f ? z : z * a.slope;
+            prob[i] = exp_flush(tl - r.y) * r.z;
+            float dt = prob[i] * (d[i] - r.w);
+            dt = z > 0.f ? dt : dt * a.slope;
+            const int e = e0 + i;
+            if (own && on[q] && ((edges >> e) & 1u) && p + e < w.len) {
+              s[q] += dt;
+              w.edge_gradient(p + e, mine[i], head[q], dt);
+            }
+          }
+          auto add = [&](int u) {
+            scale_add<W>(acc[q], v[u][q], __shfl_sync(0xffffffffu, prob[u % E], group | lane_of_edge<U, R>(u)));
+          };
+          if (edges == (1u << U) - 1u) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) add(u);
+          } else {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if ((edges >> u) & 1u) add(u);
+          }
+        }
+        q0 = q1;
+        if (p + q1 != w.stop) break;
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+#pragma unroll
+          for (int o = 1; o < R; o <<= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+        const bool row_done = p + q1 == w.rend;
+        if (row_done && w.rstart >= 0) {
+#pragma unroll
+          for (int q = 0; q < NV; ++q)
+            if (on[q]) {
+              store_floats<W>(dx + w.row * width + col[q], acc[q]);
+              if (lead) a.d_r_small[w.row * H + head[q]] = s[q];
+            }
+        } else if (w.row < n_rows) {
+          const int64_t slot = t * 2 + (w.rstart < 0 ? 0 : 1);
+#pragma unroll
+          for (int q = 0; q < NV; ++q)
+            if (on[q]) {
+              *reinterpret_cast<float4 *>(a.w.partials + slot * width + col[q]) = make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
+              if (lead) *reinterpret_cast<float2 *>(a.part_ms + (slot * H + head[q]) * 2) = make_float2(0.f, s[q]);
+            }
+        }
+        reset();
+        if (row_done) {
+          w.rstart = w.rend;
+          for (;;) {
+            w.next();
+            take_row();
+            load_row(w.row + 1);
+            if (w.rend != w.rstart) break;
+            empty_row(w.row);
+          }
+        }
+        w.stop = p + q1 == w.len ? kFar : min(w.rend, w.len);
+      } while (q0 < U);
     }
-    __syncthreads();
+  }
+}
+
+constexpr int kGatSeq = 16;  // a chain of more partials is joined in blocks of this many, then the blocks: the hub row of
+                             // 2.3 M edges (420 partials) costs 2 + 4 round trips instead of 8 + 1 with blocks of 64
+
+// Joins n elements of a chain of partials, step apart, from element k0 on, VW columns per lane, in SV pieces that lie in
+// one head each. FROM_BLOCKS: the (m, s) of the elements are those of finished blocks. Result to the row, or to the
+// block's element.
+template <int VW, int SV, bool BWD, bool FROM_BLOCKS>
+__device__ void gat_chain(const GatArgs &a, int64_t ts, int64_t k0, int64_t n, int64_t step, bool to_block, int64_t row, int lane) {
+  const int width = a.w.width, H = a.heads;
+  constexpr int PV = VW / SV;   // columns per piece
+  constexpr int kDepth = 8 / SV;  // partials requested at once
+  for (int c = lane * VW; c < width; c += 32 * VW) {
+    int h[SV];
+#pragma unroll
+    for (int j = 0; j < SV; ++j) h[j] = (c + j * PV) / a.c;
+    float acc[VW], m[SV], s[SV];
+    auto at = [&](int64_t k, float (&v)[VW], float2 (&ms)[SV]) {
+      const int64_t e = k0 + k * step, slot = (ts + e) * 2 + (e == 0 ? 1 : 0);
+      const float *p = a.w.partials + slot * width + c;
+      if constexpr (VW == 4) {
+        const float4 t = __ldcg(reinterpret_cast<const float4 *>(p));
+        v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+      } else {
+        v[0] = __ldcg(p);
+      }
+#pragma unroll
+      for (int j = 0; j < SV; ++j)
+        ms[j] = __ldcg(reinterpret_cast<const float2 *>(FROM_BLOCKS ? a.block_ms + ((ts + e) * H + h[j]) * 2
+                                                                    : a.part_ms + (slot * H + h[j]) * 2));
+    };
+    auto join = [&](const float (&v)[VW], const float2 (&ms)[SV]) {
+#pragma unroll
+      for (int j = 0; j < SV; ++j) {
+        float mine = 1.f, theirs = 1.f;
+        if (!BWD) {
+          const float mn = fmaxf(m[j], ms[j].x);
+          mine = exp_flush(m[j] - mn), theirs = exp_flush(ms[j].x - mn);
+          m[j] = mn;
+        }
+        s[j] = s[j] * mine + ms[j].y * theirs;
+#pragma unroll
+        for (int i = j * PV; i < (j + 1) * PV; ++i) acc[i] = acc[i] * mine + v[i] * theirs;
+      }
+    };
+    {
+      float2 ms[SV];
+      at(0, acc, ms);
+#pragma unroll
+      for (int j = 0; j < SV; ++j) m[j] = ms[j].x, s[j] = ms[j].y;
+    }
+    int64_t k = 1;
+    for (; k + kDepth <= n; k += kDepth) {
+      float v[kDepth][VW];
+      float2 ms[kDepth][SV];
+#pragma unroll
+      for (int u = 0; u < kDepth; ++u) at(k + u, v[u], ms[u]);
+#pragma unroll
+      for (int u = 0; u < kDepth; ++u) join(v[u], ms[u]);
+    }
+    for (; k < n; ++k) {
+      float v[VW];
+      float2 ms[SV];
+      at(k, v, ms);
+      join(v, ms);
+    }
+    float *out = to_block ? a.w.partials + ((ts + k0) * 2 + (k0 == 0 ? 1 : 0)) * width + c
+                          : static_cast<float *>(a.w.y) + row * width + c;
+#pragma unroll
+    for (int j = 0; j < SV; ++j) {
+      const float inv = BWD || to_block ? 1.f : 1.f / s[j];
+#pragma unroll
+      for (int i = j * PV; i < (j + 1) * PV; ++i) out[i] = acc[i] * inv;
+      if (c + j * PV != h[j] * a.c) continue;  // the first column of the head writes its (m, s)
+      if (to_block) {
+        *reinterpret_cast<float2 *>(a.block_ms + ((ts + k0) * H + h[j]) * 2) = make_float2(m[j], s[j]);
+      } else if (BWD) {
+        a.d_r_small[row * H + h[j]] = s[j];
+      } else {
+        a.row_max[row * H + h[j]] = m[j];
+        a.row_sum[row * H + h[j]] = s[j];
+      }
+    }
+  }
+}
+
+// Rows that tiles cut: one warp per tile, the roles of walk_fix (spmm_walk.cu).
+template <int VW, int SV, bool BWD>
+__global__ void __launch_bounds__(256, 3) gat_fix(const __grid_constant__ GatArgs a) {
+  dependency_wait();
+  const int lane = threadIdx.x & 31;
+  const WalkArgs &w = a.w;
+  const int64_t e_total = edge_total(w);
+  const int64_t n_warps = static_cast<int64_t>(gridDim.x) * 8;
+  for (int64_t t = blockIdx.x * 8ll + (threadIdx.x >> 5); t < w.max_tiles; t += n_warps) {
+    const WalkTile here = w.tiles[t], next = w.tiles[t + 1];  // not written behind the last tile, whose end is e_total
+    if (t * w.tile >= e_total || next.begin <= here.begin) continue;
+    const bool follows = next.row < w.n_dst;
+    const int64_t head_begin = load_ptr(w.ptr, here.row, w.ptr_bytes), head_end = load_ptr(w.ptr, here.row + 1, w.ptr_bytes);
+    const int64_t tail_begin = follows ? load_ptr(w.ptr, next.row, w.ptr_bytes) : next.begin;
+    const int64_t tail_end = follows ? load_ptr(w.ptr, next.row + 1, w.ptr_bytes) : next.begin;
+    for (int role = 0; role < 2; ++role) {
+      const int64_t row = role == 0 ? next.row : here.row;
+      const int64_t rb = role == 0 ? tail_begin : head_begin;
+      if (role == 0 ? (rb >= next.begin || rb < here.begin) : rb >= here.begin) continue;
+      const int64_t ts = role == 0 ? t : rb / w.tile;
+      const int64_t k = t - ts;
+      if (k % kGatSeq != 0) continue;
+      const int64_t re = min(role == 0 ? tail_end : head_end, e_total);
+      const int64_t m = (re - 1) / w.tile - ts + 1;
+      const int64_t n_blocks = (m + kGatSeq - 1) / kGatSeq;
+      gat_chain<VW, SV, BWD, false>(a, ts, k, min(static_cast<int64_t>(kGatSeq), m - k), 1, n_blocks > 1, row, lane);
+      if (n_blocks == 1) continue;
+      __threadfence();
+      __syncwarp();
+      int old = 0;
+      if (lane == 0) old = atomicAdd(w.count + ts, 1);
+      old = __shfl_sync(0xffffffffu, old, 0);
+      if (old + 1 != n_blocks) continue;
+      __threadfence();
+      gat_chain<VW, SV, BWD, true>(a, ts, 0, n_blocks, kGatSeq, false, row, lane);
+    }
   }
 }
 
 // Backward set-up, one warp per destination: stats[r, h] = {a_dst, row_max, 1 / row_sum, <dy[r,h,:], y[r,h,:]>}
-// and d a_dst[r, h] = 0 (the walk adds into it).
-template <int CB>
+// and d a_dst[r, h] = 0 (the walk adds into it). A head's columns lie with c / W neighbouring lanes.
+template <int W>
 __global__ void __launch_bounds__(256) gat_bwd_prepare(const float *dy, const float *y, const float *a_dst,
                                                        const float *row_max, const float *row_sum, float *stats,
                                                        float *d_a_dst, int64_t n_dst, int heads, int c) {
-  constexpr int EL = CB / 4;
-  constexpr int WIDTH = 32 * CB / 4;
   const int lane = threadIdx.x & 31;
-  const int lph = (c * 4) / CB;
-  const int h = lane / lph;
+  const int lph = c / W, width = heads * c;
   const int64_t gwarp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   for (int64_t r = gwarp; r < n_dst; r += nwarps) {
-    float g[EL], v[EL];
-    ldg_row<EL>(g, dy + r * WIDTH + lane * EL);
-    ldg_row<EL>(v, y + r * WIDTH + lane * EL);
-    float d = 0.f;
+    for (int c0 = 0; c0 < width; c0 += 32 * W) {
+      const int col = c0 + lane * W;
+      const bool on = col < width;
+      const int h = on ? col / c : 0;
+      float d = 0.f;
+      if (on) {
+        float g[W], v[W];
+        load_floats<W * 4>(g, dy + r * width + col);
+        load_floats<W * 4>(v, y + r * width + col);
 #pragma unroll
-    for (int i = 0; i < EL; ++i) d = fmaf(g[i], v[i], d);
-    for (int o = lph >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-    if ((lane % lph) == 0) {
-      const float sum = row_sum[r * heads + h];
-      *reinterpret_cast<float4 *>(stats + (r * heads + h) * 4) =
-          make_float4(a_dst[r * heads + h], row_max[r * heads + h], sum > 0.f ? 1.f / sum : 0.f, d);
-      d_a_dst[r * heads + h] = 0.f;
+        for (int i = 0; i < W; ++i) d = fmaf(g[i], v[i], d);
+      }
+      for (int o = lph >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+      if (on && col == h * c) {
+        const float sum = row_sum[r * heads + h];
+        *reinterpret_cast<float4 *>(stats + (r * heads + h) * 4) =
+            make_float4(a_dst[r * heads + h], row_max[r * heads + h], sum > 0.f ? 1.f / sum : 0.f, d);
+        d_a_dst[r * heads + h] = 0.f;
+      }
     }
   }
 }
@@ -690,35 +1069,18 @@ __global__ void __launch_bounds__(256) gat_dst_sum_long(const void *ptr, int ptr
 }
 
 struct GatLayout {
-  size_t hdr, tile_row, tail_row, long_tiles, part_acc, part_ms, stats, long_rows, piece_sums, d_edge, total;
-  int64_t max_tiles;
-  int max_long;
+  WalkLayout walk;
+  size_t part_ms, block_ms, stats, long_rows, piece_sums, d_edge, total;
 };
 
-int gat_tile_edges(int64_t nnz) {
-  int64_t t = nnz / (static_cast<int64_t>(kNumSM) * kGCtasPerSM * kGWarps * 4);
-  if (t > 512) t = 512;
-  if (t < 64) t = 64;
-  return static_cast<int>(t / 32 * 32);
-}
-
-void gat_layout(int64_t n_stats_rows, int64_t nnz, int heads, int c, GatLayout *L) {
-  const int64_t width = static_cast<int64_t>(heads) * c;
-  L->max_tiles = (nnz + 63) / 64 + 1;  // 64 = smallest tile
-  size_t off = 0;
-  L->hdr = off;
-  off = align_up(off + 256, 256);
-  L->tile_row = off;
-  off = align_up(off + L->max_tiles * sizeof(int64_t), 256);
-  L->tail_row = off;
-  off = align_up(off + L->max_tiles * sizeof(int64_t), 256);
-  L->max_long = static_cast<int>(L->max_tiles / kFixSeq + 1);
-  L->long_tiles = off;
-  off = align_up(off + static_cast<size_t>(L->max_long) * sizeof(int64_t), 256);
-  L->part_acc = off;
-  off = align_up(off + static_cast<size_t>(L->max_tiles) * 2 * width * sizeof(float), 256);
+int gat_layout(int64_t n_stats_rows, int64_t nnz, int heads, int c, GatLayout *L) {
+  const int rc = walk_layout(nnz, static_cast<int64_t>(heads) * c, 64, &L->walk);  // 64 = smallest tile
+  if (rc != CXG_OK) return rc;
+  size_t off = L->walk.total;
   L->part_ms = off;
-  off = align_up(off + static_cast<size_t>(L->max_tiles) * 2 * heads * 2 * sizeof(float), 256);
+  off = align_up(off + static_cast<size_t>(L->walk.max_tiles) * 2 * heads * 2 * sizeof(float), 256);
+  L->block_ms = off;
+  off = align_up(off + static_cast<size_t>(L->walk.max_tiles) * heads * 2 * sizeof(float), 256);
   L->stats = off;
   off = align_up(off + static_cast<size_t>(n_stats_rows) * heads * 4 * sizeof(float), 256);
   // ordered d a_dst of the backward: destinations of more than kLongRowEdges edges, and one value per edge and head
@@ -729,63 +1091,115 @@ void gat_layout(int64_t n_stats_rows, int64_t nnz, int heads, int c, GatLayout *
   L->d_edge = off;
   off = align_up(off + static_cast<size_t>(nnz) * heads * sizeof(float), 256);
   L->total = off;
+  return CXG_OK;
 }
 
-int check_shape(const char *who, int heads, int c) {
-  const int row_bytes = heads * c * 4;
+// Widest vector that stays inside a head, narrowed so that eight lanes, the fewest a tile is given, have one each.
+int vector_of(int heads, int c) {
+  int vb = 16;
+  while ((c * 4) % vb != 0) vb /= 2;
+  while (vb > 4 && heads * c * 4 <= 4 * vb) vb /= 2;
+  return vb;
+}
+
+int check_shape(const char *who, int heads, int c, bool backward) {
   if (heads < 1 || heads > 16 || (heads & (heads - 1)) != 0 || c < 1)
     return set_error(CXG_EUNSUPPORTED, "%s: heads = %d must be a power of two <= 16", who, heads);
-  if (row_bytes != 128 && row_bytes != 256 && row_bytes != 512)
-    return set_error(CXG_EUNSUPPORTED, "%s: a feature row of heads * c * 4 = %d bytes; 128, 256 or 512 are covered", who,
-                     row_bytes);
-  const int cb = row_bytes / 32;
-  if ((c * 4) % cb != 0)
-    return set_error(CXG_EUNSUPPORTED, "%s: c = %d leaves a lane's %d bytes across two heads", who, c, cb);
+  const int vb = vector_of(heads, c), n = heads * c * 4 / vb;
+  if (n > (vb == 4 ? 384 : 128))
+    return set_error(CXG_EUNSUPPORTED, "%s: a feature row of heads * c = %d values is too wide", who, heads * c);
+  if (backward && ((c & (c - 1)) != 0 || c * 4 / vb > 32))
+    return set_error(CXG_EUNSUPPORTED, "%s: c = %d must be a power of two of at most 128 in the backward", who, c);
   return CXG_OK;
 }
 
 void fill_args(GatArgs &a, const GatLayout &L, void *workspace, int64_t nnz, int heads, int c, float slope) {
-  char *ws = reinterpret_cast<char *>(workspace);
-  a.hdr = reinterpret_cast<int32_t *>(ws + L.hdr);
-  a.tile_row = reinterpret_cast<int64_t *>(ws + L.tile_row);
-  a.tail_row = reinterpret_cast<int64_t *>(ws + L.tail_row);
-  a.long_tiles = reinterpret_cast<int64_t *>(ws + L.long_tiles);
-  a.max_long = L.max_long;
-  a.part_acc = reinterpret_cast<float *>(ws + L.part_acc);
+  char *ws = static_cast<char *>(workspace);
+  WalkArgs &w = a.w;
+  w.hdr = reinterpret_cast<int32_t *>(ws + L.walk.hdr);
+  w.tiles = reinterpret_cast<WalkTile *>(ws + L.walk.tiles);
+  w.count = reinterpret_cast<int32_t *>(ws + L.walk.count);
+  w.partials = reinterpret_cast<float *>(ws + L.walk.partials);
+  w.nnz = nnz;
+  w.width = heads * c, w.row_bytes = heads * c * 4, w.heads = heads, w.feat = c;
+  w.whole_rows = 0;
   a.part_ms = reinterpret_cast<float *>(ws + L.part_ms);
-  a.max_tiles = L.max_tiles;
-  a.nnz = nnz;
+  a.block_ms = reinterpret_cast<float *>(ws + L.block_ms);
   a.heads = heads;
   a.c = c;
-  a.hshift = 0;
-  while ((1 << a.hshift) < heads) ++a.hshift;
   a.slope = slope;
-  a.tile = gat_tile_edges(nnz);
 }
 
-template <int CB, bool BWD>
-cudaError_t launch_walk(const GatArgs &a, cudaStream_t st) {
-  constexpr int RB = 32 * CB;
-  constexpr int B = kGStageBytes / RB > 32 ? 32 : kGStageBytes / RB;
-  const size_t smem = static_cast<size_t>(kGWarps) * (B * RB + B * a.heads * (BWD ? 16 : 4));
-  const unsigned pb = static_cast<unsigned>((a.max_tiles + 255) / 256);
-  gat_plan<<<pb, 256, 0, st>>>(a);
-  cudaError_t e;
-  if (a.idx_bytes == 8) {
-    auto k = gat_walk<CB, int64_t, BWD>;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    k<<<kNumSM * kGCtasPerSM, kGThreads, smem, st>>>(a);
+// Lane layouts by bytes per vector and vectors per row; the last number is the resident CTAs per SM that the registers of
+// that many edges in flight allow.
+template <bool BWD>
+cudaError_t launch_walk(GatArgs &a, cudaStream_t st) {
+  const int vb = vector_of(a.heads, a.c), n = a.w.row_bytes / vb;
+  cudaError_t err = cudaErrorInvalidValue;
+  auto go = [&](auto kernel, int g, int ctas) {
+    const int per_cta = kThreads / g;
+    const int64_t resident = static_cast<int64_t>(kNumSM) * ctas;
+    a.w.tile = walk_whole_waves(a.w.nnz, resident * per_cta);
+    a.w.max_tiles = (a.w.nnz + a.w.tile - 1) / a.w.tile + 1;
+    walk_plan_run(a.w, st);
+    int64_t grid = (a.w.max_tiles + per_cta - 1) / per_cta;
+    if (grid > resident) grid = resident;
+    err = launch_dependent(kernel, static_cast<unsigned>(grid), kThreads, 0, st, a);
+  };
+#define CXG_GAT(VB, G, U, CTAS) \
+  if (vb == VB && n <= G) go(gat_walk<VB, G, U, BWD, CTAS>, G, CTAS); else
+#define CXG_GAT_FWD(VB, NV, U, P, CTAS) \
+  if (vb == VB && n <= 32 * NV && U * a.heads <= 32 * P) go(gat_wide_forward<VB, NV, U, P, CTAS>, 32, CTAS); else
+#define CXG_GAT_BWD(NV, U, R, CTAS) \
+  if (vb == 16 && n <= 32 * NV && a.c / 4 >= R) go(gat_wide_backward<NV, U, R, CTAS>, 32, CTAS); else
+  if constexpr (BWD) {
+    CXG_GAT(16, 8, 4, 6)
+    CXG_GAT(16, 16, 4, 6)
+    CXG_GAT(8, 8, 4, 6)
+    CXG_GAT(8, 16, 4, 6)
+    CXG_GAT(4, 8, 4, 6)
+    CXG_GAT(4, 16, 4, 6)
+    CXG_GAT_BWD(1, 4, 4, 8)
+    CXG_GAT_BWD(1, 4, 2, 7)
+    CXG_GAT_BWD(2, 4, 4, 4)
+    CXG_GAT_BWD(4, 2, 2, 3)
+    return cudaErrorInvalidValue;
   } else {
-    auto k = gat_walk<CB, int32_t, BWD>;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    k<<<kNumSM * kGCtasPerSM, kGThreads, smem, st>>>(a);
+    CXG_GAT(16, 8, 8, 6)
+    CXG_GAT(16, 16, 8, 6)
+    CXG_GAT(8, 8, 8, 6)
+    CXG_GAT(8, 16, 8, 6)
+    CXG_GAT(4, 8, 8, 6)
+    CXG_GAT(4, 16, 8, 6)
+    CXG_GAT(16, 32, 8, 6)
+    CXG_GAT_FWD(16, 2, 4, 2, 6)
+    CXG_GAT_FWD(16, 4, 2, 1, 5)
+    CXG_GAT(8, 32, 8, 6)
+    CXG_GAT_FWD(8, 2, 8, 4, 5)
+    CXG_GAT_FWD(8, 4, 4, 2, 5)
+    CXG_GAT(4, 32, 8, 6)
+    CXG_GAT_FWD(4, 2, 8, 4, 6)
+    CXG_GAT_FWD(4, 4, 8, 4, 5)
+    CXG_GAT_FWD(4, 6, 4, 1, 5)
+    CXG_GAT_FWD(4, 6, 4, 2, 5)
+    CXG_GAT_FWD(4, 12, 2, 1, 5)
+    return cudaErrorInvalidValue;
   }
-  gat_fix<CB, BWD><<<kNumSM * 4, 256, 0, st>>>(a);
-  gat_fix_long<CB, BWD><<<kNumSM, 256, 0, st>>>(a);
-  count_launches(4);
-  return cudaSuccess;
+#undef CXG_GAT
+#undef CXG_GAT_FWD
+#undef CXG_GAT_BWD
+  if (err != cudaSuccess) return err;
+  int64_t fg = (a.w.max_tiles + 7) / 8;
+  if (fg > kNumSM * 8) fg = kNumSM * 8;
+  const unsigned grid = static_cast<unsigned>(fg);
+  if (a.c % 4 == 0)
+    err = launch_dependent(gat_fix<4, 1, BWD>, grid, 256, 0, st, a);
+  else if (a.w.width % 4 == 0)  // vectors that lie across two heads
+    err = launch_dependent(gat_fix<4, 4, BWD>, grid, 256, 0, st, a);
+  else
+    err = launch_dependent(gat_fix<1, 1, BWD>, grid, 256, 0, st, a);
+  count_launches(3);
+  return err;
 }
 
 }  // namespace
@@ -797,7 +1211,8 @@ extern "C" int cxg_gat_fused_workspace_size(int64_t n_dst, int64_t nnz, int head
   CXG_REQUIRE(bytes != nullptr, CXG_ENULL, "cxg_gat_fused_workspace_size: bytes is NULL");
   CXG_REQUIRE(n_dst >= 0 && nnz >= 0 && heads > 0 && c > 0, CXG_EINVAL, "cxg_gat_fused_workspace_size: bad sizes");
   GatLayout L;
-  gat_layout(n_dst, nnz, heads, c, &L);
+  const int rc = gat_layout(n_dst, nnz, heads, c, &L);
+  CXG_REQUIRE(rc == CXG_OK, rc, "cxg_gat_fused_workspace_size: graph too large for 32-bit tile ids");
   *bytes = L.total;
   return CXG_OK;
 }
@@ -809,7 +1224,7 @@ extern "C" int cxg_gat_fused_forward(const void *ptr, const void *idx, int ptr_b
   CXG_REQUIRE(n_dst >= 0 && nnz >= 0, CXG_EINVAL, "cxg_gat_fused_forward: negative size");
   CXG_REQUIRE((ptr_bytes == 4 || ptr_bytes == 8) && (idx_bytes == 4 || idx_bytes == 8), CXG_EINVAL,
               "cxg_gat_fused_forward: index widths %d/%d", ptr_bytes, idx_bytes);
-  int rc = check_shape("cxg_gat_fused_forward", heads, c);
+  int rc = check_shape("cxg_gat_fused_forward", heads, c, false);
   if (rc != CXG_OK) return rc;
   if (n_dst == 0) return CXG_OK;
   CXG_REQUIRE(ptr && a_dst && y && row_max && row_sum, CXG_ENULL, "cxg_gat_fused_forward: NULL argument");
@@ -817,19 +1232,18 @@ extern "C" int cxg_gat_fused_forward(const void *ptr, const void *idx, int ptr_b
   CXG_REQUIRE(reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0, CXG_EINVAL,
               "cxg_gat_fused_forward: x and y must be 16-byte aligned");
   GatLayout L;
-  gat_layout(n_dst, nnz, heads, c, &L);
+  rc = gat_layout(n_dst, nnz, heads, c, &L);
+  CXG_REQUIRE(rc == CXG_OK, rc, "cxg_gat_fused: graph too large for 32-bit tile ids");
   CXG_REQUIRE(workspace != nullptr && workspace_bytes >= L.total, CXG_EWORKSPACE,
               "cxg_gat_fused_forward: workspace %zu bytes, need %zu", workspace_bytes, L.total);
   CXG_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 16 == 0, CXG_EINVAL, "cxg_gat_fused_forward: workspace alignment");
   GatArgs a = {};
   fill_args(a, L, workspace, nnz, heads, c, slope);
-  a.ptr = ptr, a.idx = idx, a.ptr_bytes = ptr_bytes, a.idx_bytes = idx_bytes;
-  a.gathered = x, a.g_small = a_src, a.r_small = a_dst;
-  a.out = y, a.row_max = row_max, a.row_sum = row_sum;
-  a.n_rows = n_dst;
-  cudaStream_t st = as_stream(stream);
-  const int cb = heads * c * 4 / 32;
-  cudaError_t e = cb == 4 ? launch_walk<4, false>(a, st) : (cb == 8 ? launch_walk<8, false>(a, st) : launch_walk<16, false>(a, st));
+  a.w.ptr = ptr, a.w.idx = idx, a.w.ptr_bytes = ptr_bytes, a.w.idx_bytes = idx_bytes;
+  a.w.x = x, a.g_small = a_src, a.r_small = a_dst;
+  a.w.y = y, a.row_max = row_max, a.row_sum = row_sum;
+  a.w.n_dst = n_dst;
+  cudaError_t e = launch_walk<false>(a, as_stream(stream));
   if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_gat_fused_forward: %s", cudaGetErrorString(e));
   return check_launch("cxg_gat_fused_forward");
 }
@@ -843,7 +1257,7 @@ extern "C" int cxg_gat_fused_backward(const void *t_ptr, const void *t_idx, int 
   CXG_REQUIRE(n_src >= 0 && n_dst >= 0 && nnz >= 0, CXG_EINVAL, "cxg_gat_fused_backward: negative size");
   CXG_REQUIRE((ptr_bytes == 4 || ptr_bytes == 8) && (idx_bytes == 4 || idx_bytes == 8), CXG_EINVAL,
               "cxg_gat_fused_backward: index widths %d/%d", ptr_bytes, idx_bytes);
-  int rc = check_shape("cxg_gat_fused_backward", heads, c);
+  int rc = check_shape("cxg_gat_fused_backward", heads, c, true);
   if (rc != CXG_OK) return rc;
   if (n_src == 0) return CXG_OK;
   CXG_REQUIRE(t_ptr && x && a_src && dx && d_a_src && d_a_dst, CXG_ENULL, "cxg_gat_fused_backward: NULL argument");
@@ -857,45 +1271,48 @@ extern "C" int cxg_gat_fused_backward(const void *t_ptr, const void *t_idx, int 
                   reinterpret_cast<uintptr_t>(y) % 16 == 0 && reinterpret_cast<uintptr_t>(dx) % 16 == 0,
               CXG_EINVAL, "cxg_gat_fused_backward: feature matrices must be 16-byte aligned");
   GatLayout L;
-  gat_layout(n_dst, nnz, heads, c, &L);
+  rc = gat_layout(n_dst, nnz, heads, c, &L);
+  CXG_REQUIRE(rc == CXG_OK, rc, "cxg_gat_fused: graph too large for 32-bit tile ids");
   CXG_REQUIRE(workspace != nullptr && workspace_bytes >= L.total, CXG_EWORKSPACE,
               "cxg_gat_fused_backward: workspace %zu bytes, need %zu", workspace_bytes, L.total);
   CXG_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 16 == 0, CXG_EINVAL, "cxg_gat_fused_backward: workspace alignment");
   GatArgs a = {};
   fill_args(a, L, workspace, nnz, heads, c, slope);
   float *stats = reinterpret_cast<float *>(reinterpret_cast<char *>(workspace) + L.stats);
-  a.ptr = t_ptr, a.idx = t_idx, a.ptr_bytes = ptr_bytes, a.idx_bytes = idx_bytes;
-  a.gathered = dy, a.g_small = stats, a.r_small = a_src, a.r_feat = x;
-  a.out = dx, a.d_r_small = d_a_src, a.d_g_small = d_a_dst;
+  a.w.ptr = t_ptr, a.w.idx = t_idx, a.w.ptr_bytes = ptr_bytes, a.w.idx_bytes = idx_bytes;
+  a.w.x = dy, a.g_small = stats, a.r_small = a_src, a.r_feat = x;
+  a.w.y = dx, a.d_r_small = d_a_src, a.d_g_small = d_a_dst;
   const bool ordered = t_eid != nullptr && nnz > 0 && n_dst > 0;
   a.eid = ordered ? t_eid : nullptr;
   a.d_edge = ordered ? reinterpret_cast<float *>(reinterpret_cast<char *>(workspace) + L.d_edge) : nullptr;
-  a.n_rows = n_src;
+  a.w.n_dst = n_src;
+  int hshift = 0;
+  while ((1 << hshift) < heads) ++hshift;
   cudaStream_t st = as_stream(stream);
-  const int cb = heads * c * 4 / 32;
   if (n_dst > 0) {
     const unsigned pg = static_cast<unsigned>(n_dst / 8 + 1 < kNumSM * 8 ? n_dst / 8 + 1 : kNumSM * 8);
-    if (cb == 4)
-      gat_bwd_prepare<4><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, n_dst, heads, c);
-    else if (cb == 8)
-      gat_bwd_prepare<8><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, n_dst, heads, c);
+    const int vb = vector_of(heads, c);
+    if (vb == 4)
+      gat_bwd_prepare<1><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, n_dst, heads, c);
+    else if (vb == 8)
+      gat_bwd_prepare<2><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, n_dst, heads, c);
     else
-      gat_bwd_prepare<16><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, n_dst, heads, c);
+      gat_bwd_prepare<4><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, n_dst, heads, c);
     count_launches(1);
   }
-  cudaError_t e = cb == 4 ? launch_walk<4, true>(a, st) : (cb == 8 ? launch_walk<8, true>(a, st) : launch_walk<16, true>(a, st));
+  cudaError_t e = launch_walk<true>(a, st);
   if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_gat_fused_backward: %s", cudaGetErrorString(e));
   if (ordered) {
     int64_t *long_rows = reinterpret_cast<int64_t *>(reinterpret_cast<char *>(workspace) + L.long_rows);
     const int max_long = static_cast<int>(nnz / kLongRowEdges + 1);
     // one warp per destination, all of them resident at once while they fit (a row costs two dependent loads)
     const unsigned pg = static_cast<unsigned>(n_dst / 8 + 1 < kNumSM * 64 ? n_dst / 8 + 1 : kNumSM * 64);
-    gat_dst_sum_rows<<<pg, 256, 0, st>>>(fwd_ptr, fwd_ptr_bytes, a.d_edge, d_a_dst, n_dst, nnz, heads, a.hshift, a.hdr,
+    gat_dst_sum_rows<<<pg, 256, 0, st>>>(fwd_ptr, fwd_ptr_bytes, a.d_edge, d_a_dst, n_dst, nnz, heads, hshift, a.w.hdr,
                                          long_rows, max_long);
     float *piece_sums = reinterpret_cast<float *>(reinterpret_cast<char *>(workspace) + L.piece_sums);
-    gat_dst_sum_pieces<<<kNumSM * 2, 256, 0, st>>>(fwd_ptr, fwd_ptr_bytes, a.d_edge, piece_sums, nnz, heads, a.hshift,
-                                                   a.hdr, long_rows, max_long);
-    gat_dst_sum_long<<<kNumSM, 256, 0, st>>>(fwd_ptr, fwd_ptr_bytes, piece_sums, d_a_dst, nnz, heads, a.hshift, a.hdr,
+    gat_dst_sum_pieces<<<kNumSM * 2, 256, 0, st>>>(fwd_ptr, fwd_ptr_bytes, a.d_edge, piece_sums, nnz, heads, hshift,
+                                                   a.w.hdr, long_rows, max_long);
+    gat_dst_sum_long<<<kNumSM, 256, 0, st>>>(fwd_ptr, fwd_ptr_bytes, piece_sums, d_a_dst, nnz, heads, hshift, a.w.hdr,
                                              long_rows, max_long);
     count_launches(3);
   }

@@ -217,20 +217,30 @@ bool walk_eligible(const cxg_spmm_desc *d) {
   return row_bytes <= (vb == 16 ? 128 : 256) * vb;
 }
 
+void walk_plan_run(WalkArgs &a, cudaStream_t st) {
+  a.tile_magic = a.tile > 1 && a.tile < 30000 ? ~0ull / static_cast<uint64_t>(a.tile) + 1 : 0;  // exact up to 2^34 edges
+  const int64_t threads = ((a.n_dst > a.max_tiles ? a.n_dst : a.max_tiles) + kPlanRows - 1) / kPlanRows;
+  walk_plan<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(a);
+}
+
+int walk_whole_waves(int64_t nnz, int64_t resident) {
+  // Whole waves: every resident group gets the same number of tiles, so many that a tile has at most 256 edges (2.3 M
+  // edges, F = 128: 145 us with 3.1 waves of 160 edges, 131 us with 1.9 of 256). From four waves of 512 edges on the
+  // last one no longer matters and the longer tile costs less (126 M edges: 5 % over 256). At least 64 edges, so that
+  // small graphs do not become all borders.
+  if (nnz >= 2048 * resident) return 512;
+  const int64_t waves = (nnz + 256 * resident - 1) / (256 * resident);
+  const int64_t t = waves > 0 ? (nnz + waves * resident - 1) / (waves * resident) : 0;
+  return t < 64 ? 64 : static_cast<int>((t + 31) / 32 * 32);
+}
+
 int walk_tile_edges(const cxg_spmm_desc *d) {
   if (d->split_edges > 0) return d->split_edges;
   WalkArgs a;
   a.row_bytes = d->feat * d->heads * (d->dtype == CXG_F32 ? 4 : 2);
   int resident = kNumSM * 32;
   dispatch(d, a, nullptr, &resident);
-  // Whole waves: every resident group gets the same number of tiles, so many that a tile has at most 256 edges (2.3 M
-  // edges, F = 128: 145 us with 3.1 waves of 160 edges, 131 us with 1.9 of 256). From four waves of 512 edges on the
-  // last one no longer matters and the longer tile costs less (126 M edges: 5 % over 256). At least 64 edges, so that
-  // small graphs do not become all borders.
-  if (d->nnz >= 2048ll * resident) return 512;
-  const int64_t waves = (d->nnz + 256ll * resident - 1) / (256ll * resident);
-  const int64_t t = waves > 0 ? (d->nnz + waves * resident - 1) / (waves * resident) : 0;
-  return t < 64 ? 64 : static_cast<int>((t + 31) / 32 * 32);
+  return walk_whole_waves(d->nnz, resident);
 }
 
 int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t workspace_bytes, cudaStream_t st) {
@@ -255,9 +265,7 @@ int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t
   a.count = reinterpret_cast<int32_t *>(ws + L.count);
   a.partials = reinterpret_cast<float *>(ws + L.partials);
   a.max_tiles = L.max_tiles;
-  a.tile_magic = tile > 1 && tile < 30000 ? ~0ull / static_cast<uint64_t>(tile) + 1 : 0;  // exact up to 2^34 edges
-  const int64_t plan_threads = d->n_dst > L.max_tiles ? d->n_dst : L.max_tiles;
-  walk_plan<<<static_cast<unsigned>((plan_threads + 256 * kPlanRows - 1) / (256 * kPlanRows)), 256, 0, st>>>(a);
+  walk_plan_run(a, st);
   if (!dispatch(d, a, st, nullptr)) return set_error(CXG_EUNSUPPORTED, "cxg_spmm_csr: rows of %d bytes", a.row_bytes);
   int64_t fix_grid = (L.max_tiles + 7) / 8;
   if (fix_grid > kNumSM * 8) fix_grid = kNumSM * 8;

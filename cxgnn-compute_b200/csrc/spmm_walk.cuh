@@ -42,6 +42,10 @@ int walk_layout(int64_t nnz, int64_t width, int tile, WalkLayout *L);
 // True when the walk covers the descriptor: no edge mask, output rows in order and overwritten, rows that fit its lane
 // layouts.
 bool walk_eligible(const cxg_spmm_desc *d);
+// The plan kernel for a.ptr, a.tile, a.whole_rows: fills hdr, tiles, count (and sets a.tile_magic).
+void walk_plan_run(WalkArgs &a, cudaStream_t st);
+// Edges per tile when `resident` tiles are walked at the same time.
+int walk_whole_waves(int64_t nnz, int64_t resident);
 // Edges per tile for this call (desc->split_edges when set).
 int walk_tile_edges(const cxg_spmm_desc *d);
 int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t workspace_bytes, cudaStream_t st);

@@ -894,13 +894,15 @@ GAT_ORDERED_ATT_GRAD = os.environ.get("CXG_GAT_ORDERED_ATT_GRAD", "0") == "1"
 
 
 def gat_fused_supported(x_src):
-    """True when cxg_gat_fused_forward covers this [N, H, C] feature tensor (fp32, H a power of two <= 16, rows of
-    128 / 256 / 512 bytes, a lane's share of a row inside one head)."""
+    """True when cxg_gat_fused_forward covers this [N, H, C] feature tensor (fp32, H a power of two <= 16, rows of up to
+    512 values, of up to 256 / 384 where C is not a multiple of 4 / odd) and, where gradients are recorded, its
+    backward does (C a power of two, at most 128)."""
     if x_src.dim() != 3 or x_src.dtype != torch.float32 or not x_src.is_cuda:
         return False
     h, c = x_src.shape[1], x_src.shape[2]
-    row = h * c * 4
-    return h <= 16 and (h & (h - 1)) == 0 and row in (128, 256, 512) and (c * 4) % (row // 32) == 0
+    if h > 16 or h & (h - 1) or c < 1 or h * c > (512 if c % 4 == 0 else 256 if c % 2 == 0 else 384):
+        return False
+    return not torch.is_grad_enabled() or (c <= 128 and c & (c - 1) == 0)
 
 
 class _GatFusedFunction(torch.autograd.Function):

@@ -258,8 +258,9 @@ int cxg_edge_softmax_backward(const void *ptr, const void *idx, int ptr_bytes,
  *             workspace and d_a_dst[r] is the sum over row r's edges in a fixed order: every output is the
  *             same on every run (about 14 % more time for a layer's forward + backward at the GAT configuration).
  *             With both NULL d_a_dst is zeroed and added into with atomics, like the reference's grad_src.
- * x [n_src, heads, c], y / dy [n_dst, heads, c] float32; heads a power of two <= 16; heads * c * 4 must be
- * 128, 256 or 512 bytes (CXG_EUNSUPPORTED otherwise: use the separate kernels). exp is the fast __expf, like
+ * x [n_src, heads, c], y / dy [n_dst, heads, c] float32; heads a power of two <= 16; heads * c at most
+ * 512 (256 where c is even but no multiple of 4, 384 where it is odd); backward: c a power of two <= 128
+ * (CXG_EUNSUPPORTED otherwise: use the separate kernels). exp is the fast __expf, like
  * the reference's fast-math build; results agree with the three-pass formulation to fp32 rounding, not bit
  * for bit (the running maximum changes the order of the roundings).
  */
