@@ -85,6 +85,8 @@ struct TmmArgs {
   int k, n, num_rel, out_follows_src;
   int atomic;  // add the rows into a float32 C with vector reductions instead of storing them
   int tmem_cols;  // columns of ONE accumulator buffer (two are allocated)
+  int tmem_all;   // columns allocated
+  int small_off;  // compensated mode: columns from an accumulator to that of its small terms, 0 = the same one
   int stages;     // shared-memory stages of A
   int kb;         // K-block: columns of A per pipeline unit (= k unless the stage would not fit several times)
   int dense;       // dense mode: relations per CTA (0 = off); n is then dense * ncols (see below)
@@ -183,7 +185,14 @@ __device__ __forceinline__ float to_tf32(float v) {
   return __uint_as_float(r);
 }
 
-__device__ __forceinline__ float trunc_tf32(float v) { return __uint_as_float(__float_as_uint(v) & 0xffffe000u); }
+// v = hi + lo + what two bits of v cannot hold: hi the upper 19 bits of v, lo = v - hi (exact, at most 13 significant bits)
+// moved half a unit of its 19 bits up in magnitude, so that the tensor core, which ignores the other 13 bits of a word,
+// reads it rounded. Cut instead, every product would be short by 1e-7 of itself on the same side. (The addition turns a
+// NaN, which lo is where v is infinite, into -0; hi carries infinities and NaN alone.)
+__device__ __forceinline__ void split_tf32(float v, float &hi, float &lo) {
+  hi = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
+  lo = __uint_as_float(__float_as_uint(v - hi) + 0x1000u);
+}
 
 // W [R][K][N] -> Wt [R][N][K]; with `wt_lo` (fp32 only) the two TF32 terms hi = tf32(w), lo = tf32(w - hi).
 template <typename T>
@@ -255,6 +264,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t *v, uint32_t taddr) {
       : "r"(taddr));
 }
 
+// fp32 words: v += w
+template <int N>
+__device__ __forceinline__ void add_words(uint32_t *v, const uint32_t *w) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(w[i]));
+}
+
 __device__ __forceinline__ void st_global_v4(void *p, uint4 v) {
   asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -301,7 +317,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
 
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_slot)),
-                 "r"(static_cast<uint32_t>(2 * a.tmem_cols))
+                 "r"(static_cast<uint32_t>(a.tmem_all))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -447,15 +463,24 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
         if (!alive) break;
         float4 *hi = reinterpret_cast<float4 *>(smem_a + s * a_bytes);
         float4 *lo = reinterpret_cast<float4 *>(smem_a + s * a_bytes + half_bytes);
-        for (int c = ct; c < n16; c += 32 * kConvWarps) {
-          // hi = the upper 19 bits of v, lo = the upper 19 bits of v - hi: both are exact TF32 values (one
-          // logic op each instead of a conversion instruction), v - hi is exact in fp32
-          const float4 v = hi[c];
-          float4 h, l;
-          h.x = trunc_tf32(v.x), h.y = trunc_tf32(v.y), h.z = trunc_tf32(v.z), h.w = trunc_tf32(v.w);
-          l.x = trunc_tf32(v.x - h.x), l.y = trunc_tf32(v.y - h.y), l.z = trunc_tf32(v.z - h.z), l.w = trunc_tf32(v.w - h.w);
-          hi[c] = h;
-          lo[c] = l;
+        // four chunks requested at once: one after the other their round trips to shared memory bounded the kernel
+        constexpr int kStep = 32 * kConvWarps;
+        for (int c0 = ct; c0 < n16; c0 += 4 * kStep) {
+          float4 v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (c0 + u * kStep < n16) v[u] = hi[c0 + u * kStep];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (c0 + u * kStep < n16) {
+              float4 h, l;
+              split_tf32(v[u].x, h.x, l.x);
+              split_tf32(v[u].y, h.y, l.y);
+              split_tf32(v[u].z, h.z, l.z);
+              split_tf32(v[u].w, h.w, l.w);
+              hi[c0 + u * kStep] = h;
+              lo[c0 + u * kStep] = l;
+            }
         }
         // these generic-proxy writes are read by the tensor core through the async proxy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -499,9 +524,10 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
                                          : make_desc(a0 + static_cast<uint32_t>(half_bytes) + ao, lbo, sbo_a);
               const uint64_t db_hi = make_desc(bk + j * 256, lbo, sbo_b);
               const uint64_t db_lo = make_desc(bk + static_cast<uint32_t>(w_bytes) + j * 256, lbo, sbo_b);
-              mma_ss<TF32>(d, da_hi, db_lo, idesc, first);  // the two small terms first, the large one last
-              mma_ss<TF32>(d, da_lo, db_hi, idesc, 1u);
-              mma_ss<TF32>(d, da_hi, db_hi, idesc, 1u);
+              // the two small terms into an accumulator of their own where there is room for it
+              mma_ss<TF32>(d + a.small_off, da_hi, db_lo, idesc, first);
+              mma_ss<TF32>(d + a.small_off, da_lo, db_hi, idesc, 1u);
+              mma_ss<TF32>(d, da_hi, db_hi, idesc, a.small_off ? first : 1u);
             } else if (TMA) {
               // step j reads 32 bytes of K: span j / 4 of the stage (16 KiB each), 32-byte offset j % 4 inside it
               mma_ss<TF32>(d, make_desc_sw128(a0 + (j >> 2) * (kTileM * 128) + (j & 3) * 32),
@@ -568,7 +594,14 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
         for (int c0 = c_lo; c0 < c_hi; c0 += 16) {
           uint32_t v[16];
           tmem_ld16(v, taddr + c0);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (X3 && a.small_off) {
+            uint32_t sm[16];
+            tmem_ld16(sm, taddr + a.small_off + c0);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            add_words<16>(v, sm);
+          } else {
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          }
           if (c0 + 16 >= c_hi) {  // the accumulator buffer is in registers: give it back to the MMA thread
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbar_arrive(&bars.acc_empty[buf]);
@@ -594,7 +627,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
         const int64_t rel_step = dense ? a.m_valid * a.ncols : 0;
         T *row_a = C + oc_a * a.ncols + rel_lo * rel_step, *row_b = C + oc_b * a.ncols + rel_lo * rel_step;
         int cc = cc_lo;
-        constexpr int GU = TF32 ? 2 : 4;  // loads of 16 columns per round trip (fp32 kernels have fewer registers per thread)
+        constexpr int GU = X3 ? 1 : (TF32 ? 2 : 4);  // loads of 16 columns per round trip (as many as the registers hold; X3: two accumulators)
         if (c_lo >= c_hi) {  // nothing for this group (n = 16): only hand the buffer back
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           mbar_arrive(&bars.acc_empty[buf]);
@@ -604,7 +637,16 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
 #pragma unroll
           for (int u = 0; u < GU; ++u)
             if (g0 + 16 * u < c_hi) tmem_ld16(v + 16 * u, taddr + g0 + 16 * u);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (X3 && a.small_off) {
+            uint32_t sm[16 * GU];
+#pragma unroll
+            for (int u = 0; u < GU; ++u)
+              if (g0 + 16 * u < c_hi) tmem_ld16(sm + 16 * u, taddr + a.small_off + g0 + 16 * u);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            add_words<16 * GU>(v, sm);
+          } else {
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          }
           if (g0 + 16 * GU >= c_hi) {  // the accumulator buffer is in registers: give it back to the MMA thread
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbar_arrive(&bars.acc_empty[buf]);
@@ -662,7 +704,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d),
-                 "r"(static_cast<uint32_t>(2 * a.tmem_cols))
+                 "r"(static_cast<uint32_t>(a.tmem_all))
                  : "memory");
   }
 }
@@ -817,6 +859,11 @@ extern "C" int cxg_typed_matmul(const void *a, const void *w, void *c, const int
   int cols = 32;
   while (cols < n) cols <<= 1;
   t.tmem_cols = cols;  // two buffers: 2 * cols <= 512
+  // The tensor core cuts its sum at every instruction, so the error grows with the number of instructions that add to an
+  // accumulator: with the small terms in one of their own, a third as many add to the large one (K = 128: 1.0e-6 of the
+  // result with one accumulator, 0.35e-6 with two).
+  t.small_off = x3 && 4 * cols <= 512 ? 2 * cols : 0;
+  t.tmem_all = t.small_off ? 4 * cols : 2 * cols;
   t.stages = stages;
   t.kb = kb;
   if (cudaMemsetAsync(t.status, 0, 256, st) != cudaSuccess) return check_launch("cxg_typed_matmul: memset");
