@@ -16,8 +16,9 @@
 // the same bits on every run.
 //
 // fp32 inputs: plain TF32 products (precision 1) or, like the forward, error-compensated ones (precision 2): four
-// converter warps split both tiles of a stage into hi = upper 19 bits and lo = upper 19 bits of (v - hi), and the
-// tensor core accumulates A_hi.B_lo + A_lo.B_hi + A_hi.B_hi.
+// converter warps split both tiles of a stage into hi = upper 19 bits and lo = v - hi rounded to 19 bits, and the
+// tensor core accumulates A_hi.B_lo + A_lo.B_hi and A_hi.B_hi. (169,343 positions, 128 x 128, against float64: 3.8e-6 of
+// the result with one accumulator and 512 positions in it, 0.9e-6 with two and 256; an fp32 GEMM 1.4e-6.)
 //
 // Every wait is bounded; a role that waits too long raises a CTA-wide abort flag and an error status.
 #include "common.cuh"
@@ -139,7 +140,11 @@ __device__ __forceinline__ void commit_to(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-__device__ __forceinline__ float trunc_tf32(float v) { return __uint_as_float(__float_as_uint(v) & 0xffffe000u); }
+// v = hi + lo up to half a unit of lo's 19 bits (see typed_mm.cu)
+__device__ __forceinline__ void split_tf32(float v, float &hi, float &lo) {
+  hi = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
+  lo = __uint_as_float(__float_as_uint(v - hi) + 0x1000u);
+}
 
 struct Barriers {
   uint64_t full[kMaxStages];   // producers -> MMA (or converters): 256 arrivals
@@ -163,17 +168,24 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
   __shared__ int abort_slot;
   volatile int *abort_flag = &abort_slot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int spans_x = a.k * static_cast<int>(sizeof(T)) / 128, spans_g = a.n * static_cast<int>(sizeof(T)) / 128;
+  // spans that hold the rows of x and of g. The tensor core reads 128 columns of x: those behind K lie in the memory
+  // behind (g's spans, the next stage) and only reach rows of the result that are not stored.
+  const int xrow = a.k * static_cast<int>(sizeof(T)), grow = a.n * static_cast<int>(sizeof(T));
+  const int spans_x = (xrow + 127) / 128, spans_g = (grow + 127) / 128;
+  const int n_mma = spans_g * (128 / static_cast<int>(sizeof(T)));  // whole spans; columns behind N are zeros
   const uint32_t half_bytes = static_cast<uint32_t>(spans_x + spans_g) * kSpan;  // raw (or hi) tiles of x and g
   const uint32_t stage_bytes = X3 ? 2 * half_bytes : half_bytes;
   const int S = a.stages;
   uint8_t *smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);  // swizzled tiles: 1024-byte boundaries
   int tmem_cols = 32;
-  while (tmem_cols < a.n) tmem_cols <<= 1;
+  while (tmem_cols < n_mma) tmem_cols <<= 1;
+  // compensated mode: the small terms have an accumulator of their own where there is room (see typed_mm.cu)
+  const uint32_t small_off = X3 && 4 * tmem_cols <= 512 ? 2 * tmem_cols : 0;
+  const uint32_t tmem_all = small_off ? 4 * tmem_cols : 2 * tmem_cols;
 
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_slot)),
-                 "r"(static_cast<uint32_t>(2 * tmem_cols))
+                 "r"(tmem_all)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -206,7 +218,6 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     const int c16 = pt & 7;                // 16-byte chunk inside a 128-byte span
     const int prow = pt >> 3;              // row inside a pass of 32 rows
     const uint8_t *X = static_cast<const uint8_t *>(a.x), *G = static_cast<const uint8_t *>(a.g);
-    const int64_t xrow_bytes = static_cast<int64_t>(a.k) * sizeof(T), grow_bytes = static_cast<int64_t>(a.n) * sizeof(T);
     constexpr int kPass = kPos / 32;  // passes of 32 rows per tile
     auto fetch = [&](int64_t tile, int64_t (&ia)[kPass], int64_t (&ig)[kPass]) {
 #pragma unroll
@@ -242,13 +253,17 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
         const bool ok = ia[q] >= 0 && ia[q] < a.x_rows && ig[q] >= 0 && ig[q] < a.g_rows;
         const int bytes = ok ? 16 : 0;
         const uint32_t d0 = st0 + swizzled_offset<TF32>(p, c16);
-        const uint8_t *xs = ok ? X + ia[q] * xrow_bytes + c16 * 16 : X;
-        const uint8_t *gs = ok ? G + ig[q] * grow_bytes + c16 * 16 : G;
-        for (int j = 0; j < spans_x; ++j)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d0 + j * kSpan), "l"(xs + j * 128), "r"(bytes) : "memory");
-        for (int j = 0; j < spans_g; ++j)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d0 + (spans_x + j) * kSpan), "l"(gs + j * 128), "r"(bytes)
+        const uint8_t *xs = ok ? X + ia[q] * xrow : X;
+        const uint8_t *gs = ok ? G + ig[q] * grow : G;
+        // a chunk behind the row's end is written as zeros from the row's first chunk
+        auto copy = [&](const uint8_t *src, int row_bytes, int j, uint32_t dst) {
+          const int at = j * 128 + c16 * 16;
+          const bool in = at < row_bytes;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(in && ok ? src + at : src), "r"(in ? bytes : 0)
                        : "memory");
+        };
+        for (int j = 0; j < spans_x; ++j) copy(xs, xrow, j, d0 + j * kSpan);
+        for (int j = 0; j < spans_g; ++j) copy(gs, grow, j, d0 + (spans_x + j) * kSpan);
       }
       if (!(a.test_stall && it == 0))
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&bars.full[s])) : "memory");
@@ -268,13 +283,23 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
       if (!alive) break;
       float4 *hi = reinterpret_cast<float4 *>(smem + static_cast<size_t>(s) * stage_bytes);
       float4 *lo = reinterpret_cast<float4 *>(smem + static_cast<size_t>(s) * stage_bytes + half_bytes);
-      for (int c = ct; c < n16; c += 32 * kConvWarps) {
-        const float4 v = hi[c];
-        float4 h, l;
-        h.x = trunc_tf32(v.x), h.y = trunc_tf32(v.y), h.z = trunc_tf32(v.z), h.w = trunc_tf32(v.w);
-        l.x = trunc_tf32(v.x - h.x), l.y = trunc_tf32(v.y - h.y), l.z = trunc_tf32(v.z - h.z), l.w = trunc_tf32(v.w - h.w);
-        hi[c] = h;
-        lo[c] = l;
+      constexpr int kStep = 32 * kConvWarps;
+      for (int c0 = ct; c0 < n16; c0 += 4 * kStep) {  // four chunks requested at once
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (c0 + u * kStep < n16) v[u] = hi[c0 + u * kStep];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (c0 + u * kStep < n16) {
+            float4 h, l;
+            split_tf32(v[u].x, h.x, l.x);
+            split_tf32(v[u].y, h.y, l.y);
+            split_tf32(v[u].z, h.z, l.z);
+            split_tf32(v[u].w, h.w, l.w);
+            hi[c0 + u * kStep] = h;
+            lo[c0 + u * kStep] = l;
+          }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       mbar_arrive(&bars.conv[s]);
@@ -286,7 +311,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     // of positions summed in one accumulator), so an accumulator takes at most `chunk_tiles` tiles; the epilogue adds
     // the chunks of a relation with ordinary fp32 additions. Two accumulator buffers alternate.
     if (lane == 0) {
-      const uint32_t idesc = make_idesc_mn(TF32 ? 2 : 1, a.k, a.n);
+      const uint32_t idesc = make_idesc_mn(TF32 ? 2 : 1, 128, n_mma);
       const uint32_t step_bytes = kInstrK * 128;  // the next kInstrK positions of a span
       int64_t it = 0, chunk = 0;
       int in_chunk = 0;
@@ -326,9 +351,9 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
           if (X3) {
             const uint64_t xa = make_desc_mn_sw128<TF32>(x0 + off, kSpan), xl = make_desc_mn_sw128<TF32>(x0 + half_bytes + off, kSpan);
             const uint64_t ga = make_desc_mn_sw128<TF32>(g0 + off, kSpan), gl = make_desc_mn_sw128<TF32>(g0 + half_bytes + off, kSpan);
-            mma_ss<TF32>(d, xa, gl, idesc, first);  // the two small terms first, the large one last
-            mma_ss<TF32>(d, xl, ga, idesc, 1u);
-            mma_ss<TF32>(d, xa, ga, idesc, 1u);
+            mma_ss<TF32>(d + small_off, xa, gl, idesc, first);
+            mma_ss<TF32>(d + small_off, xl, ga, idesc, 1u);
+            mma_ss<TF32>(d, xa, ga, idesc, small_off ? first : 1u);
           } else {
             mma_ss<TF32>(d, make_desc_mn_sw128<TF32>(x0 + off, kSpan), make_desc_mn_sw128<TF32>(g0 + off, kSpan), idesc, first);
           }
@@ -362,7 +387,19 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
               "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
             : "r"(taddr + c0));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (X3 && small_off) {
+          uint32_t w[16];
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+              : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]), "=r"(w[8]),
+                "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
+              : "r"(taddr + small_off + c0));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(w[i]));
+        } else {
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        }
         if (row < a.k) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -407,7 +444,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
   __syncthreads();
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(static_cast<uint32_t>(2 * tmem_cols))
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(tmem_all)
                  : "memory");
   }
 }
@@ -472,8 +509,8 @@ extern "C" int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel,
               precision);
   CXG_REQUIRE(dw != nullptr, CXG_ENULL, "cxg_typed_wgrad: dw is NULL");
   const int elem = dtype == CXG_F32 ? 4 : 2;
-  CXG_REQUIRE(k == 128 && (n * elem) % 128 == 0 && n % 16 == 0 && n <= 256, CXG_EUNSUPPORTED,
-              "cxg_typed_wgrad: K = %d must be 128 and N = %d a multiple of %d up to 256", k, n, 128 / elem);
+  CXG_REQUIRE(k <= 128 && (k * elem) % 16 == 0 && n % 16 == 0 && n <= 256, CXG_EUNSUPPORTED,
+              "cxg_typed_wgrad: K = %d must be a multiple of %d up to 128 and N = %d one of 16 up to 256", k, 16 / elem, n);
   cudaStream_t st = as_stream(stream);
   const int64_t kn = static_cast<int64_t>(k) * n;
   if (m == 0) {
@@ -491,19 +528,22 @@ extern "C" int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel,
   CXG_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 16 == 0, CXG_EINVAL, "cxg_typed_wgrad: workspace alignment");
   const bool x3 = precision == 2 && dtype == CXG_F32;
   const int pos = x3 ? 64 : 128;  // positions per tile, as in the kernel
-  const size_t half = static_cast<size_t>(k + n) * elem / 128 * (128 * pos);
+  const int spans = (k * elem + 127) / 128 + (n * elem + 127) / 128;
+  const size_t half = static_cast<size_t>(spans) * (128 * pos);
   const size_t stage = x3 ? 2 * half : half;
-  int stages = static_cast<int>((kSmemBudget - 1024) / stage);
+  // the tensor core reads elem spans of x (128 columns) from a tile's start: room behind the last stage for narrow tiles
+  const size_t behind = spans < elem ? static_cast<size_t>(elem - spans) * (128 * pos) : 0;
+  int stages = static_cast<int>((kSmemBudget - 1024 - behind) / stage);
   if (stages > kMaxStages) stages = kMaxStages;
   CXG_REQUIRE(stages >= 1, CXG_EUNSUPPORTED, "cxg_typed_wgrad: one stage of %zu bytes exceeds shared memory", stage);
-  const size_t smem = 1024 + stages * stage;
+  const size_t smem = 1024 + stages * stage + behind;
 
   char *ws = static_cast<char *>(workspace);
   WgArgs a;
   a.x = x, a.g = g, a.rel = rel, a.idx = idx, a.idx_g = idx_g, a.m = m, a.x_rows = x_rows, a.g_rows = g_rows;
   a.k = k, a.n = n, a.num_rel = num_rel, a.stages = stages, a.slots = L.slots;
   a.test_stall = (flags & CXG_WGRAD_TEST_STALL) ? 1 : 0;
-  a.chunk_tiles = x3 ? 8 : 32;  // 512 / 4096 positions per accumulator: its error stays well below 1e-5 of fp32 / below
+  a.chunk_tiles = x3 ? 4 : 32;  // 256 / 4096 positions per accumulator: its error stays below that of an fp32 sum / below
                                 // the rounding of the plain products
   a.partial = reinterpret_cast<float *>(ws + L.partial);
   a.slot_rel = reinterpret_cast<int32_t *>(ws + L.slot_rel);

@@ -222,17 +222,19 @@ _wg_status = _sig("cxg_typed_wgrad_status", [_vp, _vp])
 
 
 def typed_wgrad_supported(x, g, allow_tf32=None):
-    """Shapes cxg_typed_wgrad covers: same fp32 / bf16 dtype, 128 input columns, output rows a multiple of 128 bytes,
-    one stage (both tiles, twice for the error-compensated fp32 mode) within shared memory."""
+    """Shapes cxg_typed_wgrad covers: same fp32 / bf16 dtype, up to 128 input columns in rows of whole 16-byte chunks, a
+    multiple of 16 output columns up to 256, one stage (both tiles, twice for the error-compensated fp32 mode) within
+    shared memory."""
     if not (x.is_cuda and x.dtype in (torch.float32, torch.bfloat16) and g.dtype == x.dtype and x.dim() == 2
-            and g.dim() == 2 and x.shape[1] == 128 and (g.shape[1] * g.element_size()) % 128 == 0
+            and g.dim() == 2 and x.shape[1] <= 128 and (x.shape[1] * x.element_size()) % 16 == 0
             and g.shape[1] % 16 == 0 and g.shape[1] <= 256):
         return False
     if allow_tf32 is None:
         allow_tf32 = sys.modules[__package__].ALLOW_TF32
     split = 2 if (x.dtype == torch.float32 and not allow_tf32) else 1
     positions = 64 if split == 2 else 128  # per tile, as the kernel chooses them
-    return (128 + g.shape[1]) * x.element_size() * positions * split <= 224 * 1024
+    spans = sum((t.shape[1] * t.element_size() + 127) // 128 for t in (x, g))
+    return max(spans, x.element_size()) * 128 * positions * split <= 224 * 1024
 
 
 def typed_wgrad(x, g, sorted_rel, num_rel, num_valid=None, idx=None, idx_g=None, allow_tf32=None, extra_flags=0,

@@ -140,7 +140,7 @@ int cxg_typed_matmul_status(const void *workspace, void *stream);
  * over positions, both operands MN-major) plus a fixed-order reduction of per-CTA partial sums: no atomics. An
  * accumulator in tensor memory takes a few thousand positions at most and the partial sums are added in ordinary
  * fp32, so the error does not grow with the number of rows. precision 1 = plain bf16 / TF32 products, 2 =
- * error-compensated TF32 for fp32 inputs (1e-5 class). Shapes: k == 128, n * element size a multiple of 128 bytes,
+ * error-compensated TF32 for fp32 inputs (1e-5 class). Shapes: k <= 128 in rows of whole 16-byte chunks, n a multiple of 16,
  * n <= 256, one stage within shared memory (CXG_EUNSUPPORTED otherwise). cxg_typed_wgrad_status reads back whether a
  * bounded wait ran out.
  */
