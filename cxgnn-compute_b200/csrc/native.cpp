@@ -392,6 +392,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("last_workspace", &last_workspace);
   m.def("spmm", &spmm);
   m.def("sage", &sage);
+  m.def("spmm_transposed", &spmm_transposed);
   m.def("transpose", [](const Tensor &ptr, const Tensor &idx, int64_t n, int64_t n_src, bool want_eid) {
     const Transposed t = transpose(ptr, idx, n, n_src, want_eid);
     return std::make_tuple(t.t_ptr, t.t_idx, want_eid ? optional<Tensor>(t.t_eid) : c10::nullopt, t.inv_deg);

@@ -285,7 +285,8 @@ class MyRGCNConv(torch.nn.Module):
     with `aggr_rel`, the ordering of TypedLinearS2DMMAggrOP (typed_linear.py:191-221): it moves `out` instead of
     `in` values per edge and wins when the mean degree exceeds num_rel * out / in; fp32 inputs take that GEMM in
     TF32, the precision of the typed matmul (and of the reference's `tl.dot`). "auto" (default) picks between
-    "fused_gather" and "transform_first" by the bytes each moves for the graph at hand."""
+    "fused_gather" and "transform_first" by the bytes each moves for the graph at hand; where gradients are recorded it
+    transforms the distinct (relation, source) pairs instead (cxgnncomp_backend.RelationPairs)."""
 
     def __init__(self, in_channels, hidden_channels, num_rel, norm="total", schedule="auto"):
         super().__init__()
@@ -312,6 +313,12 @@ class MyRGCNConv(torch.nn.Module):
         if idx.shape[0] > 1e8:
             return RGCNOP.apply(x, self.linear, ptr, idx, edge_types, num_node)
         num_edge = edge_types.shape[0]
+        if (self.schedule == "auto" and self.norm == "total" and num_edge > 0 and torch.is_grad_enabled()
+                and (x.requires_grad or self.linear.requires_grad)
+                and cxgnncomp_backend.relation_pairs_supported(x, self.linear)):
+            # training: only the rows that some edge reads, in both directions; never more values than "fused_gather" moves
+            # (at most one row per edge) nor, in the backward, than the table of every node under every relation
+            return cxgnncomp_backend.relation_pairs_mean(x, self.linear, ptr, idx, edge_types, num_node)
         key = (ptr.data_ptr(), ptr._version, num_node, x.dtype)
         if self._deg_cache is None or self._deg_cache[0] != key:  # per graph, not per call
             self._deg_cache = (key, (ptr[1:num_node + 1] - ptr[:num_node]).clamp(min=1).to(x.dtype), ptr)
