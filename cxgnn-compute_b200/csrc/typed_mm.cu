@@ -9,9 +9,8 @@
 // A persistent, warp-specialised CTA per SM owns a contiguous range of 128-position tiles (so the
 // relation changes at most num_rel times per CTA) and runs three roles that meet only at mbarriers:
 //   * 4 or 8 producer warps gather the 128 rows of A of a tile with 16-byte `cp.async` copies into
-//     one stage of a shared-memory ring, in the K-major "core matrix" layout the tensor core reads
-//     without swizzle (8 rows x 16 bytes per core matrix; padding rows are zero-filled by a copy
-//     of size 0), and hand the stage over with `cp.async.mbarrier.arrive.noinc`: the barrier counts
+//     one stage of a shared-memory ring, K-major in swizzled spans (padding rows are zero-filled by a
+//     copy of size 0), and hand the stage over with `cp.async.mbarrier.arrive.noinc`: the barrier counts
 //     a thread's arrival when its copies have landed, so a producer never waits for its own
 //     copies and up to `stages` tiles are in flight per CTA (waiting with `cp.async.wait_group`
 //     plus a proxy fence in the producer serialised copy and MMA latency and was 13-19 % slower).
@@ -88,7 +87,8 @@ struct TmmArgs {
   int tmem_all;   // columns allocated
   int small_off;  // compensated mode: columns from an accumulator to that of its small terms, 0 = the same one
   int stages;     // shared-memory stages of A
-  int kb;         // K-block: columns of A per pipeline unit (= k unless the stage would not fit several times)
+  int span_log;   // log2 of the 16-byte chunks in a swizzle span: 3, 2, 1 for spans of 128, 64, 32 bytes
+  int kb;         // K-block: columns of A per pipeline unit (= k unless the stage would not fit several times), whole spans
   int dense;       // dense mode: relations per CTA (0 = off); n is then dense * ncols (see below)
   int ncols;       // columns of C per relation (= n outside dense mode)
   int test_stall;  // test hook: the producers never hand over the first tile, so the waits for it run out
@@ -98,28 +98,26 @@ struct TmmArgs {
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
-// Shared-memory matrix descriptor, K-major, no swizzle: core matrices of 8 rows x 16 bytes,
-// `lbo` bytes between core matrices along K, `sbo` bytes between 8-row groups.
-__device__ __forceinline__ uint64_t make_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+// Shared-memory matrix descriptors, K-major with a swizzle: a tile is cut along K into spans of 128, 64 or 32 bytes; a
+// span holds its rows one behind the other, 8-row groups 8 * span bytes apart, and permutes the 16-byte chunks of a row by
+// the row number, so that the tensor core reads 8 rows without bank conflicts. A span starts on a multiple of 8 * span
+// bytes; K advances inside it by adding 32 bytes to the address. (As core matrices of 8 rows x 16 bytes without a swizzle,
+// which is how the copies wrote A and W before, an instruction took some 230 cycles and the tensor core bounded the kernel:
+// fp32, 2.33 M gathered rows, K = 128, N = 64 took 837 us, 564 us now; K = 64, N = 128: 495 us, now 364.)
+// What is constant in a descriptor:
+__device__ __forceinline__ uint64_t desc_base(int span_log) {
   uint64_t d = 0;
-  d |= static_cast<uint64_t>((addr >> 4) & 0x3fff);
-  d |= static_cast<uint64_t>((lbo >> 4) & 0x3fff) << 16;
-  d |= static_cast<uint64_t>((sbo >> 4) & 0x3fff) << 32;
-  d |= 1ull << 46;  // descriptor version of sm_100
+  d |= 1ull << 16;                                                  // leading offset: unused with a swizzle, canonical value 1
+  d |= static_cast<uint64_t>((128u << span_log) >> 4) << 32;        // next 8-row group
+  d |= 1ull << 46;                                                  // descriptor version of sm_100
+  d |= static_cast<uint64_t>(span_log == 3 ? 2 : span_log == 2 ? 4 : 6) << 61;  // 128-, 64- or 32-byte swizzle
   return d;
 }
-
-// The same for a tile that the bulk tensor copy unit (TMA) wrote with its 128-byte swizzle: rows of 128 bytes (one
-// swizzle span of K), 8-row groups 1024 bytes apart, the 16-byte chunks of a row permuted by (row % 8). The tile must
-// start on a 1024-byte boundary; K advances inside the span by adding bytes to `addr`.
-__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t addr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((addr >> 4) & 0x3fff);
-  d |= 1ull << 16;                                   // leading offset: unused with a swizzle, canonical value 1
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;       // next 8-row group
-  d |= 1ull << 46;                                   // descriptor version of sm_100
-  d |= 2ull << 61;                                   // layout type: 128-byte swizzle
-  return d;
+__device__ __forceinline__ uint64_t make_desc(uint64_t base, uint32_t addr) { return base | ((addr >> 4) & 0x3fff); }
+// byte offset of 16-byte chunk c of a row inside a tile whose spans are span_bytes apart
+__device__ __forceinline__ uint32_t swizzled(int row, int c, int span_log, uint32_t span_bytes) {
+  const uint32_t in = (c ^ (row >> (3 - span_log))) & ((1 << span_log) - 1);
+  return (c >> span_log) * span_bytes + (static_cast<uint32_t>(row) << (span_log + 4)) + (in << 4);
 }
 
 // One tiled 2-D bulk tensor copy global -> shared (x = element column, y = row of the tensor map's matrix); its bytes
@@ -301,19 +299,20 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
   __shared__ int abort_slot;
   volatile int *abort_flag = &abort_slot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int chunks = a.k / EPC;             // 16-byte chunks per full row (layout of W in shared memory)
-  const int chunks_blk = a.kb / EPC;        // 16-byte chunks per row of one K-block (layout of a stage of A)
+  const int chunks = a.k / EPC;             // 16-byte chunks of a row
+  const int chunks_blk = a.kb / EPC;        // 16-byte chunks per row of one K-block, whole spans
   const int nkb = a.k / a.kb;               // K-blocks per tile
-  const uint32_t lbo = 128;                 // next core matrix along K
-  const uint32_t sbo_a = chunks_blk * 128;  // next 8-row group inside a stage of A
-  const uint32_t sbo_b = chunks * 128;      // next 8-row group of W
+  const int sl = TMA ? 3 : a.span_log;
+  const uint32_t span_a = kTileM << (sl + 4);  // bytes of a span of a tile of A, and of W
+  const uint32_t span_w = a.n << (sl + 4);
   const int S = a.stages;
   const size_t half_bytes = static_cast<size_t>(kTileM) * a.kb * sizeof(T);  // one [128][kb] tile
   const size_t a_bytes = X3 ? 2 * half_bytes : half_bytes;                   // a stage: raw / hi (+ lo)
   const size_t w_bytes = static_cast<size_t>(a.n) * a.k * sizeof(T);        // n rows of W[rel]^T
-  uint8_t *smem_b = smem;                                    // W (hi), then W lo in the compensated mode
-  uint8_t *smem_a = smem + (X3 ? 2 * w_bytes : w_bytes);     // S stages
-  if (TMA) smem_a += (1024u - (smem_addr(smem_a) & 1023u)) & 1023u;  // swizzled tiles start on 1024-byte boundaries
+  // W (hi), then W lo in the compensated mode; spans start on multiples of eight of their rows
+  const uint32_t align = 128u << sl;
+  uint8_t *smem_b = smem + ((align - smem_addr(smem)) & (align - 1));
+  uint8_t *smem_a = smem_b + (X3 ? 2 * w_bytes : w_bytes);   // S stages
 
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_slot)),
@@ -393,7 +392,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
           const uint32_t bp = b0 + part * static_cast<uint32_t>(w_bytes);
           for (int row = pw * kRpi + rsub; row < a.n; row += kProdWarps * kRpi)
             for (int c = cq; c < chunks; c += kCpi)
-              cp_async16<false>(bp + (row >> 3) * sbo_b + c * 128 + (row & 7) * 16, wr + static_cast<int64_t>(row) * a.k + c * EPC, 16);
+              cp_async16<false>(bp + swizzled(row, c, sl, span_w), wr + static_cast<int64_t>(row) * a.k + c * EPC, 16);
         }
         loaded_rel = r;
       }
@@ -436,8 +435,8 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
             const bool ok = ia[gi] >= 0 && ia[gi] < a.m_valid;
             const T *src_row = ok ? A + ia[gi] * a.k + kb * a.kb : A;
             const int bytes = ok ? 16 : 0;  // size 0 writes zeros
-            const uint32_t d0 = a0 + (row >> 3) * sbo_a + (row & 7) * 16;
-            for (int c = cq; c < chunks_blk; c += kCpi) cp_async16<CA>(d0 + c * 128, src_row + c * EPC, bytes);
+            for (int c = cq; c < chunks_blk; c += kCpi)
+              cp_async16<CA>(a0 + swizzled(row, c, sl, span_a), src_row + c * EPC, bytes);
           }
         }
         // the unit's full barrier counts this thread's arrival when all copies it has issued so far (this unit's
@@ -493,6 +492,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
     if (lane == 0) {
       const uint32_t idesc = make_idesc(TF32 ? 2 : 1, kTileM, a.n);
       const uint32_t b0 = smem_addr(smem_b);
+      const uint64_t desc = desc_base(sl);
       const int steps = chunks_blk / 2;  // two chunks (32 bytes) of K per instruction
       int64_t it = 0, tile_it = 0;
       bool alive = true;
@@ -514,26 +514,21 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a0 = smem_addr(smem_a + s * a_bytes);
-          const uint32_t bk = b0 + kb * chunks_blk * 128;  // this K-block's columns of W
           for (int j = 0; j < steps; ++j) {
             const uint32_t first = (kb > 0 || j > 0) ? 1u : 0u;
+            // a step reads 32 bytes of K, of which a span holds 4, 2 or 1
+            const int g = kb * steps + j, in = (1 << (sl - 1)) - 1;
+            const uint32_t aa = a0 + (j >> (sl - 1)) * span_a + (j & in) * 32;
+            const uint32_t bb = b0 + (g >> (sl - 1)) * span_w + (g & in) * 32;
             if (X3) {
-              const uint32_t ao = TMA ? (j >> 2) * (kTileM * 128) + (j & 3) * 32 : j * 256;  // as in the plain branch below
-              const uint64_t da_hi = TMA ? make_desc_sw128(a0 + ao) : make_desc(a0 + ao, lbo, sbo_a);
-              const uint64_t da_lo = TMA ? make_desc_sw128(a0 + static_cast<uint32_t>(half_bytes) + ao)
-                                         : make_desc(a0 + static_cast<uint32_t>(half_bytes) + ao, lbo, sbo_a);
-              const uint64_t db_hi = make_desc(bk + j * 256, lbo, sbo_b);
-              const uint64_t db_lo = make_desc(bk + static_cast<uint32_t>(w_bytes) + j * 256, lbo, sbo_b);
+              const uint64_t da_hi = make_desc(desc, aa), da_lo = make_desc(desc, aa + static_cast<uint32_t>(half_bytes));
+              const uint64_t db_hi = make_desc(desc, bb), db_lo = make_desc(desc, bb + static_cast<uint32_t>(w_bytes));
               // the two small terms into an accumulator of their own where there is room for it
               mma_ss<TF32>(d + a.small_off, da_hi, db_lo, idesc, first);
               mma_ss<TF32>(d + a.small_off, da_lo, db_hi, idesc, 1u);
               mma_ss<TF32>(d, da_hi, db_hi, idesc, a.small_off ? first : 1u);
-            } else if (TMA) {
-              // step j reads 32 bytes of K: span j / 4 of the stage (16 KiB each), 32-byte offset j % 4 inside it
-              mma_ss<TF32>(d, make_desc_sw128(a0 + (j >> 2) * (kTileM * 128) + (j & 3) * 32),
-                           make_desc(bk + j * 256, lbo, sbo_b), idesc, first);
             } else {
-              mma_ss<TF32>(d, make_desc(a0 + j * 256, lbo, sbo_a), make_desc(bk + j * 256, lbo, sbo_b), idesc, first);
+              mma_ss<TF32>(d, make_desc(desc, aa), make_desc(desc, bb), idesc, first);
             }
           }
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -809,15 +804,25 @@ extern "C" int cxg_typed_matmul(const void *a, const void *w, void *c, const int
   CXG_REQUIRE(n % 16 == 0 && n >= 16 && n <= 256, CXG_EUNSUPPORTED,
               "cxg_typed_matmul: N = %d must be a multiple of 16 in [16, 256] on the tensor path", n);
   const size_t b_bytes = static_cast<size_t>(n) * k * elem * (x3 ? 2 : 1);
-  // K-block: the whole row when a stage then fits at least `want` times next to W, else halved while it stays a
-  // multiple of one instruction's K (32 bytes)
   auto stage_bytes = [&](int kb) { return static_cast<size_t>(kTileM) * kb * elem * (x3 ? 2 : 1); };
-  int kb = k;
+  // Span of the swizzle: 128 bytes, unless the row is not a multiple of it or two stages of one span do not fit next to W;
+  // then 64, then 32 (which every row here is a multiple of, and which takes what one stage of 32 bytes leaves room for).
+  // The span's alignment comes out of the budget for 128 bytes and is small enough to go on top of it below that.
+  int span_log = 3;
+  while (span_log > 1 && ((k * elem) % (16 << span_log) != 0 ||
+                          b_bytes + 2 * stage_bytes((16 << span_log) / elem) + (span_log == 3 ? 1024 : 0) > static_cast<size_t>(kSmemBudget)))
+    --span_log;
+  const size_t pad = 128u << span_log;
+  const size_t room = static_cast<size_t>(kSmemBudget) - (span_log == 3 ? pad : 0);
+  // K-block: the whole row when a stage then fits at least `want` times next to W, else fewer spans that divide it
   // (compensated dense mode: three stages of K-block 32 measured 7 % faster than six of K-block 16)
+  const int spans = k * elem / (16 << span_log);
   const int want = dense ? 3 : (x3 ? 4 : 1);
-  while (b_bytes + want * stage_bytes(kb) > static_cast<size_t>(kSmemBudget) && kb % (4 * epc) == 0) kb /= 2;
+  int parts = 1;
+  while (parts < spans && (spans % parts != 0 || b_bytes + want * stage_bytes(k / parts) > room)) ++parts;
+  const int kb = k / parts;
   const size_t a_bytes = stage_bytes(kb);
-  CXG_REQUIRE(a_bytes + b_bytes <= static_cast<size_t>(kSmemBudget), CXG_ELIMIT,
+  CXG_REQUIRE(a_bytes + b_bytes <= room, CXG_ELIMIT,
               "cxg_typed_matmul: one stage of %zu bytes plus W of %zu bytes exceeds shared memory", a_bytes, b_bytes);
   // Dense mode: the tiles of A are contiguous row blocks, which the bulk tensor copy unit fetches as swizzled boxes of
   // 128 rows x 128 bytes, one to four per K-block (CXG_TMM_NO_TMA keeps the 16-byte copies, for comparison)
@@ -828,14 +833,13 @@ extern "C" int cxg_typed_matmul(const void *a, const void *w, void *c, const int
   // 512 bytes keeps the copy unit busier than the 16-byte copies keep the producers (config 4, per-edge matmul:
   // 3.47 vs 2.07 ms in bf16, 6.95 vs 3.73 ms in TF32).
   const bool ca = src_idx != nullptr && m_valid * 2 <= m;
-  const bool tma = (dense || (!ca && (flags & CXG_TMM_GATHER4))) && (kb * elem) % 128 == 0 && kb * elem <= 512 &&
-                   !(flags & CXG_TMM_NO_TMA) &&
+  const bool tma = (dense || (!ca && (flags & CXG_TMM_GATHER4))) && span_log == 3 &&
+                   kb * elem <= 512 && !(flags & CXG_TMM_NO_TMA) &&
                    m < (1ll << 31) && m_valid < (1ll << 31) - 1 && m_valid > 0 &&
                    encode_a_map(&tmap, a, m_valid, k, elem, dense ? kTileM : 1);
-  const size_t tma_pad = tma ? 1024 : 0;  // the stages start on a 1024-byte boundary
-  int stages = static_cast<int>((kSmemBudget - b_bytes - tma_pad) / a_bytes);
+  int stages = static_cast<int>((room - b_bytes) / a_bytes);
   if (stages > kMaxStages) stages = kMaxStages;
-  const size_t smem = b_bytes + tma_pad + stages * a_bytes;
+  const size_t smem = pad + b_bytes + stages * a_bytes;
   CXG_REQUIRE(reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0 && (k * elem) % 16 == 0 &&
                   (n * elem) % 16 == 0,
               CXG_EINVAL, "cxg_typed_matmul: A, C and their rows must be 16-byte aligned");
@@ -866,6 +870,7 @@ extern "C" int cxg_typed_matmul(const void *a, const void *w, void *c, const int
   t.tmem_all = t.small_off ? 4 * cols : 2 * cols;
   t.stages = stages;
   t.kb = kb;
+  t.span_log = span_log;
   if (cudaMemsetAsync(t.status, 0, 256, st) != cudaSuccess) return check_launch("cxg_typed_matmul: memset");
   const int64_t n_tiles = (m + kTileM - 1) / kTileM;
   // one persistent CTA per SM (its shared-memory ring fills the SM), contiguous tile ranges
