@@ -449,16 +449,56 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
   }
 }
 
-// dW[r][i] = sum of partial[cta][slot][i] over the slots whose relation is r, in (cta, slot) order.
-__global__ void __launch_bounds__(256) wgrad_reduce(const float *partial, const int32_t *slot_rel, float *dw, int n_slots,
-                                                    int num_rel, int64_t kn) {
-  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  const int r = blockIdx.y;
-  if (i >= kn || r >= num_rel) return;
+// dW[r][i] = sum of partial[cta][slot][i] over the slots whose relation is r, in (cta, slot) order. A block first lists the
+// slots of its relation in order (8 slots a thread, a block scan), then adds them up with eight loads in flight. (Walking
+// all 148 * (num_rel + 1) slots with one load after the other was bound by that chain: 65 us for eight relations of
+// 128 x 64, now 5 us.) The small block spreads a small gradient over more SMs.
+constexpr int kRedThreads = 128, kRedPer = 8, kRedChunk = kRedThreads * kRedPer;
+__global__ void __launch_bounds__(kRedThreads) wgrad_reduce(const float *partial, const int32_t *slot_rel, float *dw,
+                                                            int n_slots, int num_rel, int64_t kn) {
+  __shared__ int list[kRedChunk];
+  __shared__ int warp_sum[kRedThreads / 32];
+  const int64_t i = blockIdx.x * static_cast<int64_t>(kRedThreads) + threadIdx.x;
+  const int r = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool in = i < kn;
+  const float *p = partial + (in ? i : 0);
   float s = 0.f;
-  for (int q = 0; q < n_slots; ++q)
-    if (slot_rel[q] == r) s += partial[static_cast<int64_t>(q) * kn + i];
-  dw[static_cast<int64_t>(r) * kn + i] = s;
+  for (int base = 0; base < n_slots; base += kRedChunk) {
+    const int q0 = base + static_cast<int>(threadIdx.x) * kRedPer;
+    uint32_t hit = 0;
+#pragma unroll
+    for (int u = 0; u < kRedPer; ++u)
+      if (q0 + u < n_slots && slot_rel[q0 + u] == r) hit |= 1u << u;
+    const int own = __popc(hit);
+    int at = own;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, at, d);
+      if (lane >= d) at += o;
+    }
+    if (lane == 31) warp_sum[warp] = at;
+    __syncthreads();
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < kRedThreads / 32; ++w) {
+      if (w == warp) at += total;
+      total += warp_sum[w];
+    }
+    at -= own;
+    for (; hit != 0; hit &= hit - 1) list[at++] = q0 + __ffs(hit) - 1;
+    __syncthreads();
+    int q = 0;
+    for (; q + 8 <= total; q += 8) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = p[list[q + u] * kn];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += v[u];
+    }
+    for (; q < total; ++q) s += p[list[q] * kn];
+    __syncthreads();  // the list is free for the next chunk
+  }
+  if (in) dw[static_cast<int64_t>(r) * kn + i] = s;
 }
 
 __global__ void wgrad_clear(int32_t *slot_rel, int n) {
@@ -569,8 +609,8 @@ extern "C" int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel,
     launch(typed_wgrad_tc<__nv_bfloat16, false>, kW);
   }
   if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_typed_wgrad: %s", cudaGetErrorString(e));
-  dim3 rg(static_cast<unsigned>((kn + 255) / 256), static_cast<unsigned>(num_rel));
-  wgrad_reduce<<<rg, 256, 0, st>>>(a.partial, a.slot_rel, dw, n_slots, num_rel, kn);
+  dim3 rg(static_cast<unsigned>((kn + kRedThreads - 1) / kRedThreads), static_cast<unsigned>(num_rel));
+  wgrad_reduce<<<rg, kRedThreads, 0, st>>>(a.partial, a.slot_rel, dw, n_slots, num_rel, kn);
   count_launches(3);
   return check_launch("cxg_typed_wgrad");
 }
