@@ -85,7 +85,7 @@ struct TmmArgs {
   int atomic;  // add the rows into a float32 C with vector reductions instead of storing them
   int tmem_cols;  // columns of ONE accumulator buffer (two are allocated)
   int tmem_all;   // columns allocated
-  int small_off;  // compensated mode: columns from an accumulator to that of its small terms, 0 = the same one
+  int small_off;  // compensated mode: columns from an accumulator to that of its small terms (n), 0 = the same one
   int stages;     // shared-memory stages of A
   int span_log;   // log2 of the 16-byte chunks in a swizzle span: 3, 2, 1 for spans of 128, 64, 32 bytes
   int kb;         // K-block: columns of A per pipeline unit (= k unless the stage would not fit several times), whole spans
@@ -304,12 +304,12 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
   const int nkb = a.k / a.kb;               // K-blocks per tile
   const int sl = TMA ? 3 : a.span_log;
   const uint32_t span_a = kTileM << (sl + 4);  // bytes of a span of a tile of A, and of W
-  const uint32_t span_w = a.n << (sl + 4);
+  const uint32_t span_w = (X3 ? 2 * a.n : a.n) << (sl + 4);  // compensated mode: n rows of W hi, then n rows of W lo
   const int S = a.stages;
   const size_t half_bytes = static_cast<size_t>(kTileM) * a.kb * sizeof(T);  // one [128][kb] tile
   const size_t a_bytes = X3 ? 2 * half_bytes : half_bytes;                   // a stage: raw / hi (+ lo)
   const size_t w_bytes = static_cast<size_t>(a.n) * a.k * sizeof(T);        // n rows of W[rel]^T
-  // W (hi), then W lo in the compensated mode; spans start on multiples of eight of their rows
+  // W (hi and lo in the compensated mode); spans start on multiples of eight of their rows
   const uint32_t align = 128u << sl;
   uint8_t *smem_b = smem + ((align - smem_addr(smem)) & (align - 1));
   uint8_t *smem_a = smem_b + (X3 ? 2 * w_bytes : w_bytes);   // S stages
@@ -389,10 +389,9 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
         const uint32_t b0 = smem_addr(smem_b);
         for (int part = 0; part < (X3 ? 2 : 1); ++part) {  // hi, then lo
           const T *wr = Wt + (part * static_cast<int64_t>(a.num_rel) + r) * w_elems;
-          const uint32_t bp = b0 + part * static_cast<uint32_t>(w_bytes);
           for (int row = pw * kRpi + rsub; row < a.n; row += kProdWarps * kRpi)
             for (int c = cq; c < chunks; c += kCpi)
-              cp_async16<false>(bp + swizzled(row, c, sl, span_w), wr + static_cast<int64_t>(row) * a.k + c * EPC, 16);
+              cp_async16<false>(b0 + swizzled(part * a.n + row, c, sl, span_w), wr + static_cast<int64_t>(row) * a.k + c * EPC, 16);
         }
         loaded_rel = r;
       }
@@ -492,6 +491,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
     if (lane == 0) {
       const uint32_t idesc = make_idesc(TF32 ? 2 : 1, kTileM, a.n);
       const uint32_t b0 = smem_addr(smem_b);
+      const uint32_t idesc_wide = make_idesc(2, kTileM, a.small_off ? 2 * a.n : a.n);
       const uint64_t desc = desc_base(sl);
       const int steps = chunks_blk / 2;  // two chunks (32 bytes) of K per instruction
       int64_t it = 0, tile_it = 0;
@@ -522,11 +522,16 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
             const uint32_t bb = b0 + (g >> (sl - 1)) * span_w + (g & in) * 32;
             if (X3) {
               const uint64_t da_hi = make_desc(desc, aa), da_lo = make_desc(desc, aa + static_cast<uint32_t>(half_bytes));
-              const uint64_t db_hi = make_desc(desc, bb), db_lo = make_desc(desc, bb + static_cast<uint32_t>(w_bytes));
-              // the two small terms into an accumulator of their own where there is room for it
-              mma_ss<TF32>(d + a.small_off, da_hi, db_lo, idesc, first);
-              mma_ss<TF32>(d + a.small_off, da_lo, db_hi, idesc, 1u);
-              mma_ss<TF32>(d, da_hi, db_hi, idesc, a.small_off ? first : 1u);
+              const uint64_t db_hi = make_desc(desc, bb);
+              if (a.small_off) {
+                // the small terms into an accumulator of their own, behind the large one: hi x [hi | lo] is one instruction
+                mma_ss<TF32>(d, da_hi, db_hi, idesc_wide, first);
+                mma_ss<TF32>(d + a.small_off, da_lo, db_hi, idesc, 1u);
+              } else {
+                mma_ss<TF32>(d, da_hi, make_desc(desc, bb + (a.n << (sl + 4))), idesc, first);
+                mma_ss<TF32>(d, da_lo, db_hi, idesc, 1u);
+                mma_ss<TF32>(d, da_hi, db_hi, idesc, 1u);
+              }
             } else {
               mma_ss<TF32>(d, make_desc(desc, aa), make_desc(desc, bb), idesc, first);
             }
@@ -862,12 +867,12 @@ extern "C" int cxg_typed_matmul(const void *a, const void *w, void *c, const int
   t.wt = wt;
   int cols = 32;
   while (cols < n) cols <<= 1;
-  t.tmem_cols = cols;  // two buffers: 2 * cols <= 512
   // The tensor core cuts its sum at every instruction, so the error grows with the number of instructions that add to an
   // accumulator: with the small terms in one of their own, a third as many add to the large one (K = 128: 1.0e-6 of the
   // result with one accumulator, 0.35e-6 with two).
-  t.small_off = x3 && 4 * cols <= 512 ? 2 * cols : 0;
-  t.tmem_all = t.small_off ? 4 * cols : 2 * cols;
+  t.small_off = x3 && 4 * cols <= 512 ? n : 0;
+  t.tmem_cols = t.small_off ? 2 * cols : cols;  // two buffers: at most 512 together
+  t.tmem_all = 2 * t.tmem_cols;
   t.stages = stages;
   t.kb = kb;
   t.span_log = span_log;
