@@ -49,9 +49,8 @@
 // Every wait is bounded: a role that waits longer than about a second raises a CTA-wide abort
 // flag and an error status; all roles then leave their loops, the copies in flight are waited
 // for, the tensor memory is released and the kernel returns.
-#include <cuda.h>  // CUtensorMap and its enums; the encoder is obtained through the runtime, nothing links libcuda
-
 #include "common.cuh"
+#include "tensor_core.cuh"
 
 namespace cxg {
 
@@ -60,6 +59,8 @@ int typed_rows_launch(const void *a, const void *w, void *out, const void *rel, 
                       int out_follows_src, cudaStream_t st);
 
 namespace {
+
+using namespace tc;
 
 constexpr int kTileM = 128;
 constexpr int kEpiWarps = 4;
@@ -96,39 +97,6 @@ struct TmmArgs {
   int32_t *status;  // [0] error flag
 };
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-// Shared-memory matrix descriptors, K-major with a swizzle: a tile is cut along K into spans of 128, 64 or 32 bytes; a
-// span holds its rows one behind the other, 8-row groups 8 * span bytes apart, and permutes the 16-byte chunks of a row by
-// the row number, so that the tensor core reads 8 rows without bank conflicts. A span starts on a multiple of 8 * span
-// bytes; K advances inside it by adding 32 bytes to the address. (As core matrices of 8 rows x 16 bytes without a swizzle,
-// which is how the copies wrote A and W before, an instruction took some 230 cycles and the tensor core bounded the kernel:
-// fp32, 2.33 M gathered rows, K = 128, N = 64 took 837 us, 564 us now; K = 64, N = 128: 495 us, now 364.)
-// What is constant in a descriptor:
-__device__ __forceinline__ uint64_t desc_base(int span_log) {
-  uint64_t d = 0;
-  d |= 1ull << 16;                                                  // leading offset: unused with a swizzle, canonical value 1
-  d |= static_cast<uint64_t>((128u << span_log) >> 4) << 32;        // next 8-row group
-  d |= 1ull << 46;                                                  // descriptor version of sm_100
-  d |= static_cast<uint64_t>(span_log == 3 ? 2 : span_log == 2 ? 4 : 6) << 61;  // 128-, 64- or 32-byte swizzle
-  return d;
-}
-__device__ __forceinline__ uint64_t make_desc(uint64_t base, uint32_t addr) { return base | ((addr >> 4) & 0x3fff); }
-// byte offset of 16-byte chunk c of a row inside a tile whose spans are span_bytes apart
-__device__ __forceinline__ uint32_t swizzled(int row, int c, int span_log, uint32_t span_bytes) {
-  const uint32_t in = (c ^ (row >> (3 - span_log))) & ((1 << span_log) - 1);
-  return (c >> span_log) * span_bytes + (static_cast<uint32_t>(row) << (span_log + 4)) + (in << 4);
-}
-
-// One tiled 2-D bulk tensor copy global -> shared (x = element column, y = row of the tensor map's matrix); its bytes
-// are counted on `bar`. x * element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
-
 // Four rows of the tensor map's matrix (any four: y0 .. y3), columns [x, x + box width), into 4 x 128 consecutive
 // bytes of shared memory (tile::gather4; the map's box is one row high). Rows outside the matrix arrive as zeros.
 __device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap *map, int x, int y0, int y1, int y2, int y3,
@@ -138,43 +106,6 @@ __device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap *map
       "%6, %7}], [%2];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y0), "r"(y1), "r"(y2), "r"(y3)
       : "memory");
-}
-
-// Instruction descriptor: fp32 accumulate, A and B of format `fmt` (1 = bf16, 2 = tf32), both K-major.
-__device__ __forceinline__ uint32_t make_idesc(int fmt, int m, int n) {
-  uint32_t d = 0;
-  d |= 1u << 4;                                 // D format: f32
-  d |= static_cast<uint32_t>(fmt) << 7;         // A format
-  d |= static_cast<uint32_t>(fmt) << 10;        // B format
-  d |= static_cast<uint32_t>(n >> 3) << 17;     // N / 8
-  d |= static_cast<uint32_t>(m >> 4) << 24;     // M / 16
-  return d;
-}
-
-template <bool TF32>
-__device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  if (TF32)
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-  else
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
 }
 
 __device__ __forceinline__ float to_tf32(float v) {
@@ -222,27 +153,6 @@ struct Barriers {
   uint64_t acc_empty[2];       // epilogue -> MMA (128 arrivals)
 };
 
-// Bounded wait on phase `parity`; false after a time-out here or an abort raised by another role.
-__device__ __forceinline__ bool wait_bar(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int32_t *status,
-                                         long long limit) {
-  const uint32_t b = smem_addr(bar);
-  if (mbar_try_wait(b, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait(b, parity)) {
-    if (*abort_flag) return false;
-    if (clock64() - t0 > limit) {
-      *abort_flag = 1;
-      atomicExch(status, 1);
-      return false;
-    }
-  }
-  return true;
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 // 16-byte asynchronous copy; CA = through L1 (adjacent lanes' chunks merge into one request per line, which
 // is what a gather of re-used rows wants), otherwise L2 only (faster when every row is read once).
 template <bool CA>
@@ -253,24 +163,11 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int by
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-// 16 consecutive 32-bit columns of this warp's 32 accumulator lanes; completion is awaited by the caller
-__device__ __forceinline__ void tmem_ld16(uint32_t *v, uint32_t taddr) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr));
-}
-
 // fp32 words: v += w
 template <int N>
 __device__ __forceinline__ void add_words(uint32_t *v, const uint32_t *w) {
 #pragma unroll
   for (int i = 0; i < N; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(w[i]));
-}
-
-__device__ __forceinline__ void st_global_v4(void *p, uint4 v) {
-  asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
 // PW producer warps; each copies 128 / PW rows of a tile, kSlots of them per thread. X3: error-compensated
@@ -488,69 +385,64 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
     }
   } else if (warp == kMmaWarp) {
     // ================= MMA issuer =================
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(TF32 ? 2 : 1, kTileM, a.n);
-      const uint32_t b0 = smem_addr(smem_b);
-      const uint32_t idesc_wide = make_idesc(2, kTileM, a.small_off ? 2 * a.n : a.n);
-      const uint64_t desc = desc_base(sl);
-      const int steps = chunks_blk / 2;  // two chunks (32 bytes) of K per instruction
-      int64_t it = 0, tile_it = 0;
-      bool alive = true;
-      int64_t r_next = rel_of(tile_lo);
-      for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile) {
-        const int64_t r = r_next;
-        r_next = rel_of(tile + 1);
-        if (r < 0 || r >= a.num_rel) continue;
-        const int buf = static_cast<int>(tile_it & 1);
-        const uint32_t d = tmem_d + buf * a.tmem_cols;
-        for (int kb = 0; kb < nkb && alive; ++kb) {
-          const int s = static_cast<int>(it % S);
-          alive = wait_bar(X3 ? &bars.conv[s] : &bars.full[s], static_cast<uint32_t>((it / S) & 1), abort_flag, a.status,
-                           a.wait_cycles);
-          if (alive && kb == 0 && tile_it >= 2)
-            alive = wait_bar(&bars.acc_empty[buf], static_cast<uint32_t>(((tile_it >> 1) - 1) & 1), abort_flag, a.status,
-                             a.wait_cycles);
-          if (!alive) break;
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a0 = smem_addr(smem_a + s * a_bytes);
-          for (int j = 0; j < steps; ++j) {
-            const uint32_t first = (kb > 0 || j > 0) ? 1u : 0u;
-            // a step reads 32 bytes of K, of which a span holds 4, 2 or 1
-            const int g = kb * steps + j, in = (1 << (sl - 1)) - 1;
-            const uint32_t aa = a0 + (j >> (sl - 1)) * span_a + (j & in) * 32;
-            const uint32_t bb = b0 + (g >> (sl - 1)) * span_w + (g & in) * 32;
-            if (X3) {
-              const uint64_t da_hi = make_desc(desc, aa), da_lo = make_desc(desc, aa + static_cast<uint32_t>(half_bytes));
-              const uint64_t db_hi = make_desc(desc, bb);
-              if (a.small_off) {
-                // the small terms into an accumulator of their own, behind the large one: hi x [hi | lo] is one instruction
-                mma_ss<TF32>(d, da_hi, db_hi, idesc_wide, first);
-                mma_ss<TF32>(d + a.small_off, da_lo, db_hi, idesc, 1u);
-              } else {
-                mma_ss<TF32>(d, da_hi, make_desc(desc, bb + (a.n << (sl + 4))), idesc, first);
-                mma_ss<TF32>(d, da_lo, db_hi, idesc, 1u);
-                mma_ss<TF32>(d, da_hi, db_hi, idesc, 1u);
-              }
-            } else {
-              mma_ss<TF32>(d, make_desc(desc, aa), make_desc(desc, bb), idesc, first);
-            }
-          }
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                           smem_addr(&bars.empty[s]))
-                       : "memory");
-          ++it;
-        }
+    // the whole warp walks the units together; one lane issues (mma_ss)
+    auto wait_all = [&](uint64_t *bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, a.status, a.wait_cycles)) != 0;
+    };
+    const uint32_t idesc = make_idesc(TF32 ? 2 : 1, kTileM, a.n);
+    const uint32_t b0 = smem_addr(smem_b);
+    const uint32_t idesc_wide = make_idesc(2, kTileM, a.small_off ? 2 * a.n : a.n);
+    const uint64_t desc = desc_base(sl);
+    const int steps = chunks_blk / 2;  // two chunks (32 bytes) of K per instruction
+    int64_t it = 0, tile_it = 0;
+    bool alive = true;
+    int64_t r_next = rel_of(tile_lo);
+    for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile) {
+      const int64_t r = r_next;
+      r_next = rel_of(tile + 1);
+      if (r < 0 || r >= a.num_rel) continue;
+      const int buf = static_cast<int>(tile_it & 1);
+      const uint32_t d = tmem_d + buf * a.tmem_cols;
+      for (int kb = 0; kb < nkb && alive; ++kb) {
+        const int s = static_cast<int>(it % S);
+        alive = wait_all(X3 ? &bars.conv[s] : &bars.full[s], static_cast<uint32_t>((it / S) & 1));
+        if (alive && kb == 0 && tile_it >= 2)
+          alive = wait_all(&bars.acc_empty[buf], static_cast<uint32_t>(((tile_it >> 1) - 1) & 1));
         if (!alive) break;
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                         smem_addr(&bars.acc_full[buf]))
-                     : "memory");
-        ++tile_it;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a0 = smem_addr(smem_a + s * a_bytes);
+        for (int j = 0; j < steps; ++j) {
+          const uint32_t first = (kb > 0 || j > 0) ? 1u : 0u;
+          // a step reads 32 bytes of K, of which a span holds 4, 2 or 1
+          const int g = kb * steps + j, in = (1 << (sl - 1)) - 1;
+          const uint32_t aa = a0 + (j >> (sl - 1)) * span_a + (j & in) * 32;
+          const uint32_t bb = b0 + (g >> (sl - 1)) * span_w + (g & in) * 32;
+          if (X3) {
+            const uint64_t da_hi = make_desc(desc, aa), da_lo = make_desc(desc, aa + static_cast<uint32_t>(half_bytes));
+            const uint64_t db_hi = make_desc(desc, bb);
+            if (a.small_off) {
+              // the small terms into an accumulator of their own, behind the large one: hi x [hi | lo] is one instruction
+              mma_ss<TF32>(d, da_hi, db_hi, idesc_wide, first);
+              mma_ss<TF32>(d + a.small_off, da_lo, db_hi, idesc, 1u);
+            } else {
+              mma_ss<TF32>(d, da_hi, make_desc(desc, bb + (a.n << (sl + 4))), idesc, first);
+              mma_ss<TF32>(d, da_lo, db_hi, idesc, 1u);
+              mma_ss<TF32>(d, da_hi, db_hi, idesc, 1u);
+            }
+          } else {
+            mma_ss<TF32>(d, make_desc(desc, aa), make_desc(desc, bb), idesc, first);
+          }
+        }
+        commit_to(&bars.empty[s]);
+        ++it;
       }
-      // the epilogue of the last tiles must be over before the tensor memory goes away: it arrives on
-      // acc_empty, which the final __syncthreads of the epilogue warps also orders.
+      if (!alive) break;
+      commit_to(&bars.acc_full[buf]);
+      ++tile_it;
     }
-    __syncwarp();
+    // the epilogue of the last tiles must be over before the tensor memory goes away: it arrives on
+    // acc_empty, which the final __syncthreads of the epilogue warps also orders.
   } else {
     // ================= epilogue: a warp owns accumulator lanes 32 * (warp % 4) .. + 31 = tile rows =================
     T *C = static_cast<T *>(a.c);
@@ -713,38 +605,6 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
 }  // namespace cxg
 
 using namespace cxg;
-
-namespace {
-
-// Tensor map of a row-major [rows][k] matrix of bf16 or fp32 elements for boxes of 128 rows x one 128-byte swizzle
-// span of columns (64 / 32 elements). False when the driver's encoder is not available or refuses the arguments.
-bool encode_a_map(CUtensorMap *map, const void *base, int64_t rows, int k, int elem, int box_rows) {
-  typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                               const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn fn = nullptr;
-  static bool looked = false;
-  if (!looked) {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeFn>(p);
-    else
-      (void)cudaGetLastError();
-    looked = true;
-  }
-  if (fn == nullptr) return false;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k) * elem};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / elem), static_cast<cuuint32_t>(box_rows)};
-  const cuuint32_t estr[2] = {1, 1};
-  return fn(map, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(base), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-}  // namespace
 
 extern "C" int cxg_typed_matmul_workspace_size(int num_rel, int k, int n, int dtype, size_t *bytes) {
   CXG_REQUIRE(bytes != nullptr, CXG_ENULL, "cxg_typed_matmul_workspace_size: bytes is NULL");

@@ -34,6 +34,9 @@ constexpr int kFirstProd = kMmaWarp + 1;
 constexpr int kFirstConv = kFirstProd + kProdWarps;
 constexpr int kMaxStages = 4;
 constexpr int kSmemBudget = 225 * 1024;
+// Positions per tile of the compensated mode: a stage of 128 + 128 columns takes 64 KB, so three of them are in flight (with
+// 64 positions it was one, and loading, splitting and multiplying took turns: 169,343 x 128 x 128 146 us, now 91).
+constexpr int kPosX3 = 32;
 
 struct WgArgs {
   const void *x;       // [*, k]
@@ -44,9 +47,10 @@ struct WgArgs {
   int64_t m, x_rows, g_rows;  // positions; rows with an index in [0, x_rows) / [0, g_rows) exist, others count as zero rows
   int k, n, num_rel;
   int stages, slots;
+  int dense;           // 0, or the column blocks of x: the whole matrices, one relation, a column block pair per blockIdx.y
   int chunk_tiles;     // tiles summed in one tensor-memory accumulator before the epilogue takes it over
   int test_stall;      // test hook: the producers never hand over their first tile, so the waits for it run out
-  float *partial;      // [grid][slots][k][n]
+  float *partial;      // [grid][slots][k][n]; dense: [column block pair][blockIdx.x][128][128]
   int32_t *slot_rel;   // [grid][slots]: relation of a flushed slot, -1 when unused
   int32_t *status;
   long long wait_cycles;
@@ -90,19 +94,22 @@ __device__ __forceinline__ uint32_t make_idesc_mn(int fmt, int m, int n) {
   return d;
 }
 
+// One MMA of a warp: every lane comes here with the same operands and one of them issues it. (Behind `if (lane == 0)` the
+// compiler cannot tell that the operands are the same in all active lanes and an instruction took 134 cycles whatever its
+// size; issued this way 73, and 135 for 128 x 256, which is the tensor core's own time.)
 template <bool TF32>
 __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   if (TF32)
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
         : "memory");
   else
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 
@@ -137,7 +144,10 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 }
 
 __device__ __forceinline__ void commit_to(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_addr(bar))
+      : "memory");
 }
 
 // v = hi + lo up to half a unit of lo's 19 bits (see typed_mm.cu)
@@ -159,7 +169,7 @@ struct Barriers {
 template <typename T, bool X3>
 __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConvWarps : 0)), 1) typed_wgrad_tc(WgArgs a) {
   constexpr bool TF32 = sizeof(T) == 4;
-  constexpr int kPos = X3 ? 64 : 128;
+  constexpr int kPos = X3 ? kPosX3 : 128;
   constexpr int kSpan = 128 * kPos;  // bytes of one 128-byte span of a tile (kPos rows)
   constexpr int kInstrK = TF32 ? 8 : 16;  // positions per MMA
   extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -170,7 +180,10 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // spans that hold the rows of x and of g. The tensor core reads 128 columns of x: those behind K lie in the memory
   // behind (g's spans, the next stage) and only reach rows of the result that are not stored.
-  const int xrow = a.k * static_cast<int>(sizeof(T)), grow = a.n * static_cast<int>(sizeof(T));
+  const int x_at = a.dense ? static_cast<int>(blockIdx.y % a.dense) * 128 : 0;  // first column of the block
+  const int g_at = a.dense ? static_cast<int>(blockIdx.y / a.dense) * 128 : 0;
+  const int k = a.dense ? min(128, a.k - x_at) : a.k, n = a.dense ? min(128, a.n - g_at) : a.n;
+  const int xrow = k * static_cast<int>(sizeof(T)), grow = n * static_cast<int>(sizeof(T));
   const int spans_x = (xrow + 127) / 128, spans_g = (grow + 127) / 128;
   const int n_mma = spans_g * (128 / static_cast<int>(sizeof(T)));  // whole spans; columns behind N are zeros
   const uint32_t half_bytes = static_cast<uint32_t>(spans_x + spans_g) * kSpan;  // raw (or hi) tiles of x and g
@@ -180,8 +193,9 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
   int tmem_cols = 32;
   while (tmem_cols < n_mma) tmem_cols <<= 1;
   // compensated mode: the small terms have an accumulator of their own where there is room (see typed_mm.cu)
-  const uint32_t small_off = X3 && 4 * tmem_cols <= 512 ? 2 * tmem_cols : 0;
-  const uint32_t tmem_all = small_off ? 4 * tmem_cols : 2 * tmem_cols;
+  const uint32_t small_off = X3 && 4 * tmem_cols <= 512 ? n_mma : 0;
+  if (small_off) tmem_cols *= 2;  // columns of one of the two buffers
+  const uint32_t tmem_all = 2 * tmem_cols;
 
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_slot)),
@@ -209,7 +223,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
 
   const int64_t n_tiles = (a.m + kPos - 1) / kPos;
   const int64_t tile_lo = n_tiles * blockIdx.x / gridDim.x, tile_hi = n_tiles * (blockIdx.x + 1) / gridDim.x;
-  auto rel_of = [&](int64_t tile) -> int64_t { return tile < tile_hi ? a.rel[tile * kPos] : -1; };
+  auto rel_of = [&](int64_t tile) -> int64_t { return tile < tile_hi ? (a.dense ? 0 : a.rel[tile * kPos]) : -1; };
   auto valid_rel = [&](int64_t r) { return r >= 0 && r < a.num_rel; };
 
   if (warp >= kFirstProd && warp < kFirstConv) {
@@ -217,7 +231,8 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     const int pt = tid - 32 * kFirstProd;  // 0 .. 255
     const int c16 = pt & 7;                // 16-byte chunk inside a 128-byte span
     const int prow = pt >> 3;              // row inside a pass of 32 rows
-    const uint8_t *X = static_cast<const uint8_t *>(a.x), *G = static_cast<const uint8_t *>(a.g);
+    const uint8_t *X = static_cast<const uint8_t *>(a.x) + x_at * sizeof(T), *G = static_cast<const uint8_t *>(a.g) + g_at * sizeof(T);
+    const int64_t xpitch = a.k * static_cast<int64_t>(sizeof(T)), gpitch = a.n * static_cast<int64_t>(sizeof(T));
     constexpr int kPass = kPos / 32;  // passes of 32 rows per tile
     auto fetch = [&](int64_t tile, int64_t (&ia)[kPass], int64_t (&ig)[kPass]) {
 #pragma unroll
@@ -253,8 +268,8 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
         const bool ok = ia[q] >= 0 && ia[q] < a.x_rows && ig[q] >= 0 && ig[q] < a.g_rows;
         const int bytes = ok ? 16 : 0;
         const uint32_t d0 = st0 + swizzled_offset<TF32>(p, c16);
-        const uint8_t *xs = ok ? X + ia[q] * xrow : X;
-        const uint8_t *gs = ok ? G + ig[q] * grow : G;
+        const uint8_t *xs = ok ? X + ia[q] * xpitch : X;
+        const uint8_t *gs = ok ? G + ig[q] * gpitch : G;
         // a chunk behind the row's end is written as zeros from the row's first chunk
         auto copy = [&](const uint8_t *src, int row_bytes, int j, uint32_t dst) {
           const int at = j * 128 + c16 * 16;
@@ -273,7 +288,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
   } else if (X3 && warp >= kFirstConv) {
     // ================= converters: raw fp32 tiles -> hi (in place) and lo (second half of the stage) =================
     const int ct = tid - 32 * kFirstConv;
-    const int n16 = static_cast<int>(half_bytes / 16);
+    const int n16 = static_cast<int>(half_bytes / 16), x16 = spans_x * (kSpan / 16), g16 = n16 - x16;
     int64_t it = 0;
     bool alive = true;
     for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile) {
@@ -282,6 +297,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
       alive = wait_bar(&bars.full[s], static_cast<uint32_t>((it / S) & 1), abort_flag, a.status, a.wait_cycles);
       if (!alive) break;
       float4 *hi = reinterpret_cast<float4 *>(smem + static_cast<size_t>(s) * stage_bytes);
+      // the second half holds g's lo spans first, so that they follow g's hi spans, then those of x
       float4 *lo = reinterpret_cast<float4 *>(smem + static_cast<size_t>(s) * stage_bytes + half_bytes);
       constexpr int kStep = 32 * kConvWarps;
       for (int c0 = ct; c0 < n16; c0 += 4 * kStep) {  // four chunks requested at once
@@ -297,8 +313,9 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
             split_tf32(v[u].y, h.y, l.y);
             split_tf32(v[u].z, h.z, l.z);
             split_tf32(v[u].w, h.w, l.w);
-            hi[c0 + u * kStep] = h;
-            lo[c0 + u * kStep] = l;
+            const int c = c0 + u * kStep;
+            hi[c] = h;
+            lo[c < x16 ? g16 + c : c - x16] = l;
           }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -310,62 +327,68 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     // The tensor core's fp32 accumulation loses a little on every addition (the error grows linearly with the number
     // of positions summed in one accumulator), so an accumulator takes at most `chunk_tiles` tiles; the epilogue adds
     // the chunks of a relation with ordinary fp32 additions. Two accumulator buffers alternate.
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc_mn(TF32 ? 2 : 1, 128, n_mma);
-      const uint32_t step_bytes = kInstrK * 128;  // the next kInstrK positions of a span
-      int64_t it = 0, chunk = 0;
-      int in_chunk = 0;
-      bool alive = true, open = false;  // open: the current accumulator holds tiles of relation `cur`
-      int64_t cur = -1;
-      for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile) {
-        const int64_t r = rel_of(tile);
-        if (!valid_rel(r)) continue;
-        if (open && (r != cur || in_chunk == a.chunk_tiles)) {  // hand the chunk to the epilogue
-          commit_to(&bars.acc_full[chunk & 1]);
-          open = false;
-          ++chunk;
-        }
-        const int buf = static_cast<int>(chunk & 1);
-        if (!open) {
-          if (chunk >= 2) {  // the epilogue has read the chunk that used this buffer before
-            alive = wait_bar(&bars.acc_empty[buf], static_cast<uint32_t>(((chunk >> 1) - 1) & 1), abort_flag, a.status,
-                             a.wait_cycles);
-            if (!alive) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          }
-          cur = r;
-          in_chunk = 0;
-        }
-        const uint32_t d = tmem_d + buf * tmem_cols;
-        const int s = static_cast<int>(it % S);
-        alive = wait_bar(X3 ? &bars.conv[s] : &bars.full[s], static_cast<uint32_t>((it / S) & 1), abort_flag, a.status,
-                         a.wait_cycles);
-        if (!alive) break;
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t x0 = smem_addr(smem + static_cast<size_t>(s) * stage_bytes);
-        const uint32_t g0 = x0 + spans_x * kSpan;
-        for (int j = 0; j < kPos / kInstrK; ++j) {
-          const uint32_t first = (open || j > 0) ? 1u : 0u;
-          const uint32_t off = j * step_bytes;
-          if (X3) {
-            const uint64_t xa = make_desc_mn_sw128<TF32>(x0 + off, kSpan), xl = make_desc_mn_sw128<TF32>(x0 + half_bytes + off, kSpan);
-            const uint64_t ga = make_desc_mn_sw128<TF32>(g0 + off, kSpan), gl = make_desc_mn_sw128<TF32>(g0 + half_bytes + off, kSpan);
-            mma_ss<TF32>(d + small_off, xa, gl, idesc, first);
-            mma_ss<TF32>(d + small_off, xl, ga, idesc, 1u);
-            mma_ss<TF32>(d, xa, ga, idesc, small_off ? first : 1u);
-          } else {
-            mma_ss<TF32>(d, make_desc_mn_sw128<TF32>(x0 + off, kSpan), make_desc_mn_sw128<TF32>(g0 + off, kSpan), idesc, first);
-          }
-        }
-        commit_to(&bars.empty[s]);
-        open = true;
-        ++in_chunk;
-        ++it;
+    // the whole warp walks the tiles together; one lane issues (mma_ss)
+    auto wait_all = [&](uint64_t *bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, a.status, a.wait_cycles)) != 0;
+    };
+    const uint32_t idesc = make_idesc_mn(TF32 ? 2 : 1, 128, n_mma);
+    const uint32_t idesc_wide = make_idesc_mn(2, 128, small_off ? 2 * n_mma : n_mma);
+    const uint32_t step_bytes = kInstrK * 128;  // the next kInstrK positions of a span
+    int64_t it = 0, chunk = 0;
+    int in_chunk = 0;
+    bool alive = true, open = false;  // open: the current accumulator holds tiles of relation `cur`
+    int64_t cur = -1;
+    for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile) {
+      const int64_t r = rel_of(tile);
+      if (!valid_rel(r)) continue;
+      if (open && (r != cur || in_chunk == a.chunk_tiles)) {  // hand the chunk to the epilogue
+        commit_to(&bars.acc_full[chunk & 1]);
+        open = false;
+        ++chunk;
       }
-      if (alive && open) commit_to(&bars.acc_full[chunk & 1]);
+      const int buf = static_cast<int>(chunk & 1);
+      if (!open) {
+        if (chunk >= 2) {  // the epilogue has read the chunk that used this buffer before
+          alive = wait_all(&bars.acc_empty[buf], static_cast<uint32_t>(((chunk >> 1) - 1) & 1));
+          if (!alive) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
+        cur = r;
+        in_chunk = 0;
+      }
+      const uint32_t d = tmem_d + buf * tmem_cols;
+      const int s = static_cast<int>(it % S);
+      alive = wait_all(X3 ? &bars.conv[s] : &bars.full[s], static_cast<uint32_t>((it / S) & 1));
+      if (!alive) break;
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t x0 = smem_addr(smem + static_cast<size_t>(s) * stage_bytes);
+      const uint32_t g0 = x0 + spans_x * kSpan;
+      for (int j = 0; j < kPos / kInstrK; ++j) {
+        const uint32_t first = (open || j > 0) ? 1u : 0u;
+        const uint32_t off = j * step_bytes;
+        if (X3) {
+          const uint64_t xa = make_desc_mn_sw128<TF32>(x0 + off, kSpan);
+          const uint64_t xl = make_desc_mn_sw128<TF32>(x0 + half_bytes + spans_g * kSpan + off, kSpan);
+          const uint64_t ga = make_desc_mn_sw128<TF32>(g0 + off, kSpan);
+          if (small_off) {  // hi x [hi | lo] in one instruction
+            mma_ss<TF32>(d, xa, ga, idesc_wide, first);
+            mma_ss<TF32>(d + small_off, xl, ga, idesc, 1u);
+          } else {
+            mma_ss<TF32>(d, xa, make_desc_mn_sw128<TF32>(x0 + half_bytes + off, kSpan), idesc, first);
+            mma_ss<TF32>(d, xl, ga, idesc, 1u);
+            mma_ss<TF32>(d, xa, ga, idesc, 1u);
+          }
+        } else {
+          mma_ss<TF32>(d, make_desc_mn_sw128<TF32>(x0 + off, kSpan), make_desc_mn_sw128<TF32>(g0 + off, kSpan), idesc, first);
+        }
+      }
+      commit_to(&bars.empty[s]);
+      open = true;
+      ++in_chunk;
+      ++it;
     }
-    __syncwarp();
+    if (alive && open) commit_to(&bars.acc_full[chunk & 1]);
   } else if (warp < kEpiWarps) {
     // ================= epilogue: add every chunk's accumulator into the relation segment's slot of this CTA =================
     // the chunks and segments are found by walking the same tile range as the MMA thread
@@ -378,9 +401,10 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
       alive = wait_bar(&bars.acc_full[buf], static_cast<uint32_t>((chunk >> 1) & 1), abort_flag, a.status, a.wait_cycles);
       if (!alive) return;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      float *out = a.partial + ((static_cast<int64_t>(blockIdx.x) * a.slots + seg) * a.k + row) * a.n;
+      float *out = a.dense ? a.partial + ((static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x) * 128 + row) * 128
+                           : a.partial + ((static_cast<int64_t>(blockIdx.x) * a.slots + seg) * a.k + row) * a.n;
       const uint32_t taddr = tmem_d + (static_cast<uint32_t>(warp * 32) << 16) + buf * tmem_cols;
-      for (int c0 = 0; c0 < a.n; c0 += 16) {
+      for (int c0 = 0; c0 < n; c0 += 16) {
         uint32_t v[16];
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -400,7 +424,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
         } else {
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         }
-        if (row < a.k) {
+        if (row < k) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             float4 acc = make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]), __uint_as_float(v[4 * q + 2]),
@@ -414,7 +438,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
           }
         }
       }
-      if (tid == 0 && !seg_started) a.slot_rel[static_cast<int64_t>(blockIdx.x) * a.slots + seg] = static_cast<int32_t>(cur);
+      if (tid == 0 && !seg_started && !a.dense) a.slot_rel[static_cast<int64_t>(blockIdx.x) * a.slots + seg] = static_cast<int32_t>(cur);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(&bars.acc_empty[buf]);
       seg_started = true;
@@ -506,6 +530,35 @@ __global__ void wgrad_clear(int32_t *slot_rel, int n) {
   if (i < n) slot_rel[i] = -1;
 }
 
+// Dense mode: dW[i][j] = sum of the partials of its column block pair over the blocks, in order, eight loads in flight.
+__global__ void __launch_bounds__(128) dense_reduce(const float *partial, float *dw, int k, int n, int k_blocks, int parts) {
+  const int64_t i = blockIdx.x * 128ll + threadIdx.x;
+  if (i >= static_cast<int64_t>(k) * n) return;
+  const int r = static_cast<int>(i / n), c = static_cast<int>(i % n);
+  const int64_t pair = r / 128 + static_cast<int64_t>(k_blocks) * (c / 128);
+  const float *p = partial + ((pair * parts) * 128 + r % 128) * 128 + c % 128;
+  float s = 0.f;
+  int q = 0;
+  for (; q + 8 <= parts; q += 8) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = p[static_cast<int64_t>(q + u) * (128 * 128)];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += v[u];
+  }
+  for (; q < parts; ++q) s += p[static_cast<int64_t>(q) * (128 * 128)];
+  dw[i] = s;
+}
+
+__device__ int32_t dense_status;  // set when a bounded wait of the dense mode ran out
+
+// Blocks of positions of the dense mode: one block per SM over all column block pairs.
+int dense_parts(int k, int n, int64_t m) {
+  const int64_t pairs = static_cast<int64_t>((k + 127) / 128) * ((n + 127) / 128);
+  const int64_t tiles = (m + kPosX3 - 1) / kPosX3, parts = pairs < kNumSM ? kNumSM / pairs : 1;
+  return static_cast<int>(parts < tiles ? parts : tiles);
+}
+
 struct WgLayout {
   size_t status, slot_rel, partial, total;
   int grid, slots;
@@ -567,7 +620,7 @@ extern "C" int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel,
               "cxg_typed_wgrad: workspace %zu bytes, need %zu", workspace_bytes, L.total);
   CXG_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 16 == 0, CXG_EINVAL, "cxg_typed_wgrad: workspace alignment");
   const bool x3 = precision == 2 && dtype == CXG_F32;
-  const int pos = x3 ? 64 : 128;  // positions per tile, as in the kernel
+  const int pos = x3 ? kPosX3 : 128;  // positions per tile, as in the kernel
   const int spans = (k * elem + 127) / 128 + (n * elem + 127) / 128;
   const size_t half = static_cast<size_t>(spans) * (128 * pos);
   const size_t stage = x3 ? 2 * half : half;
@@ -583,7 +636,8 @@ extern "C" int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel,
   a.x = x, a.g = g, a.rel = rel, a.idx = idx, a.idx_g = idx_g, a.m = m, a.x_rows = x_rows, a.g_rows = g_rows;
   a.k = k, a.n = n, a.num_rel = num_rel, a.stages = stages, a.slots = L.slots;
   a.test_stall = (flags & CXG_WGRAD_TEST_STALL) ? 1 : 0;
-  a.chunk_tiles = x3 ? 4 : 32;  // 256 / 4096 positions per accumulator: its error stays below that of an fp32 sum / below
+  a.dense = 0;
+  a.chunk_tiles = x3 ? 256 / kPosX3 : 32;  // 256 / 4096 positions per accumulator: its error stays below that of an fp32 sum / below
                                 // the rounding of the plain products
   a.partial = reinterpret_cast<float *>(ws + L.partial);
   a.slot_rel = reinterpret_cast<int32_t *>(ws + L.slot_rel);
@@ -613,6 +667,66 @@ extern "C" int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel,
   wgrad_reduce<<<rg, kRedThreads, 0, st>>>(a.partial, a.slot_rel, dw, n_slots, num_rel, kn);
   count_launches(3);
   return check_launch("cxg_typed_wgrad");
+}
+
+extern "C" int cxg_dense_wgrad_f32_workspace_size(int64_t m, int k, int n, size_t *bytes) {
+  CXG_REQUIRE(bytes != nullptr, CXG_ENULL, "cxg_dense_wgrad_f32_workspace_size: bytes is NULL");
+  CXG_REQUIRE(m > 0 && k > 0 && n > 0, CXG_EINVAL, "cxg_dense_wgrad_f32_workspace_size: bad sizes");
+  *bytes = static_cast<size_t>((k + 127) / 128) * ((n + 127) / 128) * dense_parts(k, n, m) * (128 * 128 * sizeof(float));
+  return CXG_OK;
+}
+
+extern "C" int cxg_dense_wgrad_f32(const float *x, const float *g, int64_t m, int k, int n, float *dw, void *workspace,
+                                   size_t workspace_bytes, void *stream) {
+  CXG_REQUIRE(m > 0 && k > 0 && n > 0, CXG_EINVAL, "cxg_dense_wgrad_f32: bad sizes");
+  CXG_REQUIRE(x && g && dw, CXG_ENULL, "cxg_dense_wgrad_f32: NULL argument");
+  const int k_blocks = (k + 127) / 128, n_blocks = (n + 127) / 128;
+  CXG_REQUIRE(k % 4 == 0 && n % 4 == 0 && k_blocks * n_blocks <= 65535, CXG_EUNSUPPORTED,
+              "cxg_dense_wgrad_f32: K = %d and N = %d must be multiples of 4", k, n);
+  CXG_REQUIRE((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g)) % 16 == 0, CXG_EINVAL,
+              "cxg_dense_wgrad_f32: x and g must be 16-byte aligned");
+  size_t need = 0;
+  cxg_dense_wgrad_f32_workspace_size(m, k, n, &need);
+  CXG_REQUIRE(workspace != nullptr && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 16 == 0,
+              CXG_EWORKSPACE, "cxg_dense_wgrad_f32: workspace %zu bytes, need %zu", workspace_bytes, need);
+  cudaStream_t st = as_stream(stream);
+  const int wk = k < 128 ? k : 128, wn = n < 128 ? n : 128;  // the widest column blocks
+  const int spans = (wk + 31) / 32 + (wn + 31) / 32;
+  const size_t stage = 2 * static_cast<size_t>(spans) * (128 * kPosX3);
+  // the tensor core reads four spans of x from a tile's start (last block of columns included)
+  const size_t behind = 4 * static_cast<size_t>(128 * kPosX3);
+  int stages = static_cast<int>((kSmemBudget - 1024 - behind) / stage);
+  if (stages > kMaxStages) stages = kMaxStages;
+  WgArgs a;
+  a.x = x, a.g = g, a.rel = nullptr, a.idx = nullptr, a.idx_g = nullptr, a.m = m, a.x_rows = m, a.g_rows = m;
+  a.k = k, a.n = n, a.num_rel = 1, a.stages = stages, a.slots = 1, a.test_stall = 0, a.dense = k_blocks;
+  a.chunk_tiles = 256 / kPosX3;
+  a.partial = static_cast<float *>(workspace);
+  a.slot_rel = nullptr;
+  a.wait_cycles = wait_limit_cycles();
+  void *word = nullptr;
+  cudaError_t e = cudaGetSymbolAddress(&word, dense_status);
+  a.status = static_cast<int32_t *>(word);
+  const int smem = static_cast<int>(1024 + stages * stage + behind);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(typed_wgrad_tc<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_dense_wgrad_f32: %s", cudaGetErrorString(e));
+  const int parts = dense_parts(k, n, m);
+  const dim3 grid(static_cast<unsigned>(parts), static_cast<unsigned>(k_blocks * n_blocks));
+  typed_wgrad_tc<float, true><<<grid, 32 * (kEpiWarps + 1 + kProdWarps + kConvWarps), smem, st>>>(a);
+  dense_reduce<<<static_cast<unsigned>((static_cast<int64_t>(k) * n + 127) / 128), 128, 0, st>>>(a.partial, dw, k, n, k_blocks,
+                                                                                            parts);
+  count_launches(2);
+  return check_launch("cxg_dense_wgrad_f32");
+}
+
+extern "C" int cxg_dense_wgrad_f32_status(void *stream) {
+  int32_t word = 0;
+  cudaStream_t st = as_stream(stream);
+  if (cudaMemcpyFromSymbolAsync(&word, dense_status, sizeof(word), 0, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess)
+    return check_launch("cxg_dense_wgrad_f32_status");
+  if (word != 0) return set_error(CXG_ETIMEOUT, "cxg_dense_wgrad_f32: a bounded wait ran out");
+  return CXG_OK;
 }
 
 extern "C" int cxg_typed_wgrad_status(const void *workspace, void *stream) {
