@@ -4,6 +4,7 @@
 //
 // The kernels stay behind the C ABI of libcxgnn_b200.so: this module opens the library it is told to (init) and calls its
 // entry points. No CUDA code, no other state than the scratch buffers per stream and the transposed graphs.
+#include <ATen/autocast_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
@@ -34,6 +35,12 @@ struct Lib {
   CXG_FN(cxg_csr_transpose_workspace_size);
   CXG_FN(cxg_csr_transpose);
   CXG_FN(cxg_gather_edges);
+  CXG_FN(cxg_linear_f32_supported);
+  CXG_FN(cxg_linear_f32);
+  CXG_FN(cxg_dense_wgrad_f32_workspace_size);
+  CXG_FN(cxg_dense_wgrad_f32);
+  CXG_FN(cxg_column_sum_workspace_size);
+  CXG_FN(cxg_column_sum);
   CXG_FN(cxg_gather_rows);
   CXG_FN(cxg_sample_batch_bounds);
   CXG_FN(cxg_sample_batch);
@@ -53,6 +60,12 @@ void init(const std::string &path) {
   CXG_FN(cxg_csr_transpose_workspace_size);
   CXG_FN(cxg_csr_transpose);
   CXG_FN(cxg_gather_edges);
+  CXG_FN(cxg_linear_f32_supported);
+  CXG_FN(cxg_linear_f32);
+  CXG_FN(cxg_dense_wgrad_f32_workspace_size);
+  CXG_FN(cxg_dense_wgrad_f32);
+  CXG_FN(cxg_column_sum_workspace_size);
+  CXG_FN(cxg_column_sum);
   CXG_FN(cxg_gather_rows);
   CXG_FN(cxg_sample_batch_bounds);
   CXG_FN(cxg_sample_batch);
@@ -335,6 +348,110 @@ Tensor gather_rows(const Tensor &x, const Tensor &rows) {
   return out;
 }
 
+// ---- linear transform ------------------------------------------------------------------------------------------------
+bool aligned16(const Tensor &t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+
+// fp32 matrices that the tensor-core kernel takes as they are
+bool dense_rows(const Tensor &t) {
+  return t.dim() == 2 && t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel() > 0 && aligned16(t);
+}
+
+// x [M, K] . w [N, K]^T (w_rows_k: w is [K, N]) + bias + add
+Tensor linear_product(const Tensor &x, const Tensor &w, bool w_rows_k, const optional<Tensor> &bias, const optional<Tensor> &add) {
+  const int64_t n = w_rows_k ? w.size(1) : w.size(0);
+  Tensor y = at::empty({x.size(0), n}, x.options());
+  check(lib.cxg_linear_f32(x.data_ptr<float>(), w.data_ptr<float>(), bias ? bias->data_ptr<float>() : nullptr,
+                           add ? add->data_ptr<float>() : nullptr, y.data_ptr<float>(), x.size(0), static_cast<int>(x.size(1)),
+                           static_cast<int>(n), w_rows_k ? 1 : 0, stream_of(x)),
+        "cxg_linear_f32");
+  return y;
+}
+
+// g [M, N]^T . x [M, K]
+Tensor linear_weight_grad(const Tensor &g, const Tensor &x) {
+  const int64_t m = x.size(0), n = g.size(1), k = x.size(1);
+  if (!dense_rows(g) || !dense_rows(x) || n % 4 != 0 || k % 4 != 0) return at::mm(g.t(), x);
+  Tensor dw = at::empty({n, k}, x.options());
+  size_t need = 0;
+  check(lib.cxg_dense_wgrad_f32_workspace_size(m, static_cast<int>(n), static_cast<int>(k), &need),
+        "cxg_dense_wgrad_f32_workspace_size");
+  void *st = stream_of(x);
+  const Tensor ws = workspace_on(x.device().index(), st, static_cast<int64_t>(need), "");
+  check(lib.cxg_dense_wgrad_f32(g.data_ptr<float>(), x.data_ptr<float>(), m, static_cast<int>(n), static_cast<int>(k),
+                                dw.data_ptr<float>(), ws.data_ptr(), static_cast<size_t>(ws.numel()), st),
+        "cxg_dense_wgrad_f32");
+  return dw;
+}
+
+Tensor rows_sum(const Tensor &g) {
+  Tensor out = at::empty({g.size(1)}, g.options());
+  size_t need = 0;
+  check(lib.cxg_column_sum_workspace_size(static_cast<int>(g.size(1)), &need), "cxg_column_sum_workspace_size");
+  void *st = stream_of(g);
+  const Tensor ws = workspace_on(g.device().index(), st, static_cast<int64_t>(need), "");
+  check(lib.cxg_column_sum(g.data_ptr(), CXG_F32, g.size(0), static_cast<int>(g.size(1)), out.data_ptr<float>(), ws.data_ptr(),
+                           static_cast<size_t>(ws.numel()), st),
+        "cxg_column_sum");
+  return out;
+}
+
+bool linear_fits(const Tensor &x, const Tensor &w) {
+  return dense_rows(x) && dense_rows(w) && x.size(1) == w.size(1) && x.device() == w.device() &&
+         lib.cxg_linear_f32_supported(x.size(0), static_cast<int>(x.size(1)), static_cast<int>(w.size(0))) == 1;
+}
+
+class LinearFunction : public torch::autograd::Function<LinearFunction> {
+ public:
+  static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &w, const optional<Tensor> &bias,
+                        const optional<Tensor> &add) {
+    ctx->save_for_backward({x, w});
+    ctx->saved_data["bias"] = bias.has_value();
+    ctx->saved_data["add"] = add.has_value();
+    return linear_product(x, w, false, bias, add);
+  }
+  static variable_list backward(AutogradContext *ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w = saved[1];
+    const Tensor g = grads[0].contiguous();
+    c10::cuda::CUDAGuard guard(g.device());
+    Tensor dx, dw, db;
+    // the edges of the node are those of the tensors that were given
+    const bool bias = ctx->saved_data["bias"].toBool(), need_db = bias && ctx->needs_input_grad(2);
+    const bool need_add = ctx->saved_data["add"].toBool() && ctx->needs_input_grad(bias ? 3 : 2);
+    if (at::GradMode::is_enabled()) {  // a graph of the backward itself is wanted
+      if (ctx->needs_input_grad(0)) dx = at::mm(g, w);
+      if (ctx->needs_input_grad(1)) dw = at::mm(g.t(), x);
+      if (need_db) db = g.sum(0);
+    } else {
+      if (ctx->needs_input_grad(0))
+        dx = dense_rows(g) && lib.cxg_linear_f32_supported(g.size(0), static_cast<int>(g.size(1)), static_cast<int>(w.size(1)))
+                 ? linear_product(g, w, true, c10::nullopt, c10::nullopt)
+                 : at::mm(g, w);
+      if (ctx->needs_input_grad(1)) dw = linear_weight_grad(g, x);
+      if (need_db) db = rows_sum(g);
+    }
+    return {dx, dw, db, need_add ? grads[0] : Tensor()};
+  }
+};
+
+// x . w^T (+ bias) (+ add): the tensor-core kernel for fp32 matrices it takes, torch otherwise (CPU, other types, autocast,
+// rows that are not whole 16-byte vectors).
+Tensor linear(const Tensor &x, const Tensor &w, const optional<Tensor> &bias, const optional<Tensor> &add) {
+  const bool fits = linear_fits(x, w) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
+                    (!bias || (bias->scalar_type() == at::kFloat && bias->is_contiguous() && bias->device() == x.device() &&
+                               bias->dim() == 1 && bias->size(0) == w.size(0)));
+  const bool add_fits = add && dense_rows(*add) && add->size(0) == x.size(0) && add->size(1) == w.size(0) && add->device() == x.device();
+  if (!fits || (add && !add_fits)) {
+    const Tensor y = at::linear(x, w, bias);
+    return add ? *add + y : y;
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad() || (bias && bias->requires_grad()) ||
+                                     (add && add->requires_grad())))
+    return LinearFunction::apply(x, w, bias, add);
+  return linear_product(x, w, false, bias, add);
+}
+
 // ---- neighbour sampling ----------------------------------------------------------------------------------------------
 // The most a call may reserve for the nodes and edges a batch can reach; above it the hops are run one by one.
 constexpr int64_t kMostSampled = 1 << 27;
@@ -404,6 +521,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("forget_graphs", &forget_graphs);
   m.def("count_graphs", &count_graphs);
   m.def("gather_rows", &gather_rows);
+  m.def("linear", &linear);
   m.def("sample_batch_fits", &sample_batch_fits);
   m.def("sample_batch", &sample_batch);
 }

@@ -24,6 +24,14 @@ def glorot(t):
         t.data.uniform_(-a, a)
 
 
+class Linear(torch.nn.Linear):
+    """torch.nn.Linear on the library's fp32 tensor-core kernel where that takes the matrices (cxgnncomp_backend.linear).
+    `add`: a matrix added to the result in the same pass."""
+
+    def forward(self, x, add=None):
+        return cxgnncomp_backend.linear(x, self.weight, self.bias, add)
+
+
 class AggrOP(torch.autograd.Function):
     """Sum aggregation through the tuner interface (graph_conv.py:34-77). Like the reference, the backward
     applies the forward operator to the gradient, which is the transpose only for a symmetric graph with as
@@ -72,9 +80,9 @@ class MySageConv(torch.nn.Module):
         self.in_channels = in_channels
         self.hidden_channels = hidden_channels
         self.root_weight = root_weight
-        self.lin_l = torch.nn.Linear(in_channels, hidden_channels, bias=bias)
+        self.lin_l = Linear(in_channels, hidden_channels, bias=bias)
         if self.root_weight:
-            self.lin_r = torch.nn.Linear(in_channels, hidden_channels, bias=False)
+            self.lin_r = Linear(in_channels, hidden_channels, bias=False)
         self.reset_parameters()
 
     def reset_parameters(self):
@@ -88,7 +96,8 @@ class MySageConv(torch.nn.Module):
         else:
             out = self.lin_l(sage_mean_forward(x, ptr, idx, num_node))
         if self.root_weight:
-            out = out + self.lin_r(x[:num_node] if num_node != 0 else x)
+            root = x[:num_node] if num_node != 0 else x
+            out = self.lin_r(root, add=out) if isinstance(self.lin_r, Linear) else out + self.lin_r(root)
         return out
 
 
@@ -99,7 +108,7 @@ class MyGINConv(torch.nn.Module):
         super().__init__()
         self.in_channels = in_channels
         self.hidden_channels = hidden_channels
-        self.nn = torch.nn.Linear(in_channels, hidden_channels, bias=False)
+        self.nn = Linear(in_channels, hidden_channels, bias=False)
         self.init_eps = 0.2
         self.eps = torch.nn.Parameter(torch.Tensor([self.init_eps]))
         self.reset_parameters()
@@ -457,7 +466,7 @@ class MyGATConv(torch.nn.Module):
         if self.tensor_core_linear:  # the layer's linear transform on the library's tensor-core kernels
             x_src = cxgnncomp_backend.dense_linear(x[:num_src], self.lin_src).view(-1, H, C)
         else:
-            x_src = F.linear(x[:num_src], self.lin_src).view(-1, H, C)
+            x_src = cxgnncomp_backend.linear(x[:num_src], self.lin_src).view(-1, H, C)
         if x_src.dtype == torch.float32 and self.fused_scores:
             alpha_src, alpha_dst = cxgnncomp_backend.gat_scores(x_src.contiguous(), self.att_src.contiguous(),
                                                                 self.att_dst.contiguous(), num_dst)
@@ -492,9 +501,9 @@ class MyGATConv(torch.nn.Module):
         edge_value = self.edge_softmax(ptr=ptr, idx=idx, att_src=alpha_src.contiguous(), att_dst=alpha_dst.contiguous(),
                                        num_edge=num_edge, relu_l=self.negative_slope).reshape(-1)
         if self.out_channels < self.in_channels:
-            out = sage_sum_forward_edge_value(torch.mm(x, self.lin_src.T), ptr, idx, edge_value, num_dst)
+            out = sage_sum_forward_edge_value(cxgnncomp_backend.linear(x, self.lin_src), ptr, idx, edge_value, num_dst)
         else:
-            out = torch.mm(sage_sum_forward_edge_value(x, ptr, idx, edge_value, num_dst), self.lin_src.T)
+            out = cxgnncomp_backend.linear(sage_sum_forward_edge_value(x, ptr, idx, edge_value, num_dst), self.lin_src)
         return cxgnncomp_backend.bias_add(out, self.bias) if self.bias is not None else out
 
     def forward(self, x, ptr, idx, num_dst, num_src, num_edge):
@@ -514,7 +523,7 @@ class MyGCNConv(torch.nn.Module):
         self.in_channels = in_channels
         self.out_channels = out_channels
         self.normalize = normalize
-        self.lin = torch.nn.Linear(in_channels, out_channels, bias=False)
+        self.lin = Linear(in_channels, out_channels, bias=False)
         self.bias = torch.nn.Parameter(torch.empty(out_channels)) if bias else None
         self.reset_parameters()
 

@@ -154,6 +154,27 @@ int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel, const int6
 int cxg_typed_wgrad_status(const void *workspace, void *stream);
 
 /*
+ * Linear transform in fp32 on the tensor cores, as close to the exact result as an fp32 multiply-add chain (every operand
+ * is taken apart into three bf16 terms): c[m, n] = a[m, :] . b[n, :] (+ bias[n]) (+ add[m, n]), all matrices row-major and
+ * contiguous. b_rows_k: b is [k, n] instead of [n, k]. k must be a multiple of 4 of which 16 rows of b fit in shared
+ * memory (about 1100 columns; cxg_linear_f32_supported tells), n up to 8192; a, b, c and add 16-byte aligned. bias and add
+ * may be NULL; add may be c. cxg_linear_f32_status reads back whether a bounded wait ran out on the current device.
+ */
+int cxg_linear_f32_supported(int64_t m, int k, int n);
+int cxg_linear_f32(const float *a, const float *b, const float *bias, const float *add, float *c, int64_t m, int k, int n,
+                   int b_rows_k, void *stream);
+int cxg_linear_f32_status(void *stream);
+
+/*
+ * Its weight gradient: dw[k, n] = x[m, k]^T . g[m, n], fp32, contiguous, k and n multiples of 4, x and g 16-byte aligned. The
+ * kernel of cxg_typed_wgrad (compensated) over blocks of 128 x 128 columns, partial sums added in a fixed order.
+ */
+int cxg_dense_wgrad_f32_workspace_size(int64_t m, int k, int n, size_t *bytes);
+int cxg_dense_wgrad_f32(const float *x, const float *g, int64_t m, int k, int n, float *dw, void *workspace,
+                        size_t workspace_bytes, void *stream);
+int cxg_dense_wgrad_f32_status(void *stream);
+
+/*
  * Scratch bytes needed by cxg_spmm_csr for a graph with n_dst rows and nnz
  * edges at row width heads*feat (split_edges as in the descriptor). Upper bound;
  * depends on sizes only.
