@@ -172,22 +172,24 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc(const __grid_constant__
 
   if (warp == kLoadWarp) {
     if (lane == 0) {
-      int64_t it = 0;
+      Ring ring(S);
       bool alive = true;
       for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile)
         for (int sp = 0; sp < spans; ++sp) {
-          const int s = static_cast<int>(it % S);
-          if (it >= S && !(alive = wait(&bars.raw_empty[s], it / S - 1))) break;
+          const int s = ring.stage;
+          if (ring.reused() && !(alive = wait(&bars.raw_empty[s], ring.emptied()))) break;
           const uint32_t bar = smem_addr(&bars.raw_full[s]);
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kRawBytes) : "memory");
           tma_load_2d(smem_addr(raw + s * kRawBytes), &tmap_a, sp * kSpan, static_cast<int>(tile * kTileM), bar);
-          ++it;
+          ring.next();
         }
       // the copies in flight land before the block ends, whatever became of their readers
-      for (int64_t j = it > S ? it - S : 0; j < it; ++j) {
-        const uint32_t bar = smem_addr(&bars.raw_full[j % S]);
+      for (int j = 0; j < S; ++j) {
+        uint32_t parity;
+        if (!ring.last(j, &parity)) continue;
+        const uint32_t bar = smem_addr(&bars.raw_full[j]);
         const long long t0 = clock64();
-        while (!mbar_try_wait(bar, static_cast<uint32_t>((j / S) & 1)) && clock64() - t0 <= a.wait_cycles) {
+        while (!mbar_try_wait(bar, parity) && clock64() - t0 <= a.wait_cycles) {
         }
       }
     }
@@ -195,17 +197,17 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc(const __grid_constant__
   } else if (warp >= kFirstConv) {
     const int ct = tid - 32 * kFirstConv;
     constexpr int kPer = kTileM * 8 / (32 * kConvWarps);  // 16-byte chunks per thread
-    int64_t it = 0;
+    Ring ring(S);
     bool alive = true;
     for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile)
-      for (int sp = 0; sp < spans; ++sp, ++it) {
-        const int s = static_cast<int>(it % S);
-        if (!(alive = wait(&bars.raw_full[s], it / S))) break;
+      for (int sp = 0; sp < spans; ++sp, ring.next()) {
+        const int s = ring.stage;
+        if (!(alive = wait(&bars.raw_full[s], ring.filled()))) break;
         const float4 *src = reinterpret_cast<const float4 *>(raw + s * kRawBytes);
         float4 v[kPer];
 #pragma unroll
         for (int u = 0; u < kPer; ++u) v[u] = src[ct + u * 32 * kConvWarps];
-        if (it >= S && !(alive = wait(&bars.term_empty[s], it / S - 1))) break;
+        if (ring.reused() && !(alive = wait(&bars.term_empty[s], ring.emptied()))) break;
         uint8_t *dst = terms + s * 3 * kTermBytes;
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
@@ -226,15 +228,16 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc(const __grid_constant__
     const uint32_t idesc = make_idesc(1, kTileM, a.nt), idesc_wide = make_idesc(1, kTileM, 2 * a.nt);
     const uint64_t desc = desc_base(2);
     const uint32_t b0 = smem_addr(smem_b);
-    int64_t it = 0, tile_it = 0;
+    Ring ring(S);
+    int64_t tile_it = 0;
     bool alive = true;
     for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile, ++tile_it) {
       const int buf = static_cast<int>(tile_it & 1);
       const uint32_t d0 = tmem_d + buf * a.acc_cols, d1 = d0 + a.nt;  // h.h, and the small products
       if (tile_it >= 2 && !(alive = wait_all(&bars.acc_empty[buf], (tile_it >> 1) - 1))) break;
-      for (int sp = 0; sp < spans; ++sp, ++it) {
-        const int s = static_cast<int>(it % S);
-        if (!(alive = wait_all(&bars.term_full[s], it / S))) break;
+      for (int sp = 0; sp < spans; ++sp, ring.next()) {
+        const int s = ring.stage;
+        if (!(alive = wait_all(&bars.term_full[s], ring.filled()))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a0 = smem_addr(terms + s * 3 * kTermBytes), bs = b0 + sp * span_b;
         const int steps = a.k - sp * kSpan > 16 ? 2 : 1;  // 16 columns of K each

@@ -109,6 +109,25 @@ __device__ __forceinline__ void commit_to(uint64_t *bar) {
       : "memory");
 }
 
+// Where a role stands in a ring of stages: the stage, and how often it has gone round. (Stage and round as remainder and
+// quotient of a 64-bit unit counter cost every role two software divisions per unit, more than the unit's MMAs.)
+struct Ring {
+  int size, stage = 0;
+  uint32_t round = 0;
+  __device__ explicit Ring(int n) : size(n) {}
+  __device__ void next() {
+    if (++stage == size) stage = 0, ++round;
+  }
+  __device__ bool reused() const { return round > 0; }
+  __device__ uint32_t filled() const { return round & 1; }        // parity of the phase that fills the stage this time
+  __device__ uint32_t emptied() const { return (round & 1) ^ 1; }  // parity of the phase that emptied it after the last time
+  // Parity of the last phase of stage i that this role has begun; false: none
+  __device__ bool last(int i, uint32_t *parity) const {
+    *parity = (i < stage ? round : round - 1) & 1;
+    return i < stage || round > 0;
+  }
+};
+
 // 16 consecutive 32-bit columns of this warp's 32 accumulator lanes; completion is awaited by the caller
 __device__ __forceinline__ void tmem_ld16(uint32_t *v, uint32_t taddr) {
   asm volatile(

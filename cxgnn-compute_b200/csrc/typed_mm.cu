@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
     const int rsub = lane / kCpi, cq = lane % kCpi;
     const T *Wt = static_cast<const T *>(a.wt);
     int64_t loaded_rel = -1;
-    int64_t it = 0;        // units (tile, K-block) issued by this CTA
+    Ring ring(S);          // units (tile, K-block) issued by this CTA
     bool alive = true;
     // the relation and the row indices of a tile are fetched one tile ahead, off the critical path
     auto fetch = [&](int64_t tile, int64_t &r, int64_t (&ia)[kIdx]) {
@@ -279,8 +279,10 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
       if (r < 0 || r >= a.num_rel) continue;  // a tile of padding only
       if (r != loaded_rel) {
         // every MMA issued so far reads the old W: let them finish
-        for (int64_t j = (it > S ? it - S : 0); j < it && alive; ++j)
-          alive = wait_bar(&bars.empty[j % S], static_cast<uint32_t>((j / S) & 1), abort_flag, a.status, a.wait_cycles);
+        for (int j = 0; j < S && alive; ++j) {
+          uint32_t parity;
+          if (ring.last(j, &parity)) alive = wait_bar(&bars.empty[j], parity, abort_flag, a.status, a.wait_cycles);
+        }
         if (!alive) break;
         const int64_t w_elems = static_cast<int64_t>(a.ncols) * a.k;  // one relation's weight (dense: P of them in a row)
         const uint32_t b0 = smem_addr(smem_b);
@@ -293,9 +295,9 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
         loaded_rel = r;
       }
       for (int kb = 0; kb < nkb && alive; ++kb) {
-        const int s = static_cast<int>(it % S);
-        if (it >= S) {
-          alive = wait_bar(&bars.empty[s], static_cast<uint32_t>(((it / S) - 1) & 1), abort_flag, a.status, a.wait_cycles);
+        const int s = ring.stage;
+        if (ring.reused()) {
+          alive = wait_bar(&bars.empty[s], ring.emptied(), abort_flag, a.status, a.wait_cycles);
           if (!alive) break;
         }
         const uint32_t a0 = smem_addr(smem_a + s * a_bytes);
@@ -337,9 +339,9 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
         }
         // the unit's full barrier counts this thread's arrival when all copies it has issued so far (this unit's
         // rows, and W when it was re-copied) have landed: the producer never waits for its own copies
-        if (!(a.test_stall && it == 0))
+        if (!(a.test_stall && ring.round == 0 && ring.stage == 0))
           asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&bars.full[s])) : "memory");
-        ++it;
+        ring.next();
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -347,14 +349,14 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
     // ================= converters: raw fp32 stage -> hi (in place) and lo (second half) =================
     const int ct = tid - 32 * kFirstConvWarp;  // 0 .. 32 * kConvWarps - 1
     const int n16 = static_cast<int>(half_bytes / 16);
-    int64_t it = 0;
+    Ring ring(S);
     bool alive = true;
     for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile) {
       const int64_t r = rel_of(tile);
       if (r < 0 || r >= a.num_rel) continue;
       for (int kb = 0; kb < nkb && alive; ++kb) {
-        const int s = static_cast<int>(it % S);
-        alive = wait_bar(&bars.full[s], static_cast<uint32_t>((it / S) & 1), abort_flag, a.status, a.wait_cycles);
+        const int s = ring.stage;
+        alive = wait_bar(&bars.full[s], ring.filled(), abort_flag, a.status, a.wait_cycles);
         if (!alive) break;
         float4 *hi = reinterpret_cast<float4 *>(smem_a + s * a_bytes);
         float4 *lo = reinterpret_cast<float4 *>(smem_a + s * a_bytes + half_bytes);
@@ -380,7 +382,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
         // these generic-proxy writes are read by the tensor core through the async proxy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_arrive(&bars.conv[s]);
-        ++it;
+        ring.next();
       }
     }
   } else if (warp == kMmaWarp) {
@@ -394,7 +396,8 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
     const uint32_t idesc_wide = make_idesc(2, kTileM, a.small_off ? 2 * a.n : a.n);
     const uint64_t desc = desc_base(sl);
     const int steps = chunks_blk / 2;  // two chunks (32 bytes) of K per instruction
-    int64_t it = 0, tile_it = 0;
+    Ring ring(S);
+    int64_t tile_it = 0;
     bool alive = true;
     int64_t r_next = rel_of(tile_lo);
     for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile) {
@@ -404,8 +407,8 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
       const int buf = static_cast<int>(tile_it & 1);
       const uint32_t d = tmem_d + buf * a.tmem_cols;
       for (int kb = 0; kb < nkb && alive; ++kb) {
-        const int s = static_cast<int>(it % S);
-        alive = wait_all(X3 ? &bars.conv[s] : &bars.full[s], static_cast<uint32_t>((it / S) & 1));
+        const int s = ring.stage;
+        alive = wait_all(X3 ? &bars.conv[s] : &bars.full[s], ring.filled());
         if (alive && kb == 0 && tile_it >= 2)
           alive = wait_all(&bars.acc_empty[buf], static_cast<uint32_t>(((tile_it >> 1) - 1) & 1));
         if (!alive) break;
@@ -435,7 +438,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
           }
         }
         commit_to(&bars.empty[s]);
-        ++it;
+        ring.next();
       }
       if (!alive) break;
       commit_to(&bars.acc_full[buf]);

@@ -22,6 +22,7 @@
 //
 // Every wait is bounded; a role that waits too long raises a CTA-wide abort flag and an error status.
 #include "common.cuh"
+#include "tensor_core.cuh"
 
 namespace cxg {
 namespace {
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     int64_t ia_next[kAhead], ig_next[kAhead];
     fetch(tile_lo, ia_next, ig_next);
     RelCursor rel(a, tile_lo);
-    int64_t it = 0;
+    tc::Ring ring(S);
     bool alive = true;
     for (int64_t tile0 = tile_lo; tile0 < tile_hi && alive; tile0 += kGroup) {
       int64_t ia[kAhead], ig[kAhead];
@@ -279,9 +280,9 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
 #pragma unroll
       for (int t = 0; t < kGroup; ++t) {
         if (tile0 + t >= tile_hi || !alive || !valid_rel(rel.at(tile0 + t))) continue;  // invalid: a tile of padding only
-        const int s = static_cast<int>(it % S);
-        if (it >= S) {
-          alive = wait_bar(&bars.empty[s], static_cast<uint32_t>(((it / S) - 1) & 1), abort_flag, a.status, a.wait_cycles);
+        const int s = ring.stage;
+        if (ring.reused()) {
+          alive = wait_bar(&bars.empty[s], ring.emptied(), abort_flag, a.status, a.wait_cycles);
           if (!alive) continue;
         }
         const uint32_t st0 = smem_addr(smem + static_cast<size_t>(s) * stage_bytes);
@@ -305,9 +306,9 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
           for (int j = 0; j < spans_x; ++j) copy(xs, xrow, j, d0 + j * kSpan);
           for (int j = 0; j < spans_g; ++j) copy(gs, grow, j, d0 + (spans_x + j) * kSpan);
         }
-        if (!(a.test_stall && it == 0))
+        if (!(a.test_stall && ring.round == 0 && ring.stage == 0))
           asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&bars.full[s])) : "memory");
-        ++it;
+        ring.next();
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -315,14 +316,14 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     // ================= converters: raw fp32 tiles -> hi (in place) and lo (second half of the stage) =================
     const int ct = tid - 32 * kFirstConv;
     const int n16 = static_cast<int>(half_bytes / 16), x16 = spans_x * (kSpan / 16), g16 = n16 - x16;
-    int64_t it = 0;
+    tc::Ring ring(S);
     bool alive = true;
     RelCursor rel(a, tile_lo);
     for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile) {
       const int64_t r = rel.at(tile);
       if (!valid_rel(r)) continue;
-      const int s = static_cast<int>(it % S);
-      alive = wait_bar(&bars.full[s], static_cast<uint32_t>((it / S) & 1), abort_flag, a.status, a.wait_cycles);
+      const int s = ring.stage;
+      alive = wait_bar(&bars.full[s], ring.filled(), abort_flag, a.status, a.wait_cycles);
       if (!alive) break;
       float4 *hi = reinterpret_cast<float4 *>(smem + static_cast<size_t>(s) * stage_bytes);
       // the second half holds g's lo spans first, so that they follow g's hi spans, then those of x
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       mbar_arrive(&bars.conv[s]);
-      ++it;
+      ring.next();
     }
   } else if (warp == kMmaWarp) {
     // ================= MMA issuer =================
@@ -362,7 +363,8 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     const uint32_t idesc = make_idesc_mn(TF32 ? 2 : 1, 128, n_mma);
     const uint32_t idesc_wide = make_idesc_mn(2, 128, small_off ? 2 * n_mma : n_mma);
     const uint32_t step_bytes = kInstrK * 128;  // the next kInstrK positions of a span
-    int64_t it = 0, chunk = 0;
+    tc::Ring ring(S);
+    int64_t chunk = 0;
     int in_chunk = 0;
     bool alive = true, open = false;  // open: the current accumulator holds tiles of relation `cur`
     int64_t cur = -1;
@@ -386,8 +388,8 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
         in_chunk = 0;
       }
       const uint32_t d = tmem_d + buf * tmem_cols;
-      const int s = static_cast<int>(it % S);
-      alive = wait_all(X3 ? &bars.conv[s] : &bars.full[s], static_cast<uint32_t>((it / S) & 1));
+      const int s = ring.stage;
+      alive = wait_all(X3 ? &bars.conv[s] : &bars.full[s], ring.filled());
       if (!alive) break;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -415,7 +417,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
       commit_to(&bars.empty[s]);
       open = true;
       ++in_chunk;
-      ++it;
+      ring.next();
     }
     if (alive && open) commit_to(&bars.acc_full[chunk & 1]);
   } else if (warp < kEpiWarps) {
