@@ -58,16 +58,32 @@ __global__ void __launch_bounds__(kCsThreads) column_sum_partial(const T *x, flo
   }
 }
 
-// Stage 2: one warp per column; lane l adds the partials of CTAs l, l + 32, ... in order, the 32 lane sums are
-// joined by a shuffle tree.
-__global__ void __launch_bounds__(kCsThreads) column_sum_final(const float *part, float *out, int n_part, int width) {
-  const int lane = threadIdx.x & 31;
-  const int col = (blockIdx.x * kCsThreads + threadIdx.x) >> 5;
-  if (col >= width) return;
+// Stage 2: warp w of a block adds the partials of CTAs w, w + 32, ... for 32 columns, the 32 sums are added in order. (A
+// warp per column read 4 bytes of every sector: 7 us for 1184 partials of 128 columns, now 4.)
+constexpr int kJoinThreads = 1024;
+__global__ void __launch_bounds__(kJoinThreads) column_sum_final(const float *part, float *out, int n_part, int width) {
+  __shared__ float sh[kJoinThreads / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.x * 32 + lane;
+  constexpr int kWarps = kJoinThreads / 32;
   float s = 0.f;
-  for (int b = lane; b < n_part; b += 32) s += part[static_cast<int64_t>(b) * width + col];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) out[col] = s;
+  if (col < width) {
+    const float *p = part + col;
+    int b = warp;
+    for (; b + 3 * kWarps < n_part; b += 4 * kWarps) {
+      float v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = p[static_cast<int64_t>(b + u * kWarps) * width];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s += v[u];
+    }
+    for (; b < n_part; b += kWarps) s += p[static_cast<int64_t>(b) * width];
+  }
+  sh[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && col < width) {
+    for (int w = 1; w < kWarps; ++w) s += sh[w][lane];
+    out[col] = s;
+  }
 }
 
 }  // namespace
@@ -93,13 +109,17 @@ extern "C" int cxg_column_sum(const void *x, int dtype, int64_t n_row, int width
               "cxg_column_sum: workspace %zu bytes, need %zu", workspace_bytes, need);
   cudaStream_t st = as_stream(stream);
   float *part = static_cast<float *>(workspace);
-  // every CTA writes its partial row (zeros when its chunk is empty), so the second stage reads no stale value
+  // every CTA writes its partial row (zeros when its chunk is empty), so the second stage reads no stale value; at least 32
+  // rows per CTA, so that a small call does not add up more partials than rows
+  int64_t ctas = (n_row + 31) / 32;
+  if (ctas > kCsCtas) ctas = kCsCtas;
+  if (ctas < 1) ctas = 1;
+  const int grid = static_cast<int>(ctas);
   if (dtype == CXG_F32)
-    column_sum_partial<float><<<kCsCtas, kCsThreads, 0, st>>>(static_cast<const float *>(x), part, n_row, width);
+    column_sum_partial<float><<<grid, kCsThreads, 0, st>>>(static_cast<const float *>(x), part, n_row, width);
   else
-    column_sum_partial<__nv_bfloat16><<<kCsCtas, kCsThreads, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), part,
-                                                                      n_row, width);
-  column_sum_final<<<(width * 32 + kCsThreads - 1) / kCsThreads, kCsThreads, 0, st>>>(part, out, kCsCtas, width);
+    column_sum_partial<__nv_bfloat16><<<grid, kCsThreads, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), part, n_row, width);
+  column_sum_final<<<(width + 31) / 32, kJoinThreads, 0, st>>>(part, out, grid, width);
   count_launches(2);
   return check_launch("cxg_column_sum");
 }

@@ -41,6 +41,13 @@ struct Lib {
   CXG_FN(cxg_dense_wgrad_f32);
   CXG_FN(cxg_column_sum_workspace_size);
   CXG_FN(cxg_column_sum);
+  CXG_FN(cxg_gat_scores);
+  CXG_FN(cxg_gat_fused_workspace_size);
+  CXG_FN(cxg_gat_fused_forward);
+  CXG_FN(cxg_gat_fused_backward);
+  CXG_FN(cxg_gat_att_grad_workspace_size);
+  CXG_FN(cxg_gat_scores_backward_add);
+  CXG_FN(cxg_head_mean_bias);
   CXG_FN(cxg_gather_rows);
   CXG_FN(cxg_sample_batch_bounds);
   CXG_FN(cxg_sample_batch);
@@ -66,6 +73,13 @@ void init(const std::string &path) {
   CXG_FN(cxg_dense_wgrad_f32);
   CXG_FN(cxg_column_sum_workspace_size);
   CXG_FN(cxg_column_sum);
+  CXG_FN(cxg_gat_scores);
+  CXG_FN(cxg_gat_fused_workspace_size);
+  CXG_FN(cxg_gat_fused_forward);
+  CXG_FN(cxg_gat_fused_backward);
+  CXG_FN(cxg_gat_att_grad_workspace_size);
+  CXG_FN(cxg_gat_scores_backward_add);
+  CXG_FN(cxg_head_mean_bias);
   CXG_FN(cxg_gather_rows);
   CXG_FN(cxg_sample_batch_bounds);
   CXG_FN(cxg_sample_batch);
@@ -452,6 +466,110 @@ Tensor linear(const Tensor &x, const Tensor &w, const optional<Tensor> &bias, co
   return linear_product(x, w, false, bias, add);
 }
 
+// ---- GAT layer -------------------------------------------------------------------------------------------------------
+Tensor head_mean_bias(const Tensor &x, const optional<Tensor> &bias, int64_t heads, int64_t c) {
+  Tensor out = at::empty({x.size(0), c}, x.options());
+  check(lib.cxg_head_mean_bias(x.data_ptr<float>(), bias ? bias->data_ptr<float>() : nullptr, out.data_ptr<float>(), x.size(0),
+                               static_cast<int>(heads), static_cast<int>(c), stream_of(x)),
+        "cxg_head_mean_bias");
+  return out;
+}
+
+// Attention scores, softmax, weighted neighbour sum, heads joined or averaged, bias: x [n_src, H, C] -> [n, H * C] or [n, C].
+class GatFunction : public torch::autograd::Function<GatFunction> {
+ public:
+  static Tensor run(const Tensor &x, const Tensor &att_src, const Tensor &att_dst, const optional<Tensor> &bias, const Tensor &ptr,
+                    const Tensor &idx, int64_t n, double slope, bool concat, variable_list *keep) {
+    const int64_t n_src = x.size(0), h = x.size(1), c = x.size(2);
+    const int hi = static_cast<int>(h), ci = static_cast<int>(c);
+    void *st = stream_of(x);
+    const Tensor a_src = at::empty({n_src, h}, x.options()), a_dst = at::empty({n, h}, x.options());
+    check(lib.cxg_gat_scores(x.data_ptr<float>(), att_src.data_ptr<float>(), att_dst.data_ptr<float>(), a_src.data_ptr<float>(),
+                             a_dst.data_ptr<float>(), n_src, n, hi, ci, st),
+          "cxg_gat_scores");
+    const Tensor y = at::empty({n, h * c}, x.options()), top = at::empty({n, h}, x.options()), sum = at::empty({n, h}, x.options());
+    size_t need = 0;
+    check(lib.cxg_gat_fused_workspace_size(n, idx.size(0), hi, ci, &need), "cxg_gat_fused_workspace_size");
+    const Tensor ws = workspace_on(x.device().index(), st, static_cast<int64_t>(need), "");
+    check(lib.cxg_gat_fused_forward(ptr.data_ptr(), idx.data_ptr(), static_cast<int>(ptr.element_size()),
+                                    static_cast<int>(idx.element_size()), x.data_ptr<float>(), a_src.data_ptr<float>(),
+                                    a_dst.data_ptr<float>(), y.data_ptr<float>(), top.data_ptr<float>(), sum.data_ptr<float>(), n,
+                                    idx.size(0), hi, ci, static_cast<float>(slope), ws.data_ptr(),
+                                    static_cast<size_t>(ws.numel()), st),
+          "cxg_gat_fused_forward");
+    if (keep != nullptr) *keep = {x, att_src, att_dst, ptr, idx, a_src, a_dst, y, top, sum};
+    if (concat) return bias ? head_mean_bias(y, bias, 1, h * c) : y;
+    return head_mean_bias(y, bias, h, c);
+  }
+  static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &att_src, const Tensor &att_dst,
+                        const optional<Tensor> &bias, const Tensor &ptr, const Tensor &idx, int64_t n, double slope, bool concat) {
+    variable_list keep;
+    Tensor out = run(x, att_src, att_dst, bias, ptr, idx, n, slope, concat, &keep);
+    if (concat && !bias) out = out.view(out.sizes());  // y itself is kept for the backward
+    ctx->save_for_backward(keep);
+    ctx->saved_data["slope"] = slope;
+    ctx->saved_data["concat"] = concat;
+    ctx->saved_data["bias"] = bias.has_value();
+    return out;
+  }
+  static variable_list backward(AutogradContext *ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &att_src = saved[1], &att_dst = saved[2], &ptr = saved[3], &idx = saved[4], &a_src = saved[5],
+                 &a_dst = saved[6], &y = saved[7], &top = saved[8], &sum = saved[9];
+    const int64_t n_src = x.size(0), h = x.size(1), c = x.size(2), n = y.size(0);
+    const int hi = static_cast<int>(h), ci = static_cast<int>(c);
+    c10::cuda::CUDAGuard guard(x.device());
+    void *st = stream_of(x);
+    const Tensor g = grads[0].contiguous();
+    Tensor db;
+    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(3)) db = rows_sum(g);
+    const Tensor dy =
+        ctx->saved_data["concat"].toBool() ? g : g.mul(1.0 / static_cast<double>(h)).unsqueeze(1).expand({n, h, c}).contiguous();
+    const Transposed t = transposed_graph(ptr, idx, n, n_src);
+    const Tensor dx = at::empty_like(x), d_src = at::empty_like(a_src), d_dst = at::empty_like(a_dst);
+    size_t need = 0, need_att = 0;
+    check(lib.cxg_gat_fused_workspace_size(n, idx.size(0), hi, ci, &need), "cxg_gat_fused_workspace_size");
+    check(lib.cxg_gat_att_grad_workspace_size(hi, ci, &need_att), "cxg_gat_att_grad_workspace_size");
+    const Tensor ws = workspace_on(x.device().index(), st, static_cast<int64_t>(std::max(need, need_att)), "");
+    check(lib.cxg_gat_fused_backward(t.t_ptr.data_ptr(), t.t_idx.data_ptr(), static_cast<int>(t.t_ptr.element_size()),
+                                     static_cast<int>(t.t_idx.element_size()), dy.data_ptr<float>(), y.data_ptr<float>(),
+                                     x.data_ptr<float>(), a_src.data_ptr<float>(), a_dst.data_ptr<float>(), top.data_ptr<float>(),
+                                     sum.data_ptr<float>(), dx.data_ptr<float>(), d_src.data_ptr<float>(), d_dst.data_ptr<float>(),
+                                     n_src, n, t.t_idx.size(0), hi, ci, static_cast<float>(ctx->saved_data["slope"].toDouble()),
+                                     nullptr, nullptr, static_cast<int>(ptr.element_size()), ws.data_ptr(),
+                                     static_cast<size_t>(ws.numel()), st),
+          "cxg_gat_fused_backward");
+    const Tensor g_as = at::empty_like(att_src), g_ad = at::empty_like(att_dst);
+    check(lib.cxg_gat_scores_backward_add(x.data_ptr<float>(), d_src.data_ptr<float>(), d_dst.data_ptr<float>(),
+                                          att_src.data_ptr<float>(), att_dst.data_ptr<float>(), dx.data_ptr<float>(),
+                                          g_as.data_ptr<float>(), g_ad.data_ptr<float>(), n_src, n, hi, ci, ws.data_ptr(),
+                                          static_cast<size_t>(ws.numel()), st),
+          "cxg_gat_scores_backward_add");
+    return {dx, g_as, g_ad, db, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor gat_layer(const Tensor &x, const Tensor &att_src, const Tensor &att_dst, const optional<Tensor> &bias, const Tensor &ptr,
+                 const Tensor &idx, int64_t num_dst, double slope, bool concat) {
+  f32(x, "x");
+  f32(att_src, "att_src");
+  f32(att_dst, "att_dst");
+  index_of(ptr, "ptr");
+  index_of(idx, "idx");
+  const int64_t n = rows_of(ptr, num_dst), h = x.size(1), c = x.size(2);
+  if (x.dim() != 3 || att_src.numel() != h * c || att_dst.numel() != h * c || n > x.size(0))
+    fail("gat_layer: x must be [n_src, H, C] with n_src >= num_dst, the attention vectors [H, C]");
+  if (bias) {
+    f32(*bias, "bias");
+    if (bias->numel() != (concat ? h * c : c)) fail("gat_layer: the bias must have one value per output column");
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  if (at::GradMode::is_enabled() &&
+      (x.requires_grad() || att_src.requires_grad() || att_dst.requires_grad() || (bias && bias->requires_grad())))
+    return GatFunction::apply(x, att_src, att_dst, bias, ptr, idx, n, slope, concat);
+  return GatFunction::run(x, att_src, att_dst, bias, ptr, idx, n, slope, concat, nullptr);
+}
+
 // ---- neighbour sampling ----------------------------------------------------------------------------------------------
 // The most a call may reserve for the nodes and edges a batch can reach; above it the hops are run one by one.
 constexpr int64_t kMostSampled = 1 << 27;
@@ -522,6 +640,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("count_graphs", &count_graphs);
   m.def("gather_rows", &gather_rows);
   m.def("linear", &linear);
+  m.def("gat_layer", &gat_layer);
+  m.def("head_mean_bias", [](const Tensor &x, const optional<Tensor> &bias, int64_t heads, int64_t c) {
+    f32(x, "x");
+    c10::cuda::CUDAGuard guard(x.device());
+    return head_mean_bias(x, bias, heads, c);
+  });
   m.def("sample_batch_fits", &sample_batch_fits);
   m.def("sample_batch", &sample_batch);
 }

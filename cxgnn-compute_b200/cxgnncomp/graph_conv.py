@@ -96,7 +96,7 @@ class MySageConv(torch.nn.Module):
         else:
             out = self.lin_l(sage_mean_forward(x, ptr, idx, num_node))
         if self.root_weight:
-            root = x[:num_node] if num_node != 0 else x
+            root = x[:num_node] if num_node not in (0, x.shape[0]) else x
             out = self.lin_r(root, add=out) if isinstance(self.lin_r, Linear) else out + self.lin_r(root)
         return out
 
@@ -463,10 +463,18 @@ class MyGATConv(torch.nn.Module):
     def forward_many(self, x, ptr, idx, num_dst, num_src, num_edge):
         H, C = self.heads, self.out_channels
         assert x.dim() == 2
+        if x.shape[0] != num_src:  # (the gradient of a slice is a copy into zeros)
+            x = x[:num_src]
         if self.tensor_core_linear:  # the layer's linear transform on the library's tensor-core kernels
-            x_src = cxgnncomp_backend.dense_linear(x[:num_src], self.lin_src).view(-1, H, C)
+            x_src = cxgnncomp_backend.dense_linear(x, self.lin_src).view(-1, H, C)
         else:
-            x_src = cxgnncomp_backend.linear(x[:num_src], self.lin_src).view(-1, H, C)
+            x_src = cxgnncomp_backend.linear(x, self.lin_src).view(-1, H, C)
+        if (x_src.dtype == torch.float32 and self.fused_scores and self.fused_aggregate
+                and self.edge_softmax_schedule == "fused" and num_dst > 0
+                and cxgnncomp_backend.gat_layer_supported(x_src, self.att_src, self.att_dst, self.bias)):
+            # scores, softmax, weighted sum, heads and bias as one operator
+            return cxgnncomp_backend.gat_layer(x_src, self.att_src, self.att_dst, self.bias, ptr, idx, num_dst,
+                                               self.negative_slope, self.concat)
         if x_src.dtype == torch.float32 and self.fused_scores:
             alpha_src, alpha_dst = cxgnncomp_backend.gat_scores(x_src.contiguous(), self.att_src.contiguous(),
                                                                 self.att_dst.contiguous(), num_dst)

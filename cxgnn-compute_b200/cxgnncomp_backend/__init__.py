@@ -1060,6 +1060,20 @@ def gat_fused(x_src, a_src, a_dst, ptr, idx, num_dst, negative_slope):
     return _GatFusedFunction.apply(x_src, a_src, a_dst, ptr, idx, int(num_dst), float(negative_slope))
 
 
+def gat_layer_supported(x_src, att_src, att_dst, bias):
+    """True when gat_layer covers these tensors (the shapes of gat_fused, fp32 parameters)."""
+    return (gat_fused_supported(x_src) and not GAT_ORDERED_ATT_GRAD and x_src.is_contiguous()
+            and all(t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous())
+                    for t in (att_src, att_dst, bias)))
+
+
+def gat_layer(x_src, att_src, att_dst, bias, ptr, idx, num_dst, negative_slope, concat):
+    """A GAT layer behind its linear transform: attention scores, softmax-weighted neighbour sum (gat_fused), heads side by
+    side (concat) or averaged, bias. x_src [n_src, H, C] -> [num_dst, H * C] or [num_dst, C]; differentiable in x_src, the
+    attention vectors and the bias."""
+    return _native.gat_layer(x_src, att_src, att_dst, bias, ptr, idx, int(num_dst), float(negative_slope), bool(concat))
+
+
 def edge_value_degree(ptr, num_dst, num_edge):
     """val[e] = 1 / in-degree of e's destination (binding.cpp:24-25)."""
     _cuda(ptr, "ptr", _INDEX_DTYPES)

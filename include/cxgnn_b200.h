@@ -360,6 +360,18 @@ int cxg_gat_att_grad(const float *feat, const float *g_src, const float *g_dst, 
                      size_t workspace_bytes, void *stream);
 
 /*
+ * Both of the above in one pass, the feature gradient added to dx: dx[n, h, :] += g_src[n, h] * att_src[h, :] +
+ * (n < n_dst) * g_dst[n, h] * att_dst[h, :]; grad_att_src and grad_att_dst as cxg_gat_att_grad, whose workspace size holds.
+ */
+int cxg_gat_scores_backward_add(const float *feat, const float *g_src, const float *g_dst, const float *att_src,
+                                const float *att_dst, float *dx, float *grad_att_src, float *grad_att_dst,
+                                int64_t n_src, int64_t n_dst, int heads, int c, void *workspace,
+                                size_t workspace_bytes, void *stream);
+
+/* out[n, :] = mean over heads of x[n, h, :] (+ bias, which may be NULL), fp32, x [n, heads, c] (cxgnncomp/graph_conv.py:487-494). */
+int cxg_head_mean_bias(const float *x, const float *bias, float *out, int64_t n, int heads, int c, void *stream);
+
+/*
  * out[c] = sum over the n_row rows of x[r, c] (x row-major [n_row, width], dtype CXG_F32 or CXG_BF16, out float32):
  * the gradient of the bias that MyGATConv / MyGCNConv add to every output row (cxgnncomp/graph_conv.py:493-494,
  * 543-545, 622-623; the reference leaves it to autograd's sum). Fixed two-level order of additions (contiguous row chunks,
