@@ -466,6 +466,98 @@ Tensor linear(const Tensor &x, const Tensor &w, const optional<Tensor> &bias, co
   return linear_product(x, w, false, bias, add);
 }
 
+// ---- SAGE layer ------------------------------------------------------------------------------------------------------
+// into += g . w, or g . w into a new matrix
+Tensor linear_input_grad(const Tensor &g, const Tensor &w, const Tensor &into) {
+  const int n = static_cast<int>(g.size(1)), k = static_cast<int>(w.size(1));
+  if (dense_rows(g) && lib.cxg_linear_f32_supported(g.size(0), n, k) && (!into.defined() || aligned16(into))) {
+    const Tensor out = into.defined() ? into : at::empty({g.size(0), k}, g.options());
+    check(lib.cxg_linear_f32(g.data_ptr<float>(), w.data_ptr<float>(), nullptr, into.defined() ? into.data_ptr<float>() : nullptr,
+                             out.data_ptr<float>(), g.size(0), n, k, 1, stream_of(g)),
+          "cxg_linear_f32");
+    return out;
+  }
+  return into.defined() ? into.addmm_(g, w) : at::mm(g, w);
+}
+
+// mean(x) . wl^T + x[:n] . wr^T + bl, the mean taken before (`first`) or behind the product with wl. As one operator the
+// gradient of x[:n] is added to that of the aggregation in place; as separate ones it was a matrix of zeros, a copy and a sum.
+class SageLayerFunction : public torch::autograd::Function<SageLayerFunction> {
+ public:
+  static Tensor run(const Tensor &x, const Tensor &ptr, const Tensor &idx, const Tensor &wl, const Tensor &wr,
+                    const optional<Tensor> &bl, int64_t n, bool first, int64_t flags, int64_t split, Tensor *mean) {
+    auto aggregate = [&](const Tensor &t) {
+      return spmm(t, ptr, idx, n, c10::nullopt, CXG_MEAN, c10::nullopt, c10::nullopt, c10::nullopt, 0, c10::nullopt, flags, split);
+    };
+    Tensor out;
+    if (first) {
+      const Tensor m = aggregate(x);
+      if (mean != nullptr) *mean = m;
+      out = linear_product(m, wl, false, bl, c10::nullopt);
+    } else {
+      out = aggregate(linear_product(x, wl, false, bl, c10::nullopt));
+    }
+    check(lib.cxg_linear_f32(x.data_ptr<float>(), wr.data_ptr<float>(), nullptr, out.data_ptr<float>(), out.data_ptr<float>(), n,
+                             static_cast<int>(x.size(1)), static_cast<int>(wr.size(0)), 0, stream_of(x)),
+          "cxg_linear_f32");
+    return out;
+  }
+  static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &ptr, const Tensor &idx, const Tensor &wl,
+                        const Tensor &wr, const optional<Tensor> &bl, int64_t n, bool first, int64_t flags, int64_t split) {
+    Tensor mean;
+    const Tensor out = run(x, ptr, idx, wl, wr, bl, n, first, flags, split, &mean);
+    ctx->save_for_backward({x, ptr, idx, wl, wr, mean});
+    ctx->saved_data["bias"] = bl.has_value();
+    ctx->saved_data["n"] = n;
+    ctx->saved_data["first"] = first;
+    ctx->saved_data["flags"] = flags;
+    ctx->saved_data["split"] = split;
+    return out;
+  }
+  static variable_list backward(AutogradContext *ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &ptr = saved[1], &idx = saved[2], &wl = saved[3], &wr = saved[4], &mean = saved[5];
+    const int64_t n = ctx->saved_data["n"].toInt(), flags = ctx->saved_data["flags"].toInt(), split = ctx->saved_data["split"].toInt();
+    const bool need_x = ctx->needs_input_grad(0), need_wl = ctx->needs_input_grad(3), need_wr = ctx->needs_input_grad(4);
+    const bool need_bl = ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(5);
+    const Tensor g = grads[0].contiguous();
+    c10::cuda::CUDAGuard guard(g.device());
+    auto back = [&](const Tensor &t) { return spmm_transposed(t, ptr, idx, n, x.size(0), c10::nullopt, CXG_MEAN, flags, split); };
+    Tensor dx, dwl, dwr, dbl;
+    if (ctx->saved_data["first"].toBool()) {
+      if (need_x) dx = back(linear_input_grad(g, wl, Tensor()));
+      if (need_wl) dwl = linear_weight_grad(g, mean);
+      if (need_bl) dbl = rows_sum(g);
+    } else if (need_x || need_wl || need_bl) {
+      const Tensor dh = back(g);
+      if (need_x) dx = linear_input_grad(dh, wl, Tensor());
+      if (need_wl) dwl = linear_weight_grad(dh, x);
+      if (need_bl) dbl = rows_sum(dh);
+    }
+    if (need_x) linear_input_grad(g, wr, dx.narrow(0, 0, n));
+    if (need_wr) dwr = linear_weight_grad(g, x.narrow(0, 0, n));
+    return {dx, Tensor(), Tensor(), dwl, dwr, dbl, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// None when the operator does not cover the arguments.
+optional<Tensor> sage_layer(const Tensor &x, const Tensor &ptr, const Tensor &idx, const Tensor &wl, const Tensor &wr,
+                            const optional<Tensor> &bl, int64_t n, bool first, int64_t flags, int64_t split) {
+  if (n < 1 || !dense_rows(x) || x.size(0) < n || idx.size(0) < 1 || ptr.size(0) - 1 < n || wl.size(0) != wr.size(0) ||
+      !linear_fits(x, wl) || !linear_fits(x, wr) ||
+      !lib.cxg_linear_f32_supported(n, static_cast<int>(x.size(1)), static_cast<int>(wl.size(0))) ||
+      at::autocast::is_autocast_enabled(at::kCUDA) ||
+      (bl && (bl->scalar_type() != at::kFloat || !bl->is_contiguous() || bl->device() != x.device() || bl->numel() != wl.size(0))))
+    return c10::nullopt;
+  index_of(ptr, "ptr");
+  index_of(idx, "idx");
+  c10::cuda::CUDAGuard guard(x.device());
+  if (at::GradMode::is_enabled() &&
+      (x.requires_grad() || wl.requires_grad() || wr.requires_grad() || (bl && bl->requires_grad())))
+    return SageLayerFunction::apply(x, ptr, idx, wl, wr, bl, n, first, flags, split);
+  return SageLayerFunction::run(x, ptr, idx, wl, wr, bl, n, first, flags, split, nullptr);
+}
+
 // ---- GAT layer -------------------------------------------------------------------------------------------------------
 Tensor head_mean_bias(const Tensor &x, const optional<Tensor> &bias, int64_t heads, int64_t c) {
   Tensor out = at::empty({x.size(0), c}, x.options());
@@ -641,6 +733,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gather_rows", &gather_rows);
   m.def("linear", &linear);
   m.def("gat_layer", &gat_layer);
+  m.def("sage_layer", &sage_layer);
   m.def("head_mean_bias", [](const Tensor &x, const optional<Tensor> &bias, int64_t heads, int64_t c) {
     f32(x, "x");
     c10::cuda::CUDAGuard guard(x.device());

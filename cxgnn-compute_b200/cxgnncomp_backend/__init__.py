@@ -1060,6 +1060,16 @@ def gat_fused(x_src, a_src, a_dst, ptr, idx, num_dst, negative_slope):
     return _GatFusedFunction.apply(x_src, a_src, a_dst, ptr, idx, int(num_dst), float(negative_slope))
 
 
+def sage_layer(x, ptr, idx, weight_neighbour, weight_root, bias, num_node, aggregate_first):
+    """mean over the neighbours of x, times weight_neighbour, + x[:num_node] times weight_root + bias as one operator (the
+    mean before or behind its product), differentiable in x and the parameters; None where it does not cover the arguments
+    (other types than fp32, row widths that linear does not take, scattered backward)."""
+    if BACKWARD_MODE == "scatter":
+        return None
+    return _native.sage_layer(x, ptr, idx, weight_neighbour, weight_root, bias, int(num_node), aggregate_first, EXTRA_SPMM_FLAGS,
+                              SPLIT_EDGES)
+
+
 def gat_layer_supported(x_src, att_src, att_dst, bias):
     """True when gat_layer covers these tensors (the shapes of gat_fused, fp32 parameters)."""
     return (gat_fused_supported(x_src) and not GAT_ORDERED_ATT_GRAD and x_src.is_contiguous()
