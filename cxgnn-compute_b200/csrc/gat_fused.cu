@@ -374,7 +374,8 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_walk(const __grid_constant
 // the edges of one row.
 //
 // Forward. Lane l scores the edges (l >> log2 H) + j * (32 >> log2 H) of a step for head l & (H - 1); P = scores per lane.
-template <int VB, int NV, int U, int P, int MINB>
+// ST: vectors that lie across two heads (C not a multiple of the vector, at least as large as one; the row is).
+template <int VB, int NV, int U, int P, int MINB, bool ST = false>
 __global__ void __launch_bounds__(kThreads, MINB) gat_wide_forward(const __grid_constant__ GatArgs a) {
   constexpr int W = VB / 4;
   __shared__ float probs[kThreads / 32][P * 32];
@@ -401,6 +402,24 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_wide_forward(const __grid_
   const float *prob_of[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q) prob_of[q] = prob + head[q];
+  int next_head[ST ? NV : 1], own[ST ? NV : 1];  // head of a vector's last value, and how many values the first head has
+  if constexpr (ST)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      next_head[q] = (col[q] + W - 1) / a.c;
+      own[q] = (head[q] + 1) * a.c - col[q];
+    }
+  // a value per head, held by the lanes of the head's index, times the accumulators
+  auto scale_heads = [&](float (&acc)[NV][W], float per_head) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      const float k = __shfl_sync(0xffffffffu, per_head, head[q]);
+      float k2 = k;
+      if constexpr (ST) k2 = __shfl_sync(0xffffffffu, per_head, next_head[q]);
+#pragma unroll
+      for (int i = 0; i < W; ++i) acc[q][i] *= ST && i >= own[q] ? k2 : k;
+    }
+  };
   const float *x = static_cast<const float *>(a.w.x);
   float *y = static_cast<float *>(a.w.y);
   auto empty_row = [&](int64_t r) {
@@ -480,12 +499,7 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_wide_forward(const __grid_
           const float keep = exp_flush(m - mn);
           m = mn;
           s *= keep;
-#pragma unroll
-          for (int q = 0; q < NV; ++q) {
-            const float k = __shfl_sync(0xffffffffu, keep, head[q]);
-#pragma unroll
-            for (int i = 0; i < W; ++i) acc[q][i] *= k;
-          }
+          scale_heads(acc, keep);
         }
 #pragma unroll
         for (int j = 0; j < P; ++j) {
@@ -496,7 +510,15 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_wide_forward(const __grid_
         __syncwarp();
         auto add = [&](int u) {
 #pragma unroll
-          for (int q = 0; q < NV; ++q) scale_add<W>(acc[q], v[u][q], prob_of[q][u << hs]);
+          for (int q = 0; q < NV; ++q) {
+            if constexpr (ST) {
+              const float k = prob_of[q][u << hs], k2 = prob[(u << hs) + next_head[q]];
+#pragma unroll
+              for (int i = 0; i < W; ++i) acc[q][i] = fmaf(v[u][q][i], i >= own[q] ? k2 : k, acc[q][i]);
+            } else {
+              scale_add<W>(acc[q], v[u][q], prob_of[q][u << hs]);
+            }
+          }
         };
         if (edges == (1u << U) - 1u) {
 #pragma unroll
@@ -513,12 +535,9 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_wide_forward(const __grid_
         for (int o = H; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         const bool row_done = p + q1 == w.rend;
         if (row_done && w.rstart >= 0) {
-          const float inv = 1.f / s;
+          scale_heads(acc, 1.f / s);
 #pragma unroll
           for (int q = 0; q < NV; ++q) {
-            const float k = __shfl_sync(0xffffffffu, inv, head[q]);
-#pragma unroll
-            for (int i = 0; i < W; ++i) acc[q][i] *= k;
             if (on[q]) store_floats<W>(y + w.row * width + col[q], acc[q]);
           }
           if (lane < H) {
@@ -866,40 +885,46 @@ __device__ void gat_chain(const GatArgs &a, int64_t ts, int64_t k0, int64_t n, i
 
 // Rows that tiles cut: one warp per tile, the roles of walk_fix (spmm_walk.cu).
 template <int VW, int SV, bool BWD>
-__global__ void __launch_bounds__(256, 3) gat_fix(const __grid_constant__ GatArgs a) {
+__global__ void __launch_bounds__(256, 3) gat_fix(const __grid_constant__ GatArgs a, int per) {
   dependency_wait();
   const int lane = threadIdx.x & 31;
   const WalkArgs &w = a.w;
   const int64_t e_total = edge_total(w);
-  const int64_t n_warps = static_cast<int64_t>(gridDim.x) * 8;
-  for (int64_t t = blockIdx.x * 8ll + (threadIdx.x >> 5); t < w.max_tiles; t += n_warps) {
+  // as walk_fix: `per` tiles are looked over at once, a lane for each of a tile's two roles
+  const int64_t t = (blockIdx.x * 8ll + (threadIdx.x >> 5)) * per + (lane & (per - 1));
+  bool lead = false;
+  int64_t row = 0;
+  int ts = 0, k = 0, m = 0;
+  if (lane < 2 * per && t < w.max_tiles && t * w.tile < e_total) {
     const WalkTile here = w.tiles[t], next = w.tiles[t + 1];  // not written behind the last tile, whose end is e_total
-    if (t * w.tile >= e_total || next.begin <= here.begin) continue;
-    const bool follows = next.row < w.n_dst;
-    const int64_t head_begin = load_ptr(w.ptr, here.row, w.ptr_bytes), head_end = load_ptr(w.ptr, here.row + 1, w.ptr_bytes);
-    const int64_t tail_begin = follows ? load_ptr(w.ptr, next.row, w.ptr_bytes) : next.begin;
-    const int64_t tail_end = follows ? load_ptr(w.ptr, next.row + 1, w.ptr_bytes) : next.begin;
-    for (int role = 0; role < 2; ++role) {
-      const int64_t row = role == 0 ? next.row : here.row;
-      const int64_t rb = role == 0 ? tail_begin : head_begin;
-      if (role == 0 ? (rb >= next.begin || rb < here.begin) : rb >= here.begin) continue;
-      const int64_t ts = role == 0 ? t : rb / w.tile;
-      const int64_t k = t - ts;
-      if (k % kGatSeq != 0) continue;
-      const int64_t re = min(role == 0 ? tail_end : head_end, e_total);
-      const int64_t m = (re - 1) / w.tile - ts + 1;
-      const int64_t n_blocks = (m + kGatSeq - 1) / kGatSeq;
-      gat_chain<VW, SV, BWD, false>(a, ts, k, min(static_cast<int64_t>(kGatSeq), m - k), 1, n_blocks > 1, row, lane);
-      if (n_blocks == 1) continue;
-      __threadfence();
-      __syncwarp();
-      int old = 0;
-      if (lane == 0) old = atomicAdd(w.count + ts, 1);
-      old = __shfl_sync(0xffffffffu, old, 0);
-      if (old + 1 != n_blocks) continue;
-      __threadfence();
-      gat_chain<VW, SV, BWD, true>(a, ts, 0, n_blocks, kGatSeq, false, row, lane);
+    const bool tail = lane < per;
+    row = tail ? next.row : here.row;
+    if (next.begin > here.begin && row < w.n_dst) {
+      const int64_t rb = load_ptr(w.ptr, row, w.ptr_bytes);
+      const int64_t re = min(load_ptr(w.ptr, row + 1, w.ptr_bytes), e_total);
+      if (tail ? (rb < next.begin && rb >= here.begin) : rb < here.begin) {
+        const int64_t first = tail ? t : rb / w.tile;
+        ts = static_cast<int>(first), k = static_cast<int>(t - first);
+        m = static_cast<int>((re - 1) / w.tile - first + 1);
+        lead = k % kGatSeq == 0;
+      }
     }
+  }
+  for (unsigned left = __ballot_sync(0xffffffffu, lead); left != 0; left &= left - 1) {
+    const int src = __ffs(left) - 1;
+    const int jts = __shfl_sync(0xffffffffu, ts, src), jk = __shfl_sync(0xffffffffu, k, src), jm = __shfl_sync(0xffffffffu, m, src);
+    const int64_t jrow = __shfl_sync(0xffffffffu, row, src);
+    const int n_blocks = (jm + kGatSeq - 1) / kGatSeq;
+    gat_chain<VW, SV, BWD, false>(a, jts, jk, min(kGatSeq, jm - jk), 1, n_blocks > 1, jrow, lane);
+    if (n_blocks == 1) continue;
+    __threadfence();
+    __syncwarp();
+    int old = 0;
+    if (lane == 0) old = atomicAdd(w.count + jts, 1);
+    old = __shfl_sync(0xffffffffu, old, 0);
+    if (old + 1 != n_blocks) continue;
+    __threadfence();
+    gat_chain<VW, SV, BWD, true>(a, jts, 0, n_blocks, kGatSeq, false, jrow, lane);
   }
 }
 
@@ -1165,6 +1190,20 @@ cudaError_t launch_walk(GatArgs &a, cudaStream_t st) {
     CXG_GAT_BWD(4, 2, 2, 3)
     return cudaErrorInvalidValue;
   } else {
+    // Rows of whole 16-byte vectors whose heads are not (class counts), from 65 values on: vectors that lie across two heads,
+    // in place of single values (16 heads of 15: 957 us, now 522; 4 of 17: 404, now 314; 4 of 47: 519, now 495) and of
+    // 8-byte ones from 16 values per head on (4 of 30: 357, now 327; 8 of 10 would take 376 instead of 344).
+    const bool across = vb < 16 && (vb == 4 || a.c >= 16) && a.w.width % 4 == 0 && a.w.width > 64 && a.c >= 4 &&
+                        (reinterpret_cast<uintptr_t>(a.w.x) | reinterpret_cast<uintptr_t>(a.w.y)) % 16 == 0;
+#define CXG_GAT_ACROSS(NV, U, P, CTAS) \
+  if (across && a.w.width <= 128 * NV && U * a.heads <= 32 * P) go(gat_wide_forward<16, NV, U, P, CTAS, true>, 32, CTAS); else
+    CXG_GAT_ACROSS(1, 8, 1, 6)
+    CXG_GAT_ACROSS(1, 8, 4, 6)
+    CXG_GAT_ACROSS(2, 8, 1, 4)
+    CXG_GAT_ACROSS(2, 4, 1, 5)
+    CXG_GAT_ACROSS(2, 4, 2, 5)
+    CXG_GAT_ACROSS(4, 4, 2, 3)
+#undef CXG_GAT_ACROSS
     CXG_GAT(16, 8, 8, 6)
     CXG_GAT(16, 16, 8, 6)
     CXG_GAT(8, 8, 8, 6)
@@ -1189,15 +1228,16 @@ cudaError_t launch_walk(GatArgs &a, cudaStream_t st) {
 #undef CXG_GAT_FWD
 #undef CXG_GAT_BWD
   if (err != cudaSuccess) return err;
-  int64_t fg = (a.w.max_tiles + 7) / 8;
-  if (fg > kNumSM * 8) fg = kNumSM * 8;
-  const unsigned grid = static_cast<unsigned>(fg);
+  // tiles a warp looks over: one while the chip holds a warp for each, up to sixteen (two roles on 32 lanes)
+  int per = 1;
+  while (per < 16 && a.w.max_tiles > static_cast<int64_t>(per) * kNumSM * 24) per *= 2;
+  const unsigned grid = static_cast<unsigned>((a.w.max_tiles + 8 * per - 1) / (8 * per));
   if (a.c % 4 == 0)
-    err = launch_dependent(gat_fix<4, 1, BWD>, grid, 256, 0, st, a);
+    err = launch_dependent(gat_fix<4, 1, BWD>, grid, 256, 0, st, a, per);
   else if (a.w.width % 4 == 0)  // vectors that lie across two heads
-    err = launch_dependent(gat_fix<4, 4, BWD>, grid, 256, 0, st, a);
+    err = launch_dependent(gat_fix<4, 4, BWD>, grid, 256, 0, st, a, per);
   else
-    err = launch_dependent(gat_fix<1, 1, BWD>, grid, 256, 0, st, a);
+    err = launch_dependent(gat_fix<1, 1, BWD>, grid, 256, 0, st, a, per);
   count_launches(3);
   return err;
 }

@@ -59,3 +59,18 @@ def test_scores_and_mean(cuda, h, c):
         assert rel_err(a_s.cpu(), (x.double() * s.double()).sum(-1)) < 2e-6
         assert rel_err(a_d.cpu(), (x.double() * d.double()).sum(-1)[:(n + 1) // 2]) < 2e-6
         assert rel_err(be._native.head_mean_bias(x.cuda(), b.cuda(), h, c).cpu(), x.double().mean(1) + b.double()) < 2e-6
+
+
+@pytest.mark.parametrize("h,c", [(4, 17), (4, 21), (4, 30), (16, 5), (16, 15), (8, 27), (8, 41), (4, 47), (4, 63), (2, 62)])
+def test_vectors_across_heads(cuda, h, c):
+    import cxgnncomp_backend as be
+    gen = torch.Generator().manual_seed(h * c)
+    n = 600
+    deg = torch.randint(0, 9, (n,), generator=gen)
+    deg[5] = 9000  # cut by many tiles
+    ptr = torch.cat([torch.zeros(1, dtype=torch.int64), deg.cumsum(0)])
+    idx = torch.randint(0, n, (int(ptr[-1]),), generator=gen)
+    args = [randn((n, h, c), 1), randn((1, h, c), 2) * 0.3, randn((1, h, c), 3) * 0.3, randn((c,), 4)]
+    with torch.no_grad():
+        got = be.gat_layer(*[t.cuda() for t in args], ptr.cuda(), idx.cuda(), n, 0.2, False)
+    assert rel_err(got.cpu(), reference(*[t.double() for t in args], ptr, idx, n, 0.2, False)) < 1e-5
