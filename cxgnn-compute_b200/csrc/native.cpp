@@ -417,11 +417,13 @@ bool linear_fits(const Tensor &x, const Tensor &w) {
 class LinearFunction : public torch::autograd::Function<LinearFunction> {
  public:
   static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &w, const optional<Tensor> &bias,
-                        const optional<Tensor> &add) {
+                        const optional<Tensor> &add, bool same_bits) {
     ctx->save_for_backward({x, w});
     ctx->saved_data["bias"] = bias.has_value();
     ctx->saved_data["add"] = add.has_value();
-    return linear_product(x, w, false, bias, add);
+    if (!same_bits) return linear_product(x, w, false, bias, add);
+    const Tensor y = at::linear(x, w, bias);
+    return add ? *add + y : y;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
@@ -444,13 +446,15 @@ class LinearFunction : public torch::autograd::Function<LinearFunction> {
       if (ctx->needs_input_grad(1)) dw = linear_weight_grad(g, x);
       if (need_db) db = rows_sum(g);
     }
-    return {dx, dw, db, need_add ? grads[0] : Tensor()};
+    return {dx, dw, db, need_add ? grads[0] : Tensor(), Tensor()};
   }
 };
 
 // x . w^T (+ bias) (+ add): the tensor-core kernel for fp32 matrices it takes, torch otherwise (CPU, other types, autocast,
-// rows that are not whole 16-byte vectors).
-Tensor linear(const Tensor &x, const Tensor &w, const optional<Tensor> &bias, const optional<Tensor> &add) {
+// rows that are not whole 16-byte vectors). same_bits: where a gradient is recorded the product itself is torch's and only
+// the gradients are the kernel's. In front of a ReLU another rounding, though a better one, puts the few activations within
+// rounding of zero on its other side, and each of them moves the gradients of a batch by up to 3e-4 of their norm.
+Tensor linear(const Tensor &x, const Tensor &w, const optional<Tensor> &bias, const optional<Tensor> &add, bool same_bits) {
   const bool fits = linear_fits(x, w) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
                     (!bias || (bias->scalar_type() == at::kFloat && bias->is_contiguous() && bias->device() == x.device() &&
                                bias->dim() == 1 && bias->size(0) == w.size(0)));
@@ -462,7 +466,7 @@ Tensor linear(const Tensor &x, const Tensor &w, const optional<Tensor> &bias, co
   c10::cuda::CUDAGuard guard(x.device());
   if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad() || (bias && bias->requires_grad()) ||
                                      (add && add->requires_grad())))
-    return LinearFunction::apply(x, w, bias, add);
+    return LinearFunction::apply(x, w, bias, add, same_bits);
   return linear_product(x, w, false, bias, add);
 }
 
@@ -485,18 +489,21 @@ Tensor linear_input_grad(const Tensor &g, const Tensor &w, const Tensor &into) {
 class SageLayerFunction : public torch::autograd::Function<SageLayerFunction> {
  public:
   static Tensor run(const Tensor &x, const Tensor &ptr, const Tensor &idx, const Tensor &wl, const Tensor &wr,
-                    const optional<Tensor> &bl, int64_t n, bool first, int64_t flags, int64_t split, Tensor *mean) {
+                    const optional<Tensor> &bl, int64_t n, bool first, int64_t flags, int64_t split, Tensor *mean, bool record) {
     auto aggregate = [&](const Tensor &t) {
       return spmm(t, ptr, idx, n, c10::nullopt, CXG_MEAN, c10::nullopt, c10::nullopt, c10::nullopt, 0, c10::nullopt, flags, split);
     };
+    // the products of a recorded pass keep torch's rounding, as in `linear`
+    auto product = [&](const Tensor &t) { return record ? at::linear(t, wl, bl) : linear_product(t, wl, false, bl, c10::nullopt); };
     Tensor out;
     if (first) {
       const Tensor m = aggregate(x);
       if (mean != nullptr) *mean = m;
-      out = linear_product(m, wl, false, bl, c10::nullopt);
+      out = product(m);
     } else {
-      out = aggregate(linear_product(x, wl, false, bl, c10::nullopt));
+      out = aggregate(product(x));
     }
+    if (record) return out.add_(at::linear(x.narrow(0, 0, n), wr));
     check(lib.cxg_linear_f32(x.data_ptr<float>(), wr.data_ptr<float>(), nullptr, out.data_ptr<float>(), out.data_ptr<float>(), n,
                              static_cast<int>(x.size(1)), static_cast<int>(wr.size(0)), 0, stream_of(x)),
           "cxg_linear_f32");
@@ -505,7 +512,7 @@ class SageLayerFunction : public torch::autograd::Function<SageLayerFunction> {
   static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &ptr, const Tensor &idx, const Tensor &wl,
                         const Tensor &wr, const optional<Tensor> &bl, int64_t n, bool first, int64_t flags, int64_t split) {
     Tensor mean;
-    const Tensor out = run(x, ptr, idx, wl, wr, bl, n, first, flags, split, &mean);
+    const Tensor out = run(x, ptr, idx, wl, wr, bl, n, first, flags, split, &mean, true);
     ctx->save_for_backward({x, ptr, idx, wl, wr, mean});
     ctx->saved_data["bias"] = bl.has_value();
     ctx->saved_data["n"] = n;
@@ -555,7 +562,7 @@ optional<Tensor> sage_layer(const Tensor &x, const Tensor &ptr, const Tensor &id
   if (at::GradMode::is_enabled() &&
       (x.requires_grad() || wl.requires_grad() || wr.requires_grad() || (bl && bl->requires_grad())))
     return SageLayerFunction::apply(x, ptr, idx, wl, wr, bl, n, first, flags, split);
-  return SageLayerFunction::run(x, ptr, idx, wl, wr, bl, n, first, flags, split, nullptr);
+  return SageLayerFunction::run(x, ptr, idx, wl, wr, bl, n, first, flags, split, nullptr, false);
 }
 
 // ---- GAT layer -------------------------------------------------------------------------------------------------------

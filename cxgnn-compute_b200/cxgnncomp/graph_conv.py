@@ -25,11 +25,11 @@ def glorot(t):
 
 
 class Linear(torch.nn.Linear):
-    """torch.nn.Linear on the library's fp32 tensor-core kernel where that takes the matrices (cxgnncomp_backend.linear).
-    `add`: a matrix added to the result in the same pass."""
+    """torch.nn.Linear on the library's fp32 tensor-core kernel where that takes the matrices (cxgnncomp_backend.linear):
+    the result where no gradient is recorded, the gradients otherwise. `add`: a matrix added to the result."""
 
     def forward(self, x, add=None):
-        return cxgnncomp_backend.linear(x, self.weight, self.bias, add)
+        return cxgnncomp_backend.linear(x, self.weight, self.bias, add, same_bits=True)
 
 
 def _plain(module):

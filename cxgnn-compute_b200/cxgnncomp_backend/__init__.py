@@ -692,10 +692,11 @@ def bias_add(y, bias):
     return _BiasAddFunction.apply(y, bias)
 
 
-def linear(x, weight, bias=None, add=None):
+def linear(x, weight, bias=None, add=None, same_bits=False):
     """torch.nn.functional.linear(x, weight, bias) (+ add), on the library's tensor-core kernel for fp32 matrices it takes
-    (error below that of an fp32 GEMM), else torch's. Differentiable in all four."""
-    return _native.linear(x, weight, bias, add)
+    (error below that of an fp32 GEMM), else torch's. Differentiable in all four. same_bits: where gradients are recorded
+    the result is torch's to the bit and the kernels serve the gradients (for what a ReLU follows)."""
+    return _native.linear(x, weight, bias, add, same_bits)
 
 
 _head_sum_c = _sig("cxg_head_sum", [_vp, _vp, _i64, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp])

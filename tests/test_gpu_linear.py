@@ -23,6 +23,7 @@ def test_linear(cuda, m, k, n, bias, add):
     assert rel_err(y.detach().cpu(), want.detach()) < 2e-6
     with torch.no_grad():
         assert torch.equal(be.linear(*dev), y)
+    assert rel_err(be.linear(*dev, same_bits=True).detach().cpu(), want.detach()) < 2e-6
     given = [i for i in range(4) if dev[i] is not None]
     got = torch.autograd.grad(y, [dev[i] for i in given], g.cuda())
     exp = torch.autograd.grad(want, [ref[i] for i in given], g.double())
