@@ -656,8 +656,10 @@ extern "C" int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel,
   const int spans = (k * elem + 127) / 128 + (n * elem + 127) / 128;
   const size_t half = static_cast<size_t>(spans) * (128 * pos);
   const size_t stage = x3 ? 2 * half : half;
-  // the tensor core reads elem spans of x (128 columns) from a tile's start: room behind the last stage for narrow tiles
-  const size_t behind = spans < elem ? static_cast<size_t>(elem - spans) * (128 * pos) : 0;
+  // The tensor core reads elem spans of x (128 columns) from the start of its spans, which for narrow x goes beyond the tile:
+  // room behind the last stage. In the compensated mode the last spans of a stage are x's lo spans.
+  const int spans_x = (k * elem + 127) / 128, over = x3 ? elem - spans_x : elem - spans;
+  const size_t behind = over > 0 ? static_cast<size_t>(over) * (128 * pos) : 0;
   int stages = static_cast<int>((kSmemBudget - 1024 - behind) / stage);
   if (stages > kMaxStages) stages = kMaxStages;
   CXG_REQUIRE(stages >= 1, CXG_EUNSUPPORTED, "cxg_typed_wgrad: one stage of %zu bytes exceeds shared memory", stage);
