@@ -536,8 +536,10 @@ namespace cxg {
 namespace {
 // alpha_src[n, h] = <feat[n, h, :], att_src[h, :]> for all n; alpha_dst[n, h] = <feat[n, h, :], att_dst[h, :]> for
 // n < n_dst: both attention scores of a GAT layer in one pass over the transformed features. One thread per
-// (node, head), the products of a row added in index order: for rows that are not whole 16-byte vectors (a few lanes per
-// row, as below, took twice as long at 47 values).
+// (node, head), the products of a row added in index order, one fused multiply-add each. The order is part of the result:
+// the sum of two scores goes through a LeakyReLU, and one within rounding of zero that changes sides changes the gradient
+// that comes back through it fivefold. VEC: whole, aligned 16-byte vectors.
+template <bool VEC>
 __global__ void __launch_bounds__(kThreads) gat_scores_kernel(const float *feat, const float *att_src, const float *att_dst,
                                                               float *alpha_src, float *alpha_dst, int64_t n_src,
                                                               int64_t n_dst, int heads, int c) {
@@ -547,60 +549,72 @@ __global__ void __launch_bounds__(kThreads) gat_scores_kernel(const float *feat,
   const int64_t n = i / heads;
   const float *f = feat + i * c, *as = att_src + h * c, *ad = att_dst + h * c;
   float s = 0.f, d = 0.f;
-  for (int j = 0; j < c; ++j) {
-    const float v = __ldg(f + j);
-    s = fmaf(v, __ldg(as + j), s), d = fmaf(v, __ldg(ad + j), d);
+  auto add = [&](float v, int j) { s = fmaf(v, __ldg(as + j), s), d = fmaf(v, __ldg(ad + j), d); };
+  if (VEC) {
+    for (int j = 0; j < c; j += 4) {
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(f + j));
+      add(v.x, j), add(v.y, j + 1), add(v.z, j + 2), add(v.w, j + 3);
+    }
+  } else {
+    for (int j = 0; j < c; ++j) add(__ldg(f + j), j);
   }
   alpha_src[i] = s;
   if (n < n_dst) alpha_dst[i] = d;
 }
 
-// The same for whole 16-byte vectors: `lanes` lanes per (node, head), eight of them in flight, the lane sums joined by a
-// shuffle tree. The number of groups is a multiple of the heads, so a group keeps its head and its attention vectors.
-// (169,343 x 4 heads of 32 values: a thread per (node, head), whose loads lie 128 bytes apart, 42 us, now 28.)
+// The same sums in the same order for heads of 32 and more columns in whole 16-byte vectors. A thread per (node, head) that
+// reads its row from memory asks for 16 bytes of 32 different lines at a time; here a warp takes one head of 32 nodes (so that the attention vectors are
+// the same address for all lanes), brings their rows in with every lane on the next vector, up to 32 columns at a time, and
+// each lane then takes its own row from shared memory. A row there is an odd number of vectors long, so that the eight
+// lanes that are served together lie in different banks. (169,343 nodes, cold: 4 heads of 32 values 37 us, 51 with a thread
+// per pair; 8 of 32 66 (127); 2 of 64 35 (47); 4 of 28, where lines are shared by pairs, 37 (31), 4 of 12 27 (14). Lanes that
+// share a row and join their sums by shuffles take 36 / 52 / 37, and another order.)
+constexpr int kScoreVecs = 8;  // vectors of a row per round
+
 __global__ void __launch_bounds__(kThreads) gat_scores_vec(const float *feat, const float *att_src, const float *att_dst,
                                                            float *alpha_src, float *alpha_dst, int64_t n_src, int64_t n_dst,
-                                                           int heads, int c, int lanes) {
-  constexpr int U = 8;
-  const int lane = threadIdx.x & (lanes - 1);
-  const int64_t total = n_src * heads, groups = static_cast<int64_t>(gridDim.x) * (kThreads / lanes);
-  const int64_t first = (blockIdx.x * static_cast<int64_t>(kThreads) + threadIdx.x) / lanes;
-  const int h = static_cast<int>(first % heads);
-  // every lane of a warp runs the same number of rounds, as the shuffles need
-  for (int64_t i0 = first; i0 - first < total; i0 += U * groups) {
-    float s[U] = {}, d[U] = {};
-    for (int j = lane * 4; j < c; j += lanes * 4) {
-      float4 f[U];
+                                                           int heads, int c) {
+  __shared__ float4 rows[kWarps][32 * (kScoreVecs + 1)];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t w = blockIdx.x * static_cast<int64_t>(kWarps) + warp, n0 = w / heads * 32;
+  if (n0 >= n_src) return;  // the whole warp
+  const int h = static_cast<int>(w % heads), nodes = n_src - n0 < 32 ? static_cast<int>(n_src - n0) : 32;
+  const int vecs = c / 4, step = heads * vecs;  // vectors of a node's head, of a node
+  const float4 *f = reinterpret_cast<const float4 *>(feat) + n0 * step + h * vecs;
+  const float4 *as = reinterpret_cast<const float4 *>(att_src) + h * vecs, *ad = reinterpret_cast<const float4 *>(att_dst) + h * vecs;
+  float4 *mine = rows[warp];
+  float s = 0.f, d = 0.f;
+  for (int j0 = 0; j0 < vecs; j0 += kScoreVecs) {
+    const int now = min(kScoreVecs, vecs - j0), pitch = now | 1;
+    const unsigned magic = 65536u / now + 1;  // q / now for q < 256
+    float4 v[kScoreVecs];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t i = i0 + u * groups;
-        f[u] = i < total ? __ldg(reinterpret_cast<const float4 *>(feat + i * c + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      float as[4], ad[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) as[k] = __ldg(att_src + h * c + j + k), ad[k] = __ldg(att_dst + h * c + j + k);
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        s[u] = fmaf(f[u].x, as[0], s[u]), d[u] = fmaf(f[u].x, ad[0], d[u]);
-        s[u] = fmaf(f[u].y, as[1], s[u]), d[u] = fmaf(f[u].y, ad[1], d[u]);
-        s[u] = fmaf(f[u].z, as[2], s[u]), d[u] = fmaf(f[u].z, ad[2], d[u]);
-        s[u] = fmaf(f[u].w, as[3], s[u]), d[u] = fmaf(f[u].w, ad[3], d[u]);
-      }
+    for (int k = 0; k < kScoreVecs; ++k) {
+      const int q = k * 32 + lane, row = static_cast<int>((q * magic) >> 16);
+      if (row < nodes) v[k] = __ldg(f + static_cast<int64_t>(row) * step + j0 + (q - row * now));
     }
-    for (int o = lanes >> 1; o > 0; o >>= 1)
+    __syncwarp();  // the lanes have read the rows of the round before
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
-        d[u] += __shfl_xor_sync(0xffffffffu, d[u], o);
-      }
-    if (lane == 0)
+    for (int k = 0; k < kScoreVecs; ++k) {
+      const int q = k * 32 + lane, row = static_cast<int>((q * magic) >> 16);
+      if (row < nodes) mine[row * pitch + (q - row * now)] = v[k];
+    }
+    __syncwarp();
+    if (lane < nodes) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t i = i0 + u * groups;
-        if (i >= total) break;
-        alpha_src[i] = s[u];
-        if (i < n_dst * heads) alpha_dst[i] = d[u];
-      }
+      for (int k = 0; k < kScoreVecs; ++k)
+        if (k < now) {
+          const float4 x = mine[lane * pitch + k], a = __ldg(as + j0 + k), b = __ldg(ad + j0 + k);
+          s = fmaf(x.x, a.x, s), d = fmaf(x.x, b.x, d);
+          s = fmaf(x.y, a.y, s), d = fmaf(x.y, b.y, d);
+          s = fmaf(x.z, a.z, s), d = fmaf(x.z, b.z, d);
+          s = fmaf(x.w, a.w, s), d = fmaf(x.w, b.w, d);
+        }
+    }
+  }
+  if (lane < nodes) {
+    alpha_src[(n0 + lane) * heads + h] = s;
+    if (n0 + lane < n_dst) alpha_dst[(n0 + lane) * heads + h] = d;
   }
 }
 
@@ -630,19 +644,14 @@ extern "C" int cxg_gat_scores(const float *feat, const float *att_src, const flo
   CXG_REQUIRE(feat && att_src && att_dst && alpha_src && (alpha_dst || n_dst == 0), CXG_ENULL,
               "cxg_gat_scores: NULL argument");
   CXG_REQUIRE(c % 4 != 0 || reinterpret_cast<uintptr_t>(feat) % 16 == 0, CXG_EINVAL, "cxg_gat_scores: feat alignment");
-  if (c % 4 != 0) {
-    const unsigned grid = static_cast<unsigned>((n_src * heads + kThreads - 1) / kThreads);
-    gat_scores_kernel<<<grid, kThreads, 0, as_stream(stream)>>>(feat, att_src, att_dst, alpha_src, alpha_dst, n_src, n_dst, heads,
-                                                                c);
+  // narrower heads share lines between neighbouring threads, which the thread per pair then finds in L1
+  if (c >= 32 && c % 4 == 0 && ((reinterpret_cast<uintptr_t>(att_src) | reinterpret_cast<uintptr_t>(att_dst)) % 16) == 0) {
+    const unsigned grid = static_cast<unsigned>(((n_src + 31) / 32 * heads + kWarps - 1) / kWarps);
+    gat_scores_vec<<<grid, kThreads, 0, as_stream(stream)>>>(feat, att_src, att_dst, alpha_src, alpha_dst, n_src, n_dst, heads, c);
   } else {
-    // as many lanes as a row of a head has vectors, rounded down to a power of two, so that few lanes idle in the last round
-    int lanes = 1;
-    while (lanes < 32 && 8 * lanes <= c) lanes *= 2;
-    int64_t grid = (n_src * heads * lanes + 8 * kThreads - 1) / (8 * kThreads);
-    if (grid > kNumSM * 16) grid = kNumSM * 16;
-    grid = (grid + heads - 1) / heads * heads;  // whole numbers of nodes between a group's rounds
-    gat_scores_vec<<<static_cast<unsigned>(grid), kThreads, 0, as_stream(stream)>>>(feat, att_src, att_dst, alpha_src, alpha_dst,
-                                                                                    n_src, n_dst, heads, c, lanes);
+    const unsigned grid = static_cast<unsigned>((n_src * heads + kThreads - 1) / kThreads);
+    auto kernel = c % 4 == 0 ? gat_scores_kernel<true> : gat_scores_kernel<false>;
+    kernel<<<grid, kThreads, 0, as_stream(stream)>>>(feat, att_src, att_dst, alpha_src, alpha_dst, n_src, n_dst, heads, c);
   }
   count_launches(1);
   return check_launch("cxg_gat_scores");

@@ -452,8 +452,9 @@ class LinearFunction : public torch::autograd::Function<LinearFunction> {
 
 // x . w^T (+ bias) (+ add): the tensor-core kernel for fp32 matrices it takes, torch otherwise (CPU, other types, autocast,
 // rows that are not whole 16-byte vectors). same_bits: where a gradient is recorded the product itself is torch's and only
-// the gradients are the kernel's. In front of a ReLU another rounding, though a better one, puts the few activations within
-// rounding of zero on its other side, and each of them moves the gradients of a batch by up to 3e-4 of their norm.
+// the gradients are the kernel's. In front of a ReLU (and of the LeakyReLU on a GAT layer's scores) another rounding, though
+// a better one, puts the few values within rounding of zero on its other side, and each of them moves the gradients: those
+// of a sampled batch by up to 3e-4 of their norm, those of a GAT layer by up to 2e-3.
 Tensor linear(const Tensor &x, const Tensor &w, const optional<Tensor> &bias, const optional<Tensor> &add, bool same_bits) {
   const bool fits = linear_fits(x, w) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
                     (!bias || (bias->scalar_type() == at::kFloat && bias->is_contiguous() && bias->device() == x.device() &&

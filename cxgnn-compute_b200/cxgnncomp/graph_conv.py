@@ -479,7 +479,8 @@ class MyGATConv(torch.nn.Module):
         if self.tensor_core_linear:  # the layer's linear transform on the library's tensor-core kernels
             x_src = cxgnncomp_backend.dense_linear(x, self.lin_src).view(-1, H, C)
         else:
-            x_src = cxgnncomp_backend.linear(x, self.lin_src).view(-1, H, C)
+            # recorded: torch's rounding, as in front of a ReLU (the sums of scores go through a LeakyReLU)
+            x_src = cxgnncomp_backend.linear(x, self.lin_src, same_bits=True).view(-1, H, C)
         if (x_src.dtype == torch.float32 and self.fused_scores and self.fused_aggregate
                 and self.edge_softmax_schedule == "fused" and num_dst > 0
                 and cxgnncomp_backend.gat_layer_supported(x_src, self.att_src, self.att_dst, self.bias)):
@@ -520,9 +521,11 @@ class MyGATConv(torch.nn.Module):
         edge_value = self.edge_softmax(ptr=ptr, idx=idx, att_src=alpha_src.contiguous(), att_dst=alpha_dst.contiguous(),
                                        num_edge=num_edge, relu_l=self.negative_slope).reshape(-1)
         if self.out_channels < self.in_channels:
-            out = sage_sum_forward_edge_value(cxgnncomp_backend.linear(x, self.lin_src), ptr, idx, edge_value, num_dst)
+            out = sage_sum_forward_edge_value(cxgnncomp_backend.linear(x, self.lin_src, same_bits=True), ptr, idx, edge_value,
+                                              num_dst)
         else:
-            out = cxgnncomp_backend.linear(sage_sum_forward_edge_value(x, ptr, idx, edge_value, num_dst), self.lin_src)
+            out = cxgnncomp_backend.linear(sage_sum_forward_edge_value(x, ptr, idx, edge_value, num_dst), self.lin_src,
+                                           same_bits=True)
         return cxgnncomp_backend.bias_add(out, self.bias) if self.bias is not None else out
 
     def forward(self, x, ptr, idx, num_dst, num_src, num_edge):

@@ -695,7 +695,7 @@ def bias_add(y, bias):
 def linear(x, weight, bias=None, add=None, same_bits=False):
     """torch.nn.functional.linear(x, weight, bias) (+ add), on the library's tensor-core kernel for fp32 matrices it takes
     (error below that of an fp32 GEMM), else torch's. Differentiable in all four. same_bits: where gradients are recorded
-    the result is torch's to the bit and the kernels serve the gradients (for what a ReLU follows)."""
+    the result is torch's to the bit and the kernels serve the gradients (for what a ReLU or a LeakyReLU follows)."""
     return _native.linear(x, weight, bias, add, same_bits)
 
 
