@@ -714,6 +714,7 @@ std::tuple<Tensor, Tensor, Tensor, std::vector<int64_t>, std::vector<int64_t>> s
     c10::cuda::getCurrentCUDAStream(seeds.device().index()).synchronize();
   }
   const int64_t *h = host_sizes.data_ptr<int64_t>();
+  if (h[0] < 0) fail("sample_batch: seeds must be node ids in [0, " + std::to_string(n_nodes) + ")");
   std::vector<int64_t> known(h, h + hops + 1), edges(h + hops + 2, h + 2 * (hops + 1));
   const int64_t rows = known[hops - 1];
   return {nodes.narrow(0, 0, known[hops]), ptr.narrow(0, 0, rows + 1), idx.narrow(0, 0, edges[hops - 1]), known, edges};

@@ -74,10 +74,23 @@ __global__ void __launch_bounds__(kThreads) start_batch(BatchArgs a, const int64
     a.row_ptr[0] = 0;
   }
   if (i < n_seeds) {
-    const int64_t v = seeds[i];
+    int64_t v = seeds[i];
+    if (v >= 0 && v < a.n_nodes)
+      a.local_of[v] = i;
+    else
+      v = -1;  // a row without neighbours; forget_nodes reports it
     a.nodes[i] = v;
-    a.local_of[v] = i;
   }
+}
+
+// First edge and number of edges of a node.
+__device__ __forceinline__ int64_t degree(const BatchArgs &a, int64_t v, int64_t *first) {
+  if (v < 0) {
+    *first = 0;
+    return 0;
+  }
+  *first = load_ptr(a.gptr, v, a.ptr_bytes);
+  return load_ptr(a.gptr, v + 1, a.ptr_bytes) - *first;
 }
 
 __device__ __forceinline__ void translate(const BatchArgs &a, int64_t from, int64_t to, int64_t tid, int64_t threads) {
@@ -96,8 +109,8 @@ __global__ void __launch_bounds__(kThreads) count_front(BatchArgs a, int hop, in
   __syncthreads();
   int32_t mine = 0;
   for (int64_t i = b0 + threadIdx.x; i < min(f1, b0 + a.per_block); i += kThreads) {
-    const int64_t v = a.nodes[i];
-    const int64_t deg = load_ptr(a.gptr, v + 1, a.ptr_bytes) - load_ptr(a.gptr, v, a.ptr_bytes);
+    int64_t lo;
+    const int64_t deg = degree(a, a.nodes[i], &lo);
     mine += static_cast<int32_t>(deg < fanout ? deg : fanout);
   }
   for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
@@ -131,8 +144,8 @@ __global__ void __launch_bounds__(kThreads) draw_front(BatchArgs a, int hop, int
     const int64_t i = c0 + threadIdx.x;
     int64_t c = 0;
     if (i < b1) {
-      const int64_t v = a.nodes[i];
-      const int64_t deg = load_ptr(a.gptr, v + 1, a.ptr_bytes) - load_ptr(a.gptr, v, a.ptr_bytes);
+      int64_t lo;
+      const int64_t deg = degree(a, a.nodes[i], &lo);
       c = deg < fanout ? deg : fanout;
     }
     int64_t inc = c;
@@ -158,7 +171,8 @@ __global__ void __launch_bounds__(kThreads) draw_front(BatchArgs a, int hop, int
   const IdxT *gidx = static_cast<const IdxT *>(a.gidx);
   for (int64_t i = b0 + threadIdx.x / GS; i < b1; i += kThreads / GS) {
     const int64_t v = a.nodes[i];
-    const int64_t lo = load_ptr(a.gptr, v, a.ptr_bytes), deg = load_ptr(a.gptr, v + 1, a.ptr_bytes) - lo;
+    int64_t lo;
+    const int64_t deg = degree(a, v, &lo);
     const int n = static_cast<int>(deg < fanout ? deg : fanout);
     const int64_t out = a.row_ptr[i + 1] - n;
     int64_t pick[PER];
@@ -267,8 +281,13 @@ __global__ void __launch_bounds__(kThreads) finish_edges(BatchArgs a, int hops) 
 }
 __global__ void __launch_bounds__(kThreads) forget_nodes(BatchArgs a, int hops) {
   const int64_t n = a.known[hops];
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(kThreads) + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * kThreads)
-    a.local_of[a.nodes[i]] = -1;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(kThreads) + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * kThreads) {
+    const int64_t v = a.nodes[i];
+    if (v >= 0)
+      a.local_of[v] = -1;
+    else
+      a.known[0] = -1;  // a seed outside the graph
+  }
 }
 
 struct BatchBounds {
@@ -288,7 +307,8 @@ int batch_bounds(int64_t n_seeds, const int *fanouts, int hops, int64_t n_nodes,
   for (int h = 0; h < hops; ++h) {
     if (fanouts[h] < 1 || fanouts[h] > kMaxFanout) return CXG_EUNSUPPORTED;
     int64_t e = b->front[h] * fanouts[h];
-    if (e > nnz) e = nnz;
+    // the nodes of a later frontier are distinct, so all of them have nnz edges at most; seeds may repeat
+    if (h > 0 && e > nnz) e = nnz;
     b->edges += e;
     b->rows += b->front[h];
     int64_t fresh = e < n_nodes ? e : n_nodes;

@@ -37,13 +37,15 @@ class NeighborSampler:
         return self._fresh_buf
 
     def sample(self, seeds, seed=0):
-        """seeds: distinct int64 global ids on the graph's device. Returns (nodes, ptr, idx, num_node_in_layer,
+        """seeds: int64 global ids on the graph's device (an id outside the graph raises). Returns (nodes, ptr, idx, num_node_in_layer,
         num_edge_in_layer) with ptr / idx int64 on the device."""
         if cxgnncomp_backend.sample_batch_fits(seeds.shape[0], self.fanouts, self.num_nodes, self.idx.shape[0]):
             # all hops in one call, sizes read back once
             return cxgnncomp_backend.sample_batch(self.ptr, self.idx, seeds, self.fanouts, seed, self.local_of,
                                                   self._marks, self._sizes)
         dev = seeds.device
+        if bool(((seeds < 0) | (seeds >= self.num_nodes)).any()):
+            raise RuntimeError(f"sample: seeds must be node ids in [0, {self.num_nodes})")
         local_of = self.local_of
         nodes = [seeds]
         n_known = seeds.shape[0]

@@ -474,7 +474,9 @@ int cxg_put_rows(const void *in, const int64_t *rows, void *const *peer_base_hos
  * batch ids in ascending order of their node id behind the ones before. nodes[batch id], row_ptr / edges = CSR rows of
  * the expanded nodes in batch ids, sizes[0 .. hops] = nodes known before hop 0, after hop 0, ..., sizes[hops + 1 ..
  * 2 hops + 1] = edges before hop 0, after hop 0, ... (device memory). local_of[n_nodes] is -1 and bitmap[ceil(n_nodes /
- * 32)] zero before and after the call. Up to 16 hops of fanout 1 to 64. cxg_sample_batch_bounds gives the lengths the
+ * 32)] zero before and after the call. Seeds may repeat (each keeps a row of its own; neighbours that are such a node get
+ * the batch id of one of them). A seed outside [0, n_nodes) gets node -1 and an empty row, and sizes[0] is -1 at the end
+ * instead of n_seeds. Up to 16 hops of fanout 1 to 64. cxg_sample_batch_bounds gives the lengths the
  * output arrays need (nodes: max_nodes, row_ptr: max_rows + 1, edges: max_edges) and the scratch bytes; fanouts and
  * hop_seeds are host memory.
  */
