@@ -111,34 +111,84 @@ void *stream_of(const Tensor &t) { return c10::cuda::getCurrentCUDAStream(t.devi
 
 // ---- scratch ---------------------------------------------------------------------------------------------------------
 // One buffer per (device, stream), grown on demand; contents never carry over. `kind` names the entry point family that
-// used it last (whose status word check_device_status can ask for). Calls of one stream are ordered, and this module runs
-// with the interpreter's lock held, so two threads on one stream do not interleave their launches.
+// used it last (whose status word check_device_status can ask for). The launches of one call hand the buffer on to each
+// other, so whoever uses it holds its lock until the last of them is issued: two threads may work on one stream (a backward
+// runs on a thread of the autograd engine, without the interpreter's lock), and launches of another call in between would
+// overwrite what the next kernel reads.
 struct Scratch {
+  std::mutex in_use;
   Tensor buf;
   std::string kind;
 };
 std::mutex scratch_lock;
 std::map<std::pair<int, void *>, Scratch> scratch;
 
-Tensor workspace_on(int device, void *stream, int64_t bytes, const char *kind) {
+Scratch &scratch_of(int device, void *stream) {
   std::lock_guard<std::mutex> hold(scratch_lock);
-  Scratch &s = scratch[{device, stream}];
-  if (!s.buf.defined() || s.buf.numel() < bytes)
-    s.buf = at::empty({std::max<int64_t>(bytes, 1 << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
-  if (s.kind != kind) s.kind = kind;
-  return s.buf;
+  return scratch[{device, stream}];
 }
 
-Tensor workspace(int device, int64_t bytes, const std::string &kind) {
-  return workspace_on(device, c10::cuda::getCurrentCUDAStream(device).stream(), bytes, kind.c_str());
+// Takes the lock without keeping other threads from the interpreter meanwhile: the holder may be Python code.
+std::unique_lock<std::mutex> lock_for_launches(std::mutex &m) {
+  std::unique_lock<std::mutex> hold(m, std::try_to_lock);
+  if (!hold.owns_lock()) {
+    if (PyGILState_Check()) {
+      py::gil_scoped_release others;
+      hold.lock();
+    } else {
+      hold.lock();
+    }
+  }
+  return hold;
 }
+
+// The stream's scratch buffer while this thread may use it.
+struct Workspace {
+  std::unique_lock<std::mutex> hold;
+  Tensor buf;
+  void *data() const { return buf.data_ptr(); }
+  size_t bytes() const { return static_cast<size_t>(buf.numel()); }
+};
+
+Workspace workspace_on(int device, void *stream, int64_t bytes, const char *kind) {
+  Scratch &s = scratch_of(device, stream);
+  Tensor grown;  // allocated without the lock
+  for (;;) {
+    Workspace w;
+    w.hold = lock_for_launches(s.in_use);
+    if (grown.defined() && (!s.buf.defined() || s.buf.numel() < grown.numel())) std::swap(s.buf, grown);
+    if (s.buf.defined() && s.buf.numel() >= bytes) {
+      if (s.kind != kind) s.kind = kind;
+      w.buf = s.buf;
+      return w;
+    }
+    w.hold.unlock();
+    grown = at::empty({std::max<int64_t>(bytes, 1 << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
+  }
+}
+
+// The same for Python: `with` the object, the buffer is the calling thread's until the block ends.
+class HeldWorkspace {
+ public:
+  HeldWorkspace(int device, int64_t bytes, std::string kind) : device_(device), bytes_(bytes), kind_(std::move(kind)) {}
+  Tensor enter() {
+    w_ = workspace_on(device_, c10::cuda::getCurrentCUDAStream(device_).stream(), bytes_, kind_.c_str());
+    return w_.buf;
+  }
+  void exit() { w_ = Workspace(); }
+
+ private:
+  int device_;
+  int64_t bytes_;
+  std::string kind_;
+  Workspace w_;
+};
 
 // (buffer or None, kind) of the current stream
 std::pair<optional<Tensor>, std::string> last_workspace(int device) {
-  std::lock_guard<std::mutex> hold(scratch_lock);
-  auto it = scratch.find({device, c10::cuda::getCurrentCUDAStream(device).stream()});
-  if (it == scratch.end()) return {c10::nullopt, ""};
-  return {it->second.buf, it->second.kind};
+  Scratch &s = scratch_of(device, c10::cuda::getCurrentCUDAStream(device).stream());
+  const auto hold = lock_for_launches(s.in_use);
+  return {s.buf.defined() ? optional<Tensor>(s.buf) : c10::nullopt, s.kind};
 }
 
 // ---- aggregation -----------------------------------------------------------------------------------------------------
@@ -171,8 +221,8 @@ void run_spmm(cxg_spmm_desc &d, const Tensor &on) {
   size_t need = 0;
   check(lib.cxg_spmm_csr_workspace_size(d.n_dst, d.nnz, d.feat, d.heads, d.split_edges, &need), "cxg_spmm_csr_workspace_size");
   void *st = stream_of(on);
-  const Tensor ws = workspace_on(on.device().index(), st, static_cast<int64_t>(need), "spmm");
-  check(lib.cxg_spmm_csr(&d, ws.data_ptr(), static_cast<size_t>(ws.numel()), st), "cxg_spmm_csr");
+  const Workspace ws = workspace_on(on.device().index(), st, static_cast<int64_t>(need), "spmm");
+  check(lib.cxg_spmm_csr(&d, ws.data(), ws.bytes(), st), "cxg_spmm_csr");
 }
 
 // y = A x for the first rows of the graph; x [N, F] or [N, H, F]
@@ -222,11 +272,11 @@ Transposed transpose(const Tensor &ptr, const Tensor &idx, int64_t num_node, int
   size_t need = 0;
   check(lib.cxg_csr_transpose_workspace_size(nnz, &need), "cxg_csr_transpose_workspace_size");
   void *st = stream_of(ptr);
-  const Tensor ws = workspace_on(ptr.device().index(), st, static_cast<int64_t>(need), "");
+  const Workspace ws = workspace_on(ptr.device().index(), st, static_cast<int64_t>(need), "");
   check(lib.cxg_csr_transpose(ptr.data_ptr(), idx.data_ptr(), static_cast<int>(ptr.element_size()),
                               static_cast<int>(idx.element_size()), n, n_src, nnz, t.t_ptr.data_ptr<int64_t>(),
                               t.t_idx.data_ptr(), want_eid ? t.t_eid.data_ptr() : nullptr, t.inv_deg.data_ptr<float>(),
-                              ws.data_ptr(), static_cast<size_t>(ws.numel()), st),
+                              ws.data(), ws.bytes(), st),
         "cxg_csr_transpose");
   return t;
 }
@@ -390,9 +440,9 @@ Tensor linear_weight_grad(const Tensor &g, const Tensor &x) {
   check(lib.cxg_dense_wgrad_f32_workspace_size(m, static_cast<int>(n), static_cast<int>(k), &need),
         "cxg_dense_wgrad_f32_workspace_size");
   void *st = stream_of(x);
-  const Tensor ws = workspace_on(x.device().index(), st, static_cast<int64_t>(need), "");
+  const Workspace ws = workspace_on(x.device().index(), st, static_cast<int64_t>(need), "");
   check(lib.cxg_dense_wgrad_f32(g.data_ptr<float>(), x.data_ptr<float>(), m, static_cast<int>(n), static_cast<int>(k),
-                                dw.data_ptr<float>(), ws.data_ptr(), static_cast<size_t>(ws.numel()), st),
+                                dw.data_ptr<float>(), ws.data(), ws.bytes(), st),
         "cxg_dense_wgrad_f32");
   return dw;
 }
@@ -402,9 +452,9 @@ Tensor rows_sum(const Tensor &g) {
   size_t need = 0;
   check(lib.cxg_column_sum_workspace_size(static_cast<int>(g.size(1)), &need), "cxg_column_sum_workspace_size");
   void *st = stream_of(g);
-  const Tensor ws = workspace_on(g.device().index(), st, static_cast<int64_t>(need), "");
-  check(lib.cxg_column_sum(g.data_ptr(), CXG_F32, g.size(0), static_cast<int>(g.size(1)), out.data_ptr<float>(), ws.data_ptr(),
-                           static_cast<size_t>(ws.numel()), st),
+  const Workspace ws = workspace_on(g.device().index(), st, static_cast<int64_t>(need), "");
+  check(lib.cxg_column_sum(g.data_ptr(), CXG_F32, g.size(0), static_cast<int>(g.size(1)), out.data_ptr<float>(), ws.data(),
+                           ws.bytes(), st),
         "cxg_column_sum");
   return out;
 }
@@ -590,13 +640,15 @@ class GatFunction : public torch::autograd::Function<GatFunction> {
     const Tensor y = at::empty({n, h * c}, x.options()), top = at::empty({n, h}, x.options()), sum = at::empty({n, h}, x.options());
     size_t need = 0;
     check(lib.cxg_gat_fused_workspace_size(n, idx.size(0), hi, ci, &need), "cxg_gat_fused_workspace_size");
-    const Tensor ws = workspace_on(x.device().index(), st, static_cast<int64_t>(need), "");
-    check(lib.cxg_gat_fused_forward(ptr.data_ptr(), idx.data_ptr(), static_cast<int>(ptr.element_size()),
-                                    static_cast<int>(idx.element_size()), x.data_ptr<float>(), a_src.data_ptr<float>(),
-                                    a_dst.data_ptr<float>(), y.data_ptr<float>(), top.data_ptr<float>(), sum.data_ptr<float>(), n,
-                                    idx.size(0), hi, ci, static_cast<float>(slope), ws.data_ptr(),
-                                    static_cast<size_t>(ws.numel()), st),
-          "cxg_gat_fused_forward");
+    {
+      const Workspace ws = workspace_on(x.device().index(), st, static_cast<int64_t>(need), "");
+      check(lib.cxg_gat_fused_forward(ptr.data_ptr(), idx.data_ptr(), static_cast<int>(ptr.element_size()),
+                                      static_cast<int>(idx.element_size()), x.data_ptr<float>(), a_src.data_ptr<float>(),
+                                      a_dst.data_ptr<float>(), y.data_ptr<float>(), top.data_ptr<float>(), sum.data_ptr<float>(), n,
+                                      idx.size(0), hi, ci, static_cast<float>(slope), ws.data(),
+                                      ws.bytes(), st),
+            "cxg_gat_fused_forward");
+    }
     if (keep != nullptr) *keep = {x, att_src, att_dst, ptr, idx, a_src, a_dst, y, top, sum};
     if (concat) return bias ? head_mean_bias(y, bias, 1, h * c) : y;
     return head_mean_bias(y, bias, h, c);
@@ -627,23 +679,23 @@ class GatFunction : public torch::autograd::Function<GatFunction> {
         ctx->saved_data["concat"].toBool() ? g : g.mul(1.0 / static_cast<double>(h)).unsqueeze(1).expand({n, h, c}).contiguous();
     const Transposed t = transposed_graph(ptr, idx, n, n_src);
     const Tensor dx = at::empty_like(x), d_src = at::empty_like(a_src), d_dst = at::empty_like(a_dst);
+    const Tensor g_as = at::empty_like(att_src), g_ad = at::empty_like(att_dst);
     size_t need = 0, need_att = 0;
     check(lib.cxg_gat_fused_workspace_size(n, idx.size(0), hi, ci, &need), "cxg_gat_fused_workspace_size");
     check(lib.cxg_gat_att_grad_workspace_size(hi, ci, &need_att), "cxg_gat_att_grad_workspace_size");
-    const Tensor ws = workspace_on(x.device().index(), st, static_cast<int64_t>(std::max(need, need_att)), "");
+    const Workspace ws = workspace_on(x.device().index(), st, static_cast<int64_t>(std::max(need, need_att)), "");
     check(lib.cxg_gat_fused_backward(t.t_ptr.data_ptr(), t.t_idx.data_ptr(), static_cast<int>(t.t_ptr.element_size()),
                                      static_cast<int>(t.t_idx.element_size()), dy.data_ptr<float>(), y.data_ptr<float>(),
                                      x.data_ptr<float>(), a_src.data_ptr<float>(), a_dst.data_ptr<float>(), top.data_ptr<float>(),
                                      sum.data_ptr<float>(), dx.data_ptr<float>(), d_src.data_ptr<float>(), d_dst.data_ptr<float>(),
                                      n_src, n, t.t_idx.size(0), hi, ci, static_cast<float>(ctx->saved_data["slope"].toDouble()),
-                                     nullptr, nullptr, static_cast<int>(ptr.element_size()), ws.data_ptr(),
-                                     static_cast<size_t>(ws.numel()), st),
+                                     nullptr, nullptr, static_cast<int>(ptr.element_size()), ws.data(),
+                                     ws.bytes(), st),
           "cxg_gat_fused_backward");
-    const Tensor g_as = at::empty_like(att_src), g_ad = at::empty_like(att_dst);
     check(lib.cxg_gat_scores_backward_add(x.data_ptr<float>(), d_src.data_ptr<float>(), d_dst.data_ptr<float>(),
                                           att_src.data_ptr<float>(), att_dst.data_ptr<float>(), dx.data_ptr<float>(),
-                                          g_as.data_ptr<float>(), g_ad.data_ptr<float>(), n_src, n, hi, ci, ws.data_ptr(),
-                                          static_cast<size_t>(ws.numel()), st),
+                                          g_as.data_ptr<float>(), g_ad.data_ptr<float>(), n_src, n, hi, ci, ws.data(),
+                                          ws.bytes(), st),
           "cxg_gat_scores_backward_add");
     return {dx, g_as, g_ad, db, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
@@ -701,13 +753,15 @@ std::tuple<Tensor, Tensor, Tensor, std::vector<int64_t>, std::vector<int64_t>> s
   Tensor nodes = at::empty({max_nodes}, opt), ptr = at::empty({max_rows + 1}, opt), idx = at::empty({max_edges}, opt);
   Tensor sizes = at::empty({2 * (hops + 1)}, opt);
   void *st = stream_of(seeds);
-  const Tensor ws = workspace_on(seeds.device().index(), st, static_cast<int64_t>(bytes), "");
-  check(lib.cxg_sample_batch(gptr.data_ptr(), gidx.data_ptr(), static_cast<int>(gptr.element_size()),
-                             static_cast<int>(gidx.element_size()), n_nodes, nnz, seeds.data_ptr<int64_t>(), seeds.size(0),
-                             fanouts.data(), hops, hop_seeds.data(), local_of.data_ptr<int64_t>(),
-                             reinterpret_cast<uint32_t *>(bitmap.data_ptr()), nodes.data_ptr<int64_t>(), ptr.data_ptr<int64_t>(),
-                             idx.data_ptr<int64_t>(), sizes.data_ptr<int64_t>(), ws.data_ptr(), static_cast<size_t>(ws.numel()), st),
-        "cxg_sample_batch");
+  {
+    const Workspace ws = workspace_on(seeds.device().index(), st, static_cast<int64_t>(bytes), "");
+    check(lib.cxg_sample_batch(gptr.data_ptr(), gidx.data_ptr(), static_cast<int>(gptr.element_size()),
+                               static_cast<int>(gidx.element_size()), n_nodes, nnz, seeds.data_ptr<int64_t>(), seeds.size(0),
+                               fanouts.data(), hops, hop_seeds.data(), local_of.data_ptr<int64_t>(),
+                               reinterpret_cast<uint32_t *>(bitmap.data_ptr()), nodes.data_ptr<int64_t>(), ptr.data_ptr<int64_t>(),
+                               idx.data_ptr<int64_t>(), sizes.data_ptr<int64_t>(), ws.data(), ws.bytes(), st),
+          "cxg_sample_batch");
+  }
   host_sizes.narrow(0, 0, sizes.size(0)).copy_(sizes, /*non_blocking=*/true);
   {
     py::gil_scoped_release other_threads;
@@ -724,7 +778,10 @@ std::tuple<Tensor, Tensor, Tensor, std::vector<int64_t>, std::vector<int64_t>> s
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("init", &init);
-  m.def("workspace", &workspace);
+  py::class_<HeldWorkspace>(m, "Workspace")
+      .def(py::init<int, int64_t, std::string>())
+      .def("__enter__", &HeldWorkspace::enter)
+      .def("__exit__", [](HeldWorkspace &w, const py::args &) { w.exit(); });
   m.def("last_workspace", &last_workspace);
   m.def("spmm", &spmm);
   m.def("sage", &sage);

@@ -153,9 +153,10 @@ EXTRA_SPMM_FLAGS = int(os.environ.get("CXG_SPMM_FLAGS", "0"))
 
 
 def _workspace(device, nbytes, kind=""):
-    """Scratch buffer per (device, stream); grows on demand, contents never carry over. `kind` names the entry
-    point family that uses it now (its status word is the one check_device_status can answer for)."""
-    return _native.workspace(_dev_index(device), nbytes, kind)
+    """`with _workspace(...) as ws`: the scratch buffer of the device's current stream, for the call inside the block alone
+    (the launches of a call of another thread on this stream wait). It grows on demand, contents never carry over. `kind`
+    names the entry point family that uses it now (its status word is the one check_device_status can answer for)."""
+    return _native.Workspace(_dev_index(device), nbytes, kind)
 
 
 def _dtype_code(t):
@@ -633,8 +634,7 @@ class _GatScoresFunction(torch.autograd.Function):
             grad_as, grad_ad = torch.empty_like(att_src), torch.empty_like(att_dst)
             need = _sz(0)
             _check(_gat_att_grad_ws(h, c, ctypes.byref(need)), "cxg_gat_att_grad_workspace_size")
-            ws = _workspace(feat.device, need.value)
-            with _on(feat.device):
+            with _on(feat.device), _workspace(feat.device, need.value) as ws:
                 _check(_gat_att_grad(_p(feat), _p(g_src), _p(g_dst), _p(grad_as), _p(grad_ad), n, ctx.num_dst, h, c,
                                      _p(ws), ws.numel(), _stream()), "cxg_gat_att_grad")
         return grad_feat, grad_as, grad_ad, None
@@ -662,8 +662,7 @@ def column_sum(x):
     out = torch.empty(width, dtype=torch.float32, device=x.device)
     need = _sz(0)
     _check(_colsum_ws(width, ctypes.byref(need)), "cxg_column_sum_workspace_size")
-    ws = _workspace(x.device, need.value)
-    with _on(x.device):
+    with _on(x.device), _workspace(x.device, need.value) as ws:
         _check(_colsum(_p(x), _dtype_code(x), n, width, _p(out), _p(ws), ws.numel(), _stream()), "cxg_column_sum")
     return out
 
@@ -946,8 +945,7 @@ class _EdgeSoftmaxFunction(torch.autograd.Function):
             raise RuntimeError("ptr has fewer rows than att_dst")
         out = torch.empty((num_edge, heads), dtype=torch.float32, device=att_dst.device)
         mask = torch.empty((num_edge, heads), dtype=torch.bool, device=att_dst.device)
-        ws = _softmax_ws(att_dst.device, n_dst, num_edge)
-        with _on(att_dst.device):
+        with _on(att_dst.device), _softmax_ws(att_dst.device, n_dst, num_edge) as ws:
             _check(_es_fwd(_p(ptr), _p(idx), ptr.element_size(), idx.element_size(), _p(att_dst), _p(att_src), _p(out),
                            _p(mask), n_dst, num_edge, heads, float(relu_l), _p(ws), ws.numel(), _stream()),
                    "cxg_edge_softmax_forward")
@@ -962,8 +960,7 @@ class _EdgeSoftmaxFunction(torch.autograd.Function):
         grad_out = _cuda(grad_out.contiguous(), "grad", (torch.float32,))
         gd = torch.zeros((n_dst, heads), dtype=torch.float32, device=out.device)
         gs = torch.zeros((n_src, heads), dtype=torch.float32, device=out.device)
-        ws = _softmax_ws(out.device, n_dst, num_edge)
-        with _on(out.device):
+        with _on(out.device), _softmax_ws(out.device, n_dst, num_edge) as ws:
             _check(_es_bwd(_p(ptr), _p(idx), ptr.element_size(), idx.element_size(), _p(grad_out), _p(mask), _p(out),
                            _p(gd), _p(gs), n_dst, num_edge, heads, relu_l, _p(ws), ws.numel(), _stream()),
                    "cxg_edge_softmax_backward")
@@ -1020,8 +1017,7 @@ class _GatFusedFunction(torch.autograd.Function):
         row_sum = torch.empty((n, h), dtype=torch.float32, device=dev)
         need = _sz(0)
         _check(_gatf_ws(n, idx.shape[0], h, c, ctypes.byref(need)), "cxg_gat_fused_workspace_size")
-        ws = _workspace(dev, need.value)
-        with _on(dev):
+        with _on(dev), _workspace(dev, need.value) as ws:
             _check(_gatf_fwd(_p(ptr), _p(idx), ptr.element_size(), idx.element_size(), _p(x_src), _p(a_src), _p(a_dst),
                              _p(y), _p(row_max), _p(row_sum), n, idx.shape[0], h, c, float(slope), _p(ws), ws.numel(),
                              _stream()), "cxg_gat_fused_forward")
@@ -1045,8 +1041,7 @@ class _GatFusedFunction(torch.autograd.Function):
             d_ad[n:].zero_()
         need = _sz(0)
         _check(_gatf_ws(n, idx.shape[0], h, c, ctypes.byref(need)), "cxg_gat_fused_workspace_size")
-        ws = _workspace(dev, need.value)
-        with _on(dev):
+        with _on(dev), _workspace(dev, need.value) as ws:
             _check(_gatf_bwd(_p(t_ptr), _p(t_idx), t_ptr.element_size(), t_idx.element_size(), _p(dy), _p(y), _p(x_src),
                              _p(a_src), _p(a_dst), _p(row_max), _p(row_sum), _p(dx), _p(d_as), _p(d_ad), n_src, n,
                              t_idx.shape[0], h, c, ctx.slope, _p(t_eid) if ordered else None,

@@ -208,8 +208,7 @@ def typed_matmul_raw(a, b, rel, m_positions, m_valid, src_idx=None, dst_idx=None
     precision = 0 if exact else (1 if (allow_tf32 or dtype == CXG_BF16) else 2)
     need = _sz(0)
     _check(_tmm_ws(num_rel, k, n, dtype, ctypes.byref(need)), "cxg_typed_matmul_workspace_size")
-    ws = _workspace(a.device, need.value, "typed_matmul")
-    with torch.cuda.device(a.device):
+    with torch.cuda.device(a.device), _workspace(a.device, need.value, "typed_matmul") as ws:
         _check(_tmm(_p(a), _p(b), _p(c), _p(rel), _p(src_idx), _p(dst_idx), int(m_positions), int(m_valid), k, n, num_rel,
                     dtype, precision, flags, _p(ws), ws.numel(), _stream()), "cxg_typed_matmul")
     return c
@@ -262,8 +261,7 @@ def typed_wgrad(x, g, sorted_rel, num_rel, num_valid=None, idx=None, idx_g=None,
     precision = 1 if (allow_tf32 or dtype == CXG_BF16) else 2
     need = _sz(0)
     _check(_wg_ws(num_rel, k, n, ctypes.byref(need)), "cxg_typed_wgrad_workspace_size")
-    ws = _workspace(x.device, need.value, "typed_wgrad")
-    with torch.cuda.device(x.device):
+    with torch.cuda.device(x.device), _workspace(x.device, need.value, "typed_wgrad") as ws:
         _check(_wg(_p(x), _p(g), _p(sorted_rel), _p(idx), _p(idx_g), m, x_rows, g_rows, k, n, num_rel, dtype, precision,
                    int(extra_flags), _p(dw), _p(ws), ws.numel(), _stream()), "cxg_typed_wgrad")
         if check_status:  # synchronises; raises when a bounded device-side wait ran out
@@ -288,8 +286,7 @@ def typed_matmul_all_relations(x, w, allow_tf32=None, extra_flags=0):
     precision = 1 if (allow_tf32 or dtype == CXG_BF16) else 2
     need = _sz(0)
     _check(_tmm_ws(num_rel, k, n, dtype, ctypes.byref(need)), "cxg_typed_matmul_workspace_size")
-    ws = _workspace(x.device, need.value, "typed_matmul")
-    with torch.cuda.device(x.device):
+    with torch.cuda.device(x.device), _workspace(x.device, need.value, "typed_matmul") as ws:
         _check(_tmm(_p(x), _p(w), _p(c), None, None, None, m, m, k, n, num_rel, dtype, precision, 8 | int(extra_flags), _p(ws), ws.numel(),
                     _stream()), "cxg_typed_matmul")
     return c
