@@ -33,6 +33,17 @@ int check_launch(const char *what) {
   return set_error(CXG_ECUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
+int take_status_word(void *word, void *stream, const char *who) {
+  int32_t v = 0;
+  cudaStream_t st = as_stream(stream);
+  cudaError_t e = cudaMemcpyAsync(&v, word, sizeof(v), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && v != 0) e = cudaMemsetAsync(word, 0, sizeof(v), st);
+  if (e != cudaSuccess) return set_error(CXG_ECUDA, "%s: reading the status: %s", who, cudaGetErrorString(e));
+  if (v != 0) return set_error(CXG_ETIMEOUT, "%s: a bounded device-side wait ran out; a result is incomplete", who);
+  return CXG_OK;
+}
+
 }  // namespace cxg
 
 extern "C" const char *cxg_last_error_string(void) { return cxg::g_last_error; }

@@ -39,7 +39,7 @@ constexpr int kThreads = 32 * (kFirstConv + kConvWarps);
 constexpr int kMaxStages = 4, kMinStages = 3;
 constexpr int kSmemBudget = 225 * 1024;  // without the alignment of the first unit
 
-__device__ int32_t linear_status;  // set when a bounded wait ran out
+__device__ int32_t linear_status;  // set when a bounded wait ran out, cleared by cxg_linear_f32_status
 
 struct LinArgs {
   const float *b, *bias, *add;
@@ -51,6 +51,7 @@ struct LinArgs {
   int b_rows_k;   // B is [K][N] instead of [N][K]
   int stages;
   int acc_cols;   // tensor-memory columns of one accumulator buffer
+  int test_stall; // test hook: the converters never hand over their first unit, so the waits for it run out
   long long wait_cycles;
 };
 
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc(const __grid_constant__
         }
         mbar_arrive(&bars.raw_empty[s]);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive(&bars.term_full[s]);
+        if (!(a.test_stall && tile == tile_lo && sp == 0)) mbar_arrive(&bars.term_full[s]);
       }
   } else if (warp == kMmaWarp) {
     const uint32_t idesc = make_idesc(1, kTileM, a.nt), idesc_wide = make_idesc(1, kTileM, 2 * a.nt);
@@ -362,6 +363,11 @@ extern "C" int cxg_linear_f32_supported(int64_t m, int k, int n) {
 
 extern "C" int cxg_linear_f32(const float *a, const float *b, const float *bias, const float *add, float *c, int64_t m, int k,
                               int n, int b_rows_k, void *stream) {
+  return cxg_linear_f32_ex(a, b, bias, add, c, m, k, n, b_rows_k ? CXG_LINEAR_B_ROWS_K : 0u, stream);
+}
+
+extern "C" int cxg_linear_f32_ex(const float *a, const float *b, const float *bias, const float *add, float *c, int64_t m, int k,
+                                 int n, uint32_t flags, void *stream) {
   CXG_REQUIRE(m >= 0 && k > 0 && n > 0, CXG_EINVAL, "cxg_linear_f32: bad sizes");
   if (m == 0) return CXG_OK;
   CXG_REQUIRE(a && b && c, CXG_ENULL, "cxg_linear_f32: NULL argument");
@@ -375,7 +381,8 @@ extern "C" int cxg_linear_f32(const float *a, const float *b, const float *bias,
   t.m = m, t.k = k, t.n = n;
   t.nt = columns_per_block(m, k, n);
   t.n_blocks = (n + t.nt - 1) / t.nt;
-  t.b_rows_k = b_rows_k;
+  t.b_rows_k = (flags & CXG_LINEAR_B_ROWS_K) ? 1 : 0;
+  t.test_stall = (flags & CXG_LINEAR_TEST_STALL) ? 1 : 0;
   t.acc_cols = 32;
   while (t.acc_cols < 2 * t.nt) t.acc_cols *= 2;
   t.wait_cycles = wait_limit_cycles();
@@ -398,11 +405,8 @@ extern "C" int cxg_linear_f32(const float *a, const float *b, const float *bias,
 }
 
 extern "C" int cxg_linear_f32_status(void *stream) {
-  int32_t word = 0;
-  cudaStream_t st = as_stream(stream);
-  if (cudaMemcpyFromSymbolAsync(&word, linear_status, sizeof(word), 0, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return check_launch("cxg_linear_f32_status");
-  if (word != 0) return set_error(CXG_ETIMEOUT, "cxg_linear_f32: a bounded wait ran out");
-  return CXG_OK;
+  void *word = nullptr;
+  const cudaError_t e = cudaGetSymbolAddress(&word, linear_status);
+  if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_linear_f32_status: %s", cudaGetErrorString(e));
+  return take_status_word(word, stream, "cxg_linear_f32");
 }

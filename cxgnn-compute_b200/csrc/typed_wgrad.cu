@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(128) dense_reduce(const float *partial, float 
   dw[i] = s;
 }
 
-__device__ int32_t dense_status;  // set when a bounded wait of the dense mode ran out
+__device__ int32_t dense_status;  // set when a bounded wait of the dense mode ran out, cleared by cxg_dense_wgrad_f32_status
 
 // Blocks of positions of the dense mode: one block per SM over all column block pairs.
 int dense_parts(int k, int n, int64_t m) {
@@ -712,6 +712,11 @@ extern "C" int cxg_dense_wgrad_f32_workspace_size(int64_t m, int k, int n, size_
 
 extern "C" int cxg_dense_wgrad_f32(const float *x, const float *g, int64_t m, int k, int n, float *dw, void *workspace,
                                    size_t workspace_bytes, void *stream) {
+  return cxg_dense_wgrad_f32_ex(x, g, m, k, n, 0u, dw, workspace, workspace_bytes, stream);
+}
+
+extern "C" int cxg_dense_wgrad_f32_ex(const float *x, const float *g, int64_t m, int k, int n, uint32_t flags, float *dw,
+                                      void *workspace, size_t workspace_bytes, void *stream) {
   CXG_REQUIRE(m > 0 && k > 0 && n > 0, CXG_EINVAL, "cxg_dense_wgrad_f32: bad sizes");
   CXG_REQUIRE(x && g && dw, CXG_ENULL, "cxg_dense_wgrad_f32: NULL argument");
   const int k_blocks = (k + 127) / 128, n_blocks = (n + 127) / 128;
@@ -733,7 +738,8 @@ extern "C" int cxg_dense_wgrad_f32(const float *x, const float *g, int64_t m, in
   if (stages > kMaxStages) stages = kMaxStages;
   WgArgs a;
   a.x = x, a.g = g, a.rel = nullptr, a.idx = nullptr, a.idx_g = nullptr, a.m = m, a.x_rows = m, a.g_rows = m;
-  a.k = k, a.n = n, a.num_rel = 1, a.stages = stages, a.slots = 1, a.test_stall = 0, a.dense = k_blocks;
+  a.k = k, a.n = n, a.num_rel = 1, a.stages = stages, a.slots = 1, a.dense = k_blocks;
+  a.test_stall = (flags & CXG_WGRAD_TEST_STALL) ? 1 : 0;
   a.chunk_tiles = 256 / kPosX3;
   a.partial = static_cast<float *>(workspace);
   a.slot_rel = nullptr;
@@ -754,13 +760,10 @@ extern "C" int cxg_dense_wgrad_f32(const float *x, const float *g, int64_t m, in
 }
 
 extern "C" int cxg_dense_wgrad_f32_status(void *stream) {
-  int32_t word = 0;
-  cudaStream_t st = as_stream(stream);
-  if (cudaMemcpyFromSymbolAsync(&word, dense_status, sizeof(word), 0, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return check_launch("cxg_dense_wgrad_f32_status");
-  if (word != 0) return set_error(CXG_ETIMEOUT, "cxg_dense_wgrad_f32: a bounded wait ran out");
-  return CXG_OK;
+  void *word = nullptr;
+  const cudaError_t e = cudaGetSymbolAddress(&word, dense_status);
+  if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_dense_wgrad_f32_status: %s", cudaGetErrorString(e));
+  return take_status_word(word, stream, "cxg_dense_wgrad_f32");
 }
 
 extern "C" int cxg_typed_wgrad_status(const void *workspace, void *stream) {

@@ -203,16 +203,31 @@ _spmm_status = _sig("cxg_spmm_csr_status", [_vp, _vp])
 _tmm_status = _sig("cxg_typed_matmul_status", [_vp, _vp])
 
 
+_wgrad_status = _sig("cxg_typed_wgrad_status", [_vp, _vp])
+_linear_status = _sig("cxg_linear_f32_status", [_vp])
+_dense_wgrad_status = _sig("cxg_dense_wgrad_f32_status", [_vp])
+
+
 def check_device_status(kind="spmm", device=None):
-    """Synchronises the current stream and raises if the LAST call on this stream was of that kind ("spmm" or
-    "typed_matmul") and a bounded device-side wait of it ran out (the kernels give up after a cycle limit instead
-    of spinning forever) or, for "spmm", ptr[num_node] exceeded the length of idx. The calls of one stream share
-    a scratch buffer, so only the last call can be asked about; for any other kind nothing is checked."""
+    """Synchronises the current stream and raises if a bounded device-side wait ran out (the kernels give up after a cycle
+    limit instead of spinning forever) or, for "spmm", ptr[num_node] exceeded the length of idx.
+    "spmm", "typed_matmul", "typed_wgrad": asks about the LAST call on this stream, if it was of that kind (the calls of one
+    stream share a scratch buffer, which holds the record; for any other last call nothing is checked).
+    "linear": asks about all fp32 linear transforms of the layers and their gradients (cxg_linear_f32, cxg_dense_wgrad_f32)
+    on this device since they were asked about last."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+    if kind == "linear":
+        with _on(device):
+            failed = [(fn(_stream()), name) for fn, name in ((_linear_status, "cxg_linear_f32_status"),
+                                                             (_dense_wgrad_status, "cxg_dense_wgrad_f32_status"))]
+        for rc, name in failed:
+            _check(rc, name)
+        return
     ws, last = _native.last_workspace(_dev_index(device))
     if ws is None or last != kind:
         return
-    fn, name = (_spmm_status, "cxg_spmm_csr_status") if kind == "spmm" else (_tmm_status, "cxg_typed_matmul_status")
+    fn, name = {"spmm": (_spmm_status, "cxg_spmm_csr_status"), "typed_matmul": (_tmm_status, "cxg_typed_matmul_status"),
+                "typed_wgrad": (_wgrad_status, "cxg_typed_wgrad_status")}[kind]
     with _on(device):
         _check(fn(_p(ws), _stream()), name)
 

@@ -158,11 +158,18 @@ int cxg_typed_wgrad_status(const void *workspace, void *stream);
  * is taken apart into three bf16 terms): c[m, n] = a[m, :] . b[n, :] (+ bias[n]) (+ add[m, n]), all matrices row-major and
  * contiguous. b_rows_k: b is [k, n] instead of [n, k]. k must be a multiple of 4 of which 16 rows of b fit in shared
  * memory (about 1100 columns; cxg_linear_f32_supported tells), n up to 8192; a, b, c and add 16-byte aligned. bias and add
- * may be NULL; add may be c. cxg_linear_f32_status reads back whether a bounded wait ran out on the current device.
+ * may be NULL; add may be c. cxg_linear_f32_status waits for everything queued on `stream`, tells whether a bounded wait of
+ * such a call ran out on the current device since it was asked last (CXG_ETIMEOUT: that call's result is incomplete), and
+ * forgets it. cxg_linear_f32_ex: the same with flags.
  */
+#define CXG_LINEAR_B_ROWS_K 1u /* b is [k, n] */
+/* Test hook: the first tile of every CTA is never handed to the tensor-core role, so the bounded waits for it run out. */
+#define CXG_LINEAR_TEST_STALL 2u
 int cxg_linear_f32_supported(int64_t m, int k, int n);
 int cxg_linear_f32(const float *a, const float *b, const float *bias, const float *add, float *c, int64_t m, int k, int n,
                    int b_rows_k, void *stream);
+int cxg_linear_f32_ex(const float *a, const float *b, const float *bias, const float *add, float *c, int64_t m, int k,
+                      int n, uint32_t flags, void *stream);
 int cxg_linear_f32_status(void *stream);
 
 /*
@@ -172,7 +179,9 @@ int cxg_linear_f32_status(void *stream);
 int cxg_dense_wgrad_f32_workspace_size(int64_t m, int k, int n, size_t *bytes);
 int cxg_dense_wgrad_f32(const float *x, const float *g, int64_t m, int k, int n, float *dw, void *workspace,
                         size_t workspace_bytes, void *stream);
-int cxg_dense_wgrad_f32_status(void *stream);
+int cxg_dense_wgrad_f32_ex(const float *x, const float *g, int64_t m, int k, int n, uint32_t flags /* CXG_WGRAD_TEST_STALL */,
+                           float *dw, void *workspace, size_t workspace_bytes, void *stream);
+int cxg_dense_wgrad_f32_status(void *stream); /* as cxg_linear_f32_status */
 
 /*
  * Scratch bytes needed by cxg_spmm_csr for a graph with n_dst rows and nnz
