@@ -38,11 +38,13 @@ constexpr int kMmaWarp = kEpiWarps, kLoadWarp = kMmaWarp + 1, kFirstConv = kLoad
 constexpr int kThreads = 32 * (kFirstConv + kConvWarps);
 constexpr int kMaxStages = 4, kMinStages = 3;
 constexpr int kSmemBudget = 225 * 1024;  // without the alignment of the first unit
+constexpr float kMostF32 = 3.402823466e38f;   // the largest finite value
+constexpr float kMostBf16 = 3.389531389e38f;  // and that of bf16
 
 __device__ int32_t linear_status;  // set when a bounded wait ran out, cleared by cxg_linear_f32_status
 
 struct LinArgs {
-  const float *b, *bias, *add;
+  const float *a, *b, *bias, *add;
   float *c;
   int64_t m;
   int k, n;
@@ -73,6 +75,22 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t &h, uint32_t &
   m = pack_bf16(a, b);
   a -= __uint_as_float(m << 16), b -= __uint_as_float(m & 0xffff0000u);
   l = pack_bf16(a, b);
+}
+
+// A[row, :] . B[col, :] as an fp32 multiply-add chain. The products of the terms cannot give an element that an infinity or
+// a value above bf16's range takes part in: Inf - Inf is no second term, and an infinity times the other operand's lower
+// terms, zeros or of either sign, is no third. Whatever comes out of the tensor core as an infinity or NaN is taken from
+// here. A chain that has become NaN stays it, so a matrix full of them ends after four steps.
+__device__ __noinline__ float exact_chain(const LinArgs &a, int64_t row, int col) {
+  const float4 *x = reinterpret_cast<const float4 *>(a.a + row * a.k);
+  const float *w = a.b + (a.b_rows_k ? col : static_cast<int64_t>(col) * a.k);
+  const int64_t step = a.b_rows_k ? a.n : 1;
+  float s = 0.f;
+  for (int k = 0; k < a.k && s == s; k += 4, w += 4 * step) {
+    const float4 v = x[k / 4];
+    s = fmaf(v.x, w[0], s), s = fmaf(v.y, w[step], s), s = fmaf(v.z, w[2 * step], s), s = fmaf(v.w, w[3 * step], s);
+  }
+  return s;
 }
 
 // 8 bytes (four columns from 4 * c4 on) of a row of a tile of bf16 rows of 64 bytes, 64-byte swizzle
@@ -123,6 +141,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc(const __grid_constant__
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // the three terms of this CTA's rows of B; rows behind N and columns behind K are zeros
+  bool b_infinite = false;  // B has a value that bf16 does not reach (or that the sum of four takes for one)
   {
     const int c4s = spans * (kSpan / 4), total = a.nt * c4s;
     constexpr int kAhead = 4;  // requested at once: this is what a call of few rows spends its time on
@@ -149,6 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc(const __grid_constant__
         if (i >= total) break;
         const int row = a.b_rows_k ? i % a.nt : i / c4s, c4 = a.b_rows_k ? i / a.nt : i % c4s;
         uint2 h, m, l;
+        b_infinite |= !((fabsf(v[u].x) + fabsf(v[u].y)) + (fabsf(v[u].z) + fabsf(v[u].w)) <= kMostBf16);
         split3(v[u].x, v[u].y, h.x, m.x, l.x);
         split3(v[u].z, v[u].w, h.y, m.y, l.y);
         uint8_t *d = smem_b + (c4 / (kSpan / 4)) * span_b + term_offset(row, c4 % (kSpan / 4));
@@ -161,7 +181,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc(const __grid_constant__
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads B through the async proxy
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  b_infinite = __syncthreads_or(b_infinite) != 0;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_d = tmem_base_slot;
   auto wait = [&](uint64_t *bar, int64_t phase) {
@@ -273,6 +293,35 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc(const __grid_constant__
       // two adjacent lanes trade 16-byte quads, so that one store of the pair writes a whole 32-byte sector
       const int64_t even = (row & ~1ll) * a.n + n0;
       const bool ok_a = (row & ~1ll) < a.m, ok_b = (row | 1) < a.m;
+      // an infinity or NaN in a row of A shows in every column of the row, the first one included. (In the loop below the
+      // calls cost the ordinary tiles 12 %, here one column read ahead.)
+      uint32_t first[2];
+      tmem_ld1(first, taddr);
+      tmem_ld1(first + 1, taddr + a.nt);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (b_infinite || !__all_sync(0xffffffffu, fabsf(__uint_as_float(first[0]) + __uint_as_float(first[1])) <= kMostF32)) {
+        for (int c0 = 0; c0 < a.nt; c0 += 16) {
+          uint32_t v[16], sm[16];
+          tmem_ld16(v, taddr + c0);
+          tmem_ld16(sm, taddr + a.nt + c0);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (row < a.m) {
+            const int64_t at = row * a.n + n0 + c0;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (c0 + i < cols) {
+                float f = __uint_as_float(v[i]) + __uint_as_float(sm[i]);
+                if (!(fabsf(f) <= kMostF32)) f = exact_chain(a, row, n0 + c0 + i);
+                f += s_bias[c0 + i];
+                a.c[at + i] = a.add != nullptr ? f + a.add[at + i] : f;
+              }
+          }
+          __syncwarp();
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        mbar_arrive(&bars.acc_empty[buf]);
+        continue;
+      }
       for (int c0 = 0; c0 < a.nt; c0 += 16) {
         // what is to be added: requested before the accumulator is read
         float4 pa[2], pb[2];
@@ -377,7 +426,7 @@ extern "C" int cxg_linear_f32_ex(const float *a, const float *b, const float *bi
                reinterpret_cast<uintptr_t>(add)) % 16 == 0,
               CXG_EINVAL, "cxg_linear_f32: A, B, C and add must be 16-byte aligned");
   LinArgs t;
-  t.b = b, t.bias = bias, t.add = add, t.c = c;
+  t.a = a, t.b = b, t.bias = bias, t.add = add, t.c = c;
   t.m = m, t.k = k, t.n = n;
   t.nt = columns_per_block(m, k, n);
   t.n_blocks = (n + t.nt - 1) / t.nt;

@@ -137,6 +137,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t *v, uint32_t taddr) {
       : "r"(taddr));
 }
 
+// one column
+__device__ __forceinline__ void tmem_ld1(uint32_t *v, uint32_t taddr) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v[0]) : "r"(taddr));
+}
+
 __device__ __forceinline__ void st_global_v4(void *p, uint4 v) {
   asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }

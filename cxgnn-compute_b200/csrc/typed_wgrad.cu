@@ -562,8 +562,11 @@ __global__ void wgrad_clear(int32_t *slot_rel, int n) {
   if (i < n) slot_rel[i] = -1;
 }
 
-// Dense mode: dW[i][j] = sum of the partials of its column block pair over the blocks, in order, eight loads in flight.
-__global__ void __launch_bounds__(128) dense_reduce(const float *partial, float *dw, int k, int n, int k_blocks, int parts) {
+// Dense mode: dW[i][j] = sum of the partials of its column block pair over the blocks, in order, eight loads in flight. An
+// infinity times the other operand's lower term, a zero or of either sign, makes NaN of what an fp32 sum gives as an
+// infinity, so an element that is not finite is summed again from x and g.
+__global__ void __launch_bounds__(128) dense_reduce(const float *partial, const float *x, const float *g, int64_t m, float *dw,
+                                                    int k, int n, int k_blocks, int parts) {
   const int64_t i = blockIdx.x * 128ll + threadIdx.x;
   if (i >= static_cast<int64_t>(k) * n) return;
   const int r = static_cast<int>(i / n), c = static_cast<int>(i % n);
@@ -579,6 +582,13 @@ __global__ void __launch_bounds__(128) dense_reduce(const float *partial, float 
     for (int u = 0; u < 8; ++u) s += v[u];
   }
   for (; q < parts; ++q) s += p[static_cast<int64_t>(q) * (128 * 128)];
+  if (!(fabsf(s) <= 3.402823466e38f)) {
+    s = 0.f;
+    for (int64_t t = 0; t < m && s == s; t += 8)  // a chain that has become NaN stays it
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (t + u < m) s = fmaf(__ldg(x + (t + u) * k + r), __ldg(g + (t + u) * n + c), s);
+  }
   dw[i] = s;
 }
 
@@ -753,8 +763,8 @@ extern "C" int cxg_dense_wgrad_f32_ex(const float *x, const float *g, int64_t m,
   const int parts = dense_parts(k, n, m);
   const dim3 grid(static_cast<unsigned>(parts), static_cast<unsigned>(k_blocks * n_blocks));
   typed_wgrad_tc<float, true><<<grid, 32 * (kEpiWarps + 1 + kProdWarps + kConvWarps), smem, st>>>(a);
-  dense_reduce<<<static_cast<unsigned>((static_cast<int64_t>(k) * n + 127) / 128), 128, 0, st>>>(a.partial, dw, k, n, k_blocks,
-                                                                                            parts);
+  dense_reduce<<<static_cast<unsigned>((static_cast<int64_t>(k) * n + 127) / 128), 128, 0, st>>>(a.partial, x, g, m, dw, k, n,
+                                                                                            k_blocks, parts);
   count_launches(2);
   return check_launch("cxg_dense_wgrad_f32");
 }

@@ -140,7 +140,7 @@ int cxg_typed_matmul_status(const void *workspace, void *stream);
  * over positions, both operands MN-major) plus a fixed-order reduction of per-CTA partial sums: no atomics. An
  * accumulator in tensor memory takes a few thousand positions at most and the partial sums are added in ordinary
  * fp32, so the error does not grow with the number of rows. precision 1 = plain bf16 / TF32 products, 2 =
- * error-compensated TF32 for fp32 inputs (1e-5 class). Shapes: k <= 128 in rows of whole 16-byte chunks, n a multiple of 16,
+ * error-compensated TF32 for fp32 inputs (1e-5 class; an infinite operand gives infinities or NaN). Shapes: k <= 128 in rows of whole 16-byte chunks, n a multiple of 16,
  * n <= 256, one stage within shared memory (CXG_EUNSUPPORTED otherwise). cxg_typed_wgrad_status reads back whether a
  * bounded wait ran out.
  */
@@ -158,7 +158,8 @@ int cxg_typed_wgrad_status(const void *workspace, void *stream);
  * is taken apart into three bf16 terms): c[m, n] = a[m, :] . b[n, :] (+ bias[n]) (+ add[m, n]), all matrices row-major and
  * contiguous. b_rows_k: b is [k, n] instead of [n, k]. k must be a multiple of 4 of which 16 rows of b fit in shared
  * memory (about 1100 columns; cxg_linear_f32_supported tells), n up to 8192; a, b, c and add 16-byte aligned. bias and add
- * may be NULL; add may be c. cxg_linear_f32_status waits for everything queued on `stream`, tells whether a bounded wait of
+ * may be NULL; add may be c. Infinities, NaN and values above bf16's range give what an fp32 chain gives.
+ * cxg_linear_f32_status waits for everything queued on `stream`, tells whether a bounded wait of
  * such a call ran out on the current device since it was asked last (CXG_ETIMEOUT: that call's result is incomplete), and
  * forgets it. cxg_linear_f32_ex: the same with flags.
  */
