@@ -85,6 +85,7 @@ __device__ __forceinline__ void finish_columns(const WalkArgs &a, T *dst, float 
   for (int i = 0; i < VW; ++i) {
     float r = s[i];
     if (a.reduce == CXG_MEAN) r = __fdiv_rn(r, static_cast<float>(deg));
+    if (a.accumulate) r += to_f32(dst[i]);
     dst[i] = from_f32<T>(r);
   }
 }
@@ -196,7 +197,9 @@ __global__ void __launch_bounds__(256, 3) walk_fix(const __grid_constant__ WalkA
 }
 
 bool dispatch(const cxg_spmm_desc *d, const WalkArgs &a, cudaStream_t st, int *resident_tiles) {
-  const int valmode = d->edge_val == nullptr ? (d->reduce == CXG_MEAN ? 3 : 0) : (d->heads == 1 ? 1 : 2);
+  const int valmode = d->flags & CXG_SPMM_ACCUMULATE ? 4
+                      : d->edge_val == nullptr       ? (d->reduce == CXG_MEAN ? 3 : 0)
+                                                     : (d->heads == 1 ? 1 : 2);
   const bool share = (d->flags & CXG_SPMM_SHARE_SMS) != 0;
   int vb = vector_bytes(d);
   // narrow rows take the vector that occupies eight lanes, the fewest a tile is given
@@ -231,7 +234,8 @@ int walk_layout(int64_t nnz, int64_t width, int tile, WalkLayout *L) {
 }
 
 bool walk_eligible(const cxg_spmm_desc *d) {
-  if (d->edge_mask != nullptr || d->targets != nullptr || (d->flags & CXG_SPMM_ACCUMULATE)) return false;
+  if (d->edge_mask != nullptr || d->targets != nullptr) return false;
+  if ((d->flags & CXG_SPMM_ACCUMULATE) && d->edge_val != nullptr) return false;
   const int elem = d->dtype == CXG_F32 ? 4 : 2;
   const int64_t row_bytes = static_cast<int64_t>(d->feat) * d->heads * elem;
   const int vb = vector_bytes(d);
@@ -274,6 +278,7 @@ int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t
   a.feat = d->feat, a.heads = d->heads, a.width = d->feat * d->heads;
   a.row_bytes = a.width * (d->dtype == CXG_F32 ? 4 : 2);
   a.ptr_bytes = d->ptr_bytes, a.idx_bytes = d->idx_bytes, a.reduce = d->reduce;
+  a.accumulate = (d->flags & CXG_SPMM_ACCUMULATE) ? 1 : 0;
   a.tile = tile;
   a.whole_rows = whole_rows ? 1 : 0;
   WalkLayout L;

@@ -25,6 +25,7 @@ struct WalkArgs {
   int64_t max_tiles;
   int row_bytes, width, feat, heads, ptr_bytes, idx_bytes, reduce;
   int tile;       // edges per tile
+  int accumulate; // 1: the output is added to
   int whole_rows; // 1: rows of up to `tile` edges are never cut (see spmm_walk_impl.cuh)
   uint64_t tile_magic;  // ceil(2^64 / tile), 0: divide
   int32_t *hdr;
@@ -39,8 +40,8 @@ struct WalkLayout {
 };
 
 int walk_layout(int64_t nnz, int64_t width, int tile, WalkLayout *L);
-// True when the walk covers the descriptor: no edge mask, output rows in order and overwritten, rows that fit its lane
-// layouts.
+// True when the walk covers the descriptor: no edge mask, output rows in order and overwritten or (without edge values)
+// added to, rows that fit its lane layouts.
 bool walk_eligible(const cxg_spmm_desc *d);
 // The plan kernel for a.ptr, a.tile, a.whole_rows: fills hdr, tiles, count (and sets a.tile_magic).
 void walk_plan_run(WalkArgs &a, cudaStream_t st);

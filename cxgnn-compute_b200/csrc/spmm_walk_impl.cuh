@@ -17,7 +17,8 @@
 // tile t then owns the pieces that START in [t*T, (t+1)*T).
 //
 // Every edge of a step has its own copy of the code at a row's end, which therefore holds nothing that is not needed there:
-// scattered (targets) and accumulating outputs take spmm_stream / spmm_rows.
+// accumulating outputs have an instantiation of their own, scattered ones (targets) and those that accumulate sums of
+// weighted rows take spmm_stream / spmm_rows.
 //
 // What bounds it: L2 and DRAM where rows are wide, the instructions per edge below 256 bytes a row (so no bounds test, no
 // address arithmetic and no wait for a row pointer per edge). Staging the rows in shared memory with 16-byte
@@ -173,8 +174,31 @@ __device__ __forceinline__ void store_row_bytes(uint8_t *dst, const float *f) {
   }
 }
 
+// Bytes of an output row that is added to (not through the read-only path: the kernel writes them).
+template <int VB>
+__device__ __forceinline__ void load_output_bytes(Words<(VB + 3) / 4> &r, const uint8_t *p) {
+  if constexpr (VB == 16) {
+    const uint4 v = __ldcs(reinterpret_cast<const uint4 *>(p));
+    r.w[0] = v.x, r.w[1] = v.y, r.w[2] = v.z, r.w[3] = v.w;
+  } else if constexpr (VB == 8) {
+    const uint2 v = __ldcs(reinterpret_cast<const uint2 *>(p));
+    r.w[0] = v.x, r.w[1] = v.y;
+  } else if constexpr (VB == 4) {
+    r.w[0] = __ldcs(reinterpret_cast<const uint32_t *>(p));
+  } else {
+    r.w[0] = __ldcs(reinterpret_cast<const uint16_t *>(p));
+  }
+}
+template <typename T, int VB>
+__device__ __forceinline__ void add_words(float *f, const Words<(VB + 3) / 4> &r) {
+#pragma unroll
+  for (int i = 0; i < VB / static_cast<int>(sizeof(T)); ++i)
+    f[i] += __uint_as_float(sizeof(T) == 4 ? r.w[i] : i % 2 == 0 ? r.w[i / 2] << 16 : r.w[i / 2] & 0xffff0000u);
+}
+
 // VB: bytes per load of a lane; NV loads per row, G lanes per tile, U edges in flight per lane. VALMODE: 0 no
-// edge values, 1 one per edge, 2 one per (edge, head), 3 none and the mean of the row.
+// edge values, 1 one per edge, 2 one per (edge, head), 3 none and the mean of the row, 4 none and the sum (or the mean) is
+// added to the output.
 template <typename T, int VB, int G, int NV, int U, int VALMODE, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constant__ WalkArgs a) {
   using A = Acc<T, VB>;
@@ -209,6 +233,7 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
       if (on(q)) store_row_bytes<T, VB>(dst + q * G * VB, f[q]);
   };
   auto zero_row = [&](uint8_t *dst) {
+    if (VALMODE == 4) return;
     float z[NV][EL];
 #pragma unroll
     for (int q = 0; q < NV; ++q)
@@ -281,6 +306,16 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
       stop = min(rend, len);
     }
     uint8_t *yr = y0 + row * rb;
+    // What rows hold that are added to is asked for a row ahead, so that it is in L2 when the walk comes to their end.
+    // (2.3 M edges, F = 128 fp32: 157 us, 171 without it, 165 with the row held in registers from its start, which at
+    // F = 256 spills: 265 / 300 / 402; overwriting 126 and 206. Through spmm_stream it took 240 and 675.)
+    auto request_old = [&]() {
+      if (VALMODE != 4 || row + 1 >= a.n_dst) return;
+#pragma unroll
+      for (int q = 0; q < NV; ++q)
+        if (on(q)) asm volatile("prefetch.global.L2 [%0];" ::"l"(yr + rb + q * G * VB));
+    };
+    if (len > 0) request_old();
     A acc[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) acc[q].zero();
@@ -294,7 +329,12 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
           acc[q].get(f[q]);
-          if (VALMODE == 3) divide_by_count<EL>(f[q], d);
+          if (VALMODE == 3 || (VALMODE == 4 && a.reduce == CXG_MEAN)) divide_by_count<EL>(f[q], d);
+          if (VALMODE == 4 && on(q)) {
+            Words<W> old;
+            load_output_bytes<VB>(old, yr + q * G * VB);
+            add_words<T, VB>(f[q], old);
+          }
         }
         store(yr, f);
       } else if (row < a.n_dst) {
@@ -321,6 +361,7 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
           if (rend != pos) break;
           zero_row(yr);  // a row without edges
         }
+        request_old();
       }
       stop = pos == len ? kFar : min(rend, len);
     };
@@ -365,7 +406,7 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
       auto add = [&](int u) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
-          if (VALMODE == 0 || VALMODE == 3)
+          if (VALMODE == 0 || VALMODE >= 3)
             acc[q].add(st.v[u][q]);
           else
             acc[q].fma(st.v[u][q], st.ev[u][VALMODE == 2 ? q : 0]);
@@ -448,6 +489,7 @@ bool launch(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *re
   if (valmode == 0) return launch_width<T, VB, 0>(a, share, st, resident_tiles);
   if (valmode == 1) return launch_width<T, VB, 1>(a, share, st, resident_tiles);
   if (valmode == 3) return launch_width<T, VB, 3>(a, share, st, resident_tiles);
+  if (valmode == 4) return launch_width<T, VB, 4>(a, share, st, resident_tiles);
   return launch_width<T, VB, 2>(a, share, st, resident_tiles);
 }
 
