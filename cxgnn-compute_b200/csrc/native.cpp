@@ -51,6 +51,9 @@ struct Lib {
   CXG_FN(cxg_gather_rows);
   CXG_FN(cxg_sample_batch_bounds);
   CXG_FN(cxg_sample_batch);
+  CXG_FN(cxg_relation_pairs_workspace_size);
+  CXG_FN(cxg_relation_pairs_count);
+  CXG_FN(cxg_relation_pairs_fill);
 #undef CXG_FN
 } lib;
 
@@ -83,6 +86,9 @@ void init(const std::string &path) {
   CXG_FN(cxg_gather_rows);
   CXG_FN(cxg_sample_batch_bounds);
   CXG_FN(cxg_sample_batch);
+  CXG_FN(cxg_relation_pairs_workspace_size);
+  CXG_FN(cxg_relation_pairs_count);
+  CXG_FN(cxg_relation_pairs_fill);
 #undef CXG_FN
 }
 
@@ -722,6 +728,41 @@ Tensor gat_layer(const Tensor &x, const Tensor &att_src, const Tensor &att_dst, 
   return GatFunction::run(x, att_src, att_dst, bias, ptr, idx, n, slope, concat, nullptr);
 }
 
+// ---- relational layer ------------------------------------------------------------------------------------------------
+// (relation, source and number of every position, first position of every source's list, the lists, position of every edge)
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> relation_pairs(const Tensor &idx, const Tensor &etype, int64_t n_src,
+                                                                          int64_t num_rel) {
+  index_of(idx, "idx");
+  index_of(etype, "edge types");
+  const int64_t nnz = std::min(idx.size(0), etype.size(0));
+  const int ib = static_cast<int>(idx.element_size()), rb = static_cast<int>(etype.element_size()), r = static_cast<int>(num_rel);
+  c10::cuda::CUDAGuard guard(idx.device());
+  const auto i64 = idx.options().dtype(at::kLong), i32 = idx.options().dtype(at::kInt);
+  size_t need = 0;
+  check(lib.cxg_relation_pairs_workspace_size(n_src, r, &need), "cxg_relation_pairs_workspace_size");
+  // a buffer of its own: the second call continues in it behind the read-back
+  const Tensor ws = at::empty({static_cast<int64_t>(need)}, idx.options().dtype(at::kByte)), sizes = at::empty({3}, i64);
+  void *st = stream_of(idx);
+  check(lib.cxg_relation_pairs_count(idx.data_ptr(), ib, etype.data_ptr(), rb, nnz, n_src, r, sizes.data_ptr<int64_t>(),
+                                     ws.data_ptr(), need, st),
+        "cxg_relation_pairs_count");
+  Tensor host;
+  {
+    py::gil_scoped_release other_threads;
+    host = sizes.cpu();
+  }
+  const int64_t *h = host.data_ptr<int64_t>();
+  if (h[2] != 0)
+    fail("edge types must lie in [0, " + std::to_string(num_rel) + ") and sources in [0, " + std::to_string(n_src) + ")");
+  Tensor rel = at::empty({h[0]}, i64), src = at::empty({h[0]}, i64), pos = at::empty({h[0]}, i64), src_ptr = at::empty({n_src + 1}, i64),
+         src_pos = at::empty({h[1]}, i32), edge_pos = at::empty({nnz}, i32);
+  check(lib.cxg_relation_pairs_fill(idx.data_ptr(), ib, etype.data_ptr(), rb, nnz, n_src, r, rel.data_ptr<int64_t>(),
+                                    src.data_ptr<int64_t>(), pos.data_ptr<int64_t>(), src_ptr.data_ptr<int64_t>(),
+                                    src_pos.data_ptr<int32_t>(), edge_pos.data_ptr<int32_t>(), ws.data_ptr(), need, st),
+        "cxg_relation_pairs_fill");
+  return {rel, src, pos, src_ptr, src_pos, edge_pos};
+}
+
 // ---- neighbour sampling ----------------------------------------------------------------------------------------------
 // The most a call may reserve for the nodes and edges a batch can reach; above it the hops are run one by one.
 constexpr int64_t kMostSampled = 1 << 27;
@@ -805,6 +846,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     c10::cuda::CUDAGuard guard(x.device());
     return head_mean_bias(x, bias, heads, c);
   });
+  m.def("relation_pairs", &relation_pairs);
   m.def("sample_batch_fits", &sample_batch_fits);
   m.def("sample_batch", &sample_batch);
 }

@@ -810,44 +810,52 @@ class RelationPairs:
     has 0.4 of num_rel * N of them). Built once per graph."""
 
     def __init__(self, idx, etype, num_src, num_rel):
-        nnz = min(idx.shape[0], etype.shape[0])
-        dev = idx.device
-        key = etype[:nnz].to(torch.int64) * num_src + idx[:nnz].to(torch.int64)
-        used = torch.zeros(num_rel * num_src, dtype=torch.bool, device=dev).index_fill_(0, key, True)
-        pairs = used.nonzero().squeeze(1)
-        rel = torch.div(pairs, num_src, rounding_mode="floor")
-        count = used.view(num_rel, num_src).sum(1)
-        padded = (count + 127) // 128 * 128
-        start, base = count.cumsum(0) - count, padded.cumsum(0) - padded
-        at = torch.arange(pairs.shape[0], device=dev) + (base - start)[rel]
-        self.num_pos = int(padded.sum())
-        # per position: its relation, its source (-1: padding), itself
-        self.rel = torch.repeat_interleave(torch.arange(num_rel, device=dev), padded, output_size=self.num_pos)
-        self.src = torch.full((self.num_pos,), -1, dtype=torch.int64, device=dev).index_copy_(0, at, pairs - rel * num_src)
-        self.pos = torch.arange(self.num_pos, device=dev)
-        where = torch.zeros(num_rel * num_src, dtype=torch.int32, device=dev).index_copy_(0, pairs, at.to(torch.int32))
-        self.idx = where[key]  # position of every edge
-        # the positions of every source, as a CSR graph over the sources
-        of_src = used.view(num_rel, num_src).t()
-        self.src_ptr = torch.zeros(num_src + 1, dtype=torch.int64, device=dev)
-        self.src_ptr[1:] = of_src.sum(1).cumsum(0)
-        self.src_idx = where.view(num_rel, num_src).t()[of_src]
+        etype = etype if etype.dtype in _INDEX_DTYPES else etype.long()
+        # per position: its relation, its source (-1: padding), itself; the positions of every source, as a CSR graph over
+        # the sources; the position of every edge
+        self.rel, self.src, self.pos, self.src_ptr, self.src_idx, self.idx = _native.relation_pairs(
+            idx.contiguous(), etype.contiguous(), num_src, num_rel)
+        self.num_pos = self.rel.shape[0]
 
 
-_pair_cache = {}
+    def tensors(self):
+        return self.rel, self.src, self.pos, self.src_ptr, self.src_idx, self.idx
+
+
+_pair_cache = {}  # key -> (RelationPairs, idx, etype, stream it was built on, event behind the build, bytes)
+_PAIR_CACHE_BYTES = 1 << 30
 
 
 def relation_pairs(idx, etype, num_src, num_rel):
-    """RelationPairs of the graph, kept for the last eight (idx, etype). An entry keeps its tensors alive, so their
-    addresses cannot be handed to another graph."""
+    """RelationPairs of the graph, kept for the last eight (idx, etype), for fewer where these take more than a gigabyte
+    together; forget_graphs() gives them back. An entry keeps its tensors alive, so their addresses cannot be handed to
+    another graph."""
     key = (idx.data_ptr(), etype.data_ptr(), idx.shape[0], etype.shape[0], idx._version, etype._version, num_src, num_rel,
            idx.device)
     hit = _pair_cache.get(key)
     if hit is None:
-        while len(_pair_cache) >= 8:
-            _pair_cache.pop(next(iter(_pair_cache)))
-        hit = _pair_cache[key] = (RelationPairs(idx, etype, num_src, num_rel), idx, etype)
+        pairs = RelationPairs(idx, etype, num_src, num_rel)
+        with _on(idx.device):
+            stream = torch.cuda.current_stream()
+            size = sum(t.numel() * t.element_size() for t in (*pairs.tensors(), idx, etype))
+            kept = list(_pair_cache.items())
+            while kept and (len(kept) >= 8 or size + sum(e[5] for _, e in kept) > _PAIR_CACHE_BYTES):
+                _pair_cache.pop(kept.pop(0)[0], None)
+            hit = _pair_cache[key] = (pairs, idx, etype, stream, stream.record_event(), size)
+    elif _raw_stream(_dev_index(idx.device)) != hit[3].cuda_stream and not torch.cuda.is_current_stream_capturing():
+        with _on(idx.device):  # built on another stream: this one waits for it, and the memory for this one
+            stream = torch.cuda.current_stream()
+            stream.wait_event(hit[4])
+            for t in hit[0].tensors():
+                t.record_stream(stream)
     return hit[0]
+
+
+def forget_graphs():
+    """Gives back what is kept per graph: transposed graphs, combined indices, (relation, source) pairs, destinations."""
+    _native.forget_graphs()
+    for kept in (_pair_cache, _cidx_cache, _DST_CACHE):
+        kept.clear()
 
 
 class _RelationPairsFunction(torch.autograd.Function):
@@ -882,7 +890,8 @@ def relation_pairs_supported(x, weights):
     """Shapes the pair table covers in both directions (tensor-core typed matmul and weight gradient)."""
     k, n = weights.shape[1], weights.shape[2]
     return (x.is_cuda and x.dtype in _FEAT_DTYPES and weights.dtype == x.dtype and k % 16 == 0 and n % 16 == 0
-            and k <= 128 and n <= 128 and weights.shape[0] * x.shape[0] < 2 ** 31)
+            and k <= 128 and n <= 128 and weights.shape[0] < 2 ** 16 - 1 and 0 < x.shape[0]
+            and weights.shape[0] * (x.shape[0] + 255) < 2 ** 31)
 
 
 def relation_pairs_mean(x, weights, ptr, idx, etype, num_node):

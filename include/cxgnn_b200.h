@@ -530,6 +530,26 @@ int cxg_topo_sort_host(const int64_t *ptr_host, const int64_t *idx_host,
                        int64_t *n_order);
 
 /*
+ * The distinct (relation, source) pairs of a graph's edges (rel[e], idx[e]), in order of relation and source, every
+ * relation's positions padded to whole blocks of 128: what cxg_typed_matmul and cxg_typed_wgrad take when every pair is
+ * transformed once. cxg_relation_pairs_count marks and counts them and leaves sizes (device memory) = {positions, pairs,
+ * 1 when an edge lies outside [0, num_rel) x [0, n_src)}; the caller reads them, allocates, and calls
+ * cxg_relation_pairs_fill with the same arguments and the same workspace, untouched, unless sizes[2] is set:
+ *   pos_rel, pos_src, pos [positions]  a position's relation, its source (-1: padding), itself
+ *   src_ptr [n_src + 1], src_pos [pairs]  the positions of every source, by relation (CSR)
+ *   edge_pos [nnz]  the position of every edge's pair
+ * num_rel * (n_src + 255) must be below 2^31, num_rel at most 65534.
+ */
+int cxg_relation_pairs_workspace_size(int64_t n_src, int num_rel, size_t *bytes);
+int cxg_relation_pairs_count(const void *idx, int idx_bytes, const void *rel, int rel_bytes, int64_t nnz,
+                             int64_t n_src, int num_rel, int64_t *sizes, void *workspace, size_t workspace_bytes,
+                             void *stream);
+int cxg_relation_pairs_fill(const void *idx, int idx_bytes, const void *rel, int rel_bytes, int64_t nnz, int64_t n_src,
+                            int num_rel, int64_t *pos_rel, int64_t *pos_src, int64_t *pos, int64_t *src_ptr,
+                            int32_t *src_pos, int32_t *edge_pos, void *workspace, size_t workspace_bytes,
+                            void *stream);
+
+/*
  * Per-relation sub-graphs on the host: rel_schedule (src/cpp/src/schedule.cu:5-63).
  * All pointers are HOST pointers; outputs are caller-allocated, row-major per relation:
  * sub_ptr [num_rel][n_dst+1], sub_idx [num_rel][nnz], sub_target [num_rel][n_dst],
