@@ -40,6 +40,15 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       : "memory");
 }
 
+// v = hi + lo + what two bits of v cannot hold: hi the upper 19 bits of v, lo = v - hi (exact, at most 13 significant bits)
+// moved half a unit of its 19 bits up in magnitude, so that the tensor core, which ignores the other 13 bits of a word,
+// reads it rounded. Cut instead, every product would be short by 1e-7 of itself on the same side. (The addition turns a
+// NaN, which lo is where v is infinite, into -0; hi carries infinities and NaN alone.)
+__device__ __forceinline__ void split_tf32(float v, float &hi, float &lo) {
+  hi = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
+  lo = __uint_as_float(__float_as_uint(v - hi) + 0x1000u);
+}
+
 // Instruction descriptor: fp32 accumulate, A and B of format `fmt` (1 = bf16, 2 = tf32), both K-major.
 __device__ __forceinline__ uint32_t make_idesc(int fmt, int m, int n) {
   uint32_t d = 0;

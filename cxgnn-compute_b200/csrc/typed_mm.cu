@@ -114,15 +114,6 @@ __device__ __forceinline__ float to_tf32(float v) {
   return __uint_as_float(r);
 }
 
-// v = hi + lo + what two bits of v cannot hold: hi the upper 19 bits of v, lo = v - hi (exact, at most 13 significant bits)
-// moved half a unit of its 19 bits up in magnitude, so that the tensor core, which ignores the other 13 bits of a word,
-// reads it rounded. Cut instead, every product would be short by 1e-7 of itself on the same side. (The addition turns a
-// NaN, which lo is where v is infinite, into -0; hi carries infinities and NaN alone.)
-__device__ __forceinline__ void split_tf32(float v, float &hi, float &lo) {
-  hi = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
-  lo = __uint_as_float(__float_as_uint(v - hi) + 0x1000u);
-}
-
 // W [R][K][N] -> Wt [R][N][K]; with `wt_lo` (fp32 only) the two TF32 terms hi = tf32(w), lo = tf32(w - hi).
 template <typename T>
 __global__ void transpose_w(const T *w, T *wt, T *wt_lo, int num_rel, int k, int n) {

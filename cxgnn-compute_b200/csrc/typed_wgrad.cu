@@ -27,6 +27,8 @@
 namespace cxg {
 namespace {
 
+using namespace tc;
+
 constexpr int kProdWarps = 8;
 constexpr int kConvWarps = 4;
 constexpr int kEpiWarps = 4;    // warps 0..3: tensor-memory lanes 32 * warp .. + 31
@@ -56,8 +58,6 @@ struct WgArgs {
   int32_t *status;
   long long wait_cycles;
 };
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 // MN-major operand in a 128-byte swizzled layout: rows of 128 bytes (one per step of the contraction index), `lbo`
 // bytes between 128-byte spans along M / N. 16-bit elements: groups of 8 rows 1024 bytes apart, the 16-byte chunks of
@@ -95,68 +95,6 @@ __device__ __forceinline__ uint32_t make_idesc_mn(int fmt, int m, int n) {
   return d;
 }
 
-// One MMA of a warp: every lane comes here with the same operands and one of them issues it. (Behind `if (lane == 0)` the
-// compiler cannot tell that the operands are the same in all active lanes and an instruction took 134 cycles whatever its
-// size; issued this way 73, and 135 for 128 x 256, which is the tensor core's own time.)
-template <bool TF32>
-__device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  if (TF32)
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-  else
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ bool wait_bar(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int32_t *status,
-                                         long long limit) {
-  const uint32_t b = smem_addr(bar);
-  if (mbar_try_wait(b, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait(b, parity)) {
-    if (*abort_flag) return false;
-    if (clock64() - t0 > limit) {
-      *abort_flag = 1;
-      atomicExch(status, 1);
-      return false;
-    }
-  }
-  return true;
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
-__device__ __forceinline__ void commit_to(uint64_t *bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_addr(bar))
-      : "memory");
-}
-
-// v = hi + lo up to half a unit of lo's 19 bits (see typed_mm.cu)
-__device__ __forceinline__ void split_tf32(float v, float &hi, float &lo) {
-  hi = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
-  lo = __uint_as_float(__float_as_uint(v - hi) + 0x1000u);
-}
-
 struct Barriers {
   uint64_t full[kMaxStages];   // producers -> MMA (or converters): 256 arrivals
   uint64_t conv[kMaxStages];   // converters -> MMA: 128 arrivals
@@ -166,7 +104,7 @@ struct Barriers {
 };
 
 // X3: error-compensated fp32. T = float or __nv_bfloat16. kPos = positions per tile, the contraction length of one
-// pipeline unit: 128, or 64 in the compensated mode, whose stages hold every tile twice.
+// pipeline unit: 128, or 32 in the compensated mode, whose stages hold every tile twice.
 template <typename T, bool X3>
 __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConvWarps : 0)), 1) typed_wgrad_tc(WgArgs a) {
   constexpr bool TF32 = sizeof(T) == 4;
@@ -270,7 +208,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     int64_t ia_next[kAhead], ig_next[kAhead];
     fetch(tile_lo, ia_next, ig_next);
     RelCursor rel(a, tile_lo);
-    tc::Ring ring(S);
+    Ring ring(S);
     bool alive = true;
     for (int64_t tile0 = tile_lo; tile0 < tile_hi && alive; tile0 += kGroup) {
       int64_t ia[kAhead], ig[kAhead];
@@ -316,7 +254,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     // ================= converters: raw fp32 tiles -> hi (in place) and lo (second half of the stage) =================
     const int ct = tid - 32 * kFirstConv;
     const int n16 = static_cast<int>(half_bytes / 16), x16 = spans_x * (kSpan / 16), g16 = n16 - x16;
-    tc::Ring ring(S);
+    Ring ring(S);
     bool alive = true;
     RelCursor rel(a, tile_lo);
     for (int64_t tile = tile_lo; tile < tile_hi && alive; ++tile) {
@@ -363,7 +301,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     const uint32_t idesc = make_idesc_mn(TF32 ? 2 : 1, 128, n_mma);
     const uint32_t idesc_wide = make_idesc_mn(2, 128, small_off ? 2 * n_mma : n_mma);
     const uint32_t step_bytes = kInstrK * 128;  // the next kInstrK positions of a span
-    tc::Ring ring(S);
+    Ring ring(S);
     int64_t chunk = 0;
     int in_chunk = 0;
     bool alive = true, open = false;  // open: the current accumulator holds tiles of relation `cur`
@@ -437,18 +375,10 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
       const uint32_t taddr = tmem_d + (static_cast<uint32_t>(warp * 32) << 16) + buf * tmem_cols;
       for (int c0 = 0; c0 < n; c0 += 16) {
         uint32_t v[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(taddr + c0));
+        tmem_ld16(v, taddr + c0);
         if (X3 && small_off) {
           uint32_t w[16];
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]), "=r"(w[8]),
-                "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
-              : "r"(taddr + small_off + c0));
+          tmem_ld16(w, taddr + small_off + c0);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(w[i]));
