@@ -246,6 +246,7 @@ Tensor spmm(const Tensor &x, const Tensor &ptr, const Tensor &idx, int64_t num_n
     const int64_t vh = edge_val->dim() == 2 ? edge_val->size(1) : 1;
     if (vh != heads) fail("edge_value has " + std::to_string(vh) + " heads, x has " + std::to_string(heads));
   }
+  if (x.size(0) > UINT32_MAX) flags |= CXG_SPMM_GENERIC_WALK;  // the default walk keeps source rows as 32-bit numbers
   c10::cuda::CUDAGuard guard(x.device());
   Tensor y = out ? *out : (x.dim() == 3 ? at::empty({n, heads, feat}, x.options()) : at::empty({n, feat}, x.options()));
   cxg_spmm_desc d = describe(ptr, idx, n, heads, feat, x.scalar_type(), reduce, flags, split);

@@ -47,27 +47,27 @@ extern "C" {
 
 /* ---- flags of cxg_spmm_csr ---------------------------------------------- */
 #define CXG_SPMM_ACCUMULATE 1u /* y[row] += result instead of y[row] = result */
-/* Row-fetch variant of the tiled kernel, kept for measurement; results are
-   bit-identical. Default: 16-byte async copies into shared memory. */
-#define CXG_SPMM_BULK_ROWS 4u /* one bulk async copy (TMA) per row into shared
-                                 memory, completion on an mbarrier             */
+/* Row-fetch variant, kept for measurement: the shared-memory-staged walk with one bulk async copy (TMA) per row, completion
+   on an mbarrier. Default: rows fetched into registers (spmm_walk_impl.cuh). Same results for the same tile size. */
+#define CXG_SPMM_BULK_ROWS 4u
 /* Test hook of the bulk-copy variant: the first stage of the first tile announces 16 bytes
    that no copy delivers, so that its bounded wait runs out and the time-out path (status
    CXG_ETIMEOUT, kernels return, nothing written out of bounds) can be exercised. Use it
    with a short cxg_set_wait_limit_cycles. */
 #define CXG_SPMM_TEST_STALL 8u
-/* Measurement aid: rows of 128 / 256 / 512 bytes without edge values normally take a leaner
-   instantiation of the tiled walk; this flag keeps them on the general one. Same results. */
+/* The shared-memory-staged walk (rows of whole 16-byte chunks up to 1 KiB) or the row-per-group kernel instead of the
+   register-staged walk. Same results for the same tile size. A call whose x has more than 2^32 - 1 rows must set it: the
+   register-staged walk keeps source rows as 32-bit numbers. */
 #define CXG_SPMM_GENERIC_WALK 16u
-/* The tiled kernel normally keeps six persistent CTAs on every SM; with this flag it keeps four, so
-   that a kernel launched from another stream meanwhile (the copy kernel of a collective that overlaps
-   this aggregation) finds room on every SM instead of waiting for this kernel to end. Same results. */
+/* The tiled kernels normally fill every SM with persistent CTAs; with this flag they keep about half of them, so that a
+   kernel launched from another stream meanwhile (the copy kernel of a collective that overlaps this aggregation) finds room
+   on every SM instead of waiting for this kernel to end. Same results for the same tile size. */
 #define CXG_SPMM_SHARE_SMS 32u
-/* Index-stream variant of the lean walk (rows of 128 / 256 / 512 bytes): the source ids of a tile are staged
-   into shared memory by the bulk-copy unit (one 512-byte `cp.async.bulk` per 128 int32 / 64 int64 ids, two
+/* Index-stream variant of the shared-memory-staged walk (rows of 128 / 256 / 512 bytes), kept for measurement: the source
+   ids of a tile are staged into shared memory by the bulk-copy unit (one 512-byte `cp.async.bulk` per 128 int32 / 64 int64 ids, two
    chunks per warp, the next one requested while the current one is read, completion on an mbarrier with a
-   bounded wait) instead of being loaded by the lanes one stage ahead. Needs a 16-byte aligned `idx`; ignored
-   otherwise and on the general walk. Same results bit for bit. CXG_SPMM_TEST_STALL makes every warp's first
+   bounded wait) instead of being loaded by the lanes one stage ahead. Needs a 16-byte aligned `idx`; without it, and for
+   other rows, the general staged walk runs. Same results for the same tile size. CXG_SPMM_TEST_STALL makes every warp's first
    chunk announce 16 bytes that never arrive. */
 #define CXG_SPMM_TMA_INDEX 64u
 
