@@ -4,10 +4,12 @@
 //
 // The kernels stay behind the C ABI of libcxgnn_b200.so: this module opens the library it is told to (init) and calls its
 // entry points. No CUDA code, no other state than the scratch buffers per stream and the transposed graphs.
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/autocast_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <list>
@@ -112,6 +114,27 @@ const Tensor &of_type(const Tensor &t, const char *name, std::initializer_list<a
 const Tensor &feature(const Tensor &t, const char *name) { return of_type(t, name, {at::kFloat, at::kBFloat16}); }
 const Tensor &index_of(const Tensor &t, const char *name) { return of_type(t, name, {at::kLong, at::kInt}); }
 const Tensor &f32(const Tensor &t, const char *name) { return of_type(t, name, {at::kFloat}); }
+
+// A tensor under forward-mode differentiation. The kernels know nothing of its tangent: torch's operators take it where
+// there is one, and the operators of this module go through their autograd function, which refuses it.
+bool has_tangent(const Tensor &t) { return t._fw_grad(/*level=*/0).defined(); }
+
+// Whether the pass has to go through the autograd function.
+bool recorded(const Tensor &t) { return (t.requires_grad() && at::GradMode::is_enabled()) || has_tangent(t); }
+bool recorded(const optional<Tensor> &t) { return t && recorded(*t); }
+template <typename A, typename... B>
+bool recorded(const A &a, const B &...b) {
+  return recorded(a) || recorded(b...);
+}
+
+// Whether torch's own operator has to be called: transforms (vmap, functionalisation, fake tensors and other subclasses),
+// forward-mode differentiation, tracing.
+bool foreign(const Tensor &t) { return at::isTensorSubclassLike(t) || has_tangent(t); }
+bool foreign(const optional<Tensor> &t) { return t && foreign(*t); }
+template <typename... T>
+bool for_torch(const T &...t) {
+  return torch::jit::tracer::isTracing() || (foreign(t) || ...);
+}
 
 void *stream_of(const Tensor &t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
@@ -403,12 +426,13 @@ class SageFunction : public torch::autograd::Function<SageFunction> {
 
 Tensor sage(const Tensor &x, const Tensor &ptr, const Tensor &idx, const optional<Tensor> &edge_val, int64_t num_node,
             int64_t reduce, int64_t flags, int64_t split, bool scatter) {
-  if (at::GradMode::is_enabled() && (x.requires_grad() || (edge_val && edge_val->requires_grad())))
+  if (recorded(x, edge_val))
     return SageFunction::apply(x, ptr, idx, edge_val, num_node, reduce, flags, split, scatter);
   return spmm(x, ptr, idx, num_node, edge_val, reduce, c10::nullopt, c10::nullopt, c10::nullopt, 0, c10::nullopt, flags, split);
 }
 
 Tensor gather_rows(const Tensor &x, const Tensor &rows) {
+  if (for_torch(x, rows)) return x.index_select(0, rows);
   cuda(x, "x");
   of_type(rows, "rows", {at::kLong});
   c10::cuda::CUDAGuard guard(x.device());
@@ -513,7 +537,7 @@ class LinearFunction : public torch::autograd::Function<LinearFunction> {
 // a better one, puts the few values within rounding of zero on its other side, and each of them moves the gradients: those
 // of a sampled batch by up to 3e-4 of their norm, those of a GAT layer by up to 2e-3.
 Tensor linear(const Tensor &x, const Tensor &w, const optional<Tensor> &bias, const optional<Tensor> &add, bool same_bits) {
-  const bool fits = linear_fits(x, w) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
+  const bool fits = !for_torch(x, w, bias, add) && linear_fits(x, w) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
                     (!bias || (bias->scalar_type() == at::kFloat && bias->is_contiguous() && bias->device() == x.device() &&
                                bias->dim() == 1 && bias->size(0) == w.size(0)));
   const bool add_fits = add && dense_rows(*add) && add->size(0) == x.size(0) && add->size(1) == w.size(0) && add->device() == x.device();
@@ -522,9 +546,7 @@ Tensor linear(const Tensor &x, const Tensor &w, const optional<Tensor> &bias, co
     return add ? *add + y : y;
   }
   c10::cuda::CUDAGuard guard(x.device());
-  if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad() || (bias && bias->requires_grad()) ||
-                                     (add && add->requires_grad())))
-    return LinearFunction::apply(x, w, bias, add, same_bits);
+  if (recorded(x, w, bias, add)) return LinearFunction::apply(x, w, bias, add, same_bits);
   return linear_product(x, w, false, bias, add);
 }
 
@@ -608,7 +630,7 @@ class SageLayerFunction : public torch::autograd::Function<SageLayerFunction> {
 // None when the operator does not cover the arguments.
 optional<Tensor> sage_layer(const Tensor &x, const Tensor &ptr, const Tensor &idx, const Tensor &wl, const Tensor &wr,
                             const optional<Tensor> &bl, int64_t n, bool first, int64_t flags, int64_t split) {
-  if (n < 1 || !dense_rows(x) || x.size(0) < n || idx.size(0) < 1 || ptr.size(0) - 1 < n || wl.size(0) != wr.size(0) ||
+  if (for_torch(x, wl, wr, bl) || n < 1 || !dense_rows(x) || x.size(0) < n || idx.size(0) < 1 || ptr.size(0) - 1 < n || wl.size(0) != wr.size(0) ||
       !linear_fits(x, wl) || !linear_fits(x, wr) ||
       !lib.cxg_linear_f32_supported(n, static_cast<int>(x.size(1)), static_cast<int>(wl.size(0))) ||
       at::autocast::is_autocast_enabled(at::kCUDA) ||
@@ -617,9 +639,7 @@ optional<Tensor> sage_layer(const Tensor &x, const Tensor &ptr, const Tensor &id
   index_of(ptr, "ptr");
   index_of(idx, "idx");
   c10::cuda::CUDAGuard guard(x.device());
-  if (at::GradMode::is_enabled() &&
-      (x.requires_grad() || wl.requires_grad() || wr.requires_grad() || (bl && bl->requires_grad())))
-    return SageLayerFunction::apply(x, ptr, idx, wl, wr, bl, n, first, flags, split);
+  if (recorded(x, wl, wr, bl)) return SageLayerFunction::apply(x, ptr, idx, wl, wr, bl, n, first, flags, split);
   return SageLayerFunction::run(x, ptr, idx, wl, wr, bl, n, first, flags, split, nullptr, false);
 }
 
@@ -723,8 +743,7 @@ Tensor gat_layer(const Tensor &x, const Tensor &att_src, const Tensor &att_dst, 
     if (bias->numel() != (concat ? h * c : c)) fail("gat_layer: the bias must have one value per output column");
   }
   c10::cuda::CUDAGuard guard(x.device());
-  if (at::GradMode::is_enabled() &&
-      (x.requires_grad() || att_src.requires_grad() || att_dst.requires_grad() || (bias && bias->requires_grad())))
+  if (recorded(x, att_src, att_dst, bias))
     return GatFunction::apply(x, att_src, att_dst, bias, ptr, idx, n, slope, concat);
   return GatFunction::run(x, att_src, att_dst, bias, ptr, idx, n, slope, concat, nullptr);
 }
