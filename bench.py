@@ -54,9 +54,9 @@ PEER_COPY_GBPS = float(os.environ.get("CXG_PEER_COPY_GBPS", "770"))
 # what --exchange auto picks when the needed rows are few enough: "needed" (pack + NCCL all-to-all), "put" (one gather
 # kernel storing into the peers' buffers) or "putcopy" (pack + copy-engine copies into the peers' buffers)
 AUTO_EXCHANGE = os.environ.get("CXG_BENCH_AUTO_EXCHANGE", "put")
-# dram__bytes_read.sum + dram__bytes_write.sum of one launch of the tiled kernel on one GPU, from ncu
-# captures of these workloads (profiles/spmm_stream_papers.md); None where no capture exists.
-NCU_DRAM_BYTES = {"papers_like": 300.59e9, "papers_tenth": 24.67e9}
+# dram__bytes_read.sum + dram__bytes_write.sum of one launch of the default kernel on one GPU, from ncu captures of these
+# workloads; None where no capture exists (the full size is not captured).
+NCU_DRAM_BYTES = {"papers_tenth": 25.19e9}
 
 
 def load_peaks():
@@ -535,9 +535,9 @@ def main():
     achieved = b_alg_local / (spmm_ms * 1e-3) / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": NCU_DRAM_BYTES.get(args.workload) if world == 1 else None,
-                "traffic_source": "ncu capture summarised in profiles/spmm_stream_papers.md (a constant, not measured by this run)",
+                "traffic_source": "ncu capture of one launch (a constant, not measured by this run)",
                 "peak_source": peak_src,
-                "kernel": "cxg_spmm_csr (plan + spmm_stream + fix kernels)",
+                "kernel": "cxg_spmm_csr (walk_plan + spmm_walk + walk_fix)",
                 "ms": spmm_ms, "algorithmic_bytes": b_alg_local}
     if roofline["traffic"]:
         # DRAM bytes actually moved (ncu, one launch) over the event-timed duration: how busy HBM is

@@ -69,7 +69,9 @@ struct GatArgs {
   float *block_ms;       // [tile][heads][2]: those of a block of a long chain
 };
 
-// exp(x): as __expf, with results below 2^-126 flushed to zero (three instructions instead of six)
+// exp(x) = 2^(x log2 e), with results below 2^-126 flushed to zero. The product and its constant are rounded once each, so
+// the exponent is off by at most |x| * 1.45 * 1.5 * 2^-24; with the 2^-22 of ex2.approx the result is off by at most
+// (1.5 |x| + 4) * 2^-24 of itself.
 __device__ __forceinline__ float exp_flush(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.4426950408889634f));

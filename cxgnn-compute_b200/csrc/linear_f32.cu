@@ -16,8 +16,8 @@
 // The five instructions per 16 columns of K read 20 KB of A and 24 KB of B from shared memory at NT = 128, 344 cycles at its
 // 128 bytes a cycle, against 384 for the products: the operands bound the kernel as much as the tensor pipe, and memory
 // traffic (173 MB for 169,343 rows of 128 -> 128, 26 us) less.
-// Measured against the fp32 library GEMM: 169,343 rows 128 -> 128 49 us (132), 1.94 M rows 128 -> 64 324 us (734), 50,952 rows
-// 256 -> 256 76 us (145), 314 rows 256 -> 256 12.4 us (11.3).
+// Measured, cold, against the fp32 library GEMM: 169,343 rows 128 -> 128 49 us (132), 1.94 M rows 128 -> 64 293 us (734),
+// 50,952 rows 256 -> 256 70 us (145), 314 rows 256 -> 256 16 us (15).
 //
 // Every wait is bounded, as in typed_mm.cu: a role that waits too long raises a CTA-wide flag and the status word, all roles
 // leave their loops, the copies in flight are waited for (bounded as well), and the tensor memory is released.

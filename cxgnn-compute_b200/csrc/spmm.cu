@@ -484,7 +484,7 @@ extern "C" int cxg_spmm_csr_workspace_size(int64_t n_dst, int64_t nnz, int32_t f
   WorkspaceLayout L;
   int rc = plan_layout(n_dst, nnz, static_cast<int64_t>(feat) * heads, split, &L);
   CXG_REQUIRE(rc == CXG_OK, rc, "cxg_spmm_csr_workspace_size: graph too large for 32-bit segment ids");
-  // the streaming path tiles the edge array; its smallest automatic tile is 64 edges
+  // the walks tile the edge array; their smallest automatic tile is 64 edges
   StreamLayout S;
   int tile = split_edges > 0 ? split_edges : 64;
   rc = stream_layout(nnz, static_cast<int64_t>(feat) * heads, tile, &S);

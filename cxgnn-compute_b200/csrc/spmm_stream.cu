@@ -1,6 +1,8 @@
-// Edge-tiled streaming CSR SpMM for sm_100a with the rows staged in shared memory: the measured variants of
-// cxg_spmm_csr that its flags select (bulk row copies, an id ring, the general walk). Without flags the
-// register-staged walk of spmm_walk_impl.cuh runs, same tiles and same bits.
+// Edge-tiled CSR SpMM for sm_100a with the rows staged in shared memory. It serves target lists and accumulating sums of
+// weighted rows (rows of whole 16-byte chunks up to 1 KiB), which the register-staged walk of spmm_walk_impl.cuh leaves to
+// it, more than 2^32 - 1 source rows, and the variants that flags select for measurement (bulk row copies, an id ring). The
+// two walks cut and add rows in the same way, so equal tile sizes give equal bits; the automatic tile sizes differ
+// (stream_tile_edges here, walk_whole_waves there), and with them the sums of rows that tiles cut.
 //
 // Work is cut by EDGES, not by rows: tile t owns edges [t*T, (t+1)*T) of the CSR
 // edge array, whatever rows they belong to, so every warp gets the same number of
@@ -9,11 +11,10 @@
 //
 // One warp walks its tile in CSR order:
 //   * the source ids of a stage are fetched kStages stages ahead (coalesced);
-//   * the feature rows of a stage are copied global -> shared asynchronously, either
-//     with ONE bulk async copy per row issued by the lane that holds the row's id
-//     (`cp.async.bulk`, completion counted on an mbarrier), or with 16-byte
-//     `cp.async` copies; up to kStages stages per warp are in flight and no register
-//     is held for them;
+//   * the feature rows of a stage are copied global -> shared asynchronously with 16-byte
+//     `cp.async` copies or (flag) with ONE bulk async copy per row issued by the lane that
+//     holds the row's id (`cp.async.bulk`, completion counted on an mbarrier); up to
+//     kStages stages per warp are in flight and no register is held for them;
 //   * the rows are added from shared memory strictly in edge order, the whole warp
 //     on one row (32 lanes x 4/8/16 bytes), into one fp32 accumulator per column
 //     (packed f32x2 adds);

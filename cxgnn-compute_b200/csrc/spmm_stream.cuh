@@ -1,4 +1,4 @@
-// Interface between cxg_spmm_csr and its edge-tiled streaming path (spmm_stream.cu).
+// Interface between cxg_spmm_csr and its walk with the rows staged in shared memory (spmm_stream.cu).
 #pragma once
 #include "common.cuh"
 
@@ -8,10 +8,9 @@ namespace cxg {
 enum { kSHdrNumLong = 0, kSHdrNumBlocks = 1, kSHdrError = 63 };  // word 63 is the error word of every SpMM workspace header
 // Values of the error word.
 enum { kSErrNone = 0, kSErrTimeout = 1, kSErrEdgeCount = 2 };
-// Row fetch variants: 16-byte async copies into shared memory (default), one bulk
-// async copy per row into shared memory.
+// Row fetch variants: 16-byte async copies into shared memory, one bulk async copy per row (CXG_SPMM_BULK_ROWS).
 enum { kModeCpAsync = 0, kModeBulk = 1 };
-// Bytes of one chunk of the id ring of the lean walk (two chunks per warp).
+// Bytes of one chunk of the id ring of CXG_SPMM_TMA_INDEX (two chunks per warp).
 constexpr int kIdxChunkBytes = 512;
 
 struct StreamArgs {
@@ -54,7 +53,7 @@ struct StreamLayout {
   int max_long, max_blocks;
 };
 
-// True when the descriptor can take the streaming path (16-byte rows up to 1 KiB, no edge mask).
+// True when this walk covers the descriptor (rows of whole 16-byte chunks up to 1 KiB, no edge mask).
 bool stream_eligible(const cxg_spmm_desc *d);
 // Edges per tile for this call (desc->split_edges when set).
 int stream_tile_edges(const cxg_spmm_desc *d);

@@ -14,13 +14,14 @@
 //     a thread's arrival when its copies have landed, so a producer never waits for its own
 //     copies and up to `stages` tiles are in flight per CTA (waiting with `cp.async.wait_group`
 //     plus a proxy fence in the producer serialised copy and MMA latency and was 13-19 % slower).
-//     The thread that issues the MMAs executes the generic-to-async proxy fence after the barrier.
+//     The warp that issues the MMAs executes the generic-to-async proxy fence after the barrier.
 //     The op is memory-bound at RGCN shapes (K = 128, N = 64: 43 flop per byte in bf16). W[rel]
 //     (pre-transposed once to [N][K]) is copied the same way when the relation changes, after
 //     the MMAs that read the previous one have drained;
-//   * one thread issues K/16 (bf16) or K/8 (tf32) `tcgen05.mma` instructions per tile with M = 128,
-//     N = n, accumulating fp32 in one of two tensor-memory buffers, and commits them to the
-//     barrier that frees the stage and to the one that hands the accumulator to the epilogue;
+//   * one warp walks the units together and an elected lane of it issues K/16 (bf16) or K/8 (tf32) `tcgen05.mma`
+//     instructions per tile with M = 128, N = n (mma_ss says why not one thread), accumulating fp32 in one of two
+//     tensor-memory buffers, and commits them to the barrier that frees the stage and to the one that hands the
+//     accumulator to the epilogue;
 //   * 8 epilogue warps (4 in the error-compensated mode, where converter warps take the other four places)
 //     read their 32 accumulator lanes with `tcgen05.ld` - two groups of four warps, each group one half of the
 //     columns, 64 (fp32: 32) columns per round trip to tensor memory - convert, and write (or atomically add)
@@ -31,9 +32,11 @@
 // fp32 inputs have two tensor-core modes. Plain TF32 (precision 1) feeds the fp32 words to `kind::tf32` as they
 // are, like the reference's tl.dot: products carry 10 mantissa bits (about 6e-4 relative on these shapes). The
 // error-compensated mode (precision 2, "3xTF32") splits every operand into hi = tf32(v) and lo = tf32(v - hi) and
-// accumulates A_hi.W_lo + A_lo.W_hi + A_hi.W_hi into the same tensor-memory accumulator, which restores fp32
-// accuracy (about 1e-6) while the tensor pipe, idle most of the time on this memory-bound op, absorbs the two
-// extra instructions. W is split once by the transposing pre-pass; a tile of A is split in shared memory by
+// accumulates A_hi.W_hi, and A_hi.W_lo + A_lo.W_hi in an accumulator of their own where tensor memory has room
+// (N up to 128: the tensor core cuts its sum at every instruction, which costs the small terms nothing there), joined by
+// the epilogue: 3.2e-7 of the result at K = 128. W_lo lies behind W_hi, so A_hi x [W_hi | W_lo] is one instruction, and
+// the tensor pipe, idle most of the time on this memory-bound op, absorbs the rest. An infinite operand gives infinities
+// or NaN (an infinity times a lower term, zero or of either sign). W is split once by the transposing pre-pass; a tile of A is split in shared memory by
 // converter warps between the producers and the MMA thread (raw -> hi in place, lo into the second half of
 // the stage). To keep several stages in flight with stages twice as large, the K dimension is cut into blocks:
 // the pipeline unit is (tile, K-block) and all blocks of a tile accumulate into one accumulator buffer.

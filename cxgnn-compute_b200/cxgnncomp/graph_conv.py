@@ -436,11 +436,11 @@ class MyGATConv(torch.nn.Module):
         # edge softmax and weighted aggregation as ONE kernel where the shape allows (the reference's sequence of
         # edge_attention + SpMMValOP otherwise, or when set to False)
         self.fused_aggregate = True
-        # True: x @ W^T, its input gradient and its weight gradient run on the library's tensor-core kernels
-        # (compensated TF32) instead of the fp32 library GEMMs torch calls: 1.48 instead of 1.69 ms for the layer's
-        # forward + backward at 169 k nodes. Off by default: in 4 of 54 processes that had also run the bulk-row
-        # measurement variant of the SpMM (CXG_SPMM_FLAGS=4) the layer's output was 3e-5 instead of 2e-6 away from the
-        # float64 result with it (same value on every call of such a process; cause not found).
+        # True: x @ W^T and its gradients run on the typed matmul's kernels with one relation (compensated TF32) instead of
+        # cxgnncomp_backend.linear. Off: it is the less exact of the two (3.2e-7 of the result against 1.2e-7), changes the
+        # rounding in front of the LeakyReLU where gradients are recorded, and gave, in 4 of 54 processes that had also run
+        # the bulk-row measurement variant of the SpMM (CXG_SPMM_FLAGS=4), an output 3e-5 instead of 2e-6 away from float64
+        # (same value on every call of such a process; cause not found).
         self.tensor_core_linear = False
         self.reset_parameters()
 
@@ -476,7 +476,7 @@ class MyGATConv(torch.nn.Module):
         assert x.dim() == 2
         if x.shape[0] != num_src:  # (the gradient of a slice is a copy into zeros)
             x = x[:num_src]
-        if self.tensor_core_linear:  # the layer's linear transform on the library's tensor-core kernels
+        if self.tensor_core_linear:
             x_src = cxgnncomp_backend.dense_linear(x, self.lin_src).view(-1, H, C)
         else:
             # recorded: torch's rounding, as in front of a ReLU (the sums of scores go through a LeakyReLU)

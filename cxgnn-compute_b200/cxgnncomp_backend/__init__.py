@@ -144,7 +144,7 @@ SPLIT_EDGES = 0
 CXG_SPMM_BULK_ROWS = 4
 CXG_SPMM_TEST_STALL = 8  # test hook, see include/cxgnn_b200.h
 CXG_SPMM_GENERIC_WALK = 16
-CXG_SPMM_TMA_INDEX = 64  # source ids staged by bulk copies into a ring in shared memory (lean walk)
+CXG_SPMM_TMA_INDEX = 64  # source ids staged by bulk copies into a ring in shared memory (for measurement)
 CXG_SPMM_SHARE_SMS = 32
 CXG_TMM_TEST_STALL = 4
 CXG_TMM_NO_TMA = 16  # dense mode: 16-byte copies instead of tiled bulk tensor copies for A
@@ -789,7 +789,7 @@ _cidx_cache = []  # (idx, etype, versions, stride, combined), most recent last
 def _combined_index(idx, etype, stride, num_rel):
     """etype[e] * stride + idx[e]: the row of the [num_rel * stride, F] table that edge e reads. Built once per
     (idx, etype) pair and kept (cache of 8), so that the relational aggregation is a plain aggregation over the
-    table and takes the lean walk and the transposed-graph backward; int32 when the table has fewer than 2^31 rows."""
+    table and takes its walk and the transposed-graph backward; int32 when the table has fewer than 2^31 rows."""
     ver = (idx._version, etype._version)
     for it in _cidx_cache:
         if it[0] is idx and it[1] is etype and it[2] == ver and it[3] == stride:

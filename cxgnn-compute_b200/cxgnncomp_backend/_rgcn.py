@@ -231,7 +231,7 @@ def typed_wgrad_supported(x, g, allow_tf32=None):
     if allow_tf32 is None:
         allow_tf32 = sys.modules[__package__].ALLOW_TF32
     split = 2 if (x.dtype == torch.float32 and not allow_tf32) else 1
-    positions = 64 if split == 2 else 128  # per tile, as the kernel chooses them
+    positions = 32 if split == 2 else 128  # per tile, as the kernel chooses them
     spans = sum((t.shape[1] * t.element_size() + 127) // 128 for t in (x, g))
     return max(spans, x.element_size()) * 128 * positions * split <= 224 * 1024
 
