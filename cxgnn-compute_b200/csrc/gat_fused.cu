@@ -219,9 +219,9 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_walk(const __grid_constant
   auto fetch = [&](int64_t t) {
     next_begin = next_stop = 0;
     if (t < n_tiles) {
-      next_row = a.w.tiles[t].row;
-      next_begin = a.w.tiles[t].begin;
-      next_stop = a.w.tiles[t + 1].begin;
+      next_row = static_cast<const WideTile *>(a.w.tiles)[t].row;
+      next_begin = static_cast<const WideTile *>(a.w.tiles)[t].begin;
+      next_stop = static_cast<const WideTile *>(a.w.tiles)[t + 1].begin;
     }
   };
   fetch(wid * NG + lane / G);
@@ -442,9 +442,9 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_wide_forward(const __grid_
   }
   for (int64_t t = wid; t < n_tiles; t += n_warps) {
     TileWalk w{a};
-    w.begin = a.w.tiles[t].begin;
-    w.row = a.w.tiles[t].row;
-    const int64_t end = a.w.tiles[t + 1].begin;
+    w.begin = static_cast<const WideTile *>(a.w.tiles)[t].begin;
+    w.row = static_cast<const WideTile *>(a.w.tiles)[t].row;
+    const int64_t end = static_cast<const WideTile *>(a.w.tiles)[t + 1].begin;
     if (end <= w.begin) continue;
     w.len = static_cast<int>(end - w.begin);
     if (t == 0)
@@ -640,9 +640,9 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_wide_backward(const __grid
   }
   for (int64_t t = wid; t < n_tiles; t += n_warps) {
     TileWalk w{a};
-    w.begin = a.w.tiles[t].begin;
-    w.row = a.w.tiles[t].row;
-    const int64_t end = a.w.tiles[t + 1].begin;
+    w.begin = static_cast<const WideTile *>(a.w.tiles)[t].begin;
+    w.row = static_cast<const WideTile *>(a.w.tiles)[t].row;
+    const int64_t end = static_cast<const WideTile *>(a.w.tiles)[t + 1].begin;
     if (end <= w.begin) continue;
     w.len = static_cast<int>(end - w.begin);
     if (t == 0)
@@ -898,7 +898,7 @@ __global__ void __launch_bounds__(256, 3) gat_fix(const __grid_constant__ GatArg
   int64_t row = 0;
   int ts = 0, k = 0, m = 0;
   if (lane < 2 * per && t < w.max_tiles && t * w.tile < e_total) {
-    const WalkTile here = w.tiles[t], next = w.tiles[t + 1];  // not written behind the last tile, whose end is e_total
+    const WideTile here = static_cast<const WideTile *>(w.tiles)[t], next = static_cast<const WideTile *>(w.tiles)[t + 1];  // not written behind the last tile, whose end is e_total
     const bool tail = lane < per;
     row = tail ? next.row : here.row;
     if (next.begin > here.begin && row < w.n_dst) {
@@ -1144,12 +1144,13 @@ void fill_args(GatArgs &a, const GatLayout &L, void *workspace, int64_t nnz, int
   char *ws = static_cast<char *>(workspace);
   WalkArgs &w = a.w;
   w.hdr = reinterpret_cast<int32_t *>(ws + L.walk.hdr);
-  w.tiles = reinterpret_cast<WalkTile *>(ws + L.walk.tiles);
+  w.tiles = ws + L.walk.tiles;
   w.count = reinterpret_cast<int32_t *>(ws + L.walk.count);
   w.partials = reinterpret_cast<float *>(ws + L.walk.partials);
   w.nnz = nnz;
   w.width = heads * c, w.row_bytes = heads * c * 4, w.heads = heads, w.feat = c;
   w.whole_rows = 0;
+  w.wide_tiles = 1;
   a.part_ms = reinterpret_cast<float *>(ws + L.part_ms);
   a.block_ms = reinterpret_cast<float *>(ws + L.block_ms);
   a.heads = heads;
@@ -1166,7 +1167,7 @@ cudaError_t launch_walk(GatArgs &a, cudaStream_t st) {
   auto go = [&](auto kernel, int g, int ctas) {
     const int per_cta = kThreads / g;
     const int64_t resident = static_cast<int64_t>(kNumSM) * ctas;
-    a.w.tile = walk_whole_waves(a.w.nnz, resident * per_cta);
+    a.w.tile = walk_whole_waves(a.w.nnz, resident * per_cta, 32);
     a.w.max_tiles = (a.w.nnz + a.w.tile - 1) / a.w.tile + 1;
     walk_plan_run(a.w, st);
     int64_t grid = (a.w.max_tiles + per_cta - 1) / per_cta;

@@ -490,7 +490,7 @@ extern "C" int cxg_spmm_csr_workspace_size(int64_t n_dst, int64_t nnz, int32_t f
   rc = stream_layout(nnz, static_cast<int64_t>(feat) * heads, tile, &S);
   CXG_REQUIRE(rc == CXG_OK, rc, "cxg_spmm_csr_workspace_size: graph too large for 32-bit tile ids");
   WalkLayout W;
-  rc = walk_layout(nnz, static_cast<int64_t>(feat) * heads, tile, &W);
+  rc = walk_layout(nnz, walk_part_stride(static_cast<int64_t>(feat) * heads), tile, &W);
   CXG_REQUIRE(rc == CXG_OK, rc, "cxg_spmm_csr_workspace_size: graph too large for 32-bit tile ids");
   *bytes = L.total > S.total ? L.total : S.total;
   if (W.total > *bytes) *bytes = W.total;

@@ -72,9 +72,11 @@ extern "C" int cxg_spmm_csr_static(const cxg_spmm_desc *d, void *stream) {
               (long long)d->nnz, d->feat, d->heads);
   // Scratch this request needs: exact for the tiled kernel, the published upper bound otherwise.
   size_t need = 0;
+  cxg_spmm_desc tiled = *d;
   if (!(d->flags & (CXG_SPMM_BULK_ROWS | CXG_SPMM_TMA_INDEX | CXG_SPMM_GENERIC_WALK)) && walk_eligible(d)) {
     WalkLayout L;
-    int rc = walk_layout(d->nnz, static_cast<int64_t>(d->feat) * d->heads, walk_tile_edges(d), &L);
+    tiled.split_edges = walk_static_tile_edges(d);
+    int rc = walk_layout(d->nnz, static_cast<int64_t>(d->feat) * d->heads, tiled.split_edges, &L);
     CXG_REQUIRE(rc == CXG_OK, rc, "cxg_spmm_csr_static: graph too large for 32-bit tile ids");
     need = L.total;
   } else if (stream_eligible(d)) {
@@ -93,7 +95,7 @@ extern "C" int cxg_spmm_csr_static(const cxg_spmm_desc *d, void *stream) {
   void *scratch = nullptr;
   int rc = static_scratch(&scratch);
   if (rc != CXG_OK) return rc;
-  return cxg_spmm_csr(d, scratch, kStaticScratchBytes, stream);
+  return cxg_spmm_csr(&tiled, scratch, kStaticScratchBytes, stream);
 }
 
 extern "C" int cxg_spmm_csr_static_status(void *stream) {

@@ -23,18 +23,20 @@ __device__ __forceinline__ int64_t tile_of(const WalkArgs &a, int64_t e) {
 }
 
 // Rows that own the first edge of a tile write the tile's record; a hub row that owns many is shared by its warp. One
-// pass over ptr, so it costs what reading ptr costs (1 us for 170,000 rows, 17 us for 14 M), where a search per tile
-// is a chain of 18 dependent loads (10 us). Also clears what the later kernels count in.
-constexpr int kPlanRows = 4;  // rows per thread
+// pass over ptr, so it costs what reading ptr costs (1 us for 170,000 rows, 17 us for 14 M) and the time that its code takes to
+// arrive, where a search per tile is a chain of 18 dependent loads (10 us). Also clears what the later kernels count in.
+constexpr int kFixThreads = 64;  // of walk_fix
 
+template <int kPlanRows>
 __global__ void __launch_bounds__(256) walk_plan(const __grid_constant__ WalkArgs a) {
   const int64_t i0 = blockIdx.x * (256ll * kPlanRows) + threadIdx.x;
-  int64_t raw_b[kPlanRows], raw_e[kPlanRows];
+  int64_t raw_b[kPlanRows], raw_e[kPlanRows], raw_n[kPlanRows];  // of the row, its end, that of the row behind it
 #pragma unroll
   for (int k = 0; k < kPlanRows; ++k) {
     const int64_t r = min(i0 + k * 256, a.n_dst - 1);
     raw_b[k] = load_ptr(a.ptr, r, a.ptr_bytes);
     raw_e[k] = load_ptr(a.ptr, r + 1, a.ptr_bytes);
+    raw_n[k] = a.whole_rows ? load_ptr(a.ptr, min(r + 2, a.n_dst), a.ptr_bytes) : 0;
   }
   const int64_t last = load_ptr(a.ptr, a.n_dst, a.ptr_bytes);
   const int64_t e_total = min(last, a.nnz);
@@ -42,51 +44,70 @@ __global__ void __launch_bounds__(256) walk_plan(const __grid_constant__ WalkArg
 #pragma unroll
   for (int k = 0; k < kPlanRows; ++k)
     if (i0 + k * 256 < a.max_tiles) a.count[i0 + k * 256] = 0;
-  if (i0 == 0) a.tiles[(e_total + a.tile - 1) / a.tile] = WalkTile{a.n_dst, e_total};
-  auto record = [&](int64_t t, int64_t r, int64_t b, int64_t e) {
+  auto put = [&](int64_t t, int64_t row, int64_t begin, int64_t row_begin, int64_t row_end) {
+    if (a.wide_tiles)
+      static_cast<WideTile *>(a.tiles)[t] = WideTile{row, begin};
+    else
+      static_cast<WalkTile *>(a.tiles)[t] = WalkTile{static_cast<uint32_t>(row), static_cast<uint32_t>(begin),
+                                                     static_cast<uint32_t>(row_begin), static_cast<uint32_t>(row_end)};
+  };
+  if (i0 == 0) put((e_total + a.tile - 1) / a.tile, a.n_dst, e_total, e_total, e_total);
+  auto record = [&](int64_t t, int64_t r, int64_t b, int64_t e, int64_t n) {
     const int64_t pos = t * a.tile;
-    WalkTile w{r, pos};
     if (a.whole_rows && pos != b) {
       const int64_t at = b + tile_of(a, pos - b + a.tile - 1) * a.tile;
       if (e - b > a.tile && at < e)
-        w.begin = at;
+        put(t, r, at, b, e);
       else
-        w = WalkTile{r + 1, e};
+        put(t, r + 1, e, e, n);
+    } else {
+      put(t, r, pos, b, e);
     }
-    a.tiles[t] = w;
   };
 #pragma unroll
   for (int k = 0; k < kPlanRows; ++k) {
     const int64_t i = i0 + k * 256;
     const int64_t rb = min(raw_b[k], e_total), re = i < a.n_dst ? min(raw_e[k], e_total) : rb;
+    const int64_t rn = min(raw_n[k], e_total);
     // tiles whose first edge lies in [rb, re)
     const int64_t t0 = tile_of(a, rb + a.tile - 1), t1 = re > rb ? tile_of(a, re + a.tile - 1) : t0;
     const bool many = t1 - t0 > 4;
     if (!many)
-      for (int64_t t = t0; t < t1; ++t) record(t, i, rb, re);
+      for (int64_t t = t0; t < t1; ++t) record(t, i, rb, re, rn);
     for (unsigned left = __ballot_sync(0xffffffffu, many); left != 0; left &= left - 1) {
       const int src = __ffs(left) - 1;
       const int64_t r = __shfl_sync(0xffffffffu, i, src), b = __shfl_sync(0xffffffffu, rb, src),
-                    e = __shfl_sync(0xffffffffu, re, src), u0 = __shfl_sync(0xffffffffu, t0, src),
+                    e = __shfl_sync(0xffffffffu, re, src), n = __shfl_sync(0xffffffffu, rn, src), u0 = __shfl_sync(0xffffffffu, t0, src),
                     u1 = __shfl_sync(0xffffffffu, t1, src);
-      for (int64_t t = u0 + (threadIdx.x & 31); t < u1; t += 32) record(t, r, b, e);
+      for (int64_t t = u0 + (threadIdx.x & 31); t < u1; t += 32) record(t, r, b, e, n);
     }
   }
 }
 
 // Partial sums of the row's chain: element k > 0 is the head partial of tile ts + k, element 0 the tail partial of ts.
 __device__ __forceinline__ float *chain_at(const WalkArgs &a, int64_t ts, int64_t k) {
-  return a.partials + ((ts + k) * 2 + (k == 0 ? 1 : 0)) * a.width;
+  return a.partials + ((ts + k) * 2 + (k == 0 ? 1 : 0)) * a.part_stride;
 }
 
 template <typename T, int VW>
-__device__ __forceinline__ void finish_columns(const WalkArgs &a, T *dst, float (&s)[VW], int64_t deg) {
+__device__ __forceinline__ void finish_columns(const WalkArgs &a, T *dst, int left, float (&s)[VW], int64_t deg) {
 #pragma unroll
   for (int i = 0; i < VW; ++i) {
+    if (i >= left) break;
     float r = s[i];
     if (a.reduce == CXG_MEAN) r = __fdiv_rn(r, static_cast<float>(deg));
     if (a.accumulate) r += to_f32(dst[i]);
     dst[i] = from_f32<T>(r);
+  }
+}
+
+template <int VW>
+__device__ __forceinline__ void load_partial(float (&v)[VW], const float *p) {
+  if constexpr (VW == 4) {
+    const float4 t = __ldcg(reinterpret_cast<const float4 *>(p));
+    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+  } else {
+    v[0] = __ldcg(p);
   }
 }
 
@@ -95,26 +116,18 @@ __device__ __forceinline__ void finish_columns(const WalkArgs &a, T *dst, float 
 template <typename T, int VW>
 __device__ __forceinline__ void chain_sum(const WalkArgs &a, int64_t ts, int64_t k0, int n, int step, float *into, int64_t row, int64_t deg,
                           int lane, int lanes) {
-  constexpr int kDepth = 8;  // partials requested at once (16 halve the resident warps and cost more than they save)
+  constexpr int kDepth = 8;  // partials requested at once (16 take a third of the resident warps and cost more than they save)
   for (int c = lane * VW; c < a.width; c += lanes * VW) {
     float s[VW];
-    auto load = [&](float (&v)[VW], const float *p) {
-      if (VW == 4) {
-        const float4 t = __ldcg(reinterpret_cast<const float4 *>(p));
-        v[0] = t.x, v[1 % VW] = t.y, v[2 % VW] = t.z, v[3 % VW] = t.w;
-      } else {
-        v[0] = __ldcg(p);
-      }
-    };
-    load(s, chain_at(a, ts, k0) + c);
-    const int64_t stride = 2ll * step * a.width;
-    const float *p = a.partials + (ts + k0) * 2 * a.width + c;
+    const int64_t stride = 2ll * step * a.part_stride;
+    const float *p = a.partials + (ts + k0) * 2 * a.part_stride + c;
+    load_partial(s, chain_at(a, ts, k0) + c);
     for (int k = 1; k < n; k += kDepth) {
       float v[kDepth][VW];
 #pragma unroll
       for (int u = 0; u < kDepth; ++u) {
         p += stride;
-        if (k + u < n) load(v[u], p);
+        if (k + u < n) load_partial(v[u], p);
       }
 #pragma unroll
       for (int u = 0; u < kDepth; ++u)
@@ -123,10 +136,12 @@ __device__ __forceinline__ void chain_sum(const WalkArgs &a, int64_t ts, int64_t
           for (int i = 0; i < VW; ++i) s[i] += v[u][i];
     }
     if (into != nullptr) {
-#pragma unroll
-      for (int i = 0; i < VW; ++i) into[c + i] = s[i];
+      if constexpr (VW == 4)
+        *reinterpret_cast<float4 *>(into + c) = make_float4(s[0], s[1], s[2], s[3]);
+      else
+        into[c] = s[0];
     } else {
-      finish_columns<T, VW>(a, static_cast<T *>(a.y) + row * a.width + c, s, deg);
+      finish_columns<T, VW>(a, static_cast<T *>(a.y) + row * a.width + c, a.width - c, s, deg);
     }
   }
 }
@@ -137,22 +152,25 @@ __device__ __forceinline__ void chain_sum(const WalkArgs &a, int64_t ts, int64_t
 // A chain is a handful of loads that depend on one another, so latency is what counts: a warp looks `per` tiles over at
 // once, a lane for each of a tile's two roles, and then adds as many chains side by side as there are `lanes`-wide groups
 // in it (one tile after the other, a warp each: 72 us for 74,500 tiles of rows of 64 columns, now 33 us; 182,000 tiles of 128: 152 us).
+// Nearly every chain has two elements, which lie next to each other: those go first, kPairs per group in flight (2.3 M edges,
+// F = 128: 16.6 us, 20.7 without). Partials lie whole vectors apart, whatever the width. Small blocks, so that the warp with the
+// longest chain does not keep the places of others.
 template <typename T, int VW>
-__global__ void __launch_bounds__(256, 3) walk_fix(const __grid_constant__ WalkArgs a, int per, int lanes) {
+__global__ void __launch_bounds__(kFixThreads, 12) walk_fix(const __grid_constant__ WalkArgs a, int per, int lanes) {
+  constexpr int kPairs = 4;
   dependency_wait();
   const int lane = threadIdx.x & 31;
   const int64_t e_total = edge_total(a);
-  const int64_t t = (blockIdx.x * 8ll + (threadIdx.x >> 5)) * per + (lane & (per - 1));
+  const int64_t t = (blockIdx.x * static_cast<int64_t>(kFixThreads / 32) + (threadIdx.x >> 5)) * per + (lane & (per - 1));
   bool lead = false;
   int64_t row = 0, deg = 0;
   int ts = 0, k = 0, m = 0;
-  if (lane < 2 * per && t < a.max_tiles && t * a.tile < e_total) {
-    const WalkTile here = a.tiles[t], next = a.tiles[t + 1];  // not written behind the last tile, whose end is e_total
+  const WalkTile here = load_tile(a, min(t, a.max_tiles - 1)), next = load_tile(a, min(t, a.max_tiles - 1) + 1);
+  if (lane < 2 * per && t < a.max_tiles && t * a.tile < e_total) {  // behind the last tile, whose end is e_total, nothing is written
     const bool tail = lane < per;
     row = tail ? next.row : here.row;
     if (next.begin > here.begin && row < a.n_dst) {
-      const int64_t rb = load_ptr(a.ptr, row, a.ptr_bytes);
-      const int64_t re = min(load_ptr(a.ptr, row + 1, a.ptr_bytes), e_total);
+      const int64_t rb = tail ? next.row_begin : here.row_begin, re = tail ? next.row_end : here.row_end;
       // cut by this tile's end, or by its start
       if (tail ? (rb < next.begin && rb >= here.begin) : rb < here.begin) {
         const int64_t first = tail ? t : tile_of(a, rb);
@@ -165,16 +183,50 @@ __global__ void __launch_bounds__(256, 3) walk_fix(const __grid_constant__ WalkA
   }
   const int group = lane / lanes, groups = 32 / lanes, in_group = lane & (lanes - 1);
   const unsigned members = (lanes == 32 ? 0xffffffffu : ((1u << lanes) - 1) << (group * lanes));
-  unsigned left = __ballot_sync(0xffffffffu, lead);
-  while (left != 0) {
-    unsigned mine = left;  // group g takes the g-th of the chains that are left
+  // group g takes the g-th of the chains that are left, and so on; -1: none
+  auto take = [&](unsigned &left) {
+    unsigned mine = left;
     for (int i = 0; i < group; ++i) mine &= mine - 1;
     for (int i = 0; i < groups; ++i) left &= left - 1;
-    const int src = mine != 0 ? __ffs(mine) - 1 : 0;
+    return mine != 0 ? __ffs(mine) - 1 : -1;
+  };
+  unsigned left = __ballot_sync(0xffffffffu, lead && m == 2);
+  while (left != 0) {
+    int64_t jrow[kPairs], jdeg[kPairs];
+    int jts[kPairs];
+#pragma unroll
+    for (int j = 0; j < kPairs; ++j) {
+      const int src = take(left);
+      jts[j] = __shfl_sync(0xffffffffu, ts, src & 31);
+      jrow[j] = __shfl_sync(0xffffffffu, row, src & 31);
+      jdeg[j] = __shfl_sync(0xffffffffu, deg, src & 31);
+      if (src < 0) jts[j] = -1;
+    }
+    for (int c = in_group * VW; c < a.width; c += lanes * VW) {
+      float s[kPairs][VW], v[kPairs][VW];
+#pragma unroll
+      for (int j = 0; j < kPairs; ++j)
+        if (jts[j] >= 0) {
+          const float *p = chain_at(a, jts[j], 0) + c;  // element 1 lies a row further on
+          load_partial(s[j], p);
+          load_partial(v[j], p + a.part_stride);
+        }
+#pragma unroll
+      for (int j = 0; j < kPairs; ++j)
+        if (jts[j] >= 0) {
+#pragma unroll
+          for (int i = 0; i < VW; ++i) s[j][i] += v[j][i];
+          finish_columns<T, VW>(a, static_cast<T *>(a.y) + jrow[j] * a.width + c, a.width - c, s[j], jdeg[j]);
+        }
+    }
+  }
+  left = __ballot_sync(0xffffffffu, lead && m != 2);
+  while (left != 0) {
+    const int got = take(left), src = got & 31;
     const int jts = __shfl_sync(0xffffffffu, ts, src), jk = __shfl_sync(0xffffffffu, k, src),
               jm = __shfl_sync(0xffffffffu, m, src);
     const int64_t jrow = __shfl_sync(0xffffffffu, row, src), jdeg = __shfl_sync(0xffffffffu, deg, src);
-    if (mine != 0) {
+    if (got >= 0) {
       const int n_blocks = (jm + kWalkSeqPartials - 1) / kWalkSeqPartials;
       int k0 = jk, n = min(kWalkSeqPartials, jm - jk), step = 1;
       float *into = n_blocks == 1 ? nullptr : chain_at(a, jts, jk);
@@ -216,7 +268,7 @@ bool dispatch(const cxg_spmm_desc *d, const WalkArgs &a, cudaStream_t st, int *r
 
 }  // namespace
 
-int walk_layout(int64_t nnz, int64_t width, int tile, WalkLayout *L) {
+int walk_layout(int64_t nnz, int64_t part_stride, int tile, WalkLayout *L) {
   const int64_t max_tiles = (nnz + tile - 1) / tile + 1;
   if (max_tiles > INT32_MAX) return CXG_ELIMIT;
   size_t off = 0;
@@ -227,7 +279,7 @@ int walk_layout(int64_t nnz, int64_t width, int tile, WalkLayout *L) {
   L->count = off;
   off = align_up(off + static_cast<size_t>(max_tiles) * sizeof(int32_t), 256);
   L->partials = off;
-  off = align_up(off + static_cast<size_t>(max_tiles) * 2 * width * sizeof(float), 256);
+  off = align_up(off + static_cast<size_t>(max_tiles) * 2 * part_stride * sizeof(float), 256);
   L->total = off;
   L->max_tiles = max_tiles;
   return CXG_OK;
@@ -240,25 +292,42 @@ bool walk_eligible(const cxg_spmm_desc *d) {
   const int64_t row_bytes = static_cast<int64_t>(d->feat) * d->heads * elem;
   const int vb = vector_bytes(d);
   if (vb < elem) return false;
+  // the walk counts rows, edges and tiles in 32 bits (and a round of tiles beyond)
+  if (d->n_dst > INT32_MAX - (1 << 20) || d->nnz > INT32_MAX - (1 << 20)) return false;
   return row_bytes <= (vb == 16 ? 128 : 256) * vb;
 }
 
 void walk_plan_run(WalkArgs &a, cudaStream_t st) {
   a.tile_magic = a.tile > 1 && a.tile < 30000 ? ~0ull / static_cast<uint64_t>(a.tile) + 1 : 0;  // exact up to 2^34 edges
-  const int64_t threads = ((a.n_dst > a.max_tiles ? a.n_dst : a.max_tiles) + kPlanRows - 1) / kPlanRows;
-  walk_plan<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(a);
+  // a row per thread while the chip holds a thread for each (a quarter of the code: 5.2 -> 2.8 us for 20,000 rows), then four
+  const int64_t rows = a.n_dst > a.max_tiles ? a.n_dst : a.max_tiles;
+  if (rows <= kNumSM * 2048)
+    walk_plan<1><<<static_cast<unsigned>((rows + 255) / 256), 256, 0, st>>>(a);
+  else
+    walk_plan<4><<<static_cast<unsigned>((rows + 1023) / 1024), 256, 0, st>>>(a);
 }
 
-int walk_whole_waves(int64_t nnz, int64_t resident) {
-  // Whole waves: every resident group gets the same number of tiles, so many that a tile has at most 256 edges (2.3 M
-  // edges, F = 128: 145 us with 3.1 waves of 160 edges, 131 us with 1.9 of 256). From four waves of 512 edges on the
-  // last one no longer matters and the longer tile costs less (126 M edges: 5 % over 256). At least 64 edges, so that
-  // small graphs do not become all borders.
+int walk_whole_waves(int64_t nnz, int64_t resident, int round) {
   if (nnz >= 2048 * resident) return 512;
   const int64_t waves = (nnz + 256 * resident - 1) / (256 * resident);
   const int64_t t = waves > 0 ? (nnz + waves * resident - 1) / (waves * resident) : 0;
-  return t < 64 ? 64 : static_cast<int>((t + 31) / 32 * 32);
+  return t < 64 ? 64 : static_cast<int>((t + round - 1) / round * round);
 }
+
+namespace {
+int tile_of_waves(int64_t nnz, int64_t resident) {
+  // One wave of tiles of up to 256 edges where that is enough (2.3 M edges, F = 64: 71 us, two waves of 128 edges 78), behind
+  // that whole waves of up to 128, which even out what the groups get through (1.2 M edges, F = 201 bf16: 270 us with two
+  // waves of 136, 250 with three of 88; 12.6 M, F = 47: 296 with six of 224, 290 with eleven of 128). From four waves of 512
+  // edges on the longer tile costs less (126 M edges: 10 % less than 128). At least 64 edges, so that small graphs do not become all
+  // borders.
+  if (nnz >= 2048 * resident) return 512;
+  const int64_t most = nnz <= 256 * resident ? 256 : 128;
+  const int64_t waves = (nnz + most * resident - 1) / (most * resident);
+  const int64_t t = waves > 0 ? (nnz + waves * resident - 1) / (waves * resident) : 0;
+  return t < 64 ? 64 : static_cast<int>((t + 7) / 8 * 8);
+}
+}  // namespace
 
 int walk_tile_edges(const cxg_spmm_desc *d) {
   if (d->split_edges > 0) return d->split_edges;
@@ -266,7 +335,16 @@ int walk_tile_edges(const cxg_spmm_desc *d) {
   a.row_bytes = d->feat * d->heads * (d->dtype == CXG_F32 ? 4 : 2);
   int resident = kNumSM * 32;
   dispatch(d, a, nullptr, &resident);
-  return walk_whole_waves(d->nnz, resident);
+  return tile_of_waves(d->nnz, resident);
+}
+
+int walk_static_tile_edges(const cxg_spmm_desc *d) {
+  if (d->split_edges > 0) return d->split_edges;
+  WalkArgs a;
+  a.row_bytes = d->feat * d->heads * (d->dtype == CXG_F32 ? 4 : 2);
+  int resident = kNumSM * 32;
+  dispatch(d, a, nullptr, &resident);
+  return walk_whole_waves(d->nnz, resident, 32);
 }
 
 int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t workspace_bytes, cudaStream_t st) {
@@ -281,14 +359,20 @@ int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t
   a.accumulate = (d->flags & CXG_SPMM_ACCUMULATE) ? 1 : 0;
   a.tile = tile;
   a.whole_rows = whole_rows ? 1 : 0;
+  a.wide_tiles = 0;
   WalkLayout L;
-  const int rc = walk_layout(d->nnz, a.width, tile, &L);
+  a.part_stride = static_cast<int>(walk_part_stride(a.width));
+  int rc = walk_layout(d->nnz, a.part_stride, tile, &L);
+  if (rc == CXG_OK && workspace_bytes < L.total) {  // scratch of a fixed size
+    a.part_stride = a.width;
+    rc = walk_layout(d->nnz, a.part_stride, tile, &L);
+  }
   if (rc != CXG_OK) return set_error(rc, "cxg_spmm_csr: graph too large for 32-bit tile ids");
   if (workspace == nullptr || workspace_bytes < L.total)
     return set_error(CXG_EWORKSPACE, "cxg_spmm_csr: workspace %zu bytes, need %zu", workspace_bytes, L.total);
   char *ws = reinterpret_cast<char *>(workspace);
   a.hdr = reinterpret_cast<int32_t *>(ws + L.hdr);
-  a.tiles = reinterpret_cast<WalkTile *>(ws + L.tiles);
+  a.tiles = ws + L.tiles;
   a.count = reinterpret_cast<int32_t *>(ws + L.count);
   a.partials = reinterpret_cast<float *>(ws + L.partials);
   a.max_tiles = L.max_tiles;
@@ -297,17 +381,18 @@ int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t
   // tiles a warp looks over: one while the chip holds a warp for each, up to sixteen (two roles on 32 lanes)
   int per = 1;
   while (per < 16 && L.max_tiles > static_cast<int64_t>(per) * kNumSM * 24) per *= 2;
-  const unsigned fg = static_cast<unsigned>((L.max_tiles + 8 * per - 1) / (8 * per));
-  const bool v4 = a.width % 4 == 0;
+  const int per_block = kFixThreads / 32 * per;
+  const unsigned fg = static_cast<unsigned>((L.max_tiles + per_block - 1) / per_block);
+  const bool v4 = a.part_stride % 4 == 0;
   int lanes = 1;  // per chain
   while (lanes < 32 && lanes * (v4 ? 4 : 1) < a.width) lanes *= 2;
   cudaError_t e;
   if (d->dtype == CXG_F32)
-    e = v4 ? launch_dependent(walk_fix<float, 4>, fg, 256, 0, st, a, per, lanes)
-           : launch_dependent(walk_fix<float, 1>, fg, 256, 0, st, a, per, lanes);
+    e = v4 ? launch_dependent(walk_fix<float, 4>, fg, kFixThreads, 0, st, a, per, lanes)
+           : launch_dependent(walk_fix<float, 1>, fg, kFixThreads, 0, st, a, per, lanes);
   else
-    e = v4 ? launch_dependent(walk_fix<__nv_bfloat16, 4>, fg, 256, 0, st, a, per, lanes)
-           : launch_dependent(walk_fix<__nv_bfloat16, 1>, fg, 256, 0, st, a, per, lanes);
+    e = v4 ? launch_dependent(walk_fix<__nv_bfloat16, 4>, fg, kFixThreads, 0, st, a, per, lanes)
+           : launch_dependent(walk_fix<__nv_bfloat16, 1>, fg, kFixThreads, 0, st, a, per, lanes);
   if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_spmm_csr: %s", cudaGetErrorString(e));
   count_launches(3);
   return check_launch("cxg_spmm_csr (walk)");

@@ -7,10 +7,19 @@ namespace cxg {
 // Longer chains of partial rows are added in ordered blocks of this many partials.
 constexpr int kWalkSeqPartials = 64;
 
-// What the plan leaves per tile: its first row and its first edge. The entry behind the last tile ends the last one.
-struct WalkTile {
+// Word of the header that counts the tiles handed out behind the first round.
+constexpr int kWalkHdrNext = 8;
+
+// What the plan leaves per tile: its first row, its first edge and that row's range of edges (what the walk and the fix-up
+// would otherwise fetch from ptr, one round trip behind the record). The entry behind the last tile ends the last one.
+struct __align__(16) WalkTile {
+  uint32_t row, begin, row_begin, row_end;
+};
+// The same of the fused GAT walks, which count in 64 bits.
+struct __align__(16) WideTile {
   int64_t row, begin;
 };
+static_assert(sizeof(WalkTile) == sizeof(WideTile), "one layout holds either");
 
 struct WalkArgs {
   const void *ptr;
@@ -26,12 +35,14 @@ struct WalkArgs {
   int row_bytes, width, feat, heads, ptr_bytes, idx_bytes, reduce;
   int tile;       // edges per tile
   int accumulate; // 1: the output is added to
+  int wide_tiles;
   int whole_rows; // 1: rows of up to `tile` edges are never cut (see spmm_walk_impl.cuh)
   uint64_t tile_magic;  // ceil(2^64 / tile), 0: divide
   int32_t *hdr;
-  WalkTile *tiles;  // [tile + 1]
+  void *tiles;      // [tile + 1] WalkTile or (wide_tiles) WideTile
   int32_t *count;   // [tile] finished blocks of the long chain that starts in the tile
-  float *partials;  // [tile][2][width]: head partial, tail partial
+  float *partials;  // [tile][2][part_stride]: head partial, tail partial
+  int part_stride;  // width in whole 16-byte vectors, or width
 };
 
 struct WalkLayout {
@@ -39,14 +50,19 @@ struct WalkLayout {
   int64_t max_tiles;
 };
 
-int walk_layout(int64_t nnz, int64_t width, int tile, WalkLayout *L);
+// part_stride: floats per partial, at least the width.
+int walk_layout(int64_t nnz, int64_t part_stride, int tile, WalkLayout *L);
+// Floats per partial where there is room: whole 16-byte vectors.
+constexpr int64_t walk_part_stride(int64_t width) { return (width + 3) / 4 * 4; }
 // True when the walk covers the descriptor: no edge mask, output rows in order and overwritten or (without edge values)
 // added to, rows that fit its lane layouts.
 bool walk_eligible(const cxg_spmm_desc *d);
 // The plan kernel for a.ptr, a.tile, a.whole_rows: fills hdr, tiles, count (and sets a.tile_magic).
 void walk_plan_run(WalkArgs &a, cudaStream_t st);
-// Edges per tile when `resident` tiles are walked at the same time.
-int walk_whole_waves(int64_t nnz, int64_t resident);
+// Edges per tile when `resident` tiles are walked at the same time: whole waves of up to 256 edges, or 512.
+int walk_whole_waves(int64_t nnz, int64_t resident, int round);
+// Edges per tile of cxg_spmm_csr_static, whose scratch has a fixed size: these decide which graphs it takes.
+int walk_static_tile_edges(const cxg_spmm_desc *d);
 // Edges per tile for this call (desc->split_edges when set).
 int walk_tile_edges(const cxg_spmm_desc *d);
 int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t workspace_bytes, cudaStream_t st);
@@ -62,6 +78,10 @@ bool walk_launch_bf16_4(const WalkArgs &a, int valmode, bool share, cudaStream_t
 bool walk_launch_bf16_2(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
 
 #ifdef __CUDACC__
+__device__ __forceinline__ WalkTile load_tile(const WalkArgs &a, int64_t t) {
+  const uint4 v = reinterpret_cast<const uint4 *>(a.tiles)[t];
+  return WalkTile{v.x, v.y, v.z, v.w};
+}
 // Edges the kernels walk: ptr[n_dst], but never more than the caller declared.
 __device__ __forceinline__ int64_t edge_total(const WalkArgs &a) {
   const int64_t e = load_ptr(a.ptr, a.n_dst, a.ptr_bytes);

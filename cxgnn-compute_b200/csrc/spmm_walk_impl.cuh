@@ -3,16 +3,17 @@
 // Work is cut by EDGES: tile t owns the edges [t*T, (t+1)*T) of the CSR edge array. A tile is walked by a GROUP of G
 // lanes, 32 / G tiles side by side in a warp. A lane holds NV vectors of VB bytes of every row, so that narrow rows do
 // not cost a whole warp instruction per load and rows of any width (F = 47, 100 ...) keep most of their lanes busy.
-// Feature rows go global -> registers through L1 (where the hub rows of a power-law graph are found again: 32 % of the
-// sectors), U edges in flight per lane, and are added strictly in edge order, one fp32 accumulator per column. When the walk passes the end of a row the accumulators are written and reset; rows
-// without edges get zeros on the way.
+// Feature rows go global -> registers through L1 (where the hub rows of a power-law graph are found again: 32 to 43 % of the
+// sectors), U edges in flight per lane, and are added strictly in edge order, one fp32 accumulator per column. When the walk
+// passes the end of a row the accumulators are written and reset; rows without edges get zeros on the way.
 //
 // A row inside one tile is therefore summed like a sequential loop. A row that crosses tile borders leaves one fp32
 // partial per tile; walk_fix adds the partials in tile order (sequentially up to 64; longer chains in blocks of 64
 // consecutive partials, whose sums are then added in block order). No atomics touch feature data. (Letting the tile that
 // arrives last add them inside this kernel measured 30 % slower: the fence and the counter cost every tile two round
 // trips to L2 while the gather saturates it. The same holds for a search of the tile's first row in here: walk_plan
-// leaves it, and the record of a group's next tile is fetched a tile ahead.)
+// leaves it. Neighbouring tiles walked as one piece, so that ids and row ends go on, measured 3 % slower below 3 M edges and no
+// faster above: what a tile costs is its partials, not its start.)
 // whole_rows: tile borders are moved so that only rows longer than T are cut, at multiples of T from their own start:
 // tile t then owns the pieces that START in [t*T, (t+1)*T).
 //
@@ -20,12 +21,17 @@
 // accumulating outputs have an instantiation of their own, scattered ones (targets) and those that accumulate sums of
 // weighted rows take spmm_stream / spmm_rows.
 //
-// What bounds it: L2 and DRAM where rows are wide, the instructions per edge below 256 bytes a row (so no bounds test, no
-// address arithmetic and no wait for a row pointer per edge). Staging the rows in shared memory with 16-byte
+// What bounds it: DRAM where x is far larger than L2 (126 M edges, F = 100: 90 % of copy bandwidth), L2 for wide rows, and in
+// between the data stage of the load path, which takes one pass per line and eight lanes: 5.4 passes per edge of 12.6 M edges
+// with F = 48 and edge values kept it 87 % busy. So lanes behind a row read what their neighbours read, ids and edge values
+// come four at a time out of shared memory (a shuffle is a pass per edge), and 32-bit counters keep everything in 64
+// registers (8 blocks per SM; the 64-bit ones spilled 100 to 200 bytes per lane, which are passes too). Tiles are handed
+// out as warps come for them: SMs differ by 20 % in what they get through. Measured, whole call, before -> now: 12.6 M
+// edges, F = 128 407 -> 357 us, with edge values 577 -> 386; F = 48 251 -> 223 and 374 -> 241; F = 47 389 -> 337 and 442 ->
+// 356; 126 M edges, F = 100 mean 5.19 -> 4.78 ms; 200 M, F = 128 bf16 6.23 -> 5.69 ms; 2.3 M, F = 128 117 -> 109 us.
+// Staging the rows in shared memory with 16-byte
 // asynchronous copies was the form before: it needs a load, an address and a barrier more per edge, and rows that do not
 // start at a multiple of 128 bytes land there at half the rate (F = 100: 12.9 ms for 126 M edges; here 4.9 ms).
-// Measured, whole call, before -> now: 126 M edges, F = 100 fp32 12.9 -> 4.9 ms, F = 64 3.8 -> 2.9, F = 128 5.5 -> 5.1,
-// F = 128 bf16 3.8 -> 3.2 ms; 12.6 M edges, F = 47 1.20 -> 0.43 ms; 2.3 M edges, F = 128 172 -> 131 us, F = 256 562 -> 205 us.
 #pragma once
 #include "spmm_stream.cuh"
 #include "spmm_walk.cuh"
@@ -64,6 +70,31 @@ __device__ __forceinline__ int32_t load_id_stream(const int32_t *p) {
   int32_t v;
   asm volatile("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
+}
+
+// The low 32 bits of an id (a row number below 2^32) and of a row pointer (an edge number below 2^32), of either width.
+__device__ __forceinline__ uint32_t load_id_low(const uint8_t *p) {
+  uint32_t v;
+  asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t load_ptr_low(const void *ptr, int i, int ptr_bytes) {
+  return __ldg(reinterpret_cast<const uint32_t *>(static_cast<const uint8_t *>(ptr) + static_cast<uint64_t>(static_cast<uint32_t>(i)) * static_cast<uint32_t>(ptr_bytes)));
+}
+
+// Two or four words of shared memory.
+template <int N, typename V>
+__device__ __forceinline__ void load_ids(V (&v)[N], const V *p) {
+  static_assert(N == 2 || N == 4, "");
+  if constexpr (N == 4) {
+    const uint4 t = *reinterpret_cast<const uint4 *>(p);
+    const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+    __builtin_memcpy(v, w, 16);
+  } else {
+    const uint2 t = *reinterpret_cast<const uint2 *>(p);
+    const uint32_t w[2] = {t.x, t.y};
+    __builtin_memcpy(v, w, 8);
+  }
 }
 
 // EL = fp32 values in VB bytes of T
@@ -208,19 +239,20 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
   const int lane = threadIdx.x & 31;
   const int lg = lane & (G - 1);
   dependency_wait();
-  const int64_t e_total = edge_total(a);
-  const int64_t n_tiles = (e_total + a.tile - 1) / a.tile;
-  const int64_t wid = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
-  const int64_t n_warps = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
+  const uint32_t e_total = static_cast<uint32_t>(edge_total(a));
+  const int n_dst = static_cast<int>(a.n_dst);
+  const int n_tiles = static_cast<int>((e_total + static_cast<int64_t>(a.tile) - 1) / a.tile);
+  const int step = static_cast<int>(gridDim.x) * (kThreads / 32) * NG;  // tiles that are walked at the same time
   const int rb = a.row_bytes;
-  // vector q of this lane covers bytes [(lg + q * G) * VB, +VB) of a row; one that lies behind the row reads the lane's
-  // first vector again (or the row's; no other sectors) and is not stored
+  const uint32_t pitch = static_cast<uint32_t>(rb);
+  // vector q of this lane covers bytes [(lg + q * G) * VB, +VB) of a row; one that lies behind the row reads the row's last
+  // vector again (the line its neighbours read: a load takes a pass per line and eight lanes) and is not stored
   auto on = [&](int q) { return (lg + q * G) * VB < rb; };
   const uint8_t *xq[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q)
-    xq[q] = static_cast<const uint8_t *>(a.x) + (on(q) ? (lg + q * G) * VB : (on(0) ? lg * VB : 0));
-  uint8_t *y0 = static_cast<uint8_t *>(a.y) + lg * VB;
+    xq[q] = static_cast<const uint8_t *>(a.x) + (on(q) ? (lg + q * G) * VB : (rb - 1) / VB * VB);
+  auto row_of_y = [&](int r) { return static_cast<uint8_t *>(a.y) + static_cast<uint64_t>(r) * static_cast<uint32_t>(rb) + lg * VB; };
   int head[NV];
   if (VALMODE == 2) {
 #pragma unroll
@@ -232,42 +264,48 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
     for (int q = 0; q < NV; ++q)
       if (on(q)) store_row_bytes<T, VB>(dst + q * G * VB, f[q]);
   };
-  auto zero_row = [&](uint8_t *dst) {
+  auto zero_row = [&](int r) {
     if (VALMODE == 4) return;
     float z[NV][EL];
 #pragma unroll
     for (int q = 0; q < NV; ++q)
 #pragma unroll
       for (int i = 0; i < EL; ++i) z[q][i] = 0.f;
-    store(dst, z);
+    store(row_of_y(r), z);
   };
+  const int t_first = static_cast<int>((blockIdx.x * static_cast<unsigned>(kThreads) + threadIdx.x) / G);
   if (e_total == 0) {  // no edge at all: every row is empty
-    for (int64_t r = wid * NG + lane / G; r < a.n_dst; r += n_warps * NG) zero_row(y0 + r * rb);
+    for (int r = t_first; r < n_dst; r += step) zero_row(r);
     return;
   }
 
-  // what the plan left for this group's next tile: its first row and first edge, and the first edge behind it
-  int64_t next_row = 0, next_begin = 0, next_stop = 0;
-  auto fetch = [&](int64_t t) {
-    next_begin = next_stop = 0;
-    if (t < n_tiles) {
-      next_row = a.tiles[t].row;
-      next_begin = a.tiles[t].begin;
-      next_stop = a.tiles[t + 1].begin;
+  // Ids (and values) of a batch of 32 edges per group, read four at a time by all lanes of the group: a shuffle per edge
+  // takes the load path's data stage as often as a quarter of a 512-byte row does. Groups lie 36 words apart: other banks.
+  constexpr int kBatch = 36;
+  __shared__ __align__(16) uint32_t id_stage[kThreads / 32][NG * kBatch];
+  __shared__ __align__(16) float val_stage[VALMODE == 1 ? kThreads / 32 : 1][VALMODE == 1 ? NG * kBatch : 4];
+  uint32_t *my_ids = id_stage[threadIdx.x >> 5] + lane / G * kBatch;
+  float *my_vals = VALMODE == 1 ? val_stage[threadIdx.x >> 5] + lane / G * kBatch : nullptr;
+  // the groups of a warp take neighbouring tiles: the first by the warp's number, then whichever are next
+  int t_next = 0;
+  for (int t = t_first; t - lane / G < n_tiles; t = t_next) {
+    t_next = n_tiles;
+    if (step < n_tiles) {
+      if (lane == 0) t_next = step + atomicAdd(a.hdr + kWalkHdrNext, NG);
     }
-  };
-  fetch(wid * NG + lane / G);
-  for (int64_t t0 = wid * NG; t0 < n_tiles; t0 += n_warps * NG) {
-    const int64_t t = t0 + lane / G;
-    const int64_t begin = next_begin;
-    int64_t row = next_row;
-    const int len = next_stop > begin ? static_cast<int>(next_stop - begin) : 0;
-    fetch(t + n_warps * NG);
+    uint32_t begin = 0, row_begin = 0, row_end = 0;
+    int row = 0, len = 0;
+    if (t < n_tiles) {
+      const WalkTile here = load_tile(a, t);
+      begin = here.begin, row_begin = here.row_begin, row_end = here.row_end;
+      row = static_cast<int>(here.row);
+      len = static_cast<int>(load_tile(a, t + 1).begin - begin);
+    }
 
     // Source ids (and edge values) are requested a whole batch of 32 edges ahead: lane lg holds edges j * G + lg.
     constexpr int IB = 32 / G;
-    uint32_t id_cur[IB], id_nxt[IB];
-    float val_cur[IB], val_nxt[IB];
+    uint32_t id_nxt[IB];
+    float val_nxt[IB];
     auto load_batch = [&](int first) {
 #pragma unroll
       for (int j = 0; j < IB; ++j) {
@@ -275,45 +313,46 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
         id_nxt[j] = 0u;
         val_nxt[j] = 0.f;
         if (pos < len) {
-          if (a.idx_bytes == 8)
-            id_nxt[j] = static_cast<uint32_t>(load_id_stream(static_cast<const int64_t *>(a.idx) + begin + pos));
-          else
-            id_nxt[j] = static_cast<uint32_t>(load_id_stream(static_cast<const int32_t *>(a.idx) + begin + pos));
+          const uint32_t e = begin + pos;
+          id_nxt[j] = load_id_low(static_cast<const uint8_t *>(a.idx) + static_cast<uint64_t>(e) * static_cast<uint32_t>(a.idx_bytes));
           if (a.edge_rel != nullptr)
-            id_nxt[j] += static_cast<uint32_t>(static_cast<int64_t>(__ldg(a.edge_rel + begin + pos)) * a.rel_stride);
-          if (VALMODE == 1) val_nxt[j] = __ldg(a.edge_val + begin + pos);
+            id_nxt[j] += static_cast<uint32_t>(static_cast<int64_t>(__ldg(a.edge_rel + e)) * a.rel_stride);
+          if (VALMODE == 1) val_nxt[j] = __ldg(a.edge_val + e);
         }
       }
     };
 
     // Row ends are positions relative to `begin`. The end of the row after the current one is requested a row ahead and
     // kept as it was loaded, so that nothing waits for it before it is used.
-    auto end_raw = [&](int64_t r) -> int64_t { return load_ptr(a.ptr, min(r + 1, a.n_dst), a.ptr_bytes); };
-    auto end_rel = [&](int64_t r, int64_t raw) -> int {
-      const int64_t v = raw - begin;
-      return r >= a.n_dst || v > kFar ? kFar : static_cast<int>(v);
+    auto end_raw = [&](int r) { return load_ptr_low(a.ptr, min(r + 1, n_dst), a.ptr_bytes); };
+    auto end_rel = [&](int r, uint32_t raw) -> int {
+      const uint32_t v = raw - begin;
+      return r >= n_dst || v > static_cast<uint32_t>(kFar) ? kFar : static_cast<int>(v);
     };
     int rend = kFar, rstart = 0, stop = kFar;
-    int64_t next_raw = 0;
+    uint32_t next_raw = 0;
     if (len > 0) {
       if (t == 0)
-        for (int64_t r = 0; r < row; ++r) zero_row(y0 + r * rb);  // leading rows without edges
-      rend = end_rel(row, end_raw(row));
-      while (rend == 0) ++row, rend = end_rel(row, end_raw(row));  // empty rows that the previous tile's walk wrote
+        for (int r = 0; r < row; ++r) zero_row(r);  // leading rows without edges
+      rstart = row_begin < begin ? -1 : 0;  // before the tile: how far does not matter
       next_raw = end_raw(row + 1);
-      const int64_t s = load_ptr(a.ptr, row, a.ptr_bytes) - begin;
-      rstart = s < -kFar ? -kFar : static_cast<int>(s);
+      rend = end_rel(row, row_end);
+      while (rend == 0) {  // empty rows that the previous tile's walk wrote
+        ++row;
+        rend = end_rel(row, next_raw);
+        next_raw = end_raw(row + 1);
+      }
       stop = min(rend, len);
     }
-    uint8_t *yr = y0 + row * rb;
     // What rows hold that are added to is asked for a row ahead, so that it is in L2 when the walk comes to their end.
     // (2.3 M edges, F = 128 fp32: 157 us, 171 without it, 165 with the row held in registers from its start, which at
     // F = 256 spills: 265 / 300 / 402; overwriting 126 and 206. Through spmm_stream it took 240 and 675.)
     auto request_old = [&]() {
-      if (VALMODE != 4 || row + 1 >= a.n_dst) return;
+      if (VALMODE != 4 || row + 1 >= n_dst) return;
+      const uint8_t *yr = row_of_y(row + 1);
 #pragma unroll
       for (int q = 0; q < NV; ++q)
-        if (on(q)) asm volatile("prefetch.global.L2 [%0];" ::"l"(yr + rb + q * G * VB));
+        if (on(q)) asm volatile("prefetch.global.L2 [%0];" ::"l"(yr + q * G * VB));
     };
     if (len > 0) request_old();
     A acc[NV];
@@ -325,6 +364,7 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
       const bool row_done = pos == rend;
       if (row_done && rstart >= 0) {
         const float d = static_cast<float>(rend - rstart);
+        uint8_t *yr = row_of_y(row);
         float f[NV][EL];
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
@@ -337,16 +377,20 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
           }
         }
         store(yr, f);
-      } else if (row < a.n_dst) {
+      } else if (row < n_dst) {
         // the row began in an earlier tile, or goes on in the next one
-        float *p = a.partials + (t * 2 + (rstart < 0 ? 0 : 1)) * a.width + lg * EL;
+        float *p = a.partials + (static_cast<int64_t>(t) * 2 + (rstart < 0 ? 0 : 1)) * a.part_stride + lg * EL;
 #pragma unroll
         for (int q = 0; q < NV; ++q)
           if (on(q)) {
             float f[EL];
             acc[q].get(f);
 #pragma unroll
-            for (int i = 0; i < EL; ++i) p[q * G * EL + i] = f[i];
+            for (int i = 0; i < EL; i += EL % 4 == 0 ? 4 : 1)
+              if constexpr (EL % 4 == 0)
+                *reinterpret_cast<float4 *>(p + q * G * EL + i) = make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]);
+              else
+                p[q * G * EL + i] = f[i];
           }
       }
 #pragma unroll
@@ -355,11 +399,10 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
         rstart = pos;
         for (;;) {
           ++row;
-          yr += rb;
           rend = end_rel(row, next_raw);
           next_raw = end_raw(row + 1);
           if (rend != pos) break;
-          zero_row(yr);  // a row without edges
+          zero_row(row);  // a row without edges
         }
         request_old();
       }
@@ -367,69 +410,64 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
     };
 
     const int longest = G == 32 ? len : __reduce_max_sync(0xffffffffu, len);
-    struct Step {
-      Words<W> v[U][NV];
-      float ev[U][VALMODE == 2 ? NV : 1];
-    };
-    // requests the rows of edges [p, p + U)
-    auto issue = [&](Step &st, int p) {
+    load_batch(0);
+    for (int p = 0; p < longest; p += U) {
       const int in_batch = p & 31;
       if (in_batch == 0) {
+        __syncwarp();
 #pragma unroll
-        for (int j = 0; j < IB; ++j) id_cur[j] = id_nxt[j], val_cur[j] = val_nxt[j];
+        for (int j = 0; j < IB; ++j) {
+          my_ids[j * G + lg] = id_nxt[j];
+          if (VALMODE == 1) my_vals[j * G + lg] = val_nxt[j];
+        }
+        __syncwarp();
         load_batch(p + 32);
       }
-      uint32_t id = id_cur[0];
-      float val = val_cur[0];
-#pragma unroll
-      for (int j = 1; j < IB; ++j) {
-        id = in_batch >= j * G ? id_cur[j] : id;
-        if (VALMODE == 1) val = in_batch >= j * G ? val_cur[j] : val;
-      }
-      const int lane0 = in_batch & (G - 1);
+      // the rows of edges [p, p + U)
+      Words<W> v[U][NV];
+      constexpr int W4 = U < 4 ? U : 4;
+      uint32_t ids[W4];
+      float vals[W4];
+      float ev[VALMODE == 2 ? U : 1][VALMODE == 2 ? NV : 1];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const uint32_t nid = __shfl_sync(0xffffffffu, id, lane0 + u, G);
-        const uint64_t off = static_cast<uint64_t>(nid) * static_cast<uint32_t>(rb);
+        if (u % W4 == 0) load_ids(ids, my_ids + in_batch + u);
+        const uint64_t off = static_cast<uint64_t>(ids[u % W4]) * pitch;
 #pragma unroll
-        for (int q = 0; q < NV; ++q) load_row_bytes<VB>(st.v[u][q], xq[q] + off);
-        if (VALMODE == 1) st.ev[u][0] = __shfl_sync(0xffffffffu, val, lane0 + u, G);
-        if (VALMODE == 2) {
+        for (int q = 0; q < NV; ++q) load_row_bytes<VB>(v[u][q], xq[q] + off);
+        if constexpr (VALMODE == 2) {
           const int pos = min(p + u, len - 1);
 #pragma unroll
-          for (int q = 0; q < NV; ++q) st.ev[u][q] = len > 0 ? __ldg(a.edge_val + (begin + pos) * a.heads + head[q]) : 0.f;
+          for (int q = 0; q < NV; ++q)
+            ev[u][q] = len > 0 ? __ldg(a.edge_val + (static_cast<int64_t>(begin) + pos) * a.heads + head[q]) : 0.f;
         }
       }
-    };
-    // adds them; groups that have passed the end of their tile add into accumulators that nobody reads
-    auto consume = [&](const Step &st, int p) {
+      // adds them; groups that have passed the end of their tile add into accumulators that nobody reads
       auto add = [&](int u) {
+        if (VALMODE == 1 && u % W4 == 0) load_ids(vals, my_vals + in_batch + u);
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
-          if (VALMODE == 0 || VALMODE >= 3)
-            acc[q].add(st.v[u][q]);
+          if constexpr (VALMODE == 0 || VALMODE >= 3)
+            acc[q].add(v[u][q]);
+          else if constexpr (VALMODE == 1)
+            acc[q].fma(v[u][q], vals[u % W4]);
           else
-            acc[q].fma(st.v[u][q], st.ev[u][VALMODE == 2 ? q : 0]);
+            acc[q].fma(v[u][q], ev[u][q]);
         }
       };
       // no row ends among the U edges of any group (not worth asking with four groups: one of them nearly always has one)
       if (NG <= 2 && !__any_sync(0xffffffffu, stop - p <= U)) {
 #pragma unroll
         for (int u = 0; u < U; ++u) add(u);
-        return;
-      }
+      } else {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        add(u);
-        if (p + u + 1 == stop) event(p + u + 1);
+        for (int u = 0; u < U; ++u) {
+          add(u);
+          if (p + u + 1 == stop) event(p + u + 1);
+        }
       }
-    };
-    load_batch(0);
-    Step s;
-    for (int p = 0; p < longest; p += U) {
-      issue(s, p);
-      consume(s, p);
     }
+    t_next = __shfl_sync(0xffffffffu, t_next, 0) + lane / G;
   }
 }
 
