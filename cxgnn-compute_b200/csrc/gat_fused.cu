@@ -1151,6 +1151,7 @@ void fill_args(GatArgs &a, const GatLayout &L, void *workspace, int64_t nnz, int
   w.width = heads * c, w.row_bytes = heads * c * 4, w.heads = heads, w.feat = c;
   w.whole_rows = 0;
   w.wide_tiles = 1;
+  w.x_rows = nullptr, w.copy_vectors = 0;
   a.part_ms = reinterpret_cast<float *>(ws + L.part_ms);
   a.block_ms = reinterpret_cast<float *>(ws + L.block_ms);
   a.heads = heads;

@@ -33,6 +33,8 @@ struct Lib {
   CXG_FN(cxg_last_error_string);
   CXG_FN(cxg_spmm_csr_workspace_size);
   CXG_FN(cxg_spmm_csr);
+  CXG_FN(cxg_spmm_csr_rows_size);
+  CXG_FN(cxg_spmm_csr_rows);
   CXG_FN(cxg_spmm_csr_backward);
   CXG_FN(cxg_csr_transpose_workspace_size);
   CXG_FN(cxg_csr_transpose);
@@ -68,6 +70,8 @@ void init(const std::string &path) {
   CXG_FN(cxg_last_error_string);
   CXG_FN(cxg_spmm_csr_workspace_size);
   CXG_FN(cxg_spmm_csr);
+  CXG_FN(cxg_spmm_csr_rows_size);
+  CXG_FN(cxg_spmm_csr_rows);
   CXG_FN(cxg_spmm_csr_backward);
   CXG_FN(cxg_csr_transpose_workspace_size);
   CXG_FN(cxg_csr_transpose);
@@ -246,12 +250,21 @@ cxg_spmm_desc describe(const Tensor &ptr, const Tensor &idx, int64_t n, int64_t 
   return d;
 }
 
-void run_spmm(cxg_spmm_desc &d, const Tensor &on) {
-  size_t need = 0;
+void run_spmm(cxg_spmm_desc &d, const Tensor &x) {
+  size_t need = 0, copy = 0;
   check(lib.cxg_spmm_csr_workspace_size(d.n_dst, d.nnz, d.feat, d.heads, d.split_edges, &need), "cxg_spmm_csr_workspace_size");
-  void *st = stream_of(on);
-  const Workspace ws = workspace_on(on.device().index(), st, static_cast<int64_t>(need), "spmm");
-  check(lib.cxg_spmm_csr(&d, ws.data(), ws.bytes(), st), "cxg_spmm_csr");
+  check(lib.cxg_spmm_csr_rows_size(&d, x.size(0), &copy), "cxg_spmm_csr_rows_size");
+  Tensor rows;
+  if (copy > 0) {
+    try {
+      rows = at::empty({static_cast<int64_t>(copy)}, x.options().dtype(at::kByte));
+    } catch (const c10::OutOfMemoryError &) {  // x as it is, then
+      copy = 0;
+    }
+  }
+  void *st = stream_of(x);
+  const Workspace ws = workspace_on(x.device().index(), st, static_cast<int64_t>(need), "spmm");
+  check(lib.cxg_spmm_csr_rows(&d, x.size(0), copy > 0 ? rows.data_ptr() : nullptr, copy, ws.data(), ws.bytes(), st), "cxg_spmm_csr");
 }
 
 // y = A x for the first rows of the graph; x [N, F] or [N, H, F]

@@ -474,6 +474,9 @@ int plan_layout(int64_t n_dst, int64_t nnz, int64_t width, int split, WorkspaceL
 
 using namespace cxg;
 
+// Flags that select another kernel than the register-staged walk.
+static constexpr uint32_t kNotTheWalk = CXG_SPMM_BULK_ROWS | CXG_SPMM_TMA_INDEX | CXG_SPMM_GENERIC_WALK;
+
 extern "C" int cxg_spmm_csr_workspace_size(int64_t n_dst, int64_t nnz, int32_t feat, int32_t heads,
                                            int32_t split_edges, size_t *bytes) {
   CXG_REQUIRE(bytes != nullptr, CXG_ENULL, "cxg_spmm_csr_workspace_size: bytes is NULL");
@@ -497,8 +500,8 @@ extern "C" int cxg_spmm_csr_workspace_size(int64_t n_dst, int64_t nnz, int32_t f
   return CXG_OK;
 }
 
-extern "C" int cxg_spmm_csr(const cxg_spmm_desc *d, void *workspace, size_t workspace_bytes,
-                            void *stream) {
+// rows: scratch for a copy of the n_src rows of x (walk_copy_bytes of it), or NULL.
+static int spmm_csr(const cxg_spmm_desc *d, int64_t n_src, void *rows, void *workspace, size_t workspace_bytes, void *stream) {
   CXG_REQUIRE(d != nullptr, CXG_ENULL, "cxg_spmm_csr: desc is NULL");
   CXG_REQUIRE(d->n_dst >= 0 && d->nnz >= 0, CXG_EINVAL, "cxg_spmm_csr: negative n_dst or nnz");
   CXG_REQUIRE(d->feat > 0 && d->heads > 0, CXG_EINVAL, "cxg_spmm_csr: feat=%d heads=%d", d->feat,
@@ -522,11 +525,10 @@ extern "C" int cxg_spmm_csr(const cxg_spmm_desc *d, void *workspace, size_t work
   CXG_REQUIRE(d->edge_rel == nullptr || d->rel_stride > 0, CXG_EINVAL,
               "cxg_spmm_csr: edge_rel needs rel_stride > 0");
 
-  const uint32_t variant = CXG_SPMM_BULK_ROWS | CXG_SPMM_TMA_INDEX | CXG_SPMM_GENERIC_WALK;
-  if (!(d->flags & variant) && walk_eligible(d)) {
+  if (!(d->flags & kNotTheWalk) && walk_eligible(d)) {
     CXG_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 16 == 0, CXG_EINVAL,
                 "cxg_spmm_csr: workspace must be 16-byte aligned");
-    return walk_launch(d, !stream_eligible(d), workspace, workspace_bytes, as_stream(stream));
+    return walk_launch(d, !stream_eligible(d), n_src, rows, workspace, workspace_bytes, as_stream(stream));
   }
   if (stream_eligible(d)) {
     CXG_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 16 == 0, CXG_EINVAL,
@@ -600,4 +602,27 @@ extern "C" int cxg_spmm_csr(const cxg_spmm_desc *d, void *workspace, size_t work
   }
   count_launches(may_split ? 4 : 1);
   return check_launch("cxg_spmm_csr");
+}
+
+extern "C" int cxg_spmm_csr(const cxg_spmm_desc *d, void *workspace, size_t workspace_bytes, void *stream) {
+  return spmm_csr(d, 0, nullptr, workspace, workspace_bytes, stream);
+}
+
+extern "C" int cxg_spmm_csr_rows_size(const cxg_spmm_desc *d, int64_t n_src, size_t *bytes) {
+  CXG_REQUIRE(d != nullptr && bytes != nullptr, CXG_ENULL, "cxg_spmm_csr_rows_size: desc or bytes is NULL");
+  const bool walk = d->n_dst > 0 && d->feat > 0 && d->heads > 0 && (d->dtype == CXG_F32 || d->dtype == CXG_BF16) &&
+                    !(d->flags & kNotTheWalk);
+  *bytes = walk ? walk_copy_bytes(d, n_src) : 0;
+  return CXG_OK;
+}
+
+extern "C" int cxg_spmm_csr_rows(const cxg_spmm_desc *d, int64_t n_src, void *rows, size_t rows_bytes, void *workspace,
+                                 size_t workspace_bytes, void *stream) {
+  size_t need = 0;
+  const int rc = cxg_spmm_csr_rows_size(d, n_src, &need);
+  if (rc != CXG_OK) return rc;
+  const bool copy = need > 0 && rows != nullptr;
+  CXG_REQUIRE(!copy || rows_bytes >= need, CXG_EWORKSPACE, "cxg_spmm_csr_rows: %zu bytes for the rows, need %zu", rows_bytes, need);
+  CXG_REQUIRE(!copy || reinterpret_cast<uintptr_t>(rows) % 32 == 0, CXG_EINVAL, "cxg_spmm_csr_rows: rows must be 32-byte aligned");
+  return spmm_csr(d, n_src, copy ? rows : nullptr, workspace, workspace_bytes, stream);
 }

@@ -1,4 +1,6 @@
 // Plan, fix-up and dispatch of the register-staged tiled walk (spmm_walk_impl.cuh).
+#include <type_traits>
+
 #include "spmm_stream.cuh"
 #include "spmm_walk.cuh"
 
@@ -16,19 +18,60 @@ int vector_bytes(const cxg_spmm_desc *d) {
   return vb;
 }
 
+// Bytes from a copied row to the next: whole lines, so that eight lanes' vectors lie in one.
+int64_t copy_pitch(int64_t row_bytes) { return (row_bytes + 127) / 128 * 128; }
+
 // e / tile
 __device__ __forceinline__ int64_t tile_of(const WalkArgs &a, int64_t e) {
   const uint64_t v = static_cast<uint64_t>(e);
   return static_cast<int64_t>(a.tile_magic ? __umul64hi(v, a.tile_magic) : v / a.tile);
 }
 
+// One 16-byte vector of the copy per thread, zeros behind a row's end. Words of the source are 4-byte aligned, its rows are not
+// always (bf16): a vector is put together from the words around it.
+template <typename T>
+__device__ __forceinline__ void copy_vector(const WalkArgs &a, int64_t i) {
+  constexpr int kElem = static_cast<int>(sizeof(T));
+  const int per_row = (a.row_bytes + 15) / 16;
+  const int64_t row = i / per_row;
+  const int at = static_cast<int>(i - row * per_row) * 16;
+  const int n = min(16, a.row_bytes - at) / kElem;  // values of the row in the vector
+  const T *src = reinterpret_cast<const T *>(static_cast<const uint8_t *>(a.x_rows) + row * a.row_bytes + at);
+  union {
+    uint4 v;
+    uint32_t w[4];
+    uint16_t h[8];
+  } out;
+  out.v = make_uint4(0, 0, 0, 0);
+  if (kElem == 4) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k < n) out.w[k] = __ldg(reinterpret_cast<const uint32_t *>(src) + k);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k < n) out.h[k] = __ldg(reinterpret_cast<const uint16_t *>(src) + k);
+  }
+  *reinterpret_cast<uint4 *>(static_cast<uint8_t *>(const_cast<void *>(a.x)) + row * a.x_pitch + at) = out.v;
+}
+
 // Rows that own the first edge of a tile write the tile's record; a hub row that owns many is shared by its warp. One
 // pass over ptr, so it costs what reading ptr costs (1 us for 170,000 rows, 17 us for 14 M) and the time that its code takes to
 // arrive, where a search per tile is a chain of 18 dependent loads (10 us). Also clears what the later kernels count in.
 constexpr int kFixThreads = 64;  // of walk_fix
+constexpr int kCopyVectors = 4;  // vectors of the copy per thread
 
-template <int kPlanRows>
+template <int kPlanRows, typename Copy>
 __global__ void __launch_bounds__(256) walk_plan(const __grid_constant__ WalkArgs a) {
+  if constexpr (!std::is_void_v<Copy>) {
+    if (blockIdx.x >= a.plan_blocks) {
+      const int64_t i0 = static_cast<int64_t>(blockIdx.x - a.plan_blocks) * (256ll * kCopyVectors) + threadIdx.x;
+#pragma unroll
+      for (int k = 0; k < kCopyVectors; ++k)
+        if (i0 + k * 256 < a.copy_vectors) copy_vector<Copy>(a, i0 + k * 256);
+      return;
+    }
+  }
   const int64_t i0 = blockIdx.x * (256ll * kPlanRows) + threadIdx.x;
   int64_t raw_b[kPlanRows], raw_e[kPlanRows], raw_n[kPlanRows];  // of the row, its end, that of the row behind it
 #pragma unroll
@@ -248,11 +291,14 @@ __global__ void __launch_bounds__(kFixThreads, 12) walk_fix(const __grid_constan
   }
 }
 
-bool dispatch(const cxg_spmm_desc *d, const WalkArgs &a, cudaStream_t st, int *resident_tiles) {
+bool dispatch(const cxg_spmm_desc *d, const WalkArgs &a, bool copied, cudaStream_t st, int *resident_tiles) {
   const int valmode = d->flags & CXG_SPMM_ACCUMULATE ? 4
                       : d->edge_val == nullptr       ? (d->reduce == CXG_MEAN ? 3 : 0)
                                                      : (d->heads == 1 ? 1 : 2);
   const bool share = (d->flags & CXG_SPMM_SHARE_SMS) != 0;
+  if (copied)
+    return d->dtype == CXG_F32 ? walk_launch_f32_copy(a, valmode, share, st, resident_tiles)
+                               : walk_launch_bf16_copy(a, valmode, share, st, resident_tiles);
   int vb = vector_bytes(d);
   // narrow rows take the vector that occupies eight lanes, the fewest a tile is given
   while (vb > 4 && a.row_bytes <= 4 * vb) vb /= 2;
@@ -301,10 +347,16 @@ void walk_plan_run(WalkArgs &a, cudaStream_t st) {
   a.tile_magic = a.tile > 1 && a.tile < 30000 ? ~0ull / static_cast<uint64_t>(a.tile) + 1 : 0;  // exact up to 2^34 edges
   // a row per thread while the chip holds a thread for each (a quarter of the code: 5.2 -> 2.8 us for 20,000 rows), then four
   const int64_t rows = a.n_dst > a.max_tiles ? a.n_dst : a.max_tiles;
-  if (rows <= kNumSM * 2048)
-    walk_plan<1><<<static_cast<unsigned>((rows + 255) / 256), 256, 0, st>>>(a);
+  const int per_thread = rows <= kNumSM * 2048 ? 1 : 4;
+  a.plan_blocks = static_cast<unsigned>((rows + 256 * per_thread - 1) / (256 * per_thread));
+  const unsigned grid = a.plan_blocks + static_cast<unsigned>((a.copy_vectors + 256 * kCopyVectors - 1) / (256 * kCopyVectors));
+  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(a); };
+  if (a.copy_vectors == 0)
+    per_thread == 1 ? go(walk_plan<1, void>) : go(walk_plan<4, void>);
+  else if (a.row_bytes == a.width * 4)
+    per_thread == 1 ? go(walk_plan<1, float>) : go(walk_plan<4, float>);
   else
-    walk_plan<4><<<static_cast<unsigned>((rows + 1023) / 1024), 256, 0, st>>>(a);
+    per_thread == 1 ? go(walk_plan<1, __nv_bfloat16>) : go(walk_plan<4, __nv_bfloat16>);
 }
 
 int walk_whole_waves(int64_t nnz, int64_t resident, int round) {
@@ -329,12 +381,12 @@ int tile_of_waves(int64_t nnz, int64_t resident) {
 }
 }  // namespace
 
-int walk_tile_edges(const cxg_spmm_desc *d) {
+int walk_tile_edges(const cxg_spmm_desc *d, bool copied) {
   if (d->split_edges > 0) return d->split_edges;
   WalkArgs a;
   a.row_bytes = d->feat * d->heads * (d->dtype == CXG_F32 ? 4 : 2);
   int resident = kNumSM * 32;
-  dispatch(d, a, nullptr, &resident);
+  dispatch(d, a, copied, nullptr, &resident);
   return tile_of_waves(d->nnz, resident);
 }
 
@@ -343,18 +395,44 @@ int walk_static_tile_edges(const cxg_spmm_desc *d) {
   WalkArgs a;
   a.row_bytes = d->feat * d->heads * (d->dtype == CXG_F32 ? 4 : 2);
   int resident = kNumSM * 32;
-  dispatch(d, a, nullptr, &resident);
+  dispatch(d, a, false, nullptr, &resident);
   return walk_whole_waves(d->nnz, resident, 32);
 }
 
-int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t workspace_bytes, cudaStream_t st) {
-  const int tile = walk_tile_edges(d);
+size_t walk_copy_bytes(const cxg_spmm_desc *d, int64_t n_src) {
+  const int elem = d->dtype == CXG_F32 ? 4 : 2;
+  const int64_t row_bytes = static_cast<int64_t>(d->feat) * d->heads * elem;
+  const uint64_t bits = static_cast<uint64_t>(row_bytes) | reinterpret_cast<uintptr_t>(d->x);
+  if (!walk_eligible(d) || (d->flags & CXG_SPMM_ACCUMULATE) || (d->heads > 1 && d->edge_val != nullptr)) return 0;
+  if (n_src <= 0 || n_src > UINT32_MAX || row_bytes <= 64 || bits % (row_bytes <= 128 ? 8 : 16) == 0) return 0;
+  // The copy costs a row's bytes twice per source, an edge gains what its loads cost: 245,000 sources, fp32, x as it is / copied
+  // (us): F = 19 (one line) 67 / 56 at 5 edges per source; F = 47 85 / 98 at 5, 123 / 125 at 11, 175 / 163 at 21, 337 / 290 at
+  // 51; F = 101 148 / 158, 209 / 195, 305 / 255. Odd numbers of bf16 values: F = 47 83 / 88 at 5, 120 / 102 at 11, 400 / 236 at
+  // 51; F = 201 225 / 250, 337 / 260. Small graphs do not repay the work behind the plan: 220,000 edges of 94 bytes 38 / 42, of
+  // 404 bytes 46 / 43.
+  const int64_t edges = row_bytes <= 128 ? 5 : bits % 4 != 0 ? 8 : 12;
+  if (d->nnz < edges * n_src || d->nnz * row_bytes < (40 << 20)) return 0;
+  return static_cast<size_t>(n_src) * copy_pitch(row_bytes);
+}
+
+int walk_launch(const cxg_spmm_desc *d, bool whole_rows, int64_t n_src, void *rows, void *workspace, size_t workspace_bytes,
+                cudaStream_t st) {
+  const bool copied = rows != nullptr;
+  const int tile = walk_tile_edges(d, copied);
   WalkArgs a;
   a.ptr = d->ptr, a.idx = d->idx, a.x = d->x, a.y = d->y;
   a.edge_val = d->edge_val, a.edge_rel = d->edge_rel;
   a.n_dst = d->n_dst, a.nnz = d->nnz, a.rel_stride = d->rel_stride;
   a.feat = d->feat, a.heads = d->heads, a.width = d->feat * d->heads;
   a.row_bytes = a.width * (d->dtype == CXG_F32 ? 4 : 2);
+  a.x_pitch = a.row_bytes;
+  a.x_rows = nullptr;
+  a.copy_vectors = 0;
+  if (copied) {
+    a.x_rows = d->x, a.x = rows;
+    a.x_pitch = static_cast<int>(copy_pitch(a.row_bytes));
+    a.copy_vectors = n_src * ((a.row_bytes + 15) / 16);
+  }
   a.ptr_bytes = d->ptr_bytes, a.idx_bytes = d->idx_bytes, a.reduce = d->reduce;
   a.accumulate = (d->flags & CXG_SPMM_ACCUMULATE) ? 1 : 0;
   a.tile = tile;
@@ -363,7 +441,7 @@ int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t
   WalkLayout L;
   a.part_stride = static_cast<int>(walk_part_stride(a.width));
   int rc = walk_layout(d->nnz, a.part_stride, tile, &L);
-  if (rc == CXG_OK && workspace_bytes < L.total) {  // scratch of a fixed size
+  if (rc == CXG_OK && workspace_bytes < L.total && !copied) {  // scratch of a fixed size
     a.part_stride = a.width;
     rc = walk_layout(d->nnz, a.part_stride, tile, &L);
   }
@@ -377,7 +455,7 @@ int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t
   a.partials = reinterpret_cast<float *>(ws + L.partials);
   a.max_tiles = L.max_tiles;
   walk_plan_run(a, st);
-  if (!dispatch(d, a, st, nullptr)) return set_error(CXG_EUNSUPPORTED, "cxg_spmm_csr: rows of %d bytes", a.row_bytes);
+  if (!dispatch(d, a, copied, st, nullptr)) return set_error(CXG_EUNSUPPORTED, "cxg_spmm_csr: rows of %d bytes", a.row_bytes);
   // tiles a warp looks over: one while the chip holds a warp for each, up to sixteen (two roles on 32 lanes)
   int per = 1;
   while (per < 16 && L.max_tiles > static_cast<int64_t>(per) * kNumSM * 24) per *= 2;

@@ -33,6 +33,7 @@ struct WalkArgs {
   int64_t rel_stride;
   int64_t max_tiles;
   int row_bytes, width, feat, heads, ptr_bytes, idx_bytes, reduce;
+  int x_pitch;    // bytes from a row of x to the next (row_bytes, or those of the copied rows)
   int tile;       // edges per tile
   int accumulate; // 1: the output is added to
   int wide_tiles;
@@ -43,6 +44,10 @@ struct WalkArgs {
   int32_t *count;   // [tile] finished blocks of the long chain that starts in the tile
   float *partials;  // [tile][2][part_stride]: head partial, tail partial
   int part_stride;  // width in whole 16-byte vectors, or width
+  // rows copied to whole 16-byte vectors by the plan kernel's blocks behind the first plan_blocks (x is that copy then)
+  const void *x_rows;     // the caller's rows
+  int64_t copy_vectors;   // 16-byte vectors of the copy, 0: none
+  unsigned plan_blocks;
 };
 
 struct WalkLayout {
@@ -64,8 +69,12 @@ int walk_whole_waves(int64_t nnz, int64_t resident, int round);
 // Edges per tile of cxg_spmm_csr_static, whose scratch has a fixed size: these decide which graphs it takes.
 int walk_static_tile_edges(const cxg_spmm_desc *d);
 // Edges per tile for this call (desc->split_edges when set).
-int walk_tile_edges(const cxg_spmm_desc *d);
-int walk_launch(const cxg_spmm_desc *d, bool whole_rows, void *workspace, size_t workspace_bytes, cudaStream_t st);
+int walk_tile_edges(const cxg_spmm_desc *d, bool copied);
+// rows: scratch for a copy of the n_src rows of x, of the size that walk_copy_bytes gives, or null.
+int walk_launch(const cxg_spmm_desc *d, bool whole_rows, int64_t n_src, void *rows, void *workspace, size_t workspace_bytes,
+                cudaStream_t st);
+// Bytes of a copy of x in rows of whole 16-byte vectors, where reading that copy is worth making it; otherwise 0.
+size_t walk_copy_bytes(const cxg_spmm_desc *d, int64_t n_src);
 
 // One launcher per element type and vector width, each in a translation unit of its own. False: no kernel for it. With
 // resident_tiles set nothing is launched: it receives the number of tiles that are walked at the same time.
@@ -75,6 +84,8 @@ bool walk_launch_f32_4(const WalkArgs &a, int valmode, bool share, cudaStream_t 
 bool walk_launch_bf16_16(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
 bool walk_launch_bf16_8(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
 bool walk_launch_bf16_4(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
+bool walk_launch_f32_copy(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
+bool walk_launch_bf16_copy(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
 bool walk_launch_bf16_2(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
 
 #ifdef __CUDACC__

@@ -1,0 +1,8 @@
+// Tiled walk, fp32 rows that the plan kernel has copied to whole 16-byte vectors.
+#include "spmm_walk_impl.cuh"
+
+namespace cxg {
+bool walk_launch_f32_copy(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles) {
+  return walk::launch_copy<float>(a, valmode, share, st, resident_tiles);
+}
+}  // namespace cxg

@@ -230,7 +230,9 @@ __device__ __forceinline__ void add_words(float *f, const Words<(VB + 3) / 4> &r
 // VB: bytes per load of a lane; NV loads per row, G lanes per tile, U edges in flight per lane. VALMODE: 0 no
 // edge values, 1 one per edge, 2 one per (edge, head), 3 none and the mean of the row, 4 none and the sum (or the mean) is
 // added to the output.
-template <typename T, int VB, int G, int NV, int U, int VALMODE, int MINB>
+// COPY: the rows of x are copies in whole vectors (walk_plan), those of y are not: a lane stores the values of its vector
+// that lie inside the row one by one.
+template <typename T, int VB, int G, int NV, int U, int VALMODE, int MINB, bool COPY>
 __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constant__ WalkArgs a) {
   using A = Acc<T, VB>;
   constexpr int W = (VB + 3) / 4;
@@ -244,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
   const int n_tiles = static_cast<int>((e_total + static_cast<int64_t>(a.tile) - 1) / a.tile);
   const int step = static_cast<int>(gridDim.x) * (kThreads / 32) * NG;  // tiles that are walked at the same time
   const int rb = a.row_bytes;
-  const uint32_t pitch = static_cast<uint32_t>(rb);
+  const uint32_t pitch = static_cast<uint32_t>(COPY ? a.x_pitch : rb);
   // vector q of this lane covers bytes [(lg + q * G) * VB, +VB) of a row; one that lies behind the row reads the row's last
   // vector again (the line its neighbours read: a load takes a pass per line and eight lanes) and is not stored
   auto on = [&](int q) { return (lg + q * G) * VB < rb; };
@@ -262,7 +264,15 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
   auto store = [&](uint8_t *dst, float (&f)[NV][EL]) {
 #pragma unroll
     for (int q = 0; q < NV; ++q)
-      if (on(q)) store_row_bytes<T, VB>(dst + q * G * VB, f[q]);
+      if constexpr (COPY) {
+        const int left = (rb - (lg + q * G) * VB) / static_cast<int>(sizeof(T));
+        T *out = reinterpret_cast<T *>(dst + q * G * VB);
+#pragma unroll
+        for (int i = 0; i < EL; ++i)
+          if (i < left) out[i] = from_f32<T>(f[q][i]);
+      } else if (on(q)) {
+        store_row_bytes<T, VB>(dst + q * G * VB, f[q]);
+      }
   };
   auto zero_row = [&](int r) {
     if (VALMODE == 4) return;
@@ -387,7 +397,9 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
             acc[q].get(f);
 #pragma unroll
             for (int i = 0; i < EL; i += EL % 4 == 0 ? 4 : 1)
-              if constexpr (EL % 4 == 0)
+              if (COPY && (lg + q * G) * EL + i >= a.part_stride)
+                break;
+              else if constexpr (EL % 4 == 0)
                 *reinterpret_cast<float4 *>(p + q * G * EL + i) = make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]);
               else
                 p[q * G * EL + i] = f[i];
@@ -476,7 +488,7 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
 // 3 to 25 % slower on 128- to 512-byte rows, twice the edges per step (128 registers) 40 %, and two steps in flight with
 // half the edges each 30 %. Narrow fp32 rows read one word at a time (F = 47) want four edges per step, not eight.
 // With resident_tiles set nothing is launched: it receives the tiles that are walked at the same time.
-template <typename T, int VB, int VALMODE>
+template <typename T, int VB, int VALMODE, bool COPY = false>
 bool launch_width(const WalkArgs &a, bool share, cudaStream_t st, int *resident_tiles) {
   const int n = (a.row_bytes + VB - 1) / VB;
   auto go = [&](auto kernel, int g, int ctas) {
@@ -493,7 +505,7 @@ bool launch_width(const WalkArgs &a, bool share, cudaStream_t st, int *resident_
   constexpr int kMost = VALMODE == 2 ? 6 : 8;  // a value per edge and vector: more registers
 #define CXG_WALK(G, NV, U, CTAS) \
   if (n <= G * NV)               \
-  return go(spmm_walk<T, VB, G, NV, U, VALMODE, (CTAS < kMost ? CTAS : kMost)>, G, CTAS < kMost ? CTAS : kMost)
+  return go(spmm_walk<T, VB, G, NV, U, VALMODE, (CTAS < kMost ? CTAS : kMost), COPY>, G, CTAS < kMost ? CTAS : kMost)
   if constexpr (VB == 16) {
     CXG_WALK(8, 1, 8, 8);
     CXG_WALK(16, 1, 8, 8);
@@ -529,6 +541,15 @@ bool launch(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *re
   if (valmode == 3) return launch_width<T, VB, 3>(a, share, st, resident_tiles);
   if (valmode == 4) return launch_width<T, VB, 4>(a, share, st, resident_tiles);
   return launch_width<T, VB, 2>(a, share, st, resident_tiles);
+}
+
+// Rows copied to whole 16-byte vectors: sums, means and sums weighted by one value per edge.
+template <typename T>
+bool launch_copy(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles) {
+  if (valmode == 0) return launch_width<T, 16, 0, true>(a, share, st, resident_tiles);
+  if (valmode == 1) return launch_width<T, 16, 1, true>(a, share, st, resident_tiles);
+  if (valmode == 3) return launch_width<T, 16, 3, true>(a, share, st, resident_tiles);
+  return false;
 }
 
 }  // namespace walk

@@ -209,6 +209,18 @@ int cxg_spmm_csr(const cxg_spmm_desc *desc, void *workspace,
                  size_t workspace_bytes, void *stream);
 
 /*
+ * The same with scratch for the rows of x. Rows that are not whole 16-byte vectors (47 fp32 values, an odd number of bf16
+ * values) cost a load per value or two when they are gathered; where a graph reads them several times the call first copies
+ * them, widened to whole 32-byte sectors, into `rows` and gathers from there. Sums are those of cxg_spmm_csr for the same
+ * tile size, bit for bit. n_src: rows of x (all that idx names, times the relations with edge_rel).
+ * cxg_spmm_csr_rows_size: bytes of that copy, 0 where the call reads x as it is. `rows` is 32-byte aligned; NULL is
+ * cxg_spmm_csr.
+ */
+int cxg_spmm_csr_rows_size(const cxg_spmm_desc *desc, int64_t n_src, size_t *bytes);
+int cxg_spmm_csr_rows(const cxg_spmm_desc *desc, int64_t n_src, void *rows, size_t rows_bytes, void *workspace,
+                      size_t workspace_bytes, void *stream);
+
+/*
  * CSR SpMM backward for the aggregation `desc` describes (desc->y is unused,
  * desc->x is the forward input and only needed for dval):
  *   dx[s(e),h,:]  += v[e,h] * dy[t(r),h,:]     (divided by the row's edge count for mean)
