@@ -5,7 +5,7 @@
 // (cxgnncomp/graph_conv.py:458-496: two score reductions, edge_softmax_fwd with its mask,
 // src/cpp/src/edge_softmax.cu:3-42, then gen_fwd_sum_edge_value_multi_head,
 // src/cpp/src/aggr_kernel.cu:155-186; backward: aggr_kernel.cu:443-491 and edge_softmax.cu:44-95).
-// Here per-edge values never reach memory:
+// Here no per-edge value crosses a call:
 //
 //   forward   y[r,h,:] = sum_e p[e,h] x[s(e),h,:],  p = softmax over the edges of row r of
 //             t[e,h] = leaky(a_dst[r,h] + a_src[s(e),h]).  The walk is the register-staged tiled one
@@ -14,6 +14,9 @@
 //             sum s and rescales the fp32 accumulator when the maximum grows (online softmax):
 //                 m' = max(m, t);  acc = acc * exp(m - m') + exp(t - m') * x;  s likewise.
 //             Outputs y, row_max = m and row_sum = s per (row, head): [N, H] each instead of [E, H].
+//             Larger ones first turn the scores of a tile's edges into weights ([nnz, H] in the workspace, a tile in shared
+//             memory at a time) and then run the SpMM's weighted walk over the same tiles: a lane that holds four columns
+//             of a head then loads its weight instead of computing two exponentials per edge (gat_weights).
 //             A row that crosses tile borders leaves (acc, m, s) partials per tile; a second kernel
 //             merges them in tile order with the same rescaling. No atomics: results are the same on
 //             every run.
@@ -34,9 +37,8 @@
 // the separate kernels (cxg_gat_scores, cxg_edge_softmax_forward, cxg_spmm_csr).
 //
 // What bounds it: instructions per edge and per row end, with an IPC of 0.55 to 0.65 per scheduler; the gather stays in L2
-// for graphs of this kind. 2.33 M edges, 4 heads x 32: forward 203 -> 178 us and its fix-up 52 -> 17, backward 407 -> 288
-// us and 42 -> 17 (before: rows and scores staged in shared memory, a whole warp per edge). 4 heads x 47 ran on the edge
-// softmax and the weighted aggregation before (0.79 ms; now 0.52).
+// for graphs of this kind. 2.33 M edges, 4 heads x 32: backward 288 us, forward in one step 178 (46 instructions per edge),
+// in two 34 + 104, of which the walk is bound by L2 like the sum over such rows (90).
 #include "spmm_walk_impl.cuh"
 
 namespace cxg {
@@ -65,6 +67,7 @@ struct GatArgs {
   float *d_edge;         // backward, ordered mode: [nnz, H] score gradient of every edge at its forward position
   int heads, c;
   float slope;
+  float *weights;        // forward by way of weights: [nnz, H]
   float *part_ms;        // [tile][2][heads][2]: forward (m, s); backward (unused, d a_src partial)
   float *block_ms;       // [tile][heads][2]: those of a block of a long chain
 };
@@ -800,6 +803,160 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_wide_backward(const __grid
   }
 }
 
+// Forward in two steps: the weights of a tile's edges, then the weighted walk of the SpMM over the same tiles. A warp per tile:
+// a lane per edge fetches the scores of its source into shared memory, a lane per (row, head) turns those of its row into
+// weights (rows of more than kKeep edges: the whole warp), and the tile's weights leave in one piece. Rows inside the
+// tile get their final weights; a piece of a row that crosses tile borders has weights relative to its own maximum and
+// leaves (m, s) for gat_fix, as the walks above do.
+constexpr int kKeep = 8;  // values of a row that a lane keeps in registers
+
+template <int H>
+__global__ void __launch_bounds__(kThreads, 8) gat_weights(const __grid_constant__ GatArgs a) {
+  extern __shared__ float score_stage[];
+  constexpr int R = 32 / H;  // rows that are looked at together
+  constexpr int HV = H < 4 ? H : 4;
+  const int lane = threadIdx.x & 31, h = lane & (H - 1);
+  float *p = score_stage + (threadIdx.x >> 5) * a.w.tile * H;
+  dependency_wait();
+  const uint32_t e_total = static_cast<uint32_t>(edge_total(a.w));
+  const int n_tiles = static_cast<int>((e_total + static_cast<int64_t>(a.w.tile) - 1) / a.w.tile);
+  const int n_rows = static_cast<int>(a.w.n_dst);
+  const int warps = static_cast<int>(gridDim.x * (blockDim.x >> 5)), first = static_cast<int>(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  auto end_of = [&](int r) {
+    return __ldg(reinterpret_cast<const uint32_t *>(static_cast<const uint8_t *>(a.w.ptr) + static_cast<uint64_t>(static_cast<uint32_t>(min(r, n_rows))) * static_cast<uint32_t>(a.w.ptr_bytes)));
+  };
+  auto put = [&](int r, float m, float s) {
+    a.row_max[static_cast<int64_t>(r) * H + h] = m;
+    a.row_sum[static_cast<int64_t>(r) * H + h] = s;
+  };
+  if (e_total == 0) {
+    for (int r = first * R + lane / H; r < n_rows; r += warps * R) put(r, kNegBig, 0.f);
+    return;
+  }
+  for (int t = first; t < n_tiles; t += warps) {
+    const WalkTile here = load_tile(a.w, t);
+    const uint32_t begin = here.begin;
+    const int len = static_cast<int>(load_tile(a.w, t + 1).begin - begin);
+    if (t == 0)
+      for (int r = lane / H; r < static_cast<int>(here.row); r += R) put(r, kNegBig, 0.f);
+    int r = static_cast<int>(here.row) + lane / H;
+    uint32_t raw_b = end_of(r), raw_e = end_of(r + 1);
+    float add = __ldg(a.r_small + static_cast<int64_t>(min(r, n_rows - 1)) * H + h);
+    for (int e0 = lane; e0 < len; e0 += 128) {
+      uint32_t id[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        id[u] = e0 + u * 32 < len ? walk::load_id_low(static_cast<const uint8_t *>(a.w.idx) + static_cast<uint64_t>(begin + e0 + u * 32) * static_cast<uint32_t>(a.w.idx_bytes)) : 0u;
+#pragma unroll
+      for (int i = 0; i < H; i += HV) {
+        float v[4][HV];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          load_floats<HV * 4>(v[u], a.g_small + static_cast<uint64_t>(id[u]) * H + i);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (e0 + u * 32 < len) {
+#pragma unroll
+            for (int k = 0; k < HV; ++k) p[(e0 + u * 32) * H + i + k] = v[u][k];
+          }
+      }
+    }
+    __syncwarp();
+    for (;;) {
+      // of the rows behind these
+      const uint32_t next_b = end_of(r + R), next_e = end_of(r + R + 1);
+      const float next_add = __ldg(a.r_small + static_cast<int64_t>(min(r + R, n_rows - 1)) * H + h);
+      const int b = static_cast<int>(raw_b - begin), e = static_cast<int>(raw_e - begin);
+      const bool mine = r < n_rows && (b < len || (b == len && e == len));  // rows without edges belong to the tile in front
+      const int lo = max(b, 0), hi = min(e, len), n = mine ? hi - lo : 0;
+      const bool whole = b >= 0 && e <= len;
+      float m = kNegBig, s = 0.f;
+      // `cnt` values of a row, `step` apart; KEEP of them are held in registers
+      auto weigh = [&](float *q, int cnt, int step, float plus, bool final, auto &&join_max, auto &&join_sum, float &top, float &sum) {
+        float t[kKeep];
+        top = kNegBig, sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i) {
+          t[i] = kNegBig;
+          if (i < cnt) {
+            const float z = plus + q[i * step];
+            t[i] = z > 0.f ? z : z * a.slope;
+          }
+          top = fmaxf(top, t[i]);
+        }
+        top = join_max(top);
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i) {
+          t[i] = exp_flush(t[i] - top);
+          if (i < cnt) sum += t[i];
+        }
+        sum = join_sum(sum);
+        const float inv = final ? 1.f / sum : 1.f;
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i)
+          if (i < cnt) q[i * step] = t[i] * inv;
+      };
+      if (n > 0 && n <= kKeep)
+        weigh(p + lo * H + h, n, H, add, whole, [](float v) { return v; }, [](float v) { return v; }, m, s);
+      for (unsigned left = __ballot_sync(0xffffffffu, n > kKeep && h == 0); left != 0; left &= left - 1) {
+        const int src = __ffs(left) - 1;
+        const int jlo = __shfl_sync(0xffffffffu, lo, src), jn = __shfl_sync(0xffffffffu, n, src);
+        const bool jwhole = __shfl_sync(0xffffffffu, whole, src);
+        const float jadd = __shfl_sync(0xffffffffu, add, src + h);
+        float *q = p + (jlo + lane / H) * H + h;
+        const int cnt = (jn - lane / H + R - 1) / R;  // of this lane: every R-th edge
+        auto over_max = [](float v) {
+#pragma unroll
+          for (int o = H; o < 32; o <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+          return v;
+        };
+        auto over_sum = [](float v) {
+#pragma unroll
+          for (int o = H; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          return v;
+        };
+        float jm = kNegBig, js = 0.f;
+        if (jn <= kKeep * R) {
+          weigh(q, cnt, 32, jadd, jwhole, over_max, over_sum, jm, js);
+        } else {
+#pragma unroll 4
+          for (int i = 0; i < cnt; ++i) {
+            const float z = jadd + q[i * 32];
+            jm = fmaxf(jm, z > 0.f ? z : z * a.slope);
+          }
+          jm = over_max(jm);
+#pragma unroll 4
+          for (int i = 0; i < cnt; ++i) {
+            const float z = jadd + q[i * 32];
+            const float pr = exp_flush((z > 0.f ? z : z * a.slope) - jm);
+            q[i * 32] = pr;
+            js += pr;
+          }
+          js = over_sum(js);
+          if (jwhole) {
+            const float inv = 1.f / js;
+            for (int i = 0; i < cnt; ++i) q[i * 32] *= inv;
+          }
+        }
+        if ((lane & ~(H - 1)) == src) m = jm, s = js;
+      }
+      if (mine) {
+        if (whole)
+          put(r, m, s);
+        else
+          *reinterpret_cast<float2 *>(a.part_ms + ((static_cast<int64_t>(t) * 2 + (b < 0 ? 0 : 1)) * H + h) * 2) = make_float2(m, s);
+      }
+      if (__any_sync(0xffffffffu, !mine)) break;
+      r += R;
+      raw_b = next_b, raw_e = next_e, add = next_add;
+    }
+    __syncwarp();
+    float *out = a.weights + static_cast<int64_t>(begin) * H;
+    for (int i = lane; i < len * H; i += 32) out[i] = p[i];
+    __syncwarp();
+  }
+}
+
 constexpr int kGatSeq = 16;  // a chain of more partials is joined in blocks of this many, then the blocks: the hub row of
                              // 2.3 M edges (420 partials) costs 2 + 4 round trips instead of 8 + 1 with blocks of 64
 
@@ -898,7 +1055,14 @@ __global__ void __launch_bounds__(256, 3) gat_fix(const __grid_constant__ GatArg
   int64_t row = 0;
   int ts = 0, k = 0, m = 0;
   if (lane < 2 * per && t < w.max_tiles && t * w.tile < e_total) {
-    const WideTile here = static_cast<const WideTile *>(w.tiles)[t], next = static_cast<const WideTile *>(w.tiles)[t + 1];  // not written behind the last tile, whose end is e_total
+    // not written behind the last tile, whose end is e_total
+    WideTile here, next;
+    if (w.wide_tiles) {
+      here = static_cast<const WideTile *>(w.tiles)[t], next = static_cast<const WideTile *>(w.tiles)[t + 1];
+    } else {
+      const WalkTile h = load_tile(w, t), n = load_tile(w, t + 1);
+      here = WideTile{h.row, h.begin}, next = WideTile{n.row, n.begin};
+    }
     const bool tail = lane < per;
     row = tail ? next.row : here.row;
     if (next.begin > here.begin && row < w.n_dst) {
@@ -1116,7 +1280,7 @@ int gat_layout(int64_t n_stats_rows, int64_t nnz, int heads, int c, GatLayout *L
   L->piece_sums = off;
   off = align_up(off + static_cast<size_t>(nnz / kPieceEdges + 1) * 2 * heads * sizeof(float), 256);
   L->d_edge = off;
-  off = align_up(off + static_cast<size_t>(nnz) * heads * sizeof(float), 256);
+  off = align_up(off + static_cast<size_t>(nnz) * heads * sizeof(float) + kWalkSlack, 256);
   L->total = off;
   return CXG_OK;
 }
@@ -1161,6 +1325,41 @@ void fill_args(GatArgs &a, const GatLayout &L, void *workspace, int64_t nnz, int
 
 // Lane layouts by bytes per vector and vectors per row; the last number is the resident CTAs per SM that the registers of
 // that many edges in flight allow.
+// Whether the forward goes by way of weights. Its second step is the SpMM's walk, which counts in 32 bits. It has a launch more
+// than the single walk, which keeps rows of up to 32 16-byte vectors of small graphs (430,000 edges: 4 heads of 8 38 us in one
+// step, 42 in two; 8 of 8 41 / 47; 4 of 32 51 / 47; 2.3 M edges: 99 / 98, 150 / 128, 198 / 157). Wider rows and other vectors
+// gain everywhere: 27,000 edges 4 of 64 44 / 36, 2 of 33 47 / 35; 2.3 M 4 of 64 391 / 246, 1 of 47 301 / 115, 2 of 50 323 / 249.
+bool by_weights(const GatArgs &a, int vb) {
+  const bool one_step = vb == 16 && a.w.width <= 128 && a.w.nnz * a.w.row_bytes < (128 << 20);
+  return !one_step && a.heads <= 8 && reinterpret_cast<uintptr_t>(a.g_small) % 16 == 0 && a.w.n_dst < INT32_MAX - (1 << 20) &&
+         a.w.nnz < INT32_MAX - (1 << 20) && a.w.width * 4 <= (vb == 16 ? 128 * 16 : 256 * vb);
+}
+
+cudaError_t launch_by_weights(GatArgs &a, int vb, cudaStream_t st) {
+  int resident = 0;
+  a.w.wide_tiles = 0;
+  a.w.edge_val = a.weights;
+  a.w.part_stride = a.w.width;
+  if (!walk_weighted(a.w, vb, st, &resident)) return cudaErrorInvalidValue;
+  const int tile = walk_whole_waves(a.w.nnz, resident, 8);
+  a.w.tile = tile < 256 ? tile : 256;
+  a.w.max_tiles = (a.w.nnz + a.w.tile - 1) / a.w.tile + 1;
+  walk_plan_run(a.w, st);
+  constexpr int warps = kThreads / 32;
+  int64_t grid = (a.w.max_tiles + warps - 1) / warps;  // a tile per warp while that many blocks are worth launching
+  if (grid > kNumSM * 64) grid = kNumSM * 64;
+  cudaError_t err = cudaErrorInvalidValue;
+  auto go = [&](auto kernel) {
+    err = launch_dependent(kernel, static_cast<unsigned>(grid), 32 * warps, static_cast<size_t>(warps) * a.w.tile * a.heads * sizeof(float), st, a);
+  };
+  if (a.heads == 1) go(gat_weights<1>);
+  if (a.heads == 2) go(gat_weights<2>);
+  if (a.heads == 4) go(gat_weights<4>);
+  if (a.heads == 8) go(gat_weights<8>);
+  if (err != cudaSuccess) return err;
+  return walk_weighted(a.w, vb, st, nullptr) ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 template <bool BWD>
 cudaError_t launch_walk(GatArgs &a, cudaStream_t st) {
   const int vb = vector_of(a.heads, a.c), n = a.w.row_bytes / vb;
@@ -1199,6 +1398,7 @@ cudaError_t launch_walk(GatArgs &a, cudaStream_t st) {
     // 8-byte ones from 16 values per head on (4 of 30: 357, now 327; 8 of 10 would take 376 instead of 344).
     const bool across = vb < 16 && (vb == 4 || a.c >= 16) && a.w.width % 4 == 0 && a.w.width > 64 && a.c >= 4 &&
                         (reinterpret_cast<uintptr_t>(a.w.x) | reinterpret_cast<uintptr_t>(a.w.y)) % 16 == 0;
+    if (!across && by_weights(a, vb)) err = launch_by_weights(a, vb, st); else
 #define CXG_GAT_ACROSS(NV, U, P, CTAS) \
   if (across && a.w.width <= 128 * NV && U * a.heads <= 32 * P) go(gat_wide_forward<16, NV, U, P, CTAS, true>, 32, CTAS); else
     CXG_GAT_ACROSS(1, 8, 1, 6)
@@ -1287,6 +1487,7 @@ extern "C" int cxg_gat_fused_forward(const void *ptr, const void *idx, int ptr_b
   a.w.x = x, a.g_small = a_src, a.r_small = a_dst;
   a.w.y = y, a.row_max = row_max, a.row_sum = row_sum;
   a.w.n_dst = n_dst;
+  a.weights = reinterpret_cast<float *>(static_cast<char *>(workspace) + L.d_edge);
   cudaError_t e = launch_walk<false>(a, as_stream(stream));
   if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_gat_fused_forward: %s", cudaGetErrorString(e));
   return check_launch("cxg_gat_fused_forward");

@@ -366,8 +366,7 @@ int walk_whole_waves(int64_t nnz, int64_t resident, int round) {
   return t < 64 ? 64 : static_cast<int>((t + round - 1) / round * round);
 }
 
-namespace {
-int tile_of_waves(int64_t nnz, int64_t resident) {
+int walk_tile_of_waves(int64_t nnz, int64_t resident) {
   // One wave of tiles of up to 256 edges where that is enough (2.3 M edges, F = 64: 71 us, two waves of 128 edges 78), behind
   // that whole waves of up to 128, which even out what the groups get through (1.2 M edges, F = 201 bf16: 270 us with two
   // waves of 136, 250 with three of 88; 12.6 M, F = 47: 296 with six of 224, 290 with eleven of 128). From four waves of 512
@@ -379,7 +378,13 @@ int tile_of_waves(int64_t nnz, int64_t resident) {
   const int64_t t = waves > 0 ? (nnz + waves * resident - 1) / (waves * resident) : 0;
   return t < 64 ? 64 : static_cast<int>((t + 7) / 8 * 8);
 }
-}  // namespace
+
+bool walk_weighted(const WalkArgs &a, int vb, cudaStream_t st, int *resident_tiles) {
+  const int valmode = a.heads == 1 ? 1 : vb != 16 || a.heads > 8 ? 2 : a.heads == 2 ? 5 : a.heads == 4 ? 6 : 7;
+  return vb == 16  ? walk_launch_f32_16(a, valmode, false, st, resident_tiles)
+         : vb == 8 ? walk_launch_f32_8(a, valmode, false, st, resident_tiles)
+                   : walk_launch_f32_4(a, valmode, false, st, resident_tiles);
+}
 
 int walk_tile_edges(const cxg_spmm_desc *d, bool copied) {
   if (d->split_edges > 0) return d->split_edges;
@@ -387,7 +392,7 @@ int walk_tile_edges(const cxg_spmm_desc *d, bool copied) {
   a.row_bytes = d->feat * d->heads * (d->dtype == CXG_F32 ? 4 : 2);
   int resident = kNumSM * 32;
   dispatch(d, a, copied, nullptr, &resident);
-  return tile_of_waves(d->nnz, resident);
+  return walk_tile_of_waves(d->nnz, resident);
 }
 
 int walk_static_tile_edges(const cxg_spmm_desc *d) {

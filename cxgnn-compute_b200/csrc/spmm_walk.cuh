@@ -64,6 +64,12 @@ constexpr int64_t walk_part_stride(int64_t width) { return (width + 3) / 4 * 4; 
 bool walk_eligible(const cxg_spmm_desc *d);
 // The plan kernel for a.ptr, a.tile, a.whole_rows: fills hdr, tiles, count (and sets a.tile_magic).
 void walk_plan_run(WalkArgs &a, cudaStream_t st);
+// The walk alone over the plan and the weights per (edge, head) in `a` (fp32 rows in vectors of vb bytes, heads a power of two),
+// behind which kWalkSlack bytes can be read. With resident_tiles set it only tells how many tiles are walked at the same time.
+constexpr size_t kWalkSlack = 256;  // 8 edges of 8 heads
+bool walk_weighted(const WalkArgs &a, int vb, cudaStream_t st, int *resident_tiles);
+// Edges per tile for that many.
+int walk_tile_of_waves(int64_t nnz, int64_t resident);
 // Edges per tile when `resident` tiles are walked at the same time: whole waves of up to 256 edges, or 512.
 int walk_whole_waves(int64_t nnz, int64_t resident, int round);
 // Edges per tile of cxg_spmm_csr_static, whose scratch has a fixed size: these decide which graphs it takes.

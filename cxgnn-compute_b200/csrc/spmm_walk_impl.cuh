@@ -229,7 +229,7 @@ __device__ __forceinline__ void add_words(float *f, const Words<(VB + 3) / 4> &r
 
 // VB: bytes per load of a lane; NV loads per row, G lanes per tile, U edges in flight per lane. VALMODE: 0 no
 // edge values, 1 one per edge, 2 one per (edge, head), 3 none and the mean of the row, 4 none and the sum (or the mean) is
-// added to the output.
+// added to the output, 5 to 7 as 2 with 2, 4 or 8 heads and values that may be read U edges beyond the last one.
 // COPY: the rows of x are copies in whole vectors (walk_plan), those of y are not: a lane stores the values of its vector
 // that lie inside the row one by one.
 template <typename T, int VB, int G, int NV, int U, int VALMODE, int MINB, bool COPY>
@@ -255,10 +255,12 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
   for (int q = 0; q < NV; ++q)
     xq[q] = static_cast<const uint8_t *>(a.x) + (on(q) ? (lg + q * G) * VB : (rb - 1) / VB * VB);
   auto row_of_y = [&](int r) { return static_cast<uint8_t *>(a.y) + static_cast<uint64_t>(r) * static_cast<uint32_t>(rb) + lg * VB; };
+  constexpr int kHeads = VALMODE >= 5 ? 1 << (VALMODE - 4) : 0;
+  constexpr bool kPerHead = VALMODE == 2 || kHeads > 0;
   int head[NV];
-  if (VALMODE == 2) {
+  if (kPerHead) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) head[q] = on(q) ? ((lg + q * G) * VB / static_cast<int>(sizeof(T))) / a.feat : 0;
+    for (int q = 0; q < NV; ++q) head[q] = on(q) ? ((lg + q * G) * EL) / a.feat : 0;
   }
 
   auto store = [&](uint8_t *dst, float (&f)[NV][EL]) {
@@ -440,18 +442,22 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
       constexpr int W4 = U < 4 ? U : 4;
       uint32_t ids[W4];
       float vals[W4];
-      float ev[VALMODE == 2 ? U : 1][VALMODE == 2 ? NV : 1];
+      float ev[kPerHead ? U : 1][kPerHead ? NV : 1];
+      const float *weights = kPerHead ? a.edge_val + static_cast<uint64_t>(begin + p) * static_cast<uint32_t>(kHeads > 0 ? kHeads : a.heads) : nullptr;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (u % W4 == 0) load_ids(ids, my_ids + in_batch + u);
         const uint64_t off = static_cast<uint64_t>(ids[u % W4]) * pitch;
 #pragma unroll
         for (int q = 0; q < NV; ++q) load_row_bytes<VB>(v[u][q], xq[q] + off);
-        if constexpr (VALMODE == 2) {
-          const int pos = min(p + u, len - 1);
+        if constexpr (kPerHead) {
 #pragma unroll
-          for (int q = 0; q < NV; ++q)
-            ev[u][q] = len > 0 ? __ldg(a.edge_val + (static_cast<int64_t>(begin) + pos) * a.heads + head[q]) : 0.f;
+          for (int q = 0; q < NV; ++q) {
+            if constexpr (kHeads > 0)
+              ev[u][q] = __ldg(weights + head[q] + u * kHeads);
+            else
+              ev[u][q] = p + u < len ? __ldg(weights + u * a.heads + head[q]) : 0.f;
+          }
         }
       }
       // adds them; groups that have passed the end of their tile add into accumulators that nobody reads
@@ -459,7 +465,7 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
         if (VALMODE == 1 && u % W4 == 0) load_ids(vals, my_vals + in_batch + u);
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
-          if constexpr (VALMODE == 0 || VALMODE >= 3)
+          if constexpr (VALMODE == 0 || VALMODE == 3 || VALMODE == 4)
             acc[q].add(v[u][q]);
           else if constexpr (VALMODE == 1)
             acc[q].fma(v[u][q], vals[u % W4]);
@@ -502,10 +508,9 @@ bool launch_width(const WalkArgs &a, bool share, cudaStream_t st, int *resident_
     if (grid > resident) grid = resident;
     return launch_dependent(kernel, static_cast<unsigned>(grid < 1 ? 1 : grid), kThreads, 0, st, a) == cudaSuccess;
   };
-  constexpr int kMost = VALMODE == 2 ? 6 : 8;  // a value per edge and vector: more registers
 #define CXG_WALK(G, NV, U, CTAS) \
   if (n <= G * NV)               \
-  return go(spmm_walk<T, VB, G, NV, U, VALMODE, (CTAS < kMost ? CTAS : kMost), COPY>, G, CTAS < kMost ? CTAS : kMost)
+  return go(spmm_walk<T, VB, G, NV, U, VALMODE, CTAS, COPY>, G, CTAS)
   if constexpr (VB == 16) {
     CXG_WALK(8, 1, 8, 8);
     CXG_WALK(16, 1, 8, 8);
@@ -540,6 +545,11 @@ bool launch(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *re
   if (valmode == 1) return launch_width<T, VB, 1>(a, share, st, resident_tiles);
   if (valmode == 3) return launch_width<T, VB, 3>(a, share, st, resident_tiles);
   if (valmode == 4) return launch_width<T, VB, 4>(a, share, st, resident_tiles);
+  if constexpr (sizeof(T) == 4 && VB == 16) {
+    if (valmode == 5) return launch_width<T, VB, 5>(a, share, st, resident_tiles);
+    if (valmode == 6) return launch_width<T, VB, 6>(a, share, st, resident_tiles);
+    if (valmode == 7) return launch_width<T, VB, 7>(a, share, st, resident_tiles);
+  }
   return launch_width<T, VB, 2>(a, share, st, resident_tiles);
 }
 

@@ -286,8 +286,8 @@ int cxg_edge_softmax_backward(const void *ptr, const void *idx, int ptr_bytes,
                               void *workspace, size_t workspace_bytes, void *stream);
 
 /*
- * Fused GAT aggregation: score, LeakyReLU, edge softmax and weighted neighbour sum in one walk over the edges,
- * without any [nnz, heads] array in memory. Replaces, for one layer, the sequence edge_attention ->
+ * Fused GAT aggregation: score, LeakyReLU, edge softmax and weighted neighbour sum in one walk over the edges, or
+ * (larger graphs, wide rows) in two, with the weights [nnz, heads] in the workspace in between. Replaces, for one layer, the sequence edge_attention ->
  * sage_sum_forward_edge_value / SpMMValOP of MyGATConv.forward_many (cxgnncomp/graph_conv.py:458-496,
  * src/cpp/src/edge_softmax.cu:3-95, src/cpp/src/aggr_kernel.cu:155-186,443-491).
  *   forward:  y[r,h,:] = sum_e p[e,h] x[idx[e],h,:],  p = softmax over row r of leaky(a_dst[r,h] + a_src[idx[e],h]);
