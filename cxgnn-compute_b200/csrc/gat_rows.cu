@@ -165,6 +165,50 @@ __global__ void __launch_bounds__(kRowThreads, 6) head_mean_bias(const float *x,
   }
 }
 
+// Weights [heads * c, k] and attention vectors [heads, c] with the heads padded to cp columns of zeros, so that every head of
+// the transformed features starts on a 16-byte boundary.
+__global__ void __launch_bounds__(kRowThreads) pad_heads(const float *w, const float *att_src, const float *att_dst, float *wp,
+                                                         float *src_p, float *dst_p, int heads, int c, int cp, int k) {
+  const int i = blockIdx.x * kRowThreads + threadIdx.x, rows = heads * cp;
+  if (i >= rows * (k + 2)) return;
+  const int row = i < rows * k ? i / k : (i - rows * k) % rows, at = row % cp, from = row / cp * c + at;
+  if (i < rows * k)
+    wp[i] = at < c ? w[static_cast<int64_t>(from) * k + (i - row * k)] : 0.f;
+  else if (i < rows * (k + 1))
+    src_p[row] = at < c ? att_src[from] : 0.f;
+  else
+    dst_p[row] = at < c ? att_dst[from] : 0.f;
+}
+
+// Rows of padded heads to the layer's output: the heads' mean [n, c], or the heads side by side [n, heads * c], plus the bias.
+// A thread takes a vector of one column group: all its heads' loads are in flight.
+template <bool JOIN>
+__global__ void __launch_bounds__(kRowThreads) unpad_heads(const float *x, const float *bias, float *out, int64_t n, int heads, int c,
+                                                           int cp) {
+  const int vecs = cp / 4, per_row = JOIN ? heads * vecs : vecs;
+  const int64_t total = n * per_row, step = static_cast<int64_t>(gridDim.x) * kRowThreads;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(kRowThreads) + threadIdx.x; i < total; i += step) {
+    const int64_t row = total < (1ll << 31) ? static_cast<int>(i) / per_row : i / per_row;
+    const int rest = static_cast<int>(i - row * per_row), h = JOIN ? rest / vecs : 0, col = (rest - h * vecs) * 4;
+    float s[4];
+    load_v<4>(s, x + (row * heads + h) * cp + col);
+    if (!JOIN) {
+#pragma unroll 4
+      for (int j = 1; j < heads; ++j) {
+        float v[4];
+        load_v<4>(v, x + (row * heads + j) * cp + col);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s[q] += v[q];
+      }
+    }
+    float *o = out + (JOIN ? (row * heads + h) * c : row * c) + col;
+    const float *b = bias != nullptr ? bias + (JOIN ? h * c : 0) + col : nullptr;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (col + q < c) o[q] = (JOIN || heads == 1 ? s[q] : s[q] * (1.f / heads)) + (b != nullptr ? b[q] : 0.f);
+  }
+}
+
 bool vectors(int c, const void *a, const void *b, const void *d) {
   return c % 4 == 0 &&
          ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(d)) % 16) == 0;
@@ -224,4 +268,29 @@ extern "C" int cxg_head_mean_bias(const float *x, const float *bias, float *out,
     head_mean_bias<1, int64_t><<<grid, kRowThreads, 0, st>>>(x, bias, out, n, heads, c);
   count_launches(1);
   return check_launch("cxg_head_mean_bias");
+}
+
+extern "C" int cxg_gat_pad_heads(const float *w, const float *att_src, const float *att_dst, float *w_padded, float *att_src_padded,
+                                 float *att_dst_padded, int heads, int c, int c_padded, int k, void *stream) {
+  CXG_REQUIRE(heads > 0 && c > 0 && c_padded >= c && k > 0 && static_cast<int64_t>(heads) * c_padded * (k + 2) < (1ll << 30),
+              CXG_EINVAL, "cxg_gat_pad_heads: bad sizes");
+  CXG_REQUIRE(w && att_src && att_dst && w_padded && att_src_padded && att_dst_padded, CXG_ENULL, "cxg_gat_pad_heads: NULL argument");
+  const int total = heads * c_padded * (k + 2);
+  pad_heads<<<(total + kRowThreads - 1) / kRowThreads, kRowThreads, 0, as_stream(stream)>>>(
+      w, att_src, att_dst, w_padded, att_src_padded, att_dst_padded, heads, c, c_padded, k);
+  count_launches(1);
+  return check_launch("cxg_gat_pad_heads");
+}
+
+extern "C" int cxg_gat_unpad_heads(const float *x, const float *bias, float *out, int64_t n, int heads, int c, int c_padded, int join,
+                                   void *stream) {
+  CXG_REQUIRE(n >= 0 && heads > 0 && c > 0 && c_padded >= c && c_padded % 4 == 0, CXG_EINVAL, "cxg_gat_unpad_heads: bad sizes");
+  if (n == 0) return CXG_OK;
+  CXG_REQUIRE(x && out, CXG_ENULL, "cxg_gat_unpad_heads: NULL argument");
+  CXG_REQUIRE(reinterpret_cast<uintptr_t>(x) % 16 == 0, CXG_EINVAL, "cxg_gat_unpad_heads: x must be 16-byte aligned");
+  const int64_t blocks = (n * (join ? heads : 1) * (c_padded / 4) + kRowThreads - 1) / kRowThreads;
+  const unsigned grid = static_cast<unsigned>(blocks < kNumSM * 64 ? blocks : kNumSM * 64);
+  (join ? unpad_heads<true> : unpad_heads<false>)<<<grid, kRowThreads, 0, as_stream(stream)>>>(x, bias, out, n, heads, c, c_padded);
+  count_launches(1);
+  return check_launch("cxg_gat_unpad_heads");
 }

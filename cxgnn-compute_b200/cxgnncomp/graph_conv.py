@@ -476,6 +476,12 @@ class MyGATConv(torch.nn.Module):
         assert x.dim() == 2
         if x.shape[0] != num_src:  # (the gradient of a slice is a copy into zeros)
             x = x[:num_src]
+        if (not self.tensor_core_linear and self.fused_scores and self.fused_aggregate and C % 4 != 0
+                and self.edge_softmax_schedule == "fused" and num_dst > 0):
+            out = cxgnncomp_backend.gat_layer_padded(x, self.lin_src, self.att_src, self.att_dst, self.bias, ptr, idx, num_dst, H,
+                                                     self.negative_slope, self.concat)
+            if out is not None:
+                return out
         if self.tensor_core_linear:
             x_src = cxgnncomp_backend.dense_linear(x, self.lin_src).view(-1, H, C)
         else:

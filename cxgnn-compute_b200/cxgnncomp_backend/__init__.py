@@ -1104,6 +1104,13 @@ def gat_layer(x_src, att_src, att_dst, bias, ptr, idx, num_dst, negative_slope, 
     return _native.gat_layer(x_src, att_src, att_dst, bias, ptr, idx, int(num_dst), float(negative_slope), bool(concat))
 
 
+def gat_layer_padded(x, weight, att_src, att_dst, bias, ptr, idx, num_dst, heads, negative_slope, concat):
+    """The same from the layer's input, x [n_src, K] and weight [H * C, K], where C is not a multiple of 4 and no gradient is
+    recorded; None where it does not cover the arguments (see gat_layer then)."""
+    return _native.gat_layer_padded(x, weight, att_src, att_dst, bias, ptr, idx, int(num_dst), int(heads), float(negative_slope),
+                                    bool(concat))
+
+
 def edge_value_degree(ptr, num_dst, num_edge):
     """val[e] = 1 / in-degree of e's destination (binding.cpp:24-25)."""
     _cuda(ptr, "ptr", _INDEX_DTYPES)

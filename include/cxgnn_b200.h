@@ -391,6 +391,13 @@ int cxg_gat_scores_backward_add(const float *feat, const float *g_src, const flo
                                 size_t workspace_bytes, void *stream);
 
 /* out[n, :] = mean over heads of x[n, h, :] (+ bias, which may be NULL), fp32, x [n, heads, c] (cxgnncomp/graph_conv.py:487-494). */
+/* Heads padded to c_padded columns (a multiple of 4), for layers whose heads are not whole 16-byte vectors (class counts):
+ * weights [heads * c, k] and attention vectors [heads, c] with zeros behind every head, and back from features
+ * [n, heads, c_padded] to the heads' mean [n, c] or (join) the heads side by side [n, heads * c], plus the bias (may be NULL). */
+int cxg_gat_pad_heads(const float *w, const float *att_src, const float *att_dst, float *w_padded, float *att_src_padded,
+                      float *att_dst_padded, int heads, int c, int c_padded, int k, void *stream);
+int cxg_gat_unpad_heads(const float *x, const float *bias, float *out, int64_t n, int heads, int c, int c_padded, int join,
+                        void *stream);
 int cxg_head_mean_bias(const float *x, const float *bias, float *out, int64_t n, int heads, int c, void *stream);
 
 /*
