@@ -56,13 +56,14 @@ __device__ __forceinline__ void copy_vector(const WalkArgs &a, int64_t i) {
 }
 
 // Rows that own the first edge of a tile write the tile's record; a hub row that owns many is shared by its warp. One
-// pass over ptr, so it costs what reading ptr costs (1 us for 170,000 rows, 17 us for 14 M) and the time that its code takes to
+// pass over ptr (behind the kernel in front in the stream, while which it is launched: 2 us), so it costs what reading ptr costs (1 us for 170,000 rows, 17 us for 14 M) and the time that its code takes to
 // arrive, where a search per tile is a chain of 18 dependent loads (10 us). Also clears what the later kernels count in.
 constexpr int kFixThreads = 64;  // of walk_fix
 constexpr int kCopyVectors = 4;  // vectors of the copy per thread
 
 template <int kPlanRows, typename Copy>
 __global__ void __launch_bounds__(256) walk_plan(const __grid_constant__ WalkArgs a) {
+  dependency_wait();
   if constexpr (!std::is_void_v<Copy>) {
     if (blockIdx.x >= a.plan_blocks) {
       const int64_t i0 = static_cast<int64_t>(blockIdx.x - a.plan_blocks) * (256ll * kCopyVectors) + threadIdx.x;
@@ -291,6 +292,24 @@ __global__ void __launch_bounds__(kFixThreads, 12) walk_fix(const __grid_constan
   }
 }
 
+// Bytes that a lane reads of a row: narrow rows take the vector that occupies eight lanes, the fewest a tile is given.
+int walk_vector_bytes(const cxg_spmm_desc *d) {
+  const int64_t row_bytes = static_cast<int64_t>(d->feat) * d->heads * (d->dtype == CXG_F32 ? 4 : 2);
+  int vb = vector_bytes(d);
+  while (vb > 4 && row_bytes <= 4 * vb) vb /= 2;
+  return vb;
+}
+
+// One launch of clusters instead of plan, walk and fix-up. For rows of 512 bytes the two meet at 65,000 edges (17.7 / 18.5 us; 74,000
+// 22.5 / 17.5), narrower ones gain up to 98,000 and beyond; there a graph whose edges all lie in one row, which one cluster
+// then walks alone, takes about as long as three launches do. Its tiles have 64 edges, which is what walk_tile_of_waves gives
+// graphs of this size.
+bool small_graph(const cxg_spmm_desc *d) {
+  const int64_t row_bytes = static_cast<int64_t>(d->feat) * d->heads * (d->dtype == CXG_F32 ? 4 : 2);
+  return d->nnz <= 98304 && d->nnz * row_bytes <= (32 << 20) && d->n_dst <= small_most_rows() && d->edge_rel == nullptr &&
+         !(d->flags & (CXG_SPMM_ACCUMULATE | CXG_SPMM_SHARE_SMS)) && (d->heads == 1 || d->edge_val == nullptr);
+}
+
 bool dispatch(const cxg_spmm_desc *d, const WalkArgs &a, bool copied, cudaStream_t st, int *resident_tiles) {
   const int valmode = d->flags & CXG_SPMM_ACCUMULATE ? 4
                       : d->edge_val == nullptr       ? (d->reduce == CXG_MEAN ? 3 : 0)
@@ -299,9 +318,7 @@ bool dispatch(const cxg_spmm_desc *d, const WalkArgs &a, bool copied, cudaStream
   if (copied)
     return d->dtype == CXG_F32 ? walk_launch_f32_copy(a, valmode, share, st, resident_tiles)
                                : walk_launch_bf16_copy(a, valmode, share, st, resident_tiles);
-  int vb = vector_bytes(d);
-  // narrow rows take the vector that occupies eight lanes, the fewest a tile is given
-  while (vb > 4 && a.row_bytes <= 4 * vb) vb /= 2;
+  const int vb = walk_vector_bytes(d);
   if (d->dtype == CXG_F32)
     return vb == 16  ? walk_launch_f32_16(a, valmode, share, st, resident_tiles)
            : vb == 8 ? walk_launch_f32_8(a, valmode, share, st, resident_tiles)
@@ -350,7 +367,7 @@ void walk_plan_run(WalkArgs &a, cudaStream_t st) {
   const int per_thread = rows <= kNumSM * 2048 ? 1 : 4;
   a.plan_blocks = static_cast<unsigned>((rows + 256 * per_thread - 1) / (256 * per_thread));
   const unsigned grid = a.plan_blocks + static_cast<unsigned>((a.copy_vectors + 256 * kCopyVectors - 1) / (256 * kCopyVectors));
-  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(a); };
+  auto go = [&](auto kernel) { launch_dependent(kernel, grid, 256, 0, st, a); };
   if (a.copy_vectors == 0)
     per_thread == 1 ? go(walk_plan<1, void>) : go(walk_plan<4, void>);
   else if (a.row_bytes == a.width * 4)
@@ -459,6 +476,10 @@ int walk_launch(const cxg_spmm_desc *d, bool whole_rows, int64_t n_src, void *ro
   a.count = reinterpret_cast<int32_t *>(ws + L.count);
   a.partials = reinterpret_cast<float *>(ws + L.partials);
   a.max_tiles = L.max_tiles;
+  if (small_graph(d) && tile == 64 && (d->split_edges == 0 || !whole_rows) && small_launch(a, d->dtype, walk_vector_bytes(d), st)) {
+    count_launches(1);
+    return check_launch("cxg_spmm_csr (small)");
+  }
   walk_plan_run(a, st);
   if (!dispatch(d, a, copied, st, nullptr)) return set_error(CXG_EUNSUPPORTED, "cxg_spmm_csr: rows of %d bytes", a.row_bytes);
   // tiles a warp looks over: one while the chip holds a warp for each, up to sixteen (two roles on 32 lanes)

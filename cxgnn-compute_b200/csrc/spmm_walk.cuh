@@ -82,6 +82,11 @@ int walk_launch(const cxg_spmm_desc *d, bool whole_rows, int64_t n_src, void *ro
 // Bytes of a copy of x in rows of whole 16-byte vectors, where reading that copy is worth making it; otherwise 0.
 size_t walk_copy_bytes(const cxg_spmm_desc *d, int64_t n_src);
 
+// The aggregation of a.ptr, idx, x, y, edge_val as one launch of clusters (spmm_small.cu): rows of up to 64 vectors of 16
+// bytes or 128 of fewer, up to small_most_rows() of them. False: no kernel for it.
+bool small_launch(const WalkArgs &a, int dtype, int vb, cudaStream_t st);
+int small_most_rows();
+
 // One launcher per element type and vector width, each in a translation unit of its own. False: no kernel for it. With
 // resident_tiles set nothing is launched: it receives the number of tiles that are walked at the same time.
 bool walk_launch_f32_16(const WalkArgs &a, int valmode, bool share, cudaStream_t st, int *resident_tiles);
