@@ -87,6 +87,11 @@ __global__ void __launch_bounds__(kJoinThreads) column_sum_final(const float *pa
 }
 
 }  // namespace
+
+void column_sum_join(const float *part, float *out, int n_part, int width, cudaStream_t st) {
+  column_sum_final<<<(width + 31) / 32, kJoinThreads, 0, st>>>(part, out, n_part, width);
+}
+
 }  // namespace cxg
 
 using namespace cxg;

@@ -19,6 +19,8 @@ int set_error(int code, const char *fmt, ...);
 int check_launch(const char *what);
 // Adds n to the process-wide count of kernels this library has launched.
 void count_launches(int n);
+// Adds n_part rows of partial column sums [n_part, width] in a fixed order (colsum.cu; one launch).
+void column_sum_join(const float *part, float *out, int n_part, int width, cudaStream_t st);
 // Reads a status word of the library's own (behind everything queued on `stream`) and clears it: CXG_OK or CXG_ETIMEOUT.
 int take_status_word(void *word, void *stream, const char *who);
 // Cycle limit of one bounded device-side wait (cxg_set_wait_limit_cycles; default about a second).

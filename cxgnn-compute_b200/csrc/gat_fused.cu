@@ -124,6 +124,19 @@ struct TileWalk {
   }
 };
 
+// Tiles behind the first round go to whichever warp comes for them: SMs differ in what they get through. A warp asks while it
+// walks and looks at the answer, which lane 0 holds, afterwards.
+struct NextTile {
+  int32_t *counter;
+  int64_t n_tiles, first;
+  __device__ __forceinline__ NextTile(const GatArgs &a, int64_t tiles, int64_t walked)
+      : counter(a.w.hdr + kWalkHdrNext), n_tiles(tiles), first(walked) {}
+  __device__ __forceinline__ int64_t ask(int count) const {
+    return first < n_tiles && (threadIdx.x & 31) == 0 ? first + atomicAdd(counter, count) : n_tiles;
+  }
+  __device__ __forceinline__ int64_t get(int64_t asked) const { return __shfl_sync(0xffffffffu, asked, 0); }
+};
+
 template <int VB>
 __device__ __forceinline__ void load_floats(float (&f)[VB / 4], const float *p) {
   if constexpr (VB == 16) {
@@ -443,7 +456,9 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_wide_forward(const __grid_
     for (int64_t r = wid; r < n_rows; r += n_warps) empty_row(r);
     return;
   }
-  for (int64_t t = wid; t < n_tiles; t += n_warps) {
+  const NextTile next_tile(a, n_tiles, n_warps);
+  for (int64_t t = wid, t_next; t < n_tiles; t = next_tile.get(t_next)) {
+    t_next = next_tile.ask(1);
     TileWalk w{a};
     w.begin = static_cast<const WideTile *>(a.w.tiles)[t].begin;
     w.row = static_cast<const WideTile *>(a.w.tiles)[t].row;
@@ -641,7 +656,9 @@ __global__ void __launch_bounds__(kThreads, MINB) gat_wide_backward(const __grid
     for (int64_t r = wid; r < n_rows; r += n_warps) empty_row(r);
     return;
   }
-  for (int64_t t = wid; t < n_tiles; t += n_warps) {
+  const NextTile next_tile(a, n_tiles, n_warps);
+  for (int64_t t = wid, t_next; t < n_tiles; t = next_tile.get(t_next)) {
+    t_next = next_tile.ask(1);
     TileWalk w{a};
     w.begin = static_cast<const WideTile *>(a.w.tiles)[t].begin;
     w.row = static_cast<const WideTile *>(a.w.tiles)[t].row;
@@ -1095,36 +1112,73 @@ __global__ void __launch_bounds__(256, 3) gat_fix(const __grid_constant__ GatArg
 }
 
 // Backward set-up, one warp per destination: stats[r, h] = {a_dst, row_max, 1 / row_sum, <dy[r,h,:], y[r,h,:]>}
-// and d a_dst[r, h] = 0 (the walk adds into it). A head's columns lie with c / W neighbouring lanes.
-template <int W>
+// and d a_dst[r, h] = 0 (the walk adds into it). A head's columns lie with c / W neighbouring lanes. With col_part the block
+// also leaves the sums of dy's columns over its rows [gridDim.x, width], the gradient of the layer's bias, which was a pass over
+// dy of its own (config 2: 25 us next to 35 of this kernel, now 35 together).
+template <int W, int kRounds>  // kRounds of 32 * W columns
 __global__ void __launch_bounds__(256) gat_bwd_prepare(const float *dy, const float *y, const float *a_dst,
                                                        const float *row_max, const float *row_sum, float *stats,
-                                                       float *d_a_dst, int64_t n_dst, int heads, int c) {
+                                                       float *d_a_dst, float *col_part, int64_t n_dst, int heads, int c) {
+  __shared__ float sums[8][kRounds * 32 * W];
   const int lane = threadIdx.x & 31;
   const int lph = c / W, width = heads * c;
   const int64_t gwarp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t r = gwarp; r < n_dst; r += nwarps) {
-    for (int c0 = 0; c0 < width; c0 += 32 * W) {
-      const int col = c0 + lane * W;
-      const bool on = col < width;
-      const int h = on ? col / c : 0;
-      float d = 0.f;
-      if (on) {
-        float g[W], v[W];
-        load_floats<W * 4>(g, dy + r * width + col);
-        load_floats<W * 4>(v, y + r * width + col);
+  constexpr int kRows = kRounds == 4 ? 1 : 4 / kRounds;  // rows whose loads are in flight
+  float total[kRounds][W] = {};
+  int head[kRounds];
+  bool on[kRounds], lead[kRounds];
 #pragma unroll
-        for (int i = 0; i < W; ++i) d = fmaf(g[i], v[i], d);
+  for (int j = 0; j < kRounds; ++j) {
+    const int col = (j * 32 + lane) * W;
+    on[j] = col < width;
+    head[j] = on[j] ? col / c : 0;
+    lead[j] = on[j] && col == head[j] * c;
+  }
+  for (int64_t r0 = gwarp; r0 < n_dst; r0 += kRows * nwarps) {
+    float g[kRows][kRounds][W], v[kRows][kRounds][W], sum[kRows][kRounds], top[kRows][kRounds], add[kRows][kRounds];
+#pragma unroll
+    for (int u = 0; u < kRows; ++u)
+#pragma unroll
+      for (int j = 0; j < kRounds; ++j) {
+        const int64_t r = min(r0 + u * nwarps, n_dst - 1);
+        const int col = on[j] ? (j * 32 + lane) * W : 0;
+        load_floats<W * 4>(g[u][j], dy + r * width + col);
+        load_floats<W * 4>(v[u][j], y + r * width + col);
+        if (lead[j]) sum[u][j] = __ldg(row_sum + r * heads + head[j]), top[u][j] = __ldg(row_max + r * heads + head[j]), add[u][j] = __ldg(a_dst + r * heads + head[j]);
       }
-      for (int o = lph >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-      if (on && col == h * c) {
-        const float sum = row_sum[r * heads + h];
-        *reinterpret_cast<float4 *>(stats + (r * heads + h) * 4) =
-            make_float4(a_dst[r * heads + h], row_max[r * heads + h], sum > 0.f ? 1.f / sum : 0.f, d);
-        d_a_dst[r * heads + h] = 0.f;
+#pragma unroll
+    for (int u = 0; u < kRows; ++u)
+#pragma unroll
+      for (int j = 0; j < kRounds; ++j) {
+        const int64_t r = r0 + u * nwarps;
+        float d = 0.f;
+        if (on[j]) {
+#pragma unroll
+          for (int i = 0; i < W; ++i) d = fmaf(g[u][j][i], v[u][j][i], d);
+          if (r < n_dst)
+#pragma unroll
+            for (int i = 0; i < W; ++i) total[j][i] += g[u][j][i];
+        }
+        for (int o = lph >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if (r < n_dst && lead[j]) {
+          *reinterpret_cast<float4 *>(stats + (r * heads + head[j]) * 4) =
+              make_float4(add[u][j], top[u][j], sum[u][j] > 0.f ? 1.f / sum[u][j] : 0.f, d);
+          d_a_dst[r * heads + head[j]] = 0.f;
+        }
       }
-    }
+  }
+  if (col_part == nullptr) return;
+#pragma unroll
+  for (int j = 0; j < kRounds; ++j)
+#pragma unroll
+    for (int i = 0; i < W; ++i) sums[threadIdx.x >> 5][(j * 32 + lane) * W + i] = total[j][i];
+  __syncthreads();
+  for (int col = threadIdx.x; col < width; col += 256) {
+    float s = sums[0][col];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) s += sums[w][col];
+    col_part[static_cast<int64_t>(blockIdx.x) * width + col] = s;
   }
 }
 
@@ -1261,8 +1315,11 @@ __global__ void __launch_bounds__(256) gat_dst_sum_long(const void *ptr, int ptr
 
 struct GatLayout {
   WalkLayout walk;
-  size_t part_ms, block_ms, stats, long_rows, piece_sums, d_edge, total;
+  size_t part_ms, block_ms, stats, col_part, long_rows, piece_sums, d_edge, total;
 };
+
+// Blocks of gat_bwd_prepare.
+int64_t prepare_blocks(int64_t n_dst) { return n_dst / 8 + 1 < kNumSM * 8 ? n_dst / 8 + 1 : kNumSM * 8; }
 
 int gat_layout(int64_t n_stats_rows, int64_t nnz, int heads, int c, GatLayout *L) {
   const int rc = walk_layout(nnz, static_cast<int64_t>(heads) * c, 64, &L->walk);  // 64 = smallest tile
@@ -1274,6 +1331,8 @@ int gat_layout(int64_t n_stats_rows, int64_t nnz, int heads, int c, GatLayout *L
   off = align_up(off + static_cast<size_t>(L->walk.max_tiles) * heads * 2 * sizeof(float), 256);
   L->stats = off;
   off = align_up(off + static_cast<size_t>(n_stats_rows) * heads * 4 * sizeof(float), 256);
+  L->col_part = off;
+  off = align_up(off + static_cast<size_t>(prepare_blocks(n_stats_rows)) * heads * c * sizeof(float), 256);
   // ordered d a_dst of the backward: destinations of more than kLongRowEdges edges, and one value per edge and head
   L->long_rows = off;
   off = align_up(off + static_cast<size_t>(nnz / kLongRowEdges + 1) * sizeof(int64_t), 256);
@@ -1367,7 +1426,7 @@ cudaError_t launch_walk(GatArgs &a, cudaStream_t st) {
   auto go = [&](auto kernel, int g, int ctas) {
     const int per_cta = kThreads / g;
     const int64_t resident = static_cast<int64_t>(kNumSM) * ctas;
-    a.w.tile = walk_whole_waves(a.w.nnz, resident * per_cta, 32);
+    a.w.tile = walk_tile_of_waves(a.w.nnz, resident * per_cta);
     a.w.max_tiles = (a.w.nnz + a.w.tile - 1) / a.w.tile + 1;
     walk_plan_run(a.w, st);
     int64_t grid = (a.w.max_tiles + per_cta - 1) / per_cta;
@@ -1493,11 +1552,11 @@ extern "C" int cxg_gat_fused_forward(const void *ptr, const void *idx, int ptr_b
   return check_launch("cxg_gat_fused_forward");
 }
 
-extern "C" int cxg_gat_fused_backward(const void *t_ptr, const void *t_idx, int ptr_bytes, int idx_bytes, const float *dy,
+extern "C" int cxg_gat_fused_backward_bias(const void *t_ptr, const void *t_idx, int ptr_bytes, int idx_bytes, const float *dy,
                                       const float *y, const float *x, const float *a_src, const float *a_dst,
                                       const float *row_max, const float *row_sum, float *dx, float *d_a_src,
                                       float *d_a_dst, int64_t n_src, int64_t n_dst, int64_t nnz, int heads, int c,
-                                      float slope, const void *t_eid, const void *fwd_ptr, int fwd_ptr_bytes,
+                                      float slope, const void *t_eid, const void *fwd_ptr, int fwd_ptr_bytes, float *d_bias,
                                       void *workspace, size_t workspace_bytes, void *stream) {
   CXG_REQUIRE(n_src >= 0 && n_dst >= 0 && nnz >= 0, CXG_EINVAL, "cxg_gat_fused_backward: negative size");
   CXG_REQUIRE((ptr_bytes == 4 || ptr_bytes == 8) && (idx_bytes == 4 || idx_bytes == 8), CXG_EINVAL,
@@ -1507,6 +1566,7 @@ extern "C" int cxg_gat_fused_backward(const void *t_ptr, const void *t_idx, int 
   if (n_src == 0) return CXG_OK;
   CXG_REQUIRE(t_ptr && x && a_src && dx && d_a_src && d_a_dst, CXG_ENULL, "cxg_gat_fused_backward: NULL argument");
   CXG_REQUIRE(n_dst == 0 || (dy && y && a_dst && row_max && row_sum), CXG_ENULL, "cxg_gat_fused_backward: NULL argument");
+  CXG_REQUIRE(d_bias == nullptr || n_dst > 0, CXG_EINVAL, "cxg_gat_fused_backward_bias: no rows");
   CXG_REQUIRE(nnz == 0 || t_idx, CXG_ENULL, "cxg_gat_fused_backward: t_idx is NULL");
   CXG_REQUIRE((t_eid == nullptr) == (fwd_ptr == nullptr), CXG_EINVAL,
               "cxg_gat_fused_backward: t_eid and fwd_ptr select the ordered d_a_dst together");
@@ -1535,15 +1595,20 @@ extern "C" int cxg_gat_fused_backward(const void *t_ptr, const void *t_idx, int 
   while ((1 << hshift) < heads) ++hshift;
   cudaStream_t st = as_stream(stream);
   if (n_dst > 0) {
-    const unsigned pg = static_cast<unsigned>(n_dst / 8 + 1 < kNumSM * 8 ? n_dst / 8 + 1 : kNumSM * 8);
+    const unsigned pg = static_cast<unsigned>(prepare_blocks(n_dst));
+    float *col_part = d_bias != nullptr ? reinterpret_cast<float *>(static_cast<char *>(workspace) + L.col_part) : nullptr;
     const int vb = vector_of(heads, c);
     if (vb == 4)
-      gat_bwd_prepare<1><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, n_dst, heads, c);
+      gat_bwd_prepare<1, 1><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, col_part, n_dst, heads, c);
     else if (vb == 8)
-      gat_bwd_prepare<2><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, n_dst, heads, c);
+      gat_bwd_prepare<2, 1><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, col_part, n_dst, heads, c);
     else
-      gat_bwd_prepare<4><<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, n_dst, heads, c);
+      (heads * c <= 128 ? gat_bwd_prepare<4, 1> : heads * c <= 256 ? gat_bwd_prepare<4, 2> : gat_bwd_prepare<4, 4>)<<<pg, 256, 0, st>>>(dy, y, a_dst, row_max, row_sum, stats, d_a_dst, col_part, n_dst, heads, c);
     count_launches(1);
+    if (d_bias != nullptr) {
+      column_sum_join(col_part, d_bias, static_cast<int>(pg), heads * c, st);
+      count_launches(1);
+    }
   }
   cudaError_t e = launch_walk<true>(a, st);
   if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_gat_fused_backward: %s", cudaGetErrorString(e));
@@ -1562,4 +1627,15 @@ extern "C" int cxg_gat_fused_backward(const void *t_ptr, const void *t_idx, int 
     count_launches(3);
   }
   return check_launch("cxg_gat_fused_backward");
+}
+
+extern "C" int cxg_gat_fused_backward(const void *t_ptr, const void *t_idx, int ptr_bytes, int idx_bytes, const float *dy,
+                                      const float *y, const float *x, const float *a_src, const float *a_dst,
+                                      const float *row_max, const float *row_sum, float *dx, float *d_a_src,
+                                      float *d_a_dst, int64_t n_src, int64_t n_dst, int64_t nnz, int heads, int c,
+                                      float slope, const void *t_eid, const void *fwd_ptr, int fwd_ptr_bytes,
+                                      void *workspace, size_t workspace_bytes, void *stream) {
+  return cxg_gat_fused_backward_bias(t_ptr, t_idx, ptr_bytes, idx_bytes, dy, y, x, a_src, a_dst, row_max, row_sum, dx, d_a_src,
+                                     d_a_dst, n_src, n_dst, nnz, heads, c, slope, t_eid, fwd_ptr, fwd_ptr_bytes, nullptr, workspace,
+                                     workspace_bytes, stream);
 }

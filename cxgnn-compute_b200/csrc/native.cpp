@@ -50,7 +50,7 @@ struct Lib {
   CXG_FN(cxg_gat_scores);
   CXG_FN(cxg_gat_fused_workspace_size);
   CXG_FN(cxg_gat_fused_forward);
-  CXG_FN(cxg_gat_fused_backward);
+  CXG_FN(cxg_gat_fused_backward_bias);
   CXG_FN(cxg_gat_att_grad_workspace_size);
   CXG_FN(cxg_gat_scores_backward_add);
   CXG_FN(cxg_head_mean_bias);
@@ -89,7 +89,7 @@ void init(const std::string &path) {
   CXG_FN(cxg_gat_scores);
   CXG_FN(cxg_gat_fused_workspace_size);
   CXG_FN(cxg_gat_fused_forward);
-  CXG_FN(cxg_gat_fused_backward);
+  CXG_FN(cxg_gat_fused_backward_bias);
   CXG_FN(cxg_gat_att_grad_workspace_size);
   CXG_FN(cxg_gat_scores_backward_add);
   CXG_FN(cxg_head_mean_bias);
@@ -764,9 +764,11 @@ class GatFunction : public torch::autograd::Function<GatFunction> {
     void *st = stream_of(x);
     const Tensor g = grads[0].contiguous();
     Tensor db;
-    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(3)) db = rows_sum(g);
+    const bool concat = ctx->saved_data["concat"].toBool(), need_db = ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(3);
+    // heads side by side: the columns of dy are the bias's, and the backward reads them anyway
+    if (need_db) db = concat && n > 0 && n_src > 0 ? at::empty({h * c}, x.options()) : rows_sum(g);
     const Tensor dy =
-        ctx->saved_data["concat"].toBool() ? g : g.mul(1.0 / static_cast<double>(h)).unsqueeze(1).expand({n, h, c}).contiguous();
+        concat ? g : g.mul(1.0 / static_cast<double>(h)).unsqueeze(1).expand({n, h, c}).contiguous();
     const Transposed t = transposed_graph(ptr, idx, n, n_src);
     const Tensor dx = at::empty_like(x), d_src = at::empty_like(a_src), d_dst = at::empty_like(a_dst);
     const Tensor g_as = at::empty_like(att_src), g_ad = at::empty_like(att_dst);
@@ -774,13 +776,13 @@ class GatFunction : public torch::autograd::Function<GatFunction> {
     check(lib.cxg_gat_fused_workspace_size(n, idx.size(0), hi, ci, &need), "cxg_gat_fused_workspace_size");
     check(lib.cxg_gat_att_grad_workspace_size(hi, ci, &need_att), "cxg_gat_att_grad_workspace_size");
     const Workspace ws = workspace_on(x.device().index(), st, static_cast<int64_t>(std::max(need, need_att)), "");
-    check(lib.cxg_gat_fused_backward(t.t_ptr.data_ptr(), t.t_idx.data_ptr(), static_cast<int>(t.t_ptr.element_size()),
+    check(lib.cxg_gat_fused_backward_bias(t.t_ptr.data_ptr(), t.t_idx.data_ptr(), static_cast<int>(t.t_ptr.element_size()),
                                      static_cast<int>(t.t_idx.element_size()), dy.data_ptr<float>(), y.data_ptr<float>(),
                                      x.data_ptr<float>(), a_src.data_ptr<float>(), a_dst.data_ptr<float>(), top.data_ptr<float>(),
                                      sum.data_ptr<float>(), dx.data_ptr<float>(), d_src.data_ptr<float>(), d_dst.data_ptr<float>(),
                                      n_src, n, t.t_idx.size(0), hi, ci, static_cast<float>(ctx->saved_data["slope"].toDouble()),
-                                     nullptr, nullptr, static_cast<int>(ptr.element_size()), ws.data(),
-                                     ws.bytes(), st),
+                                     nullptr, nullptr, static_cast<int>(ptr.element_size()),
+                                     need_db && concat && n > 0 && n_src > 0 ? db.data_ptr<float>() : nullptr, ws.data(), ws.bytes(), st),
           "cxg_gat_fused_backward");
     check(lib.cxg_gat_scores_backward_add(x.data_ptr<float>(), d_src.data_ptr<float>(), d_dst.data_ptr<float>(),
                                           att_src.data_ptr<float>(), att_dst.data_ptr<float>(), dx.data_ptr<float>(),

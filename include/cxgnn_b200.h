@@ -318,6 +318,13 @@ int cxg_gat_fused_backward(const void *t_ptr, const void *t_idx, int ptr_bytes, 
                            float *d_a_src, float *d_a_dst, int64_t n_src, int64_t n_dst, int64_t nnz,
                            int heads, int c, float slope, const void *t_eid, const void *fwd_ptr,
                            int fwd_ptr_bytes, void *workspace, size_t workspace_bytes, void *stream);
+/* The same, and d_bias [heads * c] = the sums of dy's columns (NULL: not wanted), from the pass that reads dy anyway. */
+int cxg_gat_fused_backward_bias(const void *t_ptr, const void *t_idx, int ptr_bytes, int idx_bytes,
+                           const float *dy, const float *y, const float *x, const float *a_src,
+                           const float *a_dst, const float *row_max, const float *row_sum, float *dx,
+                           float *d_a_src, float *d_a_dst, int64_t n_src, int64_t n_dst, int64_t nnz,
+                           int heads, int c, float slope, const void *t_eid, const void *fwd_ptr,
+                           int fwd_ptr_bytes, float *d_bias, void *workspace, size_t workspace_bytes, void *stream);
 
 /*
  * SDDMM on an edge list: out[e,h] = <src_feat[src[e],h,:], dst_feat[dst[e],:]>, src_feat
