@@ -109,26 +109,6 @@ __device__ __forceinline__ int64_t edge_total(const WalkArgs &a) {
   const int64_t e = load_ptr(a.ptr, a.n_dst, a.ptr_bytes);
   return e > a.nnz ? a.nnz : e;
 }
-
-// Waits for the kernel in front (launch_dependent lets a kernel start before that one has ended).
-__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-// Launch whose blocks may become resident while the kernel in front of it in the stream drains; that kernel's writes
-// are visible behind dependency_wait(). Takes about 2 us out of a chain of three short kernels.
-template <typename Kernel, typename... Args>
-cudaError_t launch_dependent(Kernel kernel, unsigned grid, int threads, size_t smem, cudaStream_t st, const Args &...args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(static_cast<unsigned>(threads));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
 #endif
 
 }  // namespace cxg
