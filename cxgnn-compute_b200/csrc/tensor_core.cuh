@@ -40,13 +40,13 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       : "memory");
 }
 
-// v = hi + lo + what two bits of v cannot hold: hi the upper 19 bits of v, lo = v - hi (exact, at most 13 significant bits)
-// moved half a unit of its 19 bits up in magnitude, so that the tensor core, which ignores the other 13 bits of a word,
-// reads it rounded. Cut instead, every product would be short by 1e-7 of itself on the same side. (The addition turns a
-// NaN, which lo is where v is infinite, into -0; hi carries infinities and NaN alone.)
-__device__ __forceinline__ void split_tf32(float v, float &hi, float &lo) {
-  hi = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
-  lo = __uint_as_float(__float_as_uint(v - hi) + 0x1000u);
+// v = hi + lo + what two bits of v cannot hold: hi the upper 19 bits of v, which the tensor core reads from v itself, as it
+// ignores the other 13 of a word; lo = v - hi (exact, at most 13 significant bits) moved half a unit of its 19 bits up in
+// magnitude, so that it is read rounded. Cut instead, every product would be short by 1e-7 of itself on the same side. (The
+// addition turns a NaN, which lo is where v is infinite, into -0; hi carries infinities and NaN alone.)
+__device__ __forceinline__ float tf32_rest(float v) {
+  const float hi = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
+  return __uint_as_float(__float_as_uint(v - hi) + 0x1000u);
 }
 
 // Instruction descriptor: fp32 accumulate, A and B of format `fmt` (1 = bf16, 2 = tf32), both K-major.
@@ -144,6 +144,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t *v, uint32_t taddr) {
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
         "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(taddr));
+}
+
+// 8 columns
+__device__ __forceinline__ void tmem_ld8(uint32_t *v, uint32_t taddr) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr));
 }
 
 // one column

@@ -37,7 +37,7 @@
 // the epilogue: 3.2e-7 of the result at K = 128. W_lo lies behind W_hi, so A_hi x [W_hi | W_lo] is one instruction, and
 // the tensor pipe, idle most of the time on this memory-bound op, absorbs the rest. An infinite operand gives infinities
 // or NaN (an infinity times a lower term, zero or of either sign). W is split once by the transposing pre-pass; a tile of A is split in shared memory by
-// converter warps between the producers and the MMA thread (raw -> hi in place, lo into the second half of
+// converter warps between the producers and the MMA thread (the raw words serve as hi, lo goes into the second half of
 // the stage). To keep several stages in flight with stages twice as large, the K dimension is cut into blocks:
 // the pipeline unit is (tile, K-block) and all blocks of a tile accumulate into one accumulator buffer.
 //
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (X3 && warp >= kFirstConvWarp) {
-    // ================= converters: raw fp32 stage -> hi (in place) and lo (second half) =================
+    // ================= converters: lo of the raw fp32 stage, which is hi, into its second half =================
     const int ct = tid - 32 * kFirstConvWarp;  // 0 .. 32 * kConvWarps - 1
     const int n16 = static_cast<int>(half_bytes / 16);
     Ring ring(S);
@@ -364,13 +364,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
 #pragma unroll
           for (int u = 0; u < 4; ++u)
             if (c0 + u * kStep < n16) {
-              float4 h, l;
-              split_tf32(v[u].x, h.x, l.x);
-              split_tf32(v[u].y, h.y, l.y);
-              split_tf32(v[u].z, h.z, l.z);
-              split_tf32(v[u].w, h.w, l.w);
-              hi[c0 + u * kStep] = h;
-              lo[c0 + u * kStep] = l;
+              lo[c0 + u * kStep] = make_float4(tf32_rest(v[u].x), tf32_rest(v[u].y), tf32_rest(v[u].z), tf32_rest(v[u].w));
             }
         }
         // these generic-proxy writes are read by the tensor core through the async proxy

@@ -15,10 +15,19 @@
 // a partial slot of this CTA. A second kernel adds the slots of every relation in (CTA, slot) order: no atomics,
 // the same bits on every run.
 //
-// fp32 inputs: plain TF32 products (precision 1) or, like the forward, error-compensated ones (precision 2): four
-// converter warps split both tiles of a stage into hi = upper 19 bits and lo = v - hi rounded to 19 bits, and the
-// tensor core accumulates A_hi.B_lo + A_lo.B_hi and A_hi.B_hi. (169,343 positions, 128 x 128, against float64: 3.8e-6 of
-// the result with one accumulator and 512 positions in it, 0.9e-6 with two and 256; an fp32 GEMM 1.4e-6.)
+// An accumulator takes a bounded number of positions (its error grows with them), then the epilogue adds it to the sum in
+// the slot. In rows of N columns every lane of that read-modify-write was in another line, and the four warps took longer
+// for it than the tensor core for the next accumulator. Now four columns of all rows lie side by side, eight warps share
+// the columns, and the old sums are asked for a step ahead: 169,343 positions, 128 x 128, 81 -> 54 us (a stream of both
+// operands takes 26); 2.33 M positions, 128 x 64, gathered, 551 -> 503 us (1.79 GB, 270). What is left is spread thin: with
+// no copies, conversion or epilogue the barriers and the 8 instructions of a tile alone take 354 us, without three quarters
+// of the instructions 233, and shared memory is busy for two thirds of the time.
+//
+// fp32 inputs: plain TF32 products (precision 1) or, like the forward, error-compensated ones (precision 2): of both tiles
+// of a stage, whose words the tensor core reads as hi = upper 19 bits, four converter warps write lo = v - hi rounded to 19
+// bits (they wrote hi as well until it showed that nothing depends on it: same bits, 3 % of the kernel), and the tensor core
+// accumulates A_hi.B_lo + A_lo.B_hi and A_hi.B_hi. (169,343 positions, 128 x 128, against float64: 3.8e-6 of the result with
+// one accumulator and 512 positions in it, 0.9e-6 with two and 256; an fp32 GEMM 1.4e-6.)
 //
 // Every wait is bounded; a role that waits too long raises a CTA-wide abort flag and an error status.
 #include "common.cuh"
@@ -31,7 +40,7 @@ using namespace tc;
 
 constexpr int kProdWarps = 8;
 constexpr int kConvWarps = 4;
-constexpr int kEpiWarps = 4;    // warps 0..3: tensor-memory lanes 32 * warp .. + 31
+constexpr int kEpiWarps = 8;    // warps 0..7: tensor-memory lanes 32 * (warp % 4) .. + 31, every other 16 columns
 constexpr int kMmaWarp = kEpiWarps;
 constexpr int kFirstProd = kMmaWarp + 1;
 constexpr int kFirstConv = kFirstProd + kProdWarps;
@@ -53,7 +62,7 @@ struct WgArgs {
   int dense;           // 0, or the column blocks of x: the whole matrices, one relation, a column block pair per blockIdx.y
   int chunk_tiles;     // tiles summed in one tensor-memory accumulator before the epilogue takes it over
   int test_stall;      // test hook: the producers never hand over their first tile, so the waits for it run out
-  float *partial;      // [grid][slots][k][n]; dense: [column block pair][blockIdx.x][128][128]
+  float *partial;      // [grid][slots][n / 4][k][4]; dense: [column block pair][blockIdx.x][128 / 4][128][4]
   int32_t *slot_rel;   // [grid][slots]: relation of a flushed slot, -1 when unused
   int32_t *status;
   long long wait_cycles;
@@ -191,6 +200,11 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     const uint8_t *X = static_cast<const uint8_t *>(a.x) + x_at * sizeof(T), *G = static_cast<const uint8_t *>(a.g) + g_at * sizeof(T);
     const int64_t xpitch = a.k * static_cast<int64_t>(sizeof(T)), gpitch = a.n * static_cast<int64_t>(sizeof(T));
     constexpr int kPass = kPos / 32;  // passes of 32 rows per tile
+    const uint32_t base = smem_addr(smem);
+    const bool last_x = (spans_x - 1) * 128 + c16 * 16 < xrow, last_g = (spans_g - 1) * 128 + c16 * 16 < grow;
+    auto copy = [](uint32_t dst, const uint8_t *src, bool in) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+    };
     // Row indices are fetched for 128 positions at once, 128 positions ahead: a tile ahead was not enough, a compensated
     // tile of 32 positions waited for its indices most of the time (2.33 M x 128 x 64: 776 us, now about 600).
     constexpr int kGroup = 128 / kPos, kAhead = kPass * kGroup;
@@ -223,26 +237,24 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
           alive = wait_bar(&bars.empty[s], ring.emptied(), abort_flag, a.status, a.wait_cycles);
           if (!alive) continue;
         }
-        const uint32_t st0 = smem_addr(smem + static_cast<size_t>(s) * stage_bytes);
+        const uint32_t st0 = base + static_cast<uint32_t>(s) * stage_bytes;
 #pragma unroll
         for (int q = 0; q < kPass; ++q) {
-          const int p = q * 32 + prow;
           const int64_t xr = ia[t * kPass + q], gr = ig[t * kPass + q];
           // a position contributes only when both of its rows exist; size 0 writes zeros
-          const bool ok = xr >= 0 && xr < a.x_rows && gr >= 0 && gr < a.g_rows;
-          const int bytes = ok ? 16 : 0;
-          const uint32_t d0 = st0 + swizzled_offset<TF32>(p, c16);
-          const uint8_t *xs = ok ? X + xr * xpitch : X;
-          const uint8_t *gs = ok ? G + gr * gpitch : G;
-          // a chunk behind the row's end is written as zeros from the row's first chunk
-          auto copy = [&](const uint8_t *src, int row_bytes, int j, uint32_t dst) {
-            const int at = j * 128 + c16 * 16;
-            const bool in = at < row_bytes;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(in && ok ? src + at : src), "r"(in ? bytes : 0)
-                         : "memory");
+          const bool ok = static_cast<uint64_t>(xr) < static_cast<uint64_t>(a.x_rows) &&
+                          static_cast<uint64_t>(gr) < static_cast<uint64_t>(a.g_rows);
+          const uint32_t d0 = st0 + swizzled_offset<TF32>(q * 32 + prow, c16);
+          // a chunk behind the row's end (only the last span has them) is written as zeros
+          auto row = [&](const uint8_t *src, int spans, bool last_in, uint32_t dst) {
+            for (int j = 1; j < spans; ++j, dst += kSpan) {
+              copy(dst, src, ok);
+              if (ok) src += 128;
+            }
+            copy(dst, last_in ? src : X, ok && last_in);
           };
-          for (int j = 0; j < spans_x; ++j) copy(xs, xrow, j, d0 + j * kSpan);
-          for (int j = 0; j < spans_g; ++j) copy(gs, grow, j, d0 + (spans_x + j) * kSpan);
+          row(ok ? X + xr * xpitch + c16 * 16 : X, spans_x, last_x, d0);
+          row(ok ? G + gr * gpitch + c16 * 16 : G, spans_g, last_g, d0 + spans_x * kSpan);
         }
         if (!(a.test_stall && ring.round == 0 && ring.stage == 0))
           asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&bars.full[s])) : "memory");
@@ -251,7 +263,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (X3 && warp >= kFirstConv) {
-    // ================= converters: raw fp32 tiles -> hi (in place) and lo (second half of the stage) =================
+    // ================= converters: lo of the raw fp32 tiles, which are hi, into the second half of the stage =================
     const int ct = tid - 32 * kFirstConv;
     const int n16 = static_cast<int>(half_bytes / 16), x16 = spans_x * (kSpan / 16), g16 = n16 - x16;
     Ring ring(S);
@@ -263,7 +275,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
       const int s = ring.stage;
       alive = wait_bar(&bars.full[s], ring.filled(), abort_flag, a.status, a.wait_cycles);
       if (!alive) break;
-      float4 *hi = reinterpret_cast<float4 *>(smem + static_cast<size_t>(s) * stage_bytes);
+      const float4 *hi = reinterpret_cast<const float4 *>(smem + static_cast<size_t>(s) * stage_bytes);
       // the second half holds g's lo spans first, so that they follow g's hi spans, then those of x
       float4 *lo = reinterpret_cast<float4 *>(smem + static_cast<size_t>(s) * stage_bytes + half_bytes);
       constexpr int kStep = 32 * kConvWarps;
@@ -275,14 +287,8 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
 #pragma unroll
         for (int u = 0; u < 4; ++u)
           if (c0 + u * kStep < n16) {
-            float4 h, l;
-            split_tf32(v[u].x, h.x, l.x);
-            split_tf32(v[u].y, h.y, l.y);
-            split_tf32(v[u].z, h.z, l.z);
-            split_tf32(v[u].w, h.w, l.w);
             const int c = c0 + u * kStep;
-            hi[c] = h;
-            lo[c < x16 ? g16 + c : c - x16] = l;
+            lo[c < x16 ? g16 + c : c - x16] = make_float4(tf32_rest(v[u].x), tf32_rest(v[u].y), tf32_rest(v[u].z), tf32_rest(v[u].w));
           }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -364,38 +370,45 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     int64_t chunk = 0, seg = 0, cur = -1;
     int in_chunk = 0;
     bool alive = true, open = false, seg_started = false;
-    const int row = warp * 32 + lane;  // row of dW[r] = column of x
+    const int row = (warp & 3) * 32 + lane;  // row of dW[r] = column of x
+    const int c_first = (warp >> 2) * 16, rows = a.dense ? 128 : a.k;
     auto take_chunk = [&]() {
       const int buf = static_cast<int>(chunk & 1);
+      // four columns of all rows side by side: a warp's access is 512 bytes in a row
+      float *slot = a.dense ? a.partial + (static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x) * (128 * 128)
+                            : a.partial + (static_cast<int64_t>(blockIdx.x) * a.slots + seg) * a.k * a.n;
+      float4 *out = reinterpret_cast<float4 *>(slot) + row;
+      const bool more = seg_started && row < k;  // a later chunk of the segment: ordinary fp32 additions, in chunk order
+      float4 old[2] = {}, next[2] = {};
+      auto fetch = [&](int c) {
+        if (more && c < n) next[0] = out[(c >> 2) * rows], next[1] = out[((c >> 2) + 1) * rows];
+      };
+      fetch(c_first);
       alive = wait_bar(&bars.acc_full[buf], static_cast<uint32_t>((chunk >> 1) & 1), abort_flag, a.status, a.wait_cycles);
       if (!alive) return;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      float *out = a.dense ? a.partial + ((static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x) * 128 + row) * 128
-                           : a.partial + ((static_cast<int64_t>(blockIdx.x) * a.slots + seg) * a.k + row) * a.n;
-      const uint32_t taddr = tmem_d + (static_cast<uint32_t>(warp * 32) << 16) + buf * tmem_cols;
-      for (int c0 = 0; c0 < n; c0 += 16) {
-        uint32_t v[16];
-        tmem_ld16(v, taddr + c0);
+      const uint32_t taddr = tmem_d + (static_cast<uint32_t>((warp & 3) * 32) << 16) + buf * tmem_cols;
+      for (int c = c_first; c < n; c += (c & 8) ? 24 : 8) {  // 8 columns at a time, 16 of every 32
+        old[0] = next[0], old[1] = next[1];
+        fetch(c + ((c & 8) ? 24 : 8));
+        uint32_t v[8];
+        tmem_ld8(v, taddr + c);
         if (X3 && small_off) {
-          uint32_t w[16];
-          tmem_ld16(w, taddr + small_off + c0);
+          uint32_t w[8];
+          tmem_ld8(w, taddr + small_off + c);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(w[i]));
+          for (int i = 0; i < 8; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(w[i]));
         } else {
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         }
         if (row < k) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
+          for (int q = 0; q < 2; ++q) {
             float4 acc = make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]), __uint_as_float(v[4 * q + 2]),
                                      __uint_as_float(v[4 * q + 3]));
-            float4 *dst = reinterpret_cast<float4 *>(out + c0 + 4 * q);
-            if (seg_started) {  // a later chunk of the segment: ordinary fp32 additions, in chunk order
-              const float4 old = *dst;
-              acc.x += old.x, acc.y += old.y, acc.z += old.z, acc.w += old.w;
-            }
-            *dst = acc;
+            if (seg_started) acc.x += old[q].x, acc.y += old[q].y, acc.z += old[q].z, acc.w += old[q].w;
+            out[((c >> 2) + q) * rows] = acc;
           }
         }
       }
@@ -441,8 +454,9 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
 // 128 x 64, now 5 us.) The small block spreads a small gradient over more SMs.
 constexpr int kRedThreads = 128, kRedPer = 8, kRedChunk = kRedThreads * kRedPer;
 __global__ void __launch_bounds__(kRedThreads) wgrad_reduce(const float *partial, const int32_t *slot_rel, float *dw,
-                                                            int n_slots, int num_rel, int64_t kn) {
+                                                            int n_slots, int num_rel, int k, int n) {
   __shared__ int list[kRedChunk];
+  const int64_t kn = static_cast<int64_t>(k) * n;
   __shared__ int warp_sum[kRedThreads / 32];
   const int64_t i = blockIdx.x * static_cast<int64_t>(kRedThreads) + threadIdx.x;
   const int r = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -484,7 +498,10 @@ __global__ void __launch_bounds__(kRedThreads) wgrad_reduce(const float *partial
     for (; q < total; ++q) s += p[list[q] * kn];
     __syncthreads();  // the list is free for the next chunk
   }
-  if (in) dw[static_cast<int64_t>(r) * kn + i] = s;
+  if (in) {
+    const int64_t q = i >> 2;  // four columns of all rows side by side
+    dw[r * kn + q % k * n + (q / k * 4 + (i & 3))] = s;
+  }
 }
 
 __global__ void wgrad_clear(int32_t *slot_rel, int n) {
@@ -499,9 +516,10 @@ __global__ void __launch_bounds__(128) dense_reduce(const float *partial, const 
                                                     int k, int n, int k_blocks, int parts) {
   const int64_t i = blockIdx.x * 128ll + threadIdx.x;
   if (i >= static_cast<int64_t>(k) * n) return;
-  const int r = static_cast<int>(i / n), c = static_cast<int>(i % n);
+  // neighbouring threads in the order of the partials: four columns, then the rows
+  const int r = static_cast<int>((i >> 2) % k), c = static_cast<int>((i >> 2) / k * 4 + (i & 3));
   const int64_t pair = r / 128 + static_cast<int64_t>(k_blocks) * (c / 128);
-  const float *p = partial + ((pair * parts) * 128 + r % 128) * 128 + c % 128;
+  const float *p = partial + pair * parts * (128 * 128) + (c % 128 / 4 * 128 + r % 128) * 4 + c % 4;
   float s = 0.f;
   int q = 0;
   for (; q + 8 <= parts; q += 8) {
@@ -519,7 +537,7 @@ __global__ void __launch_bounds__(128) dense_reduce(const float *partial, const 
       for (int u = 0; u < 8; ++u)
         if (t + u < m) s = fmaf(__ldg(x + (t + u) * k + r), __ldg(g + (t + u) * n + c), s);
   }
-  dw[i] = s;
+  dw[static_cast<int64_t>(r) * n + c] = s;
 }
 
 __device__ int32_t dense_status;  // set when a bounded wait of the dense mode ran out, cleared by cxg_dense_wgrad_f32_status
@@ -638,7 +656,7 @@ extern "C" int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel,
   }
   if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_typed_wgrad: %s", cudaGetErrorString(e));
   dim3 rg(static_cast<unsigned>((kn + kRedThreads - 1) / kRedThreads), static_cast<unsigned>(num_rel));
-  wgrad_reduce<<<rg, kRedThreads, 0, st>>>(a.partial, a.slot_rel, dw, n_slots, num_rel, kn);
+  wgrad_reduce<<<rg, kRedThreads, 0, st>>>(a.partial, a.slot_rel, dw, n_slots, num_rel, k, n);
   count_launches(3);
   return check_launch("cxg_typed_wgrad");
 }
