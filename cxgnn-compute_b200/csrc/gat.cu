@@ -566,33 +566,47 @@ __global__ void __launch_bounds__(kThreads) gat_scores_kernel(const float *feat,
 // reads its row from memory asks for 16 bytes of 32 different lines at a time; here a warp takes one head of 32 nodes (so that the attention vectors are
 // the same address for all lanes), brings their rows in with every lane on the next vector, up to 32 columns at a time, and
 // each lane then takes its own row from shared memory. A row there is an odd number of vectors long, so that the eight
-// lanes that are served together lie in different banks. (169,343 nodes, cold: 4 heads of 32 values 37 us, 51 with a thread
-// per pair; 8 of 32 66 (127); 2 of 64 35 (47); 4 of 28, where lines are shared by pairs, 37 (31), 4 of 12 27 (14). Lanes that
-// share a row and join their sums by shuffles take 36 / 52 / 37, and another order.)
-constexpr int kScoreVecs = 8;  // vectors of a row per round
+// lanes that are served together lie in different banks. A warp goes on to further nodes and asks for the next ones' vectors
+// before it sums, so that loading and summing overlap (169,343 nodes: 4 heads of 32 values 31 -> 22 us inside a layer, 4 of
+// 48 43 -> 36; six vectors and six instead of eight and four 38). With a round per block, cold: 4 heads of 32 values 37 us,
+// 51 with a thread per pair; 8 of 32 66 (127); 2 of 64 35 (47); 4 of 28, where lines are shared by pairs, 37 (31), 4 of 12
+// 27 (14). Lanes that share a row and join their sums by shuffles took 36 / 52 / 37, and another order.
+constexpr int kScoreVecs = 8;    // vectors of a row per round
+constexpr int kScoreBlocks = 4;  // per SM
 
-__global__ void __launch_bounds__(kThreads) gat_scores_vec(const float *feat, const float *att_src, const float *att_dst,
-                                                           float *alpha_src, float *alpha_dst, int64_t n_src, int64_t n_dst,
-                                                           int heads, int c) {
+__global__ void __launch_bounds__(kThreads, kScoreBlocks) gat_scores_vec(const float *feat, const float *att_src,
+                                                                         const float *att_dst, float *alpha_src,
+                                                                         float *alpha_dst, int64_t n_src, int64_t n_dst,
+                                                                         int heads, int c) {
   __shared__ float4 rows[kWarps][32 * (kScoreVecs + 1)];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t w = blockIdx.x * static_cast<int64_t>(kWarps) + warp, n0 = w / heads * 32;
-  if (n0 >= n_src) return;  // the whole warp
-  const int h = static_cast<int>(w % heads), nodes = n_src - n0 < 32 ? static_cast<int>(n_src - n0) : 32;
   const int vecs = c / 4, step = heads * vecs;  // vectors of a node's head, of a node
-  const float4 *f = reinterpret_cast<const float4 *>(feat) + n0 * step + h * vecs;
-  const float4 *as = reinterpret_cast<const float4 *>(att_src) + h * vecs, *ad = reinterpret_cast<const float4 *>(att_dst) + h * vecs;
+  const int64_t units = (n_src + 31) / 32 * heads, stride = static_cast<int64_t>(gridDim.x) * kWarps;
   float4 *mine = rows[warp];
-  float s = 0.f, d = 0.f;
-  for (int j0 = 0; j0 < vecs; j0 += kScoreVecs) {
-    const int now = min(kScoreVecs, vecs - j0), pitch = now | 1;
+  float4 v[kScoreVecs];
+  // 32 nodes of head w % heads, `now` vectors of each from j0 on
+  auto load = [&](int64_t w, int j0) {
+    const int64_t n0 = w / heads * 32;
+    const int h = static_cast<int>(w % heads), nodes = n_src - n0 < 32 ? static_cast<int>(n_src - n0) : 32;
+    const int now = min(kScoreVecs, vecs - j0);
     const unsigned magic = 65536u / now + 1;  // q / now for q < 256
-    float4 v[kScoreVecs];
+    const float4 *f = reinterpret_cast<const float4 *>(feat) + n0 * step + h * vecs + j0;
 #pragma unroll
     for (int k = 0; k < kScoreVecs; ++k) {
       const int q = k * 32 + lane, row = static_cast<int>((q * magic) >> 16);
-      if (row < nodes) v[k] = __ldg(f + static_cast<int64_t>(row) * step + j0 + (q - row * now));
+      if (row < nodes) v[k] = __ldg(f + static_cast<int64_t>(row) * step + (q - row * now));
     }
+  };
+  int64_t w = blockIdx.x * static_cast<int64_t>(kWarps) + warp;
+  int j0 = 0;
+  float s = 0.f, d = 0.f;
+  if (w < units) load(w, 0);
+  while (w < units) {
+    const int64_t n0 = w / heads * 32;
+    const int h = static_cast<int>(w % heads), nodes = n_src - n0 < 32 ? static_cast<int>(n_src - n0) : 32;
+    const int now = min(kScoreVecs, vecs - j0), pitch = now | 1, at = j0;
+    const unsigned magic = 65536u / now + 1;
+    const bool last = j0 + now == vecs;
     __syncwarp();  // the lanes have read the rows of the round before
 #pragma unroll
     for (int k = 0; k < kScoreVecs; ++k) {
@@ -600,21 +614,28 @@ __global__ void __launch_bounds__(kThreads) gat_scores_vec(const float *feat, co
       if (row < nodes) mine[row * pitch + (q - row * now)] = v[k];
     }
     __syncwarp();
+    // the next round is on its way while this one is summed
+    j0 = last ? 0 : j0 + now;
+    if (last) w += stride;
+    if (w < units) load(w, j0);
     if (lane < nodes) {
+      const float4 *as = reinterpret_cast<const float4 *>(att_src) + h * vecs + at;
+      const float4 *ad = reinterpret_cast<const float4 *>(att_dst) + h * vecs + at;
 #pragma unroll
       for (int k = 0; k < kScoreVecs; ++k)
         if (k < now) {
-          const float4 x = mine[lane * pitch + k], a = __ldg(as + j0 + k), b = __ldg(ad + j0 + k);
+          const float4 x = mine[lane * pitch + k], a = __ldg(as + k), b = __ldg(ad + k);
           s = fmaf(x.x, a.x, s), d = fmaf(x.x, b.x, d);
           s = fmaf(x.y, a.y, s), d = fmaf(x.y, b.y, d);
           s = fmaf(x.z, a.z, s), d = fmaf(x.z, b.z, d);
           s = fmaf(x.w, a.w, s), d = fmaf(x.w, b.w, d);
         }
+      if (last) {
+        alpha_src[(n0 + lane) * heads + h] = s;
+        if (n0 + lane < n_dst) alpha_dst[(n0 + lane) * heads + h] = d;
+      }
     }
-  }
-  if (lane < nodes) {
-    alpha_src[(n0 + lane) * heads + h] = s;
-    if (n0 + lane < n_dst) alpha_dst[(n0 + lane) * heads + h] = d;
+    if (last) s = 0.f, d = 0.f;
   }
 }
 
@@ -646,7 +667,8 @@ extern "C" int cxg_gat_scores(const float *feat, const float *att_src, const flo
   CXG_REQUIRE(c % 4 != 0 || reinterpret_cast<uintptr_t>(feat) % 16 == 0, CXG_EINVAL, "cxg_gat_scores: feat alignment");
   // narrower heads share lines between neighbouring threads, which the thread per pair then finds in L1
   if (c >= 32 && c % 4 == 0 && ((reinterpret_cast<uintptr_t>(att_src) | reinterpret_cast<uintptr_t>(att_dst)) % 16) == 0) {
-    const unsigned grid = static_cast<unsigned>(((n_src + 31) / 32 * heads + kWarps - 1) / kWarps);
+    const int64_t blocks = ((n_src + 31) / 32 * heads + kWarps - 1) / kWarps;
+    const unsigned grid = static_cast<unsigned>(blocks < kNumSM * kScoreBlocks ? blocks : kNumSM * kScoreBlocks);
     gat_scores_vec<<<grid, kThreads, 0, as_stream(stream)>>>(feat, att_src, att_dst, alpha_src, alpha_dst, n_src, n_dst, heads, c);
   } else {
     const unsigned grid = static_cast<unsigned>((n_src * heads + kThreads - 1) / kThreads);
