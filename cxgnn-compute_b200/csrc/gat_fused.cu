@@ -37,7 +37,7 @@
 // the separate kernels (cxg_gat_scores, cxg_edge_softmax_forward, cxg_spmm_csr).
 //
 // What bounds it: instructions per edge and per row end, with an IPC of 0.55 to 0.65 per scheduler; the gather stays in L2
-// for graphs of this kind. 2.33 M edges, 4 heads x 32: backward 288 us, forward in one step 178 (46 instructions per edge),
+// for graphs of this kind. 2.33 M edges, 4 heads x 32: backward 271 us, forward in one step 178 (46 instructions per edge),
 // in two 34 + 104, of which the walk is bound by L2 like the sum over such rows (90).
 #include "spmm_walk_impl.cuh"
 

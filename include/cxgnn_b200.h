@@ -211,7 +211,7 @@ int cxg_spmm_csr(const cxg_spmm_desc *desc, void *workspace,
 /*
  * The same with scratch for the rows of x. Rows that are not whole 16-byte vectors (47 fp32 values, an odd number of bf16
  * values) cost a load per value or two when they are gathered; where a graph reads them several times the call first copies
- * them, widened to whole 32-byte sectors, into `rows` and gathers from there. Sums are those of cxg_spmm_csr for the same
+ * them, widened to whole 128-byte lines, into `rows` and gathers from there. Sums are those of cxg_spmm_csr for the same
  * tile size, bit for bit. n_src: rows of x (all that idx names, times the relations with edge_rel).
  * cxg_spmm_csr_rows_size: bytes of that copy, 0 where the call reads x as it is. `rows` is 32-byte aligned; NULL is
  * cxg_spmm_csr.
@@ -397,7 +397,6 @@ int cxg_gat_scores_backward_add(const float *feat, const float *g_src, const flo
                                 int64_t n_src, int64_t n_dst, int heads, int c, void *workspace,
                                 size_t workspace_bytes, void *stream);
 
-/* out[n, :] = mean over heads of x[n, h, :] (+ bias, which may be NULL), fp32, x [n, heads, c] (cxgnncomp/graph_conv.py:487-494). */
 /* Heads padded to c_padded columns (a multiple of 4), for layers whose heads are not whole 16-byte vectors (class counts):
  * weights [heads * c, k] and attention vectors [heads, c] with zeros behind every head, and back from features
  * [n, heads, c_padded] to the heads' mean [n, c] or (join) the heads side by side [n, heads * c], plus the bias (may be NULL). */
@@ -405,6 +404,8 @@ int cxg_gat_pad_heads(const float *w, const float *att_src, const float *att_dst
                       float *att_dst_padded, int heads, int c, int c_padded, int k, void *stream);
 int cxg_gat_unpad_heads(const float *x, const float *bias, float *out, int64_t n, int heads, int c, int c_padded, int join,
                         void *stream);
+
+/* out[n, :] = mean over heads of x[n, h, :] (+ bias, which may be NULL), fp32, x [n, heads, c] (cxgnncomp/graph_conv.py:487-494). */
 int cxg_head_mean_bias(const float *x, const float *bias, float *out, int64_t n, int heads, int c, void *stream);
 
 /*
