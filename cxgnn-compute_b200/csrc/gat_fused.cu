@@ -1400,7 +1400,7 @@ cudaError_t launch_by_weights(GatArgs &a, int vb, cudaStream_t st) {
   a.w.edge_val = a.weights;
   a.w.part_stride = a.w.width;
   if (!walk_weighted(a.w, vb, st, &resident)) return cudaErrorInvalidValue;
-  const int tile = walk_whole_waves(a.w.nnz, resident, 8);
+  const int tile = walk_whole_waves(a.w.nnz, resident, 16);
   a.w.tile = tile < 256 ? tile : 256;
   a.w.max_tiles = (a.w.nnz + a.w.tile - 1) / a.w.tile + 1;
   walk_plan_run(a.w, st);

@@ -387,13 +387,15 @@ int walk_tile_of_waves(int64_t nnz, int64_t resident) {
   // One wave of tiles of up to 256 edges where that is enough (2.3 M edges, F = 64: 71 us, two waves of 128 edges 78), behind
   // that whole waves of up to 128, which even out what the groups get through (1.2 M edges, F = 201 bf16: 270 us with two
   // waves of 136, 250 with three of 88; 12.6 M, F = 47: 296 with six of 224, 290 with eleven of 128). From four waves of 512
-  // edges on the longer tile costs less (126 M edges: 10 % less than 128). At least 64 edges, so that small graphs do not become all
-  // borders.
+  // edges on the longer tile costs less (126 M edges: 10 % less than 128). At least 64 edges, so that small graphs do not become
+  // all borders. Several waves take multiples of 16 edges, whole lines of 64-bit ids (12.8 M edges, F = 16: 128 158 us, 120 172;
+  // 176 156, 232 161); in one wave they would leave groups without a tile (140,000 edges, F = 11: 80 35.1 us, 72 34.1).
   if (nnz >= 2048 * resident) return 512;
   const int64_t most = nnz <= 256 * resident ? 256 : 128;
   const int64_t waves = (nnz + most * resident - 1) / (most * resident);
   const int64_t t = waves > 0 ? (nnz + waves * resident - 1) / (waves * resident) : 0;
-  return t < 64 ? 64 : static_cast<int>((t + 7) / 8 * 8);
+  const int64_t round = waves > 1 ? 16 : 8;
+  return t < 64 ? 64 : static_cast<int>((t + round - 1) / round * round);
 }
 
 bool walk_weighted(const WalkArgs &a, int vb, cudaStream_t st, int *resident_tiles) {
