@@ -27,6 +27,7 @@ __device__ __forceinline__ float cs_load<__nv_bfloat16>(const __nv_bfloat16 *p) 
 // accumulators (j mod 4) joined as (a0 + a1) + (a2 + a3); the nsub sums of a column are added in sub order.
 template <typename T>
 __global__ void __launch_bounds__(kCsThreads) column_sum_partial(const T *x, float *part, int64_t n_row, int width) {
+  dependency_wait();
   __shared__ float sh[kCsThreads];
   const int nsub = width <= kCsThreads ? kCsThreads / width : 1;
   const int64_t per = (n_row + gridDim.x - 1) / gridDim.x;
@@ -62,6 +63,7 @@ __global__ void __launch_bounds__(kCsThreads) column_sum_partial(const T *x, flo
 // warp per column read 4 bytes of every sector: 7 us for 1184 partials of 128 columns, now 4.)
 constexpr int kJoinThreads = 1024;
 __global__ void __launch_bounds__(kJoinThreads) column_sum_final(const float *part, float *out, int n_part, int width) {
+  dependency_wait();
   __shared__ float sh[kJoinThreads / 32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.x * 32 + lane;
   constexpr int kWarps = kJoinThreads / 32;
@@ -89,7 +91,7 @@ __global__ void __launch_bounds__(kJoinThreads) column_sum_final(const float *pa
 }  // namespace
 
 void column_sum_join(const float *part, float *out, int n_part, int width, cudaStream_t st) {
-  column_sum_final<<<(width + 31) / 32, kJoinThreads, 0, st>>>(part, out, n_part, width);
+  launch_dependent(column_sum_final, (width + 31) / 32, kJoinThreads, 0, st, part, out, n_part, width);
 }
 
 }  // namespace cxg
@@ -121,10 +123,10 @@ extern "C" int cxg_column_sum(const void *x, int dtype, int64_t n_row, int width
   if (ctas < 1) ctas = 1;
   const int grid = static_cast<int>(ctas);
   if (dtype == CXG_F32)
-    column_sum_partial<float><<<grid, kCsThreads, 0, st>>>(static_cast<const float *>(x), part, n_row, width);
+    launch_dependent(column_sum_partial<float>, grid, kCsThreads, 0, st, static_cast<const float *>(x), part, n_row, width);
   else
-    column_sum_partial<__nv_bfloat16><<<grid, kCsThreads, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), part, n_row, width);
-  column_sum_final<<<(width + 31) / 32, kJoinThreads, 0, st>>>(part, out, grid, width);
+    launch_dependent(column_sum_partial<__nv_bfloat16>, grid, kCsThreads, 0, st, static_cast<const __nv_bfloat16 *>(x), part, n_row, width);
+  launch_dependent(column_sum_final, (width + 31) / 32, kJoinThreads, 0, st, part, out, grid, width);
   count_launches(2);
   return check_launch("cxg_column_sum");
 }

@@ -543,6 +543,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(kThreads) gat_scores_kernel(const float *feat, const float *att_src, const float *att_dst,
                                                               float *alpha_src, float *alpha_dst, int64_t n_src,
                                                               int64_t n_dst, int heads, int c) {
+  dependency_wait();
   const int64_t i = blockIdx.x * static_cast<int64_t>(kThreads) + threadIdx.x;
   if (i >= n_src * heads) return;
   const int h = static_cast<int>(i % heads);
@@ -578,6 +579,7 @@ __global__ void __launch_bounds__(kThreads, kScoreBlocks) gat_scores_vec(const f
                                                                          const float *att_dst, float *alpha_src,
                                                                          float *alpha_dst, int64_t n_src, int64_t n_dst,
                                                                          int heads, int c) {
+  dependency_wait();
   __shared__ float4 rows[kWarps][32 * (kScoreVecs + 1)];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int vecs = c / 4, step = heads * vecs;  // vectors of a node's head, of a node
@@ -669,11 +671,11 @@ extern "C" int cxg_gat_scores(const float *feat, const float *att_src, const flo
   if (c >= 32 && c % 4 == 0 && ((reinterpret_cast<uintptr_t>(att_src) | reinterpret_cast<uintptr_t>(att_dst)) % 16) == 0) {
     const int64_t blocks = ((n_src + 31) / 32 * heads + kWarps - 1) / kWarps;
     const unsigned grid = static_cast<unsigned>(blocks < kNumSM * kScoreBlocks ? blocks : kNumSM * kScoreBlocks);
-    gat_scores_vec<<<grid, kThreads, 0, as_stream(stream)>>>(feat, att_src, att_dst, alpha_src, alpha_dst, n_src, n_dst, heads, c);
+    launch_dependent(gat_scores_vec, grid, kThreads, 0, as_stream(stream), feat, att_src, att_dst, alpha_src, alpha_dst, n_src, n_dst, heads, c);
   } else {
     const unsigned grid = static_cast<unsigned>((n_src * heads + kThreads - 1) / kThreads);
     auto kernel = c % 4 == 0 ? gat_scores_kernel<true> : gat_scores_kernel<false>;
-    kernel<<<grid, kThreads, 0, as_stream(stream)>>>(feat, att_src, att_dst, alpha_src, alpha_dst, n_src, n_dst, heads, c);
+    launch_dependent(kernel, grid, kThreads, 0, as_stream(stream), feat, att_src, att_dst, alpha_src, alpha_dst, n_src, n_dst, heads, c);
   }
   count_launches(1);
   return check_launch("cxg_gat_scores");

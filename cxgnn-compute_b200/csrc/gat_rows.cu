@@ -34,6 +34,7 @@ template <int V>
 __global__ void __launch_bounds__(kRowThreads) scores_backward_add(const float *feat, const float *g_src, const float *g_dst,
                                                                    const float *att_src, const float *att_dst, float *dx,
                                                                    float *part, int64_t n_src, int64_t n_dst, int heads, int c) {
+  dependency_wait();
   __shared__ float sh[2][kRowThreads * V];
   const int width = heads * c, per_row = width / V;  // threads per row
   const int subs = per_row <= kRowThreads ? kRowThreads / per_row : 1;
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(kRowThreads) scores_backward_add(const float *
 constexpr int kJoinThreads = 1024;
 __global__ void __launch_bounds__(kJoinThreads) att_grad_join(const float *part, float *grad_src, float *grad_dst, int n_part,
                                                              int width) {
+  dependency_wait();
   __shared__ float sh[kJoinThreads / 32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane;  // of the 2 * width columns of a part
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(kJoinThreads) att_grad_join(const float *part,
 template <int V, typename I>  // I: 32-bit positions wherever they suffice, the divisions are half of the work
 __global__ void __launch_bounds__(kRowThreads, 6) head_mean_bias(const float *x, const float *bias, float *out, int64_t n, int heads,
                                                               int c) {
+  dependency_wait();
   const I per_row = c / V, total = static_cast<I>(n) * per_row, step = static_cast<I>(gridDim.x) * kRowThreads;
   constexpr int U = V == 4 ? 2 : 4;
   for (int64_t i0 = blockIdx.x * static_cast<int64_t>(kRowThreads) + threadIdx.x; i0 < total; i0 += U * static_cast<int64_t>(step)) {
@@ -169,6 +172,7 @@ __global__ void __launch_bounds__(kRowThreads, 6) head_mean_bias(const float *x,
 // the transformed features starts on a 16-byte boundary.
 __global__ void __launch_bounds__(kRowThreads) pad_heads(const float *w, const float *att_src, const float *att_dst, float *wp,
                                                          float *src_p, float *dst_p, int heads, int c, int cp, int k) {
+  dependency_wait();
   const int i = blockIdx.x * kRowThreads + threadIdx.x, rows = heads * cp;
   if (i >= rows * (k + 2)) return;
   const int row = i < rows * k ? i / k : (i - rows * k) % rows, at = row % cp, from = row / cp * c + at;
@@ -185,6 +189,7 @@ __global__ void __launch_bounds__(kRowThreads) pad_heads(const float *w, const f
 template <bool JOIN>
 __global__ void __launch_bounds__(kRowThreads) unpad_heads(const float *x, const float *bias, float *out, int64_t n, int heads, int c,
                                                            int cp) {
+  dependency_wait();
   const int vecs = cp / 4, per_row = JOIN ? heads * vecs : vecs;
   const int64_t total = n * per_row, step = static_cast<int64_t>(gridDim.x) * kRowThreads;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(kRowThreads) + threadIdx.x; i < total; i += step) {
@@ -241,10 +246,10 @@ extern "C" int cxg_gat_scores_backward_add(const float *feat, const float *g_src
   if (ctas < 1) ctas = 1;
   const unsigned grid = static_cast<unsigned>(ctas);
   if (vectors(c, feat, dx, workspace) && vectors(c, att_src, att_dst, nullptr))
-    scores_backward_add<4><<<grid, kRowThreads, 0, st>>>(feat, g_src, g_dst, att_src, att_dst, dx, part, n_src, n_dst, heads, c);
+    launch_dependent(scores_backward_add<4>, grid, kRowThreads, 0, st, feat, g_src, g_dst, att_src, att_dst, dx, part, n_src, n_dst, heads, c);
   else
-    scores_backward_add<1><<<grid, kRowThreads, 0, st>>>(feat, g_src, g_dst, att_src, att_dst, dx, part, n_src, n_dst, heads, c);
-  att_grad_join<<<(2 * width + 31) / 32, kJoinThreads, 0, st>>>(part, grad_att_src, grad_att_dst, static_cast<int>(grid), width);
+    launch_dependent(scores_backward_add<1>, grid, kRowThreads, 0, st, feat, g_src, g_dst, att_src, att_dst, dx, part, n_src, n_dst, heads, c);
+  launch_dependent(att_grad_join, (2 * width + 31) / 32, kJoinThreads, 0, st, part, grad_att_src, grad_att_dst, static_cast<int>(grid), width);
   count_launches(2);
   return check_launch("cxg_gat_scores_backward_add");
 }
@@ -259,13 +264,13 @@ extern "C" int cxg_head_mean_bias(const float *x, const float *bias, float *out,
   const bool narrow = n * c < (1ll << 30);
   cudaStream_t st = as_stream(stream);
   if (v4 && narrow)
-    head_mean_bias<4, int32_t><<<grid, kRowThreads, 0, st>>>(x, bias, out, n, heads, c);
+    launch_dependent(head_mean_bias<4, int32_t>, grid, kRowThreads, 0, st, x, bias, out, n, heads, c);
   else if (v4)
-    head_mean_bias<4, int64_t><<<grid, kRowThreads, 0, st>>>(x, bias, out, n, heads, c);
+    launch_dependent(head_mean_bias<4, int64_t>, grid, kRowThreads, 0, st, x, bias, out, n, heads, c);
   else if (narrow)
-    head_mean_bias<1, int32_t><<<grid, kRowThreads, 0, st>>>(x, bias, out, n, heads, c);
+    launch_dependent(head_mean_bias<1, int32_t>, grid, kRowThreads, 0, st, x, bias, out, n, heads, c);
   else
-    head_mean_bias<1, int64_t><<<grid, kRowThreads, 0, st>>>(x, bias, out, n, heads, c);
+    launch_dependent(head_mean_bias<1, int64_t>, grid, kRowThreads, 0, st, x, bias, out, n, heads, c);
   count_launches(1);
   return check_launch("cxg_head_mean_bias");
 }
@@ -276,8 +281,8 @@ extern "C" int cxg_gat_pad_heads(const float *w, const float *att_src, const flo
               CXG_EINVAL, "cxg_gat_pad_heads: bad sizes");
   CXG_REQUIRE(w && att_src && att_dst && w_padded && att_src_padded && att_dst_padded, CXG_ENULL, "cxg_gat_pad_heads: NULL argument");
   const int total = heads * c_padded * (k + 2);
-  pad_heads<<<(total + kRowThreads - 1) / kRowThreads, kRowThreads, 0, as_stream(stream)>>>(
-      w, att_src, att_dst, w_padded, att_src_padded, att_dst_padded, heads, c, c_padded, k);
+  launch_dependent(pad_heads, (total + kRowThreads - 1) / kRowThreads, kRowThreads, 0, as_stream(stream), w, att_src, att_dst, w_padded,
+                   att_src_padded, att_dst_padded, heads, c, c_padded, k);
   count_launches(1);
   return check_launch("cxg_gat_pad_heads");
 }
@@ -290,7 +295,7 @@ extern "C" int cxg_gat_unpad_heads(const float *x, const float *bias, float *out
   CXG_REQUIRE(reinterpret_cast<uintptr_t>(x) % 16 == 0, CXG_EINVAL, "cxg_gat_unpad_heads: x must be 16-byte aligned");
   const int64_t blocks = (n * (join ? heads : 1) * (c_padded / 4) + kRowThreads - 1) / kRowThreads;
   const unsigned grid = static_cast<unsigned>(blocks < kNumSM * 64 ? blocks : kNumSM * 64);
-  (join ? unpad_heads<true> : unpad_heads<false>)<<<grid, kRowThreads, 0, as_stream(stream)>>>(x, bias, out, n, heads, c, c_padded);
+  launch_dependent(join ? unpad_heads<true> : unpad_heads<false>, grid, kRowThreads, 0, as_stream(stream), x, bias, out, n, heads, c, c_padded);
   count_launches(1);
   return check_launch("cxg_gat_unpad_heads");
 }

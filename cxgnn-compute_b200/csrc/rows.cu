@@ -15,6 +15,7 @@ constexpr int kThreads = 256;
 template <typename V>
 __global__ void __launch_bounds__(kThreads) gather_rows_kernel(const V *in, const int64_t *rows, V *out, int64_t n_rows,
                                                                int vecs_per_row, int group) {
+  dependency_wait();
   const int lane = threadIdx.x % group;
   const int64_t groups = static_cast<int64_t>(gridDim.x) * (kThreads / group);
   for (int64_t i = blockIdx.x * static_cast<int64_t>(kThreads / group) + threadIdx.x / group; i < n_rows; i += groups) {
@@ -67,7 +68,7 @@ void launch(const void *in, const int64_t *rows, void *out, int64_t n_rows, int6
   while (group < vecs && group < 32) group <<= 1;
   const int64_t want = (n_rows + kThreads / group - 1) / (kThreads / group);
   const unsigned grid = static_cast<unsigned>(want < kNumSM * 16 ? want : kNumSM * 16);
-  gather_rows_kernel<V><<<grid, kThreads, 0, st>>>(static_cast<const V *>(in), rows, static_cast<V *>(out), n_rows, vecs,
+  launch_dependent(gather_rows_kernel<V>, grid, kThreads, 0, st, static_cast<const V *>(in), rows, static_cast<V *>(out), n_rows, vecs,
                                                    group);
 }
 

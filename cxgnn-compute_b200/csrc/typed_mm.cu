@@ -120,6 +120,7 @@ __device__ __forceinline__ float to_tf32(float v) {
 // W [R][K][N] -> Wt [R][N][K]; with `wt_lo` (fp32 only) the two TF32 terms hi = tf32(w), lo = tf32(w - hi).
 template <typename T>
 __global__ void transpose_w(const T *w, T *wt, T *wt_lo, int num_rel, int k, int n) {
+  dependency_wait();
   const int64_t total = static_cast<int64_t>(num_rel) * k * n;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + PW + (X3 ? kConvWarps : 
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  dependency_wait();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -743,11 +745,11 @@ extern "C" int cxg_typed_matmul(const void *a, const void *w, void *c, const int
   cudaError_t e = cudaSuccess;
   auto launch = [&](auto kernel, int warps) {
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e == cudaSuccess) kernel<<<static_cast<unsigned>(grid), 32 * warps, smem, st>>>(t, tmap);
+    if (e == cudaSuccess) launch_dependent(kernel, static_cast<unsigned>(grid), 32 * warps, smem, st, t, tmap);
   };
   if (dtype == CXG_F32) {
     float *wt_f = static_cast<float *>(wt);
-    transpose_w<float><<<kNumSM, 256, 0, st>>>(static_cast<const float *>(w), wt_f,
+    launch_dependent(transpose_w<float>, kNumSM, 256, 0, st, static_cast<const float *>(w), wt_f,
                                                x3 ? wt_f + static_cast<size_t>(num_rel) * k * ncols : nullptr, num_rel, k,
                                                ncols);
     constexpr int kW = kEpiWarps + 1 + 8;
@@ -767,7 +769,7 @@ extern "C" int cxg_typed_matmul(const void *a, const void *w, void *c, const int
         launch(typed_mm_tc<float, false, 8, false, false>, kW + kEpiWarps);
     }
   } else {
-    transpose_w<__nv_bfloat16><<<kNumSM, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(w),
+    launch_dependent(transpose_w<__nv_bfloat16>, kNumSM, 256, 0, st, static_cast<const __nv_bfloat16 *>(w),
                                                        static_cast<__nv_bfloat16 *>(wt), nullptr, num_rel, k, ncols);
     constexpr int kW = kEpiWarps + 1 + 4;
     if (tma)

@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  dependency_wait();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -455,6 +456,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 1 + kProdWarps + (X3 ? kConv
 constexpr int kRedThreads = 128, kRedPer = 8, kRedChunk = kRedThreads * kRedPer;
 __global__ void __launch_bounds__(kRedThreads) wgrad_reduce(const float *partial, const int32_t *slot_rel, float *dw,
                                                             int n_slots, int num_rel, int k, int n) {
+  dependency_wait();
   __shared__ int list[kRedChunk];
   const int64_t kn = static_cast<int64_t>(k) * n;
   __shared__ int warp_sum[kRedThreads / 32];
@@ -505,6 +507,7 @@ __global__ void __launch_bounds__(kRedThreads) wgrad_reduce(const float *partial
 }
 
 __global__ void wgrad_clear(int32_t *slot_rel, int n) {
+  dependency_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) slot_rel[i] = -1;
 }
@@ -514,6 +517,7 @@ __global__ void wgrad_clear(int32_t *slot_rel, int n) {
 // infinity, so an element that is not finite is summed again from x and g.
 __global__ void __launch_bounds__(128) dense_reduce(const float *partial, const float *x, const float *g, int64_t m, float *dw,
                                                     int k, int n, int k_blocks, int parts) {
+  dependency_wait();
   const int64_t i = blockIdx.x * 128ll + threadIdx.x;
   if (i >= static_cast<int64_t>(k) * n) return;
   // neighbouring threads in the order of the partials: four columns, then the rows
@@ -637,13 +641,13 @@ extern "C" int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel,
   a.wait_cycles = wait_limit_cycles();
   if (cudaMemsetAsync(a.status, 0, 256, st) != cudaSuccess) return check_launch("cxg_typed_wgrad: memset");
   const int n_slots = L.grid * L.slots;
-  wgrad_clear<<<(n_slots + 255) / 256, 256, 0, st>>>(a.slot_rel, n_slots);
+  launch_dependent(wgrad_clear, (n_slots + 255) / 256, 256, 0, st, a.slot_rel, n_slots);
   const int64_t n_tiles = (m + pos - 1) / pos;  // a last partial tile holds positions past the padded buckets
   const unsigned grid = static_cast<unsigned>(n_tiles < L.grid ? n_tiles : L.grid);
   cudaError_t e = cudaSuccess;
   auto launch = [&](auto kernel, int warps) {
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e == cudaSuccess) kernel<<<grid, 32 * warps, smem, st>>>(a);
+    if (e == cudaSuccess) launch_dependent(kernel, grid, 32 * warps, smem, st, a);
   };
   constexpr int kW = kEpiWarps + 1 + kProdWarps;
   if (dtype == CXG_F32) {
@@ -656,7 +660,7 @@ extern "C" int cxg_typed_wgrad(const void *x, const void *g, const int64_t *rel,
   }
   if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_typed_wgrad: %s", cudaGetErrorString(e));
   dim3 rg(static_cast<unsigned>((kn + kRedThreads - 1) / kRedThreads), static_cast<unsigned>(num_rel));
-  wgrad_reduce<<<rg, kRedThreads, 0, st>>>(a.partial, a.slot_rel, dw, n_slots, num_rel, k, n);
+  launch_dependent(wgrad_reduce, rg, kRedThreads, 0, st, a.partial, a.slot_rel, dw, n_slots, num_rel, k, n);
   count_launches(3);
   return check_launch("cxg_typed_wgrad");
 }
@@ -710,8 +714,8 @@ extern "C" int cxg_dense_wgrad_f32_ex(const float *x, const float *g, int64_t m,
   if (e != cudaSuccess) return set_error(CXG_ECUDA, "cxg_dense_wgrad_f32: %s", cudaGetErrorString(e));
   const int parts = dense_parts(k, n, m);
   const dim3 grid(static_cast<unsigned>(parts), static_cast<unsigned>(k_blocks * n_blocks));
-  typed_wgrad_tc<float, true><<<grid, 32 * (kEpiWarps + 1 + kProdWarps + kConvWarps), smem, st>>>(a);
-  dense_reduce<<<static_cast<unsigned>((static_cast<int64_t>(k) * n + 127) / 128), 128, 0, st>>>(a.partial, x, g, m, dw, k, n,
+  launch_dependent(typed_wgrad_tc<float, true>, grid, 32 * (kEpiWarps + 1 + kProdWarps + kConvWarps), smem, st, a);
+  launch_dependent(dense_reduce, static_cast<unsigned>((static_cast<int64_t>(k) * n + 127) / 128), 128, 0, st, a.partial, x, g, m, dw, k, n,
                                                                                             k_blocks, parts);
   count_launches(2);
   return check_launch("cxg_dense_wgrad_f32");
