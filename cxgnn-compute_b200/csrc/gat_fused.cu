@@ -1339,7 +1339,7 @@ int gat_layout(int64_t n_stats_rows, int64_t nnz, int heads, int c, GatLayout *L
   L->piece_sums = off;
   off = align_up(off + static_cast<size_t>(nnz / kPieceEdges + 1) * 2 * heads * sizeof(float), 256);
   L->d_edge = off;
-  off = align_up(off + static_cast<size_t>(nnz) * heads * sizeof(float) + kWalkSlack, 256);
+  off = align_up(off + static_cast<size_t>(nnz) * heads * sizeof(float) + walk_weights_slack(heads), 256);
   L->total = off;
   return CXG_OK;
 }
@@ -1382,26 +1382,38 @@ void fill_args(GatArgs &a, const GatLayout &L, void *workspace, int64_t nnz, int
   a.slope = slope;
 }
 
-// Lane layouts by bytes per vector and vectors per row; the last number is the resident CTAs per SM that the registers of
-// that many edges in flight allow.
+// Rows of whole 16-byte vectors whose heads are not (class counts), from 65 values on: vectors that lie across two heads,
+// in place of single values (16 heads of 15: 957 us, now 522; 4 of 17: 404, now 314; 4 of 47: 519, now 495) and of
+// 8-byte ones from 16 values per head on (4 of 30: 357, now 327; 8 of 10 would take 376 instead of 344).
+bool across_heads(const GatArgs &a, int vb) {
+  return vb < 16 && (vb == 4 || a.c >= 16) && a.w.width % 4 == 0 && a.w.width > 64 && a.c >= 4 &&
+         (reinterpret_cast<uintptr_t>(a.w.x) | reinterpret_cast<uintptr_t>(a.w.y)) % 16 == 0;
+}
+
 // Whether the forward goes by way of weights. Its second step is the SpMM's walk, which counts in 32 bits. It has a launch more
 // than the single walk, which keeps rows of up to 32 16-byte vectors of small graphs (430,000 edges: 4 heads of 8 38 us in one
 // step, 42 in two; 8 of 8 41 / 47; 4 of 32 51 / 47; 2.3 M edges: 99 / 98, 150 / 128, 198 / 157). Wider rows and other vectors
 // gain everywhere: 27,000 edges 4 of 64 44 / 36, 2 of 33 47 / 35; 2.3 M 4 of 64 391 / 246, 1 of 47 301 / 115, 2 of 50 323 / 249.
 bool by_weights(const GatArgs &a, int vb) {
   const bool one_step = vb == 16 && a.w.width <= 128 && a.w.nnz * a.w.row_bytes < (128 << 20);
-  return !one_step && a.heads <= 8 && reinterpret_cast<uintptr_t>(a.g_small) % 16 == 0 && a.w.n_dst < INT32_MAX - (1 << 20) &&
+  return !one_step && !across_heads(a, vb) && a.heads <= 8 && reinterpret_cast<uintptr_t>(a.g_small) % 16 == 0 && a.w.n_dst < INT32_MAX - (1 << 20) &&
          a.w.nnz < INT32_MAX - (1 << 20) && a.w.width * 4 <= (vb == 16 ? 128 * 16 : 256 * vb);
 }
 
-cudaError_t launch_by_weights(GatArgs &a, int vb, cudaStream_t st) {
+// Edges per tile of that form, 0: no lane layout for its rows.
+int weighted_tile(const GatArgs &a, int vb) {
   int resident = 0;
+  if (!walk_weighted(a.w, vb, nullptr, &resident)) return 0;
+  const int tile = walk_whole_waves(a.w.nnz, resident, 16);
+  return tile < kWeightedTile ? tile : kWeightedTile;
+}
+
+cudaError_t launch_by_weights(GatArgs &a, int vb, cudaStream_t st) {
   a.w.wide_tiles = 0;
   a.w.edge_val = a.weights;
   a.w.part_stride = a.w.width;
-  if (!walk_weighted(a.w, vb, st, &resident)) return cudaErrorInvalidValue;
-  const int tile = walk_whole_waves(a.w.nnz, resident, 16);
-  a.w.tile = tile < 256 ? tile : 256;
+  a.w.tile = weighted_tile(a, vb);
+  if (a.w.tile == 0) return cudaErrorInvalidValue;
   a.w.max_tiles = (a.w.nnz + a.w.tile - 1) / a.w.tile + 1;
   walk_plan_run(a.w, st);
   constexpr int warps = kThreads / 32;
@@ -1419,6 +1431,8 @@ cudaError_t launch_by_weights(GatArgs &a, int vb, cudaStream_t st) {
   return walk_weighted(a.w, vb, st, nullptr) ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// Lane layouts by bytes per vector and vectors per row; the last number is the resident CTAs per SM that the registers of
+// that many edges in flight allow.
 template <bool BWD>
 cudaError_t launch_walk(GatArgs &a, cudaStream_t st) {
   const int vb = vector_of(a.heads, a.c), n = a.w.row_bytes / vb;
@@ -1452,12 +1466,8 @@ cudaError_t launch_walk(GatArgs &a, cudaStream_t st) {
     CXG_GAT_BWD(4, 2, 2, 3)
     return cudaErrorInvalidValue;
   } else {
-    // Rows of whole 16-byte vectors whose heads are not (class counts), from 65 values on: vectors that lie across two heads,
-    // in place of single values (16 heads of 15: 957 us, now 522; 4 of 17: 404, now 314; 4 of 47: 519, now 495) and of
-    // 8-byte ones from 16 values per head on (4 of 30: 357, now 327; 8 of 10 would take 376 instead of 344).
-    const bool across = vb < 16 && (vb == 4 || a.c >= 16) && a.w.width % 4 == 0 && a.w.width > 64 && a.c >= 4 &&
-                        (reinterpret_cast<uintptr_t>(a.w.x) | reinterpret_cast<uintptr_t>(a.w.y)) % 16 == 0;
-    if (!across && by_weights(a, vb)) err = launch_by_weights(a, vb, st); else
+    const bool across = across_heads(a, vb);
+    if (by_weights(a, vb)) err = launch_by_weights(a, vb, st); else
 #define CXG_GAT_ACROSS(NV, U, P, CTAS) \
   if (across && a.w.width <= 128 * NV && U * a.heads <= 32 * P) go(gat_wide_forward<16, NV, U, P, CTAS, true>, 32, CTAS); else
     CXG_GAT_ACROSS(1, 8, 1, 6)
@@ -1517,6 +1527,23 @@ extern "C" int cxg_gat_fused_workspace_size(int64_t n_dst, int64_t nnz, int head
   const int rc = gat_layout(n_dst, nnz, heads, c, &L);
   CXG_REQUIRE(rc == CXG_OK, rc, "cxg_gat_fused_workspace_size: graph too large for 32-bit tile ids");
   *bytes = L.total;
+  return CXG_OK;
+}
+
+extern "C" int cxg_gat_fused_weights_room(int64_t n_dst, int64_t nnz, int heads, int c, int *tile, size_t *bytes) {
+  CXG_REQUIRE(tile != nullptr && bytes != nullptr, CXG_ENULL, "cxg_gat_fused_weights_room: NULL argument");
+  CXG_REQUIRE(n_dst >= 0 && nnz >= 0, CXG_EINVAL, "cxg_gat_fused_weights_room: negative size");
+  int rc = check_shape("cxg_gat_fused_weights_room", heads, c, false);
+  if (rc != CXG_OK) return rc;
+  GatLayout L;
+  rc = gat_layout(n_dst, nnz, heads, c, &L);
+  CXG_REQUIRE(rc == CXG_OK, rc, "cxg_gat_fused_weights_room: graph too large for 32-bit tile ids");
+  GatArgs a = {};
+  a.w.n_dst = n_dst, a.w.nnz = nnz;
+  a.w.width = heads * c, a.w.row_bytes = heads * c * 4, a.w.heads = a.heads = heads, a.w.feat = a.c = c;
+  const int vb = vector_of(heads, c);
+  *tile = by_weights(a, vb) ? weighted_tile(a, vb) : 0;
+  *bytes = L.total - L.d_edge;
   return CXG_OK;
 }
 

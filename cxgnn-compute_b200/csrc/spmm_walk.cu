@@ -399,6 +399,7 @@ int walk_tile_of_waves(int64_t nnz, int64_t resident) {
 }
 
 bool walk_weighted(const WalkArgs &a, int vb, cudaStream_t st, int *resident_tiles) {
+  if (resident_tiles == nullptr && a.tile > kWeightedTile) return false;
   const int valmode = a.heads == 1 ? 1 : vb != 16 || a.heads > 8 ? 2 : a.heads == 2 ? 5 : a.heads == 4 ? 6 : 7;
   return vb == 16  ? walk_launch_f32_16(a, valmode, false, st, resident_tiles)
          : vb == 8 ? walk_launch_f32_8(a, valmode, false, st, resident_tiles)

@@ -65,8 +65,13 @@ bool walk_eligible(const cxg_spmm_desc *d);
 // The plan kernel for a.ptr, a.tile, a.whole_rows: fills hdr, tiles, count (and sets a.tile_magic).
 void walk_plan_run(WalkArgs &a, cudaStream_t st);
 // The walk alone over the plan and the weights per (edge, head) in `a` (fp32 rows in vectors of vb bytes, heads a power of two),
-// behind which kWalkSlack bytes can be read. With resident_tiles set it only tells how many tiles are walked at the same time.
-constexpr size_t kWalkSlack = 256;  // 8 edges of 8 heads
+// behind which walk_weights_slack bytes can be read. With resident_tiles set it only tells how many tiles are walked at the
+// same time. False, too, for tiles of more than kWeightedTile edges.
+constexpr int kWeightedTile = 256;   // most edges of a tile of that walk
+constexpr int kWalkInFlight = 8;     // most edges that a lane has in flight
+// The lane groups of a warp step together until the longest of their tiles ends, and read weights at every step: a last tile
+// of one edge beside a full one is read on to where it would end if it were full, in whole steps.
+constexpr size_t walk_weights_slack(int heads) { return static_cast<size_t>(kWeightedTile + kWalkInFlight) * heads * sizeof(float); }
 bool walk_weighted(const WalkArgs &a, int vb, cudaStream_t st, int *resident_tiles);
 // Edges per tile for that many.
 int walk_tile_of_waves(int64_t nnz, int64_t resident);

@@ -229,7 +229,8 @@ __device__ __forceinline__ void add_words(float *f, const Words<(VB + 3) / 4> &r
 
 // VB: bytes per load of a lane; NV loads per row, G lanes per tile, U edges in flight per lane. VALMODE: 0 no
 // edge values, 1 one per edge, 2 one per (edge, head), 3 none and the mean of the row, 4 none and the sum (or the mean) is
-// added to the output, 5 to 7 as 2 with 2, 4 or 8 heads and values that may be read U edges beyond the last one.
+// added to the output, 5 to 7 as 2 with 2, 4 or 8 heads and walk_weights_slack bytes behind the values: what lies behind a
+// tile's end is read unasked and goes into sums that nobody reads.
 // COPY: the rows of x are copies in whole vectors (walk_plan), those of y are not: a lane stores the values of its vector
 // that lie inside the row one by one.
 template <typename T, int VB, int G, int NV, int U, int VALMODE, int MINB, bool COPY>
@@ -238,6 +239,7 @@ __global__ void __launch_bounds__(kThreads, MINB) spmm_walk(const __grid_constan
   constexpr int W = (VB + 3) / 4;
   constexpr int EL = A::EL;
   constexpr int NG = 32 / G;
+  static_assert(U <= kWalkInFlight, "walk_weights_slack covers a step");
   const int lane = threadIdx.x & 31;
   const int lg = lane & (G - 1);
   dependency_wait();

@@ -308,6 +308,9 @@ int cxg_edge_softmax_backward(const void *ptr, const void *idx, int ptr_bytes,
  * for bit (the running maximum changes the order of the roundings).
  */
 int cxg_gat_fused_workspace_size(int64_t n_dst, int64_t nnz, int heads, int c, size_t *bytes);
+/* For tests: edges per tile where the forward goes by way of weights (0: in one step), and the bytes of the workspace from the
+ * first weight on, of which the walk may read those of a last tile as if it were full. */
+int cxg_gat_fused_weights_room(int64_t n_dst, int64_t nnz, int heads, int c, int *tile, size_t *bytes);
 int cxg_gat_fused_forward(const void *ptr, const void *idx, int ptr_bytes, int idx_bytes, const float *x,
                           const float *a_src, const float *a_dst, float *y, float *row_max, float *row_sum,
                           int64_t n_dst, int64_t nnz, int heads, int c, float slope, void *workspace,

@@ -63,3 +63,28 @@ def test_no_edges(cuda):
     ptr, idx = torch.zeros(101, dtype=torch.int64).cuda(), torch.empty(0, dtype=torch.int64).cuda()
     y, _, total = be.gat_fused(randn((50, 4, 64), 1).cuda(), randn((50, 4), 2).cuda(), randn((100, 4), 3).cuda(), ptr, idx, 100, 0.2)
     assert bool((y == 0).all()) and bool((total == 0).all())
+
+
+@pytest.mark.parametrize("heads,c", [(2, 16), (2, 32), (4, 8), (4, 16), (8, 4), (8, 8), (8, 12)])
+def test_last_tile_of_one_edge(cuda, heads, c):
+    """The fewest edges from which these widths go by weights, 8 and 16 lanes per tile, and one more than whole tiles."""
+    import ctypes
+    import cxgnncomp_backend as be
+    room = be._lib.cxg_gat_fused_weights_room
+    room.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_size_t)]
+    tile, size = ctypes.c_int(0), ctypes.c_size_t(0)
+    n_src, edges = 5000, (128 << 20) // (heads * c * 4) + 1
+    assert room(1, edges, heads, c, ctypes.byref(tile), ctypes.byref(size)) == 0 and tile.value > 0
+    edges += -(edges - 1) % tile.value
+    deg = torch.randint(0, 60, (edges // 30 + 2000,), generator=torch.Generator().manual_seed(c))
+    ptr = torch.zeros(deg.numel() + 1, dtype=torch.int64)
+    ptr[1:] = torch.cumsum(deg, 0).clamp(max=edges)
+    assert int(ptr[-1]) == edges and edges % tile.value == 1
+    idx = torch.randint(0, n_src, (edges,), generator=torch.Generator().manual_seed(heads))
+    n = deg.numel()
+    x, a_s, a_d = randn((n_src, heads, c), 1), randn((n_src, heads), 2), randn((n, heads), 3)
+    p = oracle.torch_edge_softmax_opwise(ptr.cuda(), idx.cuda(), a_s.double().cuda(), a_d.double().cuda(), edges, 0.2)
+    want = oracle.torch_spmm_index_add(x.double().cuda(), ptr.cuda(), idx.cuda(), n, edge_val=p)
+    with torch.no_grad():
+        y = be.gat_fused(x.cuda(), a_s.cuda(), a_d.cuda(), ptr.cuda(), idx.cuda(), n, 0.2)[0]
+    assert rel_err(y, want) < 1e-5
