@@ -330,8 +330,36 @@ Transposed transpose(const Tensor &ptr, const Tensor &idx, int64_t num_node, int
   return t;
 }
 
+// The capture that records what the stream is given, or none.
+optional<unsigned long long> capture_of(const c10::cuda::CUDAStream &stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream.stream(), &status, &id));
+  if (status == cudaStreamCaptureStatusNone) return c10::nullopt;
+  return id;
+}
+
+// The stream that has built something for keeping, and an event behind that.
+struct Built {
+  c10::Stream stream;
+  std::shared_ptr<c10::Event> event;
+  explicit Built(c10::Stream s) : stream(s), event(std::make_shared<c10::Event>(c10::DeviceType::CUDA)) { event->record(s); }
+  // Another stream waits for the build, and the memory for that stream. A stream under capture cannot wait for what lies in
+  // front of the capture (`outside`): the host does.
+  void hand_to(const c10::Stream &other, bool outside, std::initializer_list<Tensor> tensors) const {
+    if (other == stream) return;
+    if (outside) {
+      c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+      event->synchronize();
+    } else {
+      event->block(other);
+    }
+    for (const Tensor &t : tensors) t.record_stream(other);
+  }
+};
+
 // The last eight transposed graphs, by the tensors they came from. An entry keeps ptr and idx alive, so their addresses
-// cannot be handed to another graph.
+// cannot be handed to another graph. What a graph capture has recorded is there for that capture alone.
 struct CachedGraph {
   const void *ptr_data, *idx_data;
   int64_t n, n_src;
@@ -339,11 +367,11 @@ struct CachedGraph {
   int device;
   Tensor ptr, idx;
   Transposed t;
-  // 1 / in-degree of every transposed edge's destination, when a mean's gradient has asked for it, with the stream it was
-  // made on and an event behind that
+  Built built;
+  optional<unsigned long long> capture;
+  // 1 / in-degree of every transposed edge's destination, when a mean's gradient has asked for it
   Tensor weight;
-  c10::optional<c10::Stream> weight_stream;
-  std::shared_ptr<c10::Event> weight_made;
+  optional<Built> weight_built;
 };
 std::mutex graphs_lock;
 std::list<CachedGraph> &graphs = *new std::list<CachedGraph>;  // not torn down at exit: events would outlive the driver
@@ -351,16 +379,20 @@ constexpr size_t kMostGraphs = 8;
 
 Transposed transposed_graph(const Tensor &ptr, const Tensor &idx, int64_t n, int64_t n_src) {
   const uint32_t pv = ptr._version(), iv = idx._version();
+  const auto stream = c10::cuda::getCurrentCUDAStream(ptr.device().index());
+  const auto capture = capture_of(stream);
   {
     std::lock_guard<std::mutex> hold(graphs_lock);
     for (const auto &g : graphs)
       if (g.ptr_data == ptr.data_ptr() && g.idx_data == idx.data_ptr() && g.n == n && g.n_src == n_src && g.ptr_version == pv &&
-          g.idx_version == iv && g.device == ptr.device().index())
+          g.idx_version == iv && g.device == ptr.device().index() && (!g.capture || g.capture == capture)) {
+        g.built.hand_to(stream, capture.has_value() && !g.capture, {g.t.t_ptr, g.t.t_idx, g.t.t_eid, g.t.inv_deg});
         return g.t;
+      }
   }
-  CachedGraph g{ptr.data_ptr(), idx.data_ptr(), n, n_src, pv, iv, ptr.device().index(), ptr, idx, transpose(ptr, idx, n, n_src, true),
-                Tensor(), c10::nullopt, nullptr};
-  Transposed t = g.t;
+  const Transposed t = transpose(ptr, idx, n, n_src, true);
+  CachedGraph g{ptr.data_ptr(), idx.data_ptr(), n, n_src, pv, iv, ptr.device().index(), ptr, idx, t, Built(stream), capture,
+                Tensor(), c10::nullopt};
   std::lock_guard<std::mutex> hold(graphs_lock);
   while (graphs.size() >= kMostGraphs) graphs.pop_front();
   graphs.push_back(std::move(g));
@@ -384,20 +416,16 @@ Tensor mean_weights(const Transposed &t) {
           "cxg_gather_edges");
     return w;
   };
-  // what a graph capture records is not there for others
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return make();
-  const c10::Stream stream = c10::cuda::getCurrentCUDAStream(t.t_idx.device().index()).unwrap();
+  const auto stream = c10::cuda::getCurrentCUDAStream(t.t_idx.device().index());
+  if (capture_of(stream)) return make();  // what a graph capture records is not there for others
   std::lock_guard<std::mutex> hold(graphs_lock);
   for (auto &g : graphs)
     if (g.t.t_idx.is_same(t.t_idx)) {
       if (!g.weight.defined()) {
         g.weight = make();
-        g.weight_stream = stream;
-        g.weight_made = std::make_shared<c10::Event>(c10::DeviceType::CUDA);
-        g.weight_made->record(stream);
-      } else if (*g.weight_stream != stream) {
-        g.weight_made->block(stream);
-        g.weight.record_stream(stream);
+        g.weight_built.emplace(stream);
+      } else {
+        g.weight_built->hand_to(stream, false, {g.weight});
       }
       return g.weight;
     }

@@ -159,6 +159,35 @@ def _workspace(device, nbytes, kind=""):
     return _native.Workspace(_dev_index(device), nbytes, kind)
 
 
+class _Kept:
+    """Tensors that the current stream has built and a cache keeps."""
+    __slots__ = ("tensors", "stream", "event")
+
+    def __init__(self, *tensors):
+        self.tensors = tensors
+        with _on(tensors[0].device):
+            self.stream = torch.cuda.current_stream()
+            self.event = self.stream.record_event()
+
+    def take(self):
+        """The tensors for the current stream. Where that is another one, it waits for the build and the memory for it. (A
+        stream under capture cannot wait for what was issued in front of the capture; torch.cuda.graph waits for the device
+        before it begins one.)"""
+        dev = self.tensors[0].device
+        if _raw_stream(_dev_index(dev)) != self.stream.cuda_stream and _can_keep():
+            with _on(dev):
+                stream = torch.cuda.current_stream()
+                stream.wait_event(self.event)
+                for t in self.tensors:
+                    t.record_stream(stream)
+        return self.tensors
+
+
+def _can_keep():
+    """Not while a graph capture records the work: its results are there when the graph has run, not before."""
+    return not torch.cuda.is_current_stream_capturing()
+
+
 def _dtype_code(t):
     return CXG_F32 if t.dtype == torch.float32 else CXG_BF16
 
@@ -783,7 +812,7 @@ def target_aggr_backward(grad_in, ptr, idx, targets, grad_out, num_node):
     _spmm_backward(grad_in, None, ptr, idx, num_node, grad_x=grad_out, targets=targets, x_shape=grad_out.shape)
 
 
-_cidx_cache = []  # (idx, etype, versions, stride, combined), most recent last
+_cidx_cache = []  # (idx, etype, versions, stride, kept), most recent last
 
 
 def _combined_index(idx, etype, stride, num_rel):
@@ -793,14 +822,15 @@ def _combined_index(idx, etype, stride, num_rel):
     ver = (idx._version, etype._version)
     for it in _cidx_cache:
         if it[0] is idx and it[1] is etype and it[2] == ver and it[3] == stride:
-            return it[4]
+            return it[4].take()[0]
     n = min(idx.shape[0], etype.shape[0])
     c = etype[:n].to(torch.int64) * stride + idx[:n].to(torch.int64)
     if stride * num_rel < 2 ** 31:
         c = c.to(torch.int32)
-    _cidx_cache.append((idx, etype, ver, stride, c))
-    if len(_cidx_cache) > 8:
-        _cidx_cache.pop(0)
+    if _can_keep():
+        _cidx_cache.append((idx, etype, ver, stride, _Kept(c)))
+        if len(_cidx_cache) > 8:
+            _cidx_cache.pop(0)
     return c
 
 
@@ -822,7 +852,7 @@ class RelationPairs:
         return self.rel, self.src, self.pos, self.src_ptr, self.src_idx, self.idx
 
 
-_pair_cache = {}  # key -> (RelationPairs, idx, etype, stream it was built on, event behind the build, bytes)
+_pair_cache = {}  # key -> (RelationPairs, idx, etype, kept, bytes)
 _PAIR_CACHE_BYTES = 1 << 30
 
 
@@ -835,19 +865,13 @@ def relation_pairs(idx, etype, num_src, num_rel):
     hit = _pair_cache.get(key)
     if hit is None:
         pairs = RelationPairs(idx, etype, num_src, num_rel)
-        with _on(idx.device):
-            stream = torch.cuda.current_stream()
-            size = sum(t.numel() * t.element_size() for t in (*pairs.tensors(), idx, etype))
-            kept = list(_pair_cache.items())
-            while kept and (len(kept) >= 8 or size + sum(e[5] for _, e in kept) > _PAIR_CACHE_BYTES):
-                _pair_cache.pop(kept.pop(0)[0], None)
-            hit = _pair_cache[key] = (pairs, idx, etype, stream, stream.record_event(), size)
-    elif _raw_stream(_dev_index(idx.device)) != hit[3].cuda_stream and not torch.cuda.is_current_stream_capturing():
-        with _on(idx.device):  # built on another stream: this one waits for it, and the memory for this one
-            stream = torch.cuda.current_stream()
-            stream.wait_event(hit[4])
-            for t in hit[0].tensors():
-                t.record_stream(stream)
+        size = sum(t.numel() * t.element_size() for t in (*pairs.tensors(), idx, etype))
+        kept = list(_pair_cache.items())
+        while kept and (len(kept) >= 8 or size + sum(e[4] for _, e in kept) > _PAIR_CACHE_BYTES):
+            _pair_cache.pop(kept.pop(0)[0], None)
+        hit = _pair_cache[key] = (pairs, idx, etype, _Kept(*pairs.tensors()), size)
+    else:
+        hit[3].take()
     return hit[0]
 
 
@@ -1155,11 +1179,11 @@ def _dst_of_edges(ptr, idx, n):
     hit = _DST_CACHE.get(key)
     if hit is None:
         deg = (ptr[1:n + 1] - ptr[:n]).long()
-        hit = (torch.repeat_interleave(torch.arange(n, device=ptr.device, dtype=idx.dtype), deg), ptr)
+        dst = torch.repeat_interleave(torch.arange(n, device=ptr.device, dtype=idx.dtype), deg)
         if len(_DST_CACHE) >= 8:
             _DST_CACHE.pop(next(iter(_DST_CACHE)))
-        _DST_CACHE[key] = hit
-    return hit[0]
+        hit = _DST_CACHE[key] = (_Kept(dst), ptr)  # repeat_interleave reads a size back: never under capture
+    return hit[0].take()[0]
 
 
 def run_sddmm_vertex_centric(ptr, idx, src_feat, dst_feat, num_node, *tuner_args):

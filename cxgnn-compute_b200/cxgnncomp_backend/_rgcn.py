@@ -7,7 +7,7 @@ import sys
 import torch
 
 from . import (_check, _cuda, _p, _stream, _sig, _workspace, _vp, _i64, _sz, _num_rows, _INDEX_DTYPES, CXG_F32,
-               CXG_BF16)
+               CXG_BF16, _Kept, _can_keep)
 
 _int = ctypes.c_int
 _pad = _sig("cxg_pad_rel", [_vp, _vp, _vp, _int, _int, _i64, _vp])
@@ -343,9 +343,12 @@ def _one_relation(n, device):
     """int64 zeros [n]: the position array of a weight gradient whose rows all belong to one relation (kept and
     re-sliced, it never changes)."""
     key = str(device)
-    t = _one_rel_cache.get(key)
-    if t is None or t.shape[0] < n:
-        t = _one_rel_cache[key] = torch.zeros(max(n, 1 << 16), dtype=torch.int64, device=device)
+    kept = _one_rel_cache.get(key)
+    if kept is not None and kept.tensors[0].shape[0] >= n:
+        return kept.take()[0][:n]
+    t = torch.zeros(max(n, 1 << 16), dtype=torch.int64, device=device)
+    if _can_keep():
+        _one_rel_cache[key] = _Kept(t)
     return t[:n]
 
 
