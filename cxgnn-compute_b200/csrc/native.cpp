@@ -407,7 +407,11 @@ size_t count_graphs() {
   return graphs.size();
 }
 
-// The weights of a mean's gradient, per transposed edge: kept with the graph, on whichever stream they are wanted.
+// The weights of a mean's gradient, per transposed edge: kept with the graph, on whichever stream they are wanted. All graphs'
+// together take a gigabyte at most, like the plans of the relational layers: the weights of the oldest graphs make room, and
+// those of a graph that alone has more are made for the call.
+constexpr size_t kMostWeightBytes = size_t{1} << 30;
+
 Tensor mean_weights(const Transposed &t) {
   auto make = [&]() {
     Tensor w = at::empty({t.t_idx.size(0)}, t.inv_deg.options());
@@ -417,11 +421,20 @@ Tensor mean_weights(const Transposed &t) {
     return w;
   };
   const auto stream = c10::cuda::getCurrentCUDAStream(t.t_idx.device().index());
-  if (capture_of(stream)) return make();  // what a graph capture records is not there for others
+  const size_t bytes = static_cast<size_t>(t.t_idx.size(0)) * sizeof(float);
+  if (bytes > kMostWeightBytes || capture_of(stream)) return make();  // what a graph capture records is not there for others
   std::lock_guard<std::mutex> hold(graphs_lock);
   for (auto &g : graphs)
     if (g.t.t_idx.is_same(t.t_idx)) {
       if (!g.weight.defined()) {
+        size_t kept = 0;
+        for (const auto &other : graphs) kept += other.weight.defined() ? other.weight.nbytes() : 0;
+        for (auto &other : graphs)
+          if (other.weight.defined() && kept + bytes > kMostWeightBytes) {
+            kept -= other.weight.nbytes();
+            other.weight = Tensor();
+            other.weight_built.reset();
+          }
         g.weight = make();
         g.weight_built.emplace(stream);
       } else {

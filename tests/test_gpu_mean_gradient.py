@@ -54,3 +54,33 @@ def test_other_streams(cuda):
     assert all(torch.equal(first, o) for o in others)
     be.forget_graphs()
     assert torch.equal(first, gradient())
+
+
+@pytest.mark.parametrize("degree,graphs", [(80, 3), (216, 1)])
+def test_kept_weights_have_a_limit(cuda, degree, graphs):
+    """Graphs of 100 M edges, whose weights take 0.4 GB each, and one whose weights alone exceed the limit of a gigabyte."""
+    import cxgnncomp_backend as be
+    n = 1_250_000
+    be.forget_graphs()
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(n, 384, device="cuda", generator=gen).to(torch.bfloat16).requires_grad_(True)
+    g = torch.randn(n, 384, device="cuda", generator=gen).to(torch.bfloat16)
+    ptr = torch.arange(n + 1, device="cuda") * degree
+    ids = [torch.randint(0, n, (n * degree,), device="cuda", generator=gen, dtype=torch.int32) for _ in range(graphs)]
+
+    def gradient(idx):
+        return torch.autograd.grad(be.sage_mean_forward(x, ptr, idx, n), [x], g)[0]
+
+    gradient(ids[0])  # grows the stream's scratch
+    be.forget_graphs()
+    start = torch.cuda.memory_allocated()
+    be._transposed_graph(ptr, ids[0], n, n)
+    one = torch.cuda.memory_allocated() - start  # a transposed graph without weights
+    be.forget_graphs()
+    first = [gradient(idx) for idx in ids]
+    kept = torch.cuda.memory_allocated() - start - sum(t.numel() * 2 for t in first) - graphs * one
+    assert len(be._TRANSPOSE_CACHE) == graphs
+    assert abs(kept - (2 * 4 * n * degree if graphs > 1 else 0)) < 32 << 20  # blocks are cut to a megabyte
+    for want, idx in zip(first, ids):  # weights that have made room are made again
+        assert torch.equal(gradient(idx), want)
+    be.forget_graphs()
