@@ -292,6 +292,12 @@ __global__ void __launch_bounds__(kFixThreads, 12) walk_fix(const __grid_constan
   }
 }
 
+// Most bytes of a copy of x, a limit of memory and not of speed: the copy comes on top of x and y, and a caller that is short
+// of memory has its allocator give everything back before it hears that there is none. 111 M rows of 47 fp32 values (20.9 GB)
+// would be copied to 28.4. (x as it is / copied: 15 M rows of 201 bf16 values, 199 M edges, 7.7 GB 19.9 / 13.0 ms; 20 M rows,
+// 10.2 GB 21.1 / 15.3, the first of them beyond the limit; 60 M rows of 47 bf16, 7.7 GB 17.1 / 14.4.)
+constexpr int64_t kMostCopyBytes = int64_t{8} << 30;
+
 // Bytes that a lane reads of a row: narrow rows take the vector that occupies eight lanes, the fewest a tile is given.
 int walk_vector_bytes(const cxg_spmm_desc *d) {
   const int64_t row_bytes = static_cast<int64_t>(d->feat) * d->heads * (d->dtype == CXG_F32 ? 4 : 2);
@@ -436,7 +442,7 @@ size_t walk_copy_bytes(const cxg_spmm_desc *d, int64_t n_src) {
   // 51; F = 201 225 / 250, 337 / 260. Small graphs do not repay the work behind the plan: 220,000 edges of 94 bytes 38 / 42, of
   // 404 bytes 46 / 43.
   const int64_t edges = row_bytes <= 128 ? 5 : bits % 4 != 0 ? 8 : 12;
-  if (d->nnz < edges * n_src || d->nnz * row_bytes < (40 << 20)) return 0;
+  if (d->nnz < edges * n_src || d->nnz * row_bytes < (40 << 20) || n_src * copy_pitch(row_bytes) > kMostCopyBytes) return 0;
   return static_cast<size_t>(n_src) * copy_pitch(row_bytes);
 }
 

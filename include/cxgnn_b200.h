@@ -213,7 +213,7 @@ int cxg_spmm_csr(const cxg_spmm_desc *desc, void *workspace,
  * values) cost a load per value or two when they are gathered; where a graph reads them several times the call first copies
  * them, widened to whole 128-byte lines, into `rows` and gathers from there. Sums are those of cxg_spmm_csr for the same
  * tile size, bit for bit. n_src: rows of x (all that idx names, times the relations with edge_rel).
- * cxg_spmm_csr_rows_size: bytes of that copy, 0 where the call reads x as it is. `rows` is 32-byte aligned; NULL is
+ * cxg_spmm_csr_rows_size: bytes of that copy (8 GiB at most), 0 where the call reads x as it is. `rows` is 32-byte aligned; NULL is
  * cxg_spmm_csr.
  */
 int cxg_spmm_csr_rows_size(const cxg_spmm_desc *desc, int64_t n_src, size_t *bytes);
