@@ -14,6 +14,7 @@
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <list>
 #include <map>
 #include <mutex>
@@ -148,12 +149,22 @@ bool for_torch(const T &...t) {
 
 void *stream_of(const Tensor &t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
+// The capture that records what the stream is given, or none.
+optional<unsigned long long> capture_of(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream, &status, &id));
+  if (status == cudaStreamCaptureStatusNone) return c10::nullopt;
+  return id;
+}
+
 // ---- scratch ---------------------------------------------------------------------------------------------------------
 // One buffer per (device, stream), grown on demand; contents never carry over. `kind` names the entry point family that
 // used it last (whose status word check_device_status can ask for). The launches of one call hand the buffer on to each
 // other, so whoever uses it holds its lock until the last of them is issued: two threads may work on one stream (a backward
 // runs on a thread of the autograd engine, without the interpreter's lock), and launches of another call in between would
-// overwrite what the next kernel reads.
+// overwrite what the next kernel reads. A call that a graph capture records gets a buffer of its own out of the capture's
+// memory: the graph runs it again when the stream's buffer has long been replaced, or is in use.
 struct Scratch {
   std::mutex in_use;
   Tensor buf;
@@ -190,6 +201,14 @@ struct Workspace {
 };
 
 Workspace workspace_on(int device, void *stream, int64_t bytes, const char *kind) {
+  auto buffer = [&]() {
+    return at::empty({std::max<int64_t>(bytes, 1 << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
+  };
+  if (capture_of(static_cast<cudaStream_t>(stream))) {
+    Workspace w;
+    w.buf = buffer();
+    return w;
+  }
   Scratch &s = scratch_of(device, stream);
   Tensor grown;  // allocated without the lock
   for (;;) {
@@ -202,7 +221,7 @@ Workspace workspace_on(int device, void *stream, int64_t bytes, const char *kind
       return w;
     }
     w.hold.unlock();
-    grown = at::empty({std::max<int64_t>(bytes, 1 << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
+    grown = buffer();
   }
 }
 
@@ -330,15 +349,6 @@ Transposed transpose(const Tensor &ptr, const Tensor &idx, int64_t num_node, int
   return t;
 }
 
-// The capture that records what the stream is given, or none.
-optional<unsigned long long> capture_of(const c10::cuda::CUDAStream &stream) {
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  unsigned long long id = 0;
-  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream.stream(), &status, &id));
-  if (status == cudaStreamCaptureStatusNone) return c10::nullopt;
-  return id;
-}
-
 // The stream that has built something for keeping, and an event behind that.
 struct Built {
   c10::Stream stream;
@@ -375,18 +385,22 @@ struct CachedGraph {
 };
 std::mutex graphs_lock;
 std::list<CachedGraph> &graphs = *new std::list<CachedGraph>;  // not torn down at exit: events would outlive the driver
+std::list<Transposed> &captured_graphs = *new std::list<Transposed>;  // those that captures have taken: replays read them
 constexpr size_t kMostGraphs = 8;
 
 Transposed transposed_graph(const Tensor &ptr, const Tensor &idx, int64_t n, int64_t n_src) {
   const uint32_t pv = ptr._version(), iv = idx._version();
   const auto stream = c10::cuda::getCurrentCUDAStream(ptr.device().index());
-  const auto capture = capture_of(stream);
+  const auto capture = capture_of(stream.stream());
   {
     std::lock_guard<std::mutex> hold(graphs_lock);
     for (const auto &g : graphs)
       if (g.ptr_data == ptr.data_ptr() && g.idx_data == idx.data_ptr() && g.n == n && g.n_src == n_src && g.ptr_version == pv &&
           g.idx_version == iv && g.device == ptr.device().index() && (!g.capture || g.capture == capture)) {
-        g.built.hand_to(stream, capture.has_value() && !g.capture, {g.t.t_ptr, g.t.t_idx, g.t.t_eid, g.t.inv_deg});
+        const bool outside = capture && !g.capture;
+        if (outside && std::none_of(captured_graphs.begin(), captured_graphs.end(), [&](const Transposed &c) { return c.t_idx.is_same(g.t.t_idx); }))
+          captured_graphs.push_back(g.t);
+        g.built.hand_to(stream, outside, {g.t.t_ptr, g.t.t_idx, g.t.t_eid, g.t.inv_deg});
         return g.t;
       }
   }
@@ -401,6 +415,7 @@ Transposed transposed_graph(const Tensor &ptr, const Tensor &idx, int64_t n, int
 void forget_graphs() {
   std::lock_guard<std::mutex> hold(graphs_lock);
   graphs.clear();
+  captured_graphs.clear();
 }
 size_t count_graphs() {
   std::lock_guard<std::mutex> hold(graphs_lock);
@@ -422,7 +437,7 @@ Tensor mean_weights(const Transposed &t) {
   };
   const auto stream = c10::cuda::getCurrentCUDAStream(t.t_idx.device().index());
   const size_t bytes = static_cast<size_t>(t.t_idx.size(0)) * sizeof(float);
-  if (bytes > kMostWeightBytes || capture_of(stream)) return make();  // what a graph capture records is not there for others
+  if (bytes > kMostWeightBytes || capture_of(stream.stream())) return make();  // what a graph capture records is not there for others
   std::lock_guard<std::mutex> hold(graphs_lock);
   for (auto &g : graphs)
     if (g.t.t_idx.is_same(t.t_idx)) {

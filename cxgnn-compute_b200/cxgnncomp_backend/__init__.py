@@ -174,8 +174,11 @@ class _Kept:
         stream under capture cannot wait for what was issued in front of the capture; torch.cuda.graph waits for the device
         before it begins one.)"""
         dev = self.tensors[0].device
-        if _raw_stream(_dev_index(dev)) != self.stream.cuda_stream and _can_keep():
-            with _on(dev):
+        with _on(dev):
+            if not _can_keep():
+                if self not in _captured:
+                    _captured.append(self)
+            elif _raw_stream(_dev_index(dev)) != self.stream.cuda_stream:
                 stream = torch.cuda.current_stream()
                 stream.wait_event(self.event)
                 for t in self.tensors:
@@ -183,9 +186,12 @@ class _Kept:
         return self.tensors
 
 
+_captured = []  # what captures have taken: their graphs read it again when it may have left its cache
+
+
 def _can_keep():
     """Not while a graph capture records the work: its results are there when the graph has run, not before."""
-    return not torch.cuda.is_current_stream_capturing()
+    return not torch._C._cuda_isCurrentStreamCapturing()
 
 
 def _dtype_code(t):
@@ -876,9 +882,10 @@ def relation_pairs(idx, etype, num_src, num_rel):
 
 
 def forget_graphs():
-    """Gives back what is kept per graph: transposed graphs, combined indices, (relation, source) pairs, destinations."""
+    """Gives back what is kept per graph: transposed graphs, combined indices, (relation, source) pairs, destinations. Not to be
+    called while CUDA graphs that were captured over them are still to run."""
     _native.forget_graphs()
-    for kept in (_pair_cache, _cidx_cache, _DST_CACHE):
+    for kept in (_pair_cache, _cidx_cache, _DST_CACHE, _captured):
         kept.clear()
 
 

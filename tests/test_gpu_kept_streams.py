@@ -81,3 +81,32 @@ def test_capture(cuda, kind, kept_before):
     torch.cuda.synchronize()
     assert _same(got, want) and _same(run(), want)
     be.forget_graphs()
+
+
+@pytest.mark.parametrize("kind", ["sum", "mean", "relation", "gat"])
+def test_replay_after_others(cuda, kind):
+    """What a capture has taken or used as scratch stays its own: nine other graphs, larger calls on its stream and other tensors
+    come between the capture and its replay."""
+    import cxgnncomp_backend as be
+    be.forget_graphs()
+    side = torch.cuda.Stream()
+    run = _aggregation(kind, *_graph(3))
+    others = [_aggregation(kind, *_graph(10 + i)) for i in range(9)]
+    large = [t.cuda() for t in random_csr(40_000, 40_000, 30, seed=4)]
+    with torch.cuda.stream(side):
+        want = run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        got = run()
+    with torch.cuda.stream(side):
+        for other in others:
+            other()
+        be.sage_sum_forward(randn((40_000, 256), 5).cuda(), *large, 40_000)
+        waste = [torch.full((1 << k,), 7, dtype=torch.int64, device="cuda") for k in range(9, 20) for _ in range(8)]
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert _same(got, want) and all(bool((w == 7).all()) for w in waste)
+    del graph
+    be.forget_graphs()
