@@ -351,13 +351,13 @@ Transposed transpose(const Tensor &ptr, const Tensor &idx, int64_t num_node, int
 
 // The stream that has built something for keeping, and an event behind that.
 struct Built {
-  c10::Stream stream;
+  c10::cuda::CUDAStream stream;
   std::shared_ptr<c10::Event> event;
-  explicit Built(c10::Stream s) : stream(s), event(std::make_shared<c10::Event>(c10::DeviceType::CUDA)) { event->record(s); }
+  explicit Built(const c10::cuda::CUDAStream &s) : stream(s), event(std::make_shared<c10::Event>(c10::DeviceType::CUDA)) { event->record(s); }
   // Another stream waits for the build, and the memory for that stream. A stream under capture cannot wait for what lies in
   // front of the capture (`outside`): the host does.
-  void hand_to(const c10::Stream &other, bool outside, std::initializer_list<Tensor> tensors) const {
-    if (other == stream) return;
+  template <typename Tensors>
+  void hand_to(const c10::cuda::CUDAStream &other, bool outside, const Tensors &tensors) const {
     if (outside) {
       c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
       event->synchronize();
@@ -366,6 +366,25 @@ struct Built {
     }
     for (const Tensor &t : tensors) t.record_stream(other);
   }
+};
+
+// Tensors that the current stream has built and a cache of the Python side keeps.
+class Kept {
+ public:
+  explicit Kept(std::vector<Tensor> tensors)
+      : tensors_(std::move(tensors)), device_(tensors_.at(0).device().index()), built_(c10::cuda::getCurrentCUDAStream(device_)) {}
+  // They are about to be used on the current stream. True: under a capture, whose replays use them again.
+  bool take() const {
+    const auto stream = c10::cuda::getCurrentCUDAStream(device_);
+    const bool capturing = capture_of(stream.stream()).has_value();
+    if (stream != built_.stream) built_.hand_to(stream, capturing, tensors_);
+    return capturing;
+  }
+
+ private:
+  std::vector<Tensor> tensors_;
+  c10::DeviceIndex device_;
+  Built built_;
 };
 
 // The last eight transposed graphs, by the tensors they came from. An entry keeps ptr and idx alive, so their addresses
@@ -400,7 +419,8 @@ Transposed transposed_graph(const Tensor &ptr, const Tensor &idx, int64_t n, int
         const bool outside = capture && !g.capture;
         if (outside && std::none_of(captured_graphs.begin(), captured_graphs.end(), [&](const Transposed &c) { return c.t_idx.is_same(g.t.t_idx); }))
           captured_graphs.push_back(g.t);
-        g.built.hand_to(stream, outside, {g.t.t_ptr, g.t.t_idx, g.t.t_eid, g.t.inv_deg});
+        if (stream != g.built.stream)
+          g.built.hand_to(stream, outside, std::initializer_list<Tensor>{g.t.t_ptr, g.t.t_idx, g.t.t_eid, g.t.inv_deg});
         return g.t;
       }
   }
@@ -452,8 +472,8 @@ Tensor mean_weights(const Transposed &t) {
           }
         g.weight = make();
         g.weight_built.emplace(stream);
-      } else {
-        g.weight_built->hand_to(stream, false, {g.weight});
+      } else if (stream != g.weight_built->stream) {
+        g.weight_built->hand_to(stream, false, std::initializer_list<Tensor>{g.weight});
       }
       return g.weight;
     }
@@ -1002,6 +1022,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("__enter__", &HeldWorkspace::enter)
       .def("__exit__", [](HeldWorkspace &w, const py::args &) { w.exit(); });
   m.def("last_workspace", &last_workspace);
+  py::class_<Kept>(m, "Kept").def(py::init<std::vector<Tensor>>()).def("take", &Kept::take);
+  m.def("capturing", [](int device) { return capture_of(c10::cuda::getCurrentCUDAStream(device).stream()).has_value(); });
   m.def("spmm", &spmm);
   m.def("sage", &sage);
   m.def("spmm_transposed", &spmm_transposed);

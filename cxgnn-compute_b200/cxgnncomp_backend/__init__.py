@@ -161,37 +161,25 @@ def _workspace(device, nbytes, kind=""):
 
 class _Kept:
     """Tensors that the current stream has built and a cache keeps."""
-    __slots__ = ("tensors", "stream", "event")
+    __slots__ = ("tensors", "built")
 
     def __init__(self, *tensors):
         self.tensors = tensors
-        with _on(tensors[0].device):
-            self.stream = torch.cuda.current_stream()
-            self.event = self.stream.record_event()
+        self.built = _native.Kept(tensors)
 
     def take(self):
-        """The tensors for the current stream. Where that is another one, it waits for the build and the memory for it. (A
-        stream under capture cannot wait for what was issued in front of the capture; torch.cuda.graph waits for the device
-        before it begins one.)"""
-        dev = self.tensors[0].device
-        with _on(dev):
-            if not _can_keep():
-                if self not in _captured:
-                    _captured.append(self)
-            elif _raw_stream(_dev_index(dev)) != self.stream.cuda_stream:
-                stream = torch.cuda.current_stream()
-                stream.wait_event(self.event)
-                for t in self.tensors:
-                    t.record_stream(stream)
+        """The tensors for the current stream. Where that is another one, it waits for the build and the memory for it."""
+        if self.built.take() and self not in _captured:
+            _captured.append(self)
         return self.tensors
 
 
-_captured = []  # what captures have taken: their graphs read it again when it may have left its cache
+_captured = []  # what graph captures have taken: their replays read it when it may have left its cache
 
 
-def _can_keep():
+def _can_keep(device):
     """Not while a graph capture records the work: its results are there when the graph has run, not before."""
-    return not torch._C._cuda_isCurrentStreamCapturing()
+    return not _native.capturing(_dev_index(device))
 
 
 def _dtype_code(t):
@@ -833,7 +821,7 @@ def _combined_index(idx, etype, stride, num_rel):
     c = etype[:n].to(torch.int64) * stride + idx[:n].to(torch.int64)
     if stride * num_rel < 2 ** 31:
         c = c.to(torch.int32)
-    if _can_keep():
+    if _can_keep(idx.device):
         _cidx_cache.append((idx, etype, ver, stride, _Kept(c)))
         if len(_cidx_cache) > 8:
             _cidx_cache.pop(0)

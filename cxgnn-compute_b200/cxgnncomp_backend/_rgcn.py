@@ -347,7 +347,7 @@ def _one_relation(n, device):
     if kept is not None and kept.tensors[0].shape[0] >= n:
         return kept.take()[0][:n]
     t = torch.zeros(max(n, 1 << 16), dtype=torch.int64, device=device)
-    if _can_keep():
+    if _can_keep(device):
         _one_rel_cache[key] = _Kept(t)
     return t[:n]
 
