@@ -18,8 +18,8 @@
 //
 // Small batches are a chain of launches and of loads that wait for one another, so the kernels' blocks become resident while
 // the one in front drains, and small frontiers are spread over blocks of one node per group. 32 seeds, fanouts 15 / 10 / 5,
-// 245 K nodes: the three draws 33 -> 18 us, inference of the sampled SAGE batch 292 -> 244 us; 1,024 seeds, 2.4 M nodes: a
-// training step 1354 -> 1292 us.
+// 245 K nodes: the three draws 33 -> 18 us, inference of the sampled SAGE batch 292 -> 244 us. (A training step of 1,024 seeds
+// and 2.4 M nodes, 1.25 to 1.4 ms, is bound by host work behind the batch, which varies by more than sampling gained.)
 #include "common.cuh"
 
 namespace cxg {

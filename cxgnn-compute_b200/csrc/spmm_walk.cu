@@ -55,12 +55,13 @@ __device__ __forceinline__ void copy_vector(const WalkArgs &a, int64_t i) {
   *reinterpret_cast<uint4 *>(static_cast<uint8_t *>(const_cast<void *>(a.x)) + row * a.x_pitch + at) = out.v;
 }
 
-// Rows that own the first edge of a tile write the tile's record; a hub row that owns many is shared by its warp. One
-// pass over ptr (behind the kernel in front in the stream, while which it is launched: 2 us), so it costs what reading ptr costs (1 us for 170,000 rows, 17 us for 14 M) and the time that its code takes to
-// arrive, where a search per tile is a chain of 18 dependent loads (10 us). Also clears what the later kernels count in.
 constexpr int kFixThreads = 64;  // of walk_fix
 constexpr int kCopyVectors = 4;  // vectors of the copy per thread
 
+// Rows that own the first edge of a tile write the tile's record; a hub row that owns many is shared by its warp. One pass
+// over ptr costs what reading ptr costs (1 us for 170,000 rows, 17 us for 14 M) and the time that its code takes to arrive;
+// a search per tile is a chain of 18 dependent loads (10 us). It is launched while the kernel in front of it in the stream
+// still runs, which saves 2 us. Also clears what the later kernels count in.
 template <int kPlanRows, typename Copy>
 __global__ void __launch_bounds__(256) walk_plan(const __grid_constant__ WalkArgs a) {
   dependency_wait();

@@ -145,7 +145,7 @@ struct Barriers {
   uint64_t conv[kMaxStages];   // converters -> MMA: hi / lo halves of the stage are written (128 arrivals)
   uint64_t empty[kMaxStages];  // MMA -> producers: the MMAs that read the stage are done (1 commit)
   uint64_t acc_full[2];        // MMA -> epilogue (1 commit)
-  uint64_t acc_empty[2];       // epilogue -> MMA (128 arrivals)
+  uint64_t acc_empty[2];       // epilogue -> MMA (32 arrivals per epilogue warp: 128, or 256 with two groups)
 };
 
 // 16-byte asynchronous copy; CA = through L1 (adjacent lanes' chunks merge into one request per line, which

@@ -109,7 +109,7 @@ struct Barriers {
   uint64_t conv[kMaxStages];   // converters -> MMA: 128 arrivals
   uint64_t empty[kMaxStages];  // MMA -> producers: 1 commit
   uint64_t acc_full[2];        // MMA -> epilogue: the accumulator buffer holds a finished chunk (1 commit)
-  uint64_t acc_empty[2];       // epilogue -> MMA: the buffer has been read (128 arrivals)
+  uint64_t acc_empty[2];       // epilogue -> MMA: the buffer has been read (256 arrivals)
 };
 
 // X3: error-compensated fp32. T = float or __nv_bfloat16. kPos = positions per tile, the contraction length of one

@@ -1,5 +1,5 @@
-"""The fused GAT forward by way of weights (cxg_gat_fused_forward on graphs that are large enough): rows of one edge to
-thousands, on both sides of what a lane and a warp keep in registers, rows that cross tiles, empty rows, every vector width
+"""The fused GAT forward by way of weights (cxg_gat_fused_forward, all widths but vectors across heads, narrow rows of whole
+vectors from 128 MB of gathered rows on): rows of one edge to thousands, on both sides of what a lane and a warp keep in registers, rows that cross tiles, empty rows, every vector width
 and number of heads, against float64."""
 import pytest
 import torch
@@ -18,7 +18,8 @@ def _graph(degrees, n_src, seed):
     return ptr, torch.randint(0, n_src, (int(ptr[-1]),), generator=g)
 
 
-@pytest.mark.parametrize("heads,c", [(1, 47), (1, 50), (1, 256), (2, 33), (2, 15), (2, 66), (4, 64), (4, 33), (8, 20), (8, 64)])
+@pytest.mark.parametrize("heads,c", [(1, 47), (1, 50), (1, 256), (2, 33), (2, 15), (2, 66), (4, 64), (4, 33), (8, 20), (8, 64),
+                                     (2, 10), (4, 6), (8, 2), (4, 5), (8, 7)])
 @pytest.mark.parametrize("idx_dtype", [torch.int64, torch.int32])
 def test_forward(cuda, heads, c, idx_dtype):
     import cxgnncomp_backend as be
